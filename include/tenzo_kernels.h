@@ -110,8 +110,8 @@ TENZO_API int tenzo_cuda_rmsnorm_quant(const float* x, const float* norm_w, int 
  * rope_cos/sin: [max_seq][head_dim/2] tables (built on the host with the reference's float
  * expressions so rotations are bit-identical); NULL skips RoPE. head_dim must be 128.
  * The kernel reproduces the reference's fp32 operation order (sequential sums over t, glibc expf
- * bits), so its output is bit-identical, not merely close. No scratch memory: score vectors live
- * in shared memory, which bounds max_len at 36864 keys. */
+ * bits), so its output is bit-identical, not merely close. max_len is bounded at 36864 keys (without a workspace the score
+ * vectors live in shared memory). */
 typedef struct {
     const float* q;        /* [batch][q_stride]  n_q*128 used, pre-RoPE */
     const float* k;        /* [batch][kv_stride] n_kv*128 used, pre-RoPE new key */
@@ -134,7 +134,8 @@ typedef struct {
     int tiles;             /* 0 = choose automatically; 1 = force the variant whose scoring warps read K through TMA tiles
                               (two keys per lane; for many (sequence, kv head) items; returns -5 if it does not fit:
                               needs four 16 KB tile rings beside the weights, n_q/n_kv <= 4 heads per CTA, cache_k and
-                              seq_stride_kv 16-byte aligned); 2 = force per-lane global loads */
+                              seq_stride_kv 16-byte aligned); 2 = force per-lane global loads; 3 = force the three kernels that
+                              spread one launch's keys over all SMs (needs `workspace`; returns -5 if they do not fit) */
     /* kv_mode "paged_int8" (PagedKVCache of the reference, TenzoEngine.cpp:220-445, TenzoEngine.h:154-193). A non-NULL
      * block_table selects it: cache_k/cache_v are then the block pools int8 [block][n_layers][kv_head][16][128] and
      * scale_k/scale_v fp32 [block][n_layers][kv_head][16]; token t of sequence s lives in block
@@ -157,8 +158,11 @@ typedef struct {
      * returns -5 otherwise. */
     int mode;
     int split_keys;         /* mode 1: keys per CTA (rounded up to 128); 0 = choose automatically */
-    void* workspace;        /* mode 1: tenzo_cuda_attention_workspace_bytes(...) bytes, 16-byte aligned, for the partial
-                               results of the splits (contents need not be kept) */
+    void* workspace;        /* 16-byte aligned, contents need not be kept. Mode 1: tenzo_cuda_attention_workspace_bytes(...)
+                               bytes for the partial results of the splits. Mode 0: optional,
+                               tenzo_cuda_attention_exact_workspace_bytes(...) bytes for the score vectors (room for one
+                               sequence at least); NULL keeps them in shared memory, which is slower for all but short
+                               contexts of few sequences. Same results either way */
     size_t workspace_bytes;
 } tenzo_attention_args;
 
@@ -168,6 +172,8 @@ TENZO_API int tenzo_cuda_attention_int8(const tenzo_attention_args* args, void* 
 TENZO_API int tenzo_cuda_attention_take_timeouts(void);
 /* Scratch bytes mode 1 may need for these sizes (an upper bound over every split it can choose). */
 TENZO_API size_t tenzo_cuda_attention_workspace_bytes(int batch, int n_q, int n_kv, int max_len);
+/* Scratch bytes with which mode 0 takes whole batches at its best; bounded (about 64 MB, or one sequence's scores). */
+TENZO_API size_t tenzo_cuda_attention_exact_workspace_bytes(int batch, int n_q, int n_kv, int max_len);
 /* Query heads one CTA will process for this shape (1..n_q/n_kv); informational. */
 TENZO_API int tenzo_cuda_attention_heads_per_cta(int batch, int n_q, int n_kv, int max_len);
 

@@ -678,6 +678,17 @@ namespace tz {
 bool attn_fast_applicable(const tenzo_attention_args& a);
 int attn_fast_run(const tenzo_attention_args& a, cudaStream_t st);
 int attn_fast_take_timeouts();
+// exact order over the whole machine, with scratch (attention_split.cu)
+bool attn_split_possible(const tenzo_attention_args& a);
+bool attn_split_preferred(const tenzo_attention_args& a);
+int attn_split_kernels(const tenzo_attention_args& a);
+int attn_split_run(const tenzo_attention_args& a, cudaStream_t st);
+int attn_split_take_timeouts();
+
+static bool attn_split_chosen(const tenzo_attention_args& a) {
+    return a.tiles == 3 || (a.tiles == 0 && a.heads_per_cta == 0 && attn_split_possible(a) && attn_split_preferred(a));
+}
+int attn_kernels(const tenzo_attention_args& a) { return a.mode == 1 ? 3 : attn_split_chosen(a) ? attn_split_kernels(a) : 1; }
 }
 
 extern "C" int tenzo_cuda_attention_take_timeouts(void) {
@@ -685,8 +696,9 @@ extern "C" int tenzo_cuda_attention_take_timeouts(void) {
     if (cudaMemcpyFromSymbol(&v, tz::g_attn_timeouts, sizeof v) != cudaSuccess) return -1;
     if (v) cudaMemcpyToSymbol(tz::g_attn_timeouts, &zero, sizeof zero);
     const int f = tz::attn_fast_take_timeouts();
-    if (f < 0) return -1;
-    return v > f ? v : f;
+    const int p = tz::attn_split_take_timeouts();
+    if (f < 0 || p < 0) return -1;
+    return v > f ? (v > p ? v : p) : (f > p ? f : p);
 }
 
 extern "C" int tenzo_cuda_attention_heads_per_cta(int batch, int n_q, int n_kv, int max_len) {
@@ -709,6 +721,8 @@ extern "C" int tenzo_cuda_attention_int8(const tenzo_attention_args* args, void*
     if (a.mode == 1) return attn_fast_applicable(a) ? attn_fast_run(a, static_cast<cudaStream_t>(stream)) : -5;
     if (a.mode != 0) return -1;
     if ((size_t)a.max_len * sizeof(float) > (size_t)kScoreSmemBytes) return -5;   // one head's scores must fit on chip
+    if (a.tiles == 3 && !attn_split_possible(a)) return -5;
+    if (attn_split_chosen(a)) return attn_split_run(a, static_cast<cudaStream_t>(stream));
     AttnLaunch L;
     L.a = a;
     if (L.a.q_stride <= 0) L.a.q_stride = a.n_q * kHd;
@@ -755,7 +769,7 @@ extern "C" int tenzo_cuda_attention_int8(const tenzo_attention_args* args, void*
         case 4: tw = tile_warps_for<4>(a.max_len); break;
         default: tw = 0; break;          // eight heads per CTA need more registers than the tiled variant has
     }
-    const bool tiled = a.tiles != 2 && tw >= 4 && (a.tiles == 1 || a.batch * a.n_kv >= 64) && a.seq_stride_kv % 16 == 0 &&
+    const bool tiled = a.tiles != 2 && tw >= 4 && (a.tiles == 1 || a.batch * a.n_kv >= 64) && a.seq_stride_kv % 16 == 0 && (a.batch == 1 || a.seq_stride_kv > 0) &&
                        (reinterpret_cast<uintptr_t>(a.cache_k) & 15) == 0;
     if (a.tiles == 1 && !tiled) return -5;
     L.n_tile_warps = tiled ? tw : 0;

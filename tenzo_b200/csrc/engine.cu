@@ -35,6 +35,8 @@
 
 namespace tz {
 
+int attn_kernels(const tenzo_attention_args& a);         // how many kernels one attention call launches (attention.cu)
+
 // cos/sin [max_seq][head_dim/2] with the reference's float expressions (TenzoEngine.cpp:466-469).
 void rope_tables_host(int max_seq, int head_dim, float theta, float* cs, float* sn) {
     const int half = head_dim / 2;
@@ -253,9 +255,11 @@ void Engine::init(const tenzo_config_t& c, const tenzo_ext_options_t& o) {
         if (paged) throw std::invalid_argument("attention_mode 1 needs the contiguous KV cache (kv_mode int8_fused)");
         if (cfg.max_seq_len % 4) throw std::invalid_argument("attention_mode 1 needs max_seq_len to be a multiple of 4 (16-byte rows of scales)");
         attn_ws_bytes = tenzo_cuda_attention_workspace_bytes(batch, cfg.num_q_heads, cfg.num_kv_heads, cfg.max_seq_len);
-        attn_ws = dalloc(attn_ws_bytes);
         persistent = 0;                                   // the one-kernel form has only the exact-order attention
+    } else {
+        attn_ws_bytes = tenzo_cuda_attention_exact_workspace_bytes(batch, cfg.num_q_heads, cfg.num_kv_heads, cfg.max_seq_len);
     }
+    attn_ws = dalloc(attn_ws_bytes);
 
     TZ_CUDA(cudaMallocHost(&h_pin, (3 * B + 16) * sizeof(int)));
     h_tokens = h_pin;
@@ -291,7 +295,7 @@ void Engine::release_all() {
 Engine::~Engine() { release_all(); }
 
 void Engine::free_prefill_rows() {
-    void** ptrs[] = {(void**)&pf_x, (void**)&pf_qkv, (void**)&pf_attn, (void**)&pf_h1, (void**)&pf_act, (void**)&pf_tokens, (void**)&pf_pos, &pf_ws};
+    void** ptrs[] = {(void**)&pf_x, (void**)&pf_qkv, (void**)&pf_attn, (void**)&pf_h1, (void**)&pf_act, (void**)&pf_tokens, (void**)&pf_pos, &pf_ws, &pf_attn_ws};
     for (void** p : ptrs) {
         if (*p) cudaFree(*p);
         *p = nullptr;
@@ -456,7 +460,7 @@ void Engine::enqueue_layer(int l, int max_len, bool gemv_only) {
     a.mode = attention_mode; a.workspace = attn_ws; a.workspace_bytes = attn_ws_bytes;
     if (!gemv_only) {
         TZ_KERNEL(tenzo_cuda_attention_int8(&a, stream));
-        launches += attention_mode == 1 ? 3 : 1;          // tolerance mode: append, split kernel, merge
+        launches += attn_kernels(a);
     }
 
     // out projection + residual
@@ -532,6 +536,8 @@ void Engine::prefill_chunk(const int* tokens, int M) {
             TZ_CUDA(cudaMalloc((void**)&pf_tokens, m * 4));
             TZ_CUDA(cudaMalloc((void**)&pf_pos, m * 4));
             TZ_CUDA(cudaMalloc(&pf_ws, tenzo_cuda_tl1_gemv_workspace_bytes(M > 1 ? M : 2, h > ffn ? h : ffn)));
+            pf_attn_ws_bytes = tenzo_cuda_attention_exact_workspace_bytes(M, cfg.num_q_heads, cfg.num_kv_heads, cfg.max_seq_len);
+            TZ_CUDA(cudaMalloc(&pf_attn_ws, pf_attn_ws_bytes));
         } catch (...) {
             free_prefill_rows();
             throw;
@@ -573,14 +579,15 @@ void Engine::prefill_chunk(const int* tokens, int M) {
         a.seq_stride_kv = 0; a.seq_stride_sc = 0;          // every query row reads the one sequence's cache
         a.pos = pf_pos; a.rope_cos = rope_cos; a.rope_sin = rope_sin;
         a.layer = l; a.n_q = cfg.num_q_heads; a.n_kv = cfg.num_kv_heads; a.head_dim = 128;
-        a.max_seq = cfg.max_seq_len; a.batch = M; a.max_len = max_len; a.append = 0; a.tiles = 2;
+        a.max_seq = cfg.max_seq_len; a.batch = M; a.max_len = max_len; a.append = 0;
+        a.workspace = pf_attn_ws; a.workspace_bytes = pf_attn_ws_bytes;
         if (paged) { a.block_table = d_table; a.table_stride = 0; a.n_layers = L; a.n_pool_blocks = total_blocks; }      // every query row reads sequence 0's table
         TZ_KERNEL(tenzo_cuda_attention_int8(&a, stream));
         g.x = pf_attn; g.x_stride = qd; g.norm_w = d.attn_sub_norm; g.w = d.o; g.K = h;
         g.n_blocks = h / 64; g.seg_end[0] = g.seg_end[1] = g.seg_end[2] = g.n_blocks; g.seg_scale[0] = d.s_o;
         g.epilogue = TENZO_EPI_RESIDUAL; g.resid = pf_x; g.out = pf_h1; g.out_stride = h;
         TZ_KERNEL(tenzo_cuda_tl1_gemv(&g, stream));
-        launches += 2 * gemv_kernels + 2;
+        launches += 2 * gemv_kernels + 1 + attn_kernels(a);
         if (d.has_mlp) {
             g.x = pf_h1; g.x_stride = h; g.norm_w = d.post_norm; g.w = d.gateup; g.K = h;
             g.n_blocks = 2 * ffn / 64; g.seg_end[0] = ffn / 64; g.seg_end[1] = g.seg_end[2] = g.n_blocks;

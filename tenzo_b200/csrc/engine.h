@@ -112,7 +112,8 @@ public:
     size_t attn_ws_bytes = 0;
     float *pf_x = nullptr, *pf_qkv = nullptr, *pf_attn = nullptr, *pf_h1 = nullptr, *pf_act = nullptr;   // chunked prefill rows
     int *pf_tokens = nullptr, *pf_pos = nullptr, pf_cap = 0;
-    void* pf_ws = nullptr;
+    void *pf_ws = nullptr, *pf_attn_ws = nullptr;
+    size_t pf_attn_ws_bytes = 0;
     void *d_cand = nullptr, *h_cand = nullptr;           // sampler: candidate count + (value, index) pairs
     int* d_sample_past = nullptr;
     size_t sample_past_cap = 0;

@@ -63,25 +63,44 @@ __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[1
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// Tensor maps through the driver entry point, fetched once by way of the runtime.
+typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                      const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                      CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static inline TensorMapEncodeFn tensor_map_encoder() {
+    static const TensorMapEncodeFn encode = []() -> TensorMapEncodeFn {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess) return nullptr;
+        return reinterpret_cast<TensorMapEncodeFn>(fn);
+    }();
+    return encode;
+}
+
 // 2-D row-major tensor map: `inner` elements per row, `rows` rows `row_stride_bytes` apart, box {box_inner, box_rows}.
 static inline int encode_2d(CUtensorMap* out, CUtensorMapDataType type, const void* base, uint64_t inner, uint64_t rows, uint64_t row_stride_bytes,
                      uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) != cudaSuccess || qr != cudaDriverEntryPointSuccess || !fn)
-            return -4;
-        encode = reinterpret_cast<EncodeFn>(fn);
-    }
+    const TensorMapEncodeFn encode = tensor_map_encoder();
+    if (!encode) return -4;
     const cuuint64_t dims[2] = {inner, rows};
     const cuuint64_t strides[1] = {row_stride_bytes};
     const cuuint32_t box[2] = {box_inner, box_rows};
     const cuuint32_t estr[2] = {1u, 1u};
     const CUresult r = encode(out, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : -4;
+}
+
+// 3-D byte tensor {inner, rows, planes}, rows `inner` bytes apart, planes `plane_stride` bytes apart, box {box_inner, box_rows, 1}.
+static inline int encode_3d_bytes(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t plane_stride,
+                                  uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
+    const TensorMapEncodeFn encode = tensor_map_encoder();
+    if (!encode) return -4;
+    const cuuint64_t dims[3] = {inner, rows, planes};
+    const cuuint64_t strides[2] = {inner, plane_stride};
+    const cuuint32_t box[3] = {box_inner, box_rows, 1u};
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : -4;
 }

@@ -84,10 +84,7 @@ def rmsnorm_quant(x: torch.Tensor, norm_w=None, *, do_norm=True, eps=1e-5, qmax=
 
 
 def attention_workspace_bytes(batch, n_q, n_kv, max_len) -> int:
-    lib = load_library()
-    lib.tenzo_cuda_attention_workspace_bytes.restype = C.c_size_t
-    lib.tenzo_cuda_attention_workspace_bytes.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int]
-    return int(lib.tenzo_cuda_attention_workspace_bytes(batch, n_q, n_kv, max_len))
+    return int(load_library().tenzo_cuda_attention_workspace_bytes(batch, n_q, n_kv, max_len))
 
 
 def attention_int8(q, k, v, cache_k, cache_v, scale_k, scale_v, pos, *, layer, n_q, n_kv, max_seq, rope_cos=None,
@@ -116,10 +113,12 @@ def attention_int8(q, k, v, cache_k, cache_v, scale_k, scale_v, pos, *, layer, n
         assert block_table.dtype == torch.int32 and block_table.is_contiguous()
         a.block_table, a.table_stride, a.n_layers = _ptr(block_table), (block_table.stride(0) if block_table.dim() == 2 else 0), n_layers
         a.n_pool_blocks = cache_k.shape[0]
-    if mode == 1:
-        if workspace is None:
-            workspace = torch.empty(attention_workspace_bytes(batch, n_q, n_kv, max_len), dtype=torch.uint8, device=q.device)
-        a.mode, a.split_keys, a.workspace, a.workspace_bytes = 1, split_keys, _ptr(workspace), workspace.numel()
+    if workspace is None and (mode == 1 or tiles in (0, 3)):
+        need = lib.tenzo_cuda_attention_workspace_bytes if mode == 1 else lib.tenzo_cuda_attention_exact_workspace_bytes
+        workspace = torch.empty(need(batch, n_q, n_kv, max_len), dtype=torch.uint8, device=q.device)
+    if workspace is not None:
+        a.workspace, a.workspace_bytes = _ptr(workspace), workspace.numel()
+    a.mode, a.split_keys = mode, split_keys
     _ok(lib.tenzo_cuda_attention_int8(C.byref(a), _stream()), "tenzo_cuda_attention_int8")
     return out
 
