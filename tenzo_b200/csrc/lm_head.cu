@@ -228,7 +228,7 @@ __global__ void tl1_pack_rows2bit_kernel(const uint8_t* __restrict__ raw, int N,
 }  // namespace tz
 
 namespace tz {
-// tensor-core path for 16 or more sequences (lm_head_umma.cu)
+// tensor-core path for two or more sequences (lm_head_umma.cu)
 bool lm_head_umma_applicable(int vocab, int hidden, int batch, const int8_t* w, const float* logits);
 int launch_lm_head_umma(const int8_t* q8, const float* sx, const int8_t* w, const float* row_scales, int vocab, int hidden, int batch,
                         float* logits, int32_t* acc_out, LmBest* cand, int use_pdl, cudaStream_t st);

@@ -1,4 +1,4 @@
-// INT8 LM head for 16 or more sequences on tcgen05 (kind::i8, accumulators in tensor memory), sm_100a.
+// INT8 LM head for two or more sequences on tcgen05 (kind::i8, accumulators in tensor memory), sm_100a.
 //
 // Same computation as lm_head_kernel (compute_logits' int8 branch and the greedy argmax of the
 // reference, src/runtime/TenzoEngine.cpp:1661-1719 and :1745-1755): the activations arrive already
@@ -25,6 +25,7 @@ constexpr int kLmuStages = 4;
 constexpr int kLmuKc = 128;                    // bytes of K per stage
 constexpr int kLmuRows = 128;                  // vocabulary rows per CTA
 constexpr int kLmuMaxN = 256;
+constexpr int kLmuMinBatch = 2;                // the warp-per-row kernel reads a row once for eight sequences, but at 211 us a pass (128256 x 2560); here 88
 
 struct LmUmmaLaunch {
     const float* sx;             // [batch] activation scales m/127
@@ -183,7 +184,7 @@ __global__ void __launch_bounds__(kLmuThreads, 1) lm_head_umma_kernel(const LmUm
 }
 
 bool lm_head_umma_applicable(int vocab, int hidden, int batch, const int8_t* w, const float* logits) {
-    return batch >= 16 && hidden % kLmuKc == 0 && hidden >= kLmuKc && vocab % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
+    return batch >= kLmuMinBatch && hidden % kLmuKc == 0 && hidden >= kLmuKc && vocab % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
            (reinterpret_cast<uintptr_t>(logits) & 15) == 0 && (vocab + kLmuRows - 1) / kLmuRows <= kLmuMaxTiles;
 }
 

@@ -542,7 +542,7 @@ static int pick_ksplit(int n_blocks, int K, int epilogue, int batch) {
 // act_quant_kernel lives in norm_quant.cu
 cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, float eps, int K, int batch, int x_stride,
                              uint32_t* words, float* inv, int8_t* a_out, int* sum_out, int use_pdl, cudaStream_t st);
-// tcgen05 GEMM for 16 or more sequences (tl1_umma.cu)
+// tcgen05 GEMM for nine or more sequences (tl1_umma.cu)
 bool tl1_umma_applicable(const tenzo_tl1_gemv_args& a);
 int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float* inv, const int* sum_a, cudaStream_t st);
 int tl1_umma_take_timeouts();

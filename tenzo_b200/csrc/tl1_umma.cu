@@ -1,5 +1,5 @@
 // Batched TL1 bitlinear on the 5th-generation tensor cores (tcgen05.mma kind::i8, accumulators AND the weight
-// operand in tensor memory) for sm_100a. Used by tenzo_cuda_tl1_gemv when there are at least 16 sequences.
+// operand in tensor memory) for sm_100a. Used by tenzo_cuda_tl1_gemv when there are at least nine sequences.
 //
 // Replaces, for many sequences at once, the same reference code as tl1_gemv.cu
 // (src/runtime/TenzoEngine.cpp:22-166 and the call shapes :1547-1628 of the reference): integer
@@ -56,6 +56,9 @@ namespace tz {
 
 constexpr int kExpandGroups = 4;               // groups of four warps that expand alternate chunks (and run the epilogue)
 constexpr int kUmmaThreads = 32 * (2 + 4 * kExpandGroups + 3);   // warp 0 producer, warp 1 and the last three MMA issue, the rest expand
+// From nine sequences on: up to eight, one mma.sync column group holds them all (8.8 us for quantiser and 3840 x 2560 product,
+// 11.9 for 2560 x 6912; here 8.9 and 13.2), with more it takes four (21 and 25 us; here 9.0 and 13.5).
+constexpr int kUmmaMinBatch = 9;
 constexpr int kMmaThreads = 4;
 constexpr int kMaxSlots = 16;                  // ring of chunk slots: as many as tensor memory and shared memory allow (4 at 256 sequences, 12 at 64)
 constexpr int kPGroup = 8;                     // chunks of packed weights per bulk copy (16 KB per row block)
@@ -544,7 +547,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
 }
 
 bool tl1_umma_applicable(const tenzo_tl1_gemv_args& a) {
-    return a.batch >= 16 && a.K % kKc == 0 && a.K >= kKc && a.out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+    return a.batch >= kUmmaMinBatch && a.K % kKc == 0 && a.K >= kKc && a.out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
 // CTAs of a cluster that split one tile's K range: doubled while the grid still fits the SMs (one CTA per SM) and
@@ -658,7 +661,7 @@ extern "C" int tenzo_cuda_tl1_gemm_layout(int batch, int* slots, int* weight_gro
 }
 
 extern "C" int tenzo_cuda_tl1_gemm_ksplit(int n_blocks, int K, int batch, int epilogue) {
-    if (n_blocks <= 0 || K < tz::kKc || K % tz::kKc || batch < 16) return 0;       // the tensor-core path does not apply
+    if (n_blocks <= 0 || K < tz::kKc || K % tz::kKc || batch < tz::kUmmaMinBatch) return 0;       // the tensor-core path does not apply
     const int units = epilogue == TENZO_EPI_RELU2_GLU ? n_blocks / 2 : (n_blocks + 1) / 2;
     return tz::pick_umma_ksplit(units * ((batch + tz::kMaxN - 1) / tz::kMaxN), K / tz::kKc);
 }
