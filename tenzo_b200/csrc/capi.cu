@@ -185,9 +185,8 @@ int tenzo_generate_step(tenzo_engine_t engine, int cur_token, const tenzo_sampli
         tz::Engine& e = *engine->impl;
         if (e.batch != 1) throw std::invalid_argument("batched engine: use tenzo_ext_generate_step");
         const tenzo_sampling_params_t p = params ? *params : tenzo_default_sampling_params();   // :1729-1732
-        e.generate(&cur_token, &out);
         const bool penalised = p.repetition_penalty != 1.0f && past_tokens && past_tokens_len > 0;
-        if (p.temperature > 0.0f || penalised) out = e.sample(p, past_tokens, past_tokens_len);
+        e.generate(&cur_token, &out, p.temperature > 0.0f || penalised ? &p : nullptr, past_tokens, past_tokens_len);
         return TENZO_SUCCESS;
     });
     return st == TENZO_SUCCESS ? out : -1;

@@ -282,9 +282,9 @@ void Engine::release_all() {
     if (pc_host) cudaFreeHost(pc_host);
     h_pin = nullptr; h_table = nullptr; h_cand = nullptr; pc_host = nullptr;
     free_prefill_rows();
-    if (d_sample_past) cudaFree(d_sample_past);
+    if (h_sample_past) cudaFreeHost(h_sample_past);
     if (d_history) cudaFree(d_history);
-    d_sample_past = nullptr; d_history = nullptr;
+    h_sample_past = nullptr; d_history = nullptr;
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     if (stream) cudaStreamDestroy(stream);
@@ -501,7 +501,7 @@ void Engine::enqueue_step(bool with_logits, bool feed_back, int max_len) {
     if (with_logits) {
         TZ_KERNEL(tenzo_cuda_lm_head_i8(b_x, final_norm, 1, 1e-5f, lm_w, lm_scales, V, h, batch, h, b_logits, nullptr,
                                         d_next, lm_scratch, use_pdl, stream));
-        launches += batch >= 16 && h % 128 == 0 ? 3 : 2;   // (quantiser +) LM head + argmax finish
+        launches += batch >= 2 && h % 128 == 0 ? 3 : 2;   // (quantiser +) LM head + argmax finish
     }
     advance_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(d_pos, d_tokens, d_next, batch, feed_back ? 1 : 0, V);
     TZ_CUDA(cudaGetLastError());
@@ -694,7 +694,7 @@ void Engine::prefill(const int* tokens) {
     pc_check();
 }
 
-void Engine::generate(const int* cur, int* out) {
+void Engine::generate(const int* cur, int* out, const tenzo_sampling_params_t* p, const int* past, int n_past) {
     NvtxRange range("tenzo.generate_step");
     if (pc_usable() && seq_len[0] + 1 <= pc_score_cap(bucket_for(seq_len[0] + 1, cfg.max_seq_len))) {
         // persistent kernel: token and position travel as kernel arguments, the result comes back through a mapped
@@ -713,13 +713,17 @@ void Engine::generate(const int* cur, int* out) {
         TZ_CUDA(cudaEventRecord(ev1, stream));
         TZ_CUDA(cudaStreamSynchronize(stream));
         pc_check();
-        out[0] = pc_host[1];
+        out[0] = p ? sample(*p, past, n_past) : pc_host[1];
         return;
     }
     push_state(cur);
     TZ_CUDA(cudaEventRecord(ev0, stream));
     run_step(true, false);
     TZ_CUDA(cudaEventRecord(ev1, stream));
+    if (p) {
+        out[0] = sample(*p, past, n_past);
+        return;
+    }
     TZ_CUDA(cudaMemcpyAsync(h_next, d_next, (size_t)batch * 4, cudaMemcpyDeviceToHost, stream));
     TZ_CUDA(cudaStreamSynchronize(stream));
     check_device_status(false);
@@ -943,47 +947,48 @@ int sample_pairs(const float* vals, const int* idxs, int n_in, const tenzo_sampl
     return ci[0];
 }
 
-// Penalty, k-th-largest selection and candidate compaction on the device (sampler.cu), the rest on the host.
+// Penalty, k-th-largest selection and candidate compaction on the device (sampler.cu), the rest on the host. Behind the step
+// on the engine's stream, one synchronisation for both: the kernels read the penalised tokens from pinned memory and write
+// the candidates to it (no copies).
 int Engine::sample(const tenzo_sampling_params_t& p, const int* past, int n_past) {
     if (batch != 1) throw std::invalid_argument("sampling with parameters is per sequence");
+    if (!h_cand) TZ_CUDA(cudaMallocHost((void**)&h_cand, 16 + (size_t)kMaxCandidates * 8));
     if (p.repetition_penalty != 1.0f && past && n_past > 0) {
-        std::map<int, int> mult;                          // once per occurrence (:1736-1742)
-        for (int i = 0; i < n_past; ++i) ++mult[past[i]];
-        std::vector<int> toks, cnts;
-        for (auto& kv : mult) { toks.push_back(kv.first); cnts.push_back(kv.second); }
-        const size_t n = toks.size();
-        if (n > sample_past_cap) {
-            if (d_sample_past) cudaFree(d_sample_past);
-            sample_past_cap = n * 2;
-            TZ_CUDA(cudaMalloc((void**)&d_sample_past, sample_past_cap * 2 * sizeof(int)));
+        if (past_count.empty()) past_count.assign(V, 0);
+        if ((size_t)n_past > sample_past_cap) {
+            TZ_CUDA(cudaStreamSynchronize(stream));
+            if (h_sample_past) cudaFreeHost(h_sample_past);
+            h_sample_past = nullptr;
+            sample_past_cap = 0;
+            TZ_CUDA(cudaMallocHost((void**)&h_sample_past, (size_t)n_past * 4 * sizeof(int)));
+            sample_past_cap = (size_t)n_past * 2;
         }
-        TZ_CUDA(cudaMemcpyAsync(d_sample_past, toks.data(), n * 4, cudaMemcpyHostToDevice, stream));
-        TZ_CUDA(cudaMemcpyAsync(d_sample_past + sample_past_cap, cnts.data(), n * 4, cudaMemcpyHostToDevice, stream));
-        TZ_CUDA(launch_penalty(b_logits, V, d_sample_past, d_sample_past + sample_past_cap, (int)n, p.repetition_penalty, stream));
-        launches += 1;
+        int* toks = h_sample_past;                        // distinct tokens and how often each occurs: once per occurrence (:1736-1742)
+        int* cnts = h_sample_past + sample_past_cap;
+        int n = 0;
+        for (int i = 0; i < n_past; ++i)
+            if (past[i] >= 0 && past[i] < V && past_count[past[i]]++ == 0) toks[n++] = past[i];
+        for (int i = 0; i < n; ++i) {
+            cnts[i] = past_count[toks[i]];
+            past_count[toks[i]] = 0;
+        }
+        TZ_CUDA(launch_penalty(b_logits, V, toks, cnts, n, p.repetition_penalty, stream));
+        launches += n > 0;
     }
     const int k = p.temperature <= 0.0f ? 1 : (p.top_k < 1 ? 1 : (p.top_k > 64 ? 64 : p.top_k));
-    if (!d_cand) {
-        TZ_CUDA(cudaMalloc((void**)&d_cand, 16 + (size_t)kMaxCandidates * 8));
-        owned.push_back(d_cand);
-        TZ_CUDA(cudaMallocHost((void**)&h_cand, 16 + (size_t)kMaxCandidates * 8));
-    }
-    int* d_count = reinterpret_cast<int*>(d_cand);
-    float* d_val = reinterpret_cast<float*>(static_cast<unsigned char*>(d_cand) + 16);
-    int* d_idx = reinterpret_cast<int*>(d_val + kMaxCandidates);
-    TZ_CUDA(launch_select_candidates(b_logits, V, k, d_count, d_val, d_idx, stream));
+    int* c_count = reinterpret_cast<int*>(h_cand);
+    float* c_val = reinterpret_cast<float*>(static_cast<unsigned char*>(h_cand) + 16);
+    int* c_idx = reinterpret_cast<int*>(c_val + kMaxCandidates);
+    TZ_CUDA(launch_select_candidates(b_logits, V, k < V ? k : V, c_count, c_val, c_idx, stream));
     launches += 1;
-    TZ_CUDA(cudaMemcpyAsync(h_cand, d_cand, 16 + (size_t)kMaxCandidates * 8, cudaMemcpyDeviceToHost, stream));
     TZ_CUDA(cudaStreamSynchronize(stream));
-    const int count = *reinterpret_cast<const int*>(h_cand);
-    const float* hv = reinterpret_cast<const float*>(static_cast<unsigned char*>(h_cand) + 16);
-    const int* hi = reinterpret_cast<const int*>(hv + kMaxCandidates);
-    if (count > kMaxCandidates) {                         // a huge tie at the threshold: take the whole vector
+    check_device_status(false);
+    if (*c_count > kMaxCandidates) {                      // a huge tie at the threshold: take the whole vector
         std::vector<float> lg((size_t)V);
         TZ_CUDA(cudaMemcpy(lg.data(), b_logits, lg.size() * 4, cudaMemcpyDeviceToHost));
         return sample_pairs(lg.data(), nullptr, V, p, -1.0f);
     }
-    return sample_pairs(hv, hi, count, p, -1.0f);
+    return sample_pairs(c_val, c_idx, *c_count, p, -1.0f);
 }
 
 }  // namespace tz

@@ -54,7 +54,8 @@ public:
 
     void prefill(const int* tokens);                       // one token per sequence, no logits
     void prefill_chunk(const int* tokens, int n);          // n consecutive tokens of the one sequence, together
-    void generate(const int* cur, int* out);               // device argmax
+    // one token a sequence: the device argmax, or (one sequence) drawn with `p` from the candidates the device selects
+    void generate(const int* cur, int* out, const tenzo_sampling_params_t* p = nullptr, const int* past = nullptr, int n_past = 0);
     void decode_greedy(const int* first, int n_steps, int* out);
     int sample(const tenzo_sampling_params_t& p, const int* past, int n_past);   // on the logits of the last step
 
@@ -114,8 +115,9 @@ public:
     int *pf_tokens = nullptr, *pf_pos = nullptr, pf_cap = 0;
     void *pf_ws = nullptr, *pf_attn_ws = nullptr;
     size_t pf_attn_ws_bytes = 0;
-    void *d_cand = nullptr, *h_cand = nullptr;           // sampler: candidate count + (value, index) pairs
-    int* d_sample_past = nullptr;
+    void* h_cand = nullptr;                              // sampler, pinned: candidate count + (value, index) pairs
+    int* h_sample_past = nullptr;                        // pinned: distinct past tokens, then their counts
+    std::vector<int> past_count;                         // [V], zero between calls
     size_t sample_past_cap = 0;
     int *h_pin = nullptr, *h_tokens = nullptr, *h_pos = nullptr, *h_next = nullptr;
     std::vector<int> seq_len;
