@@ -68,13 +68,20 @@ __device__ long long g_aq_trace[8];
 #else
 #define AQT(i) ((void)0)
 #endif
-constexpr int kAqVec = 7;     // float4 values a thread of act_quant_kernel holds: rows up to 7168 floats stay in registers
 
-__global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
+// Row stride of the squares in chain-major order: a chain of K/8 a row, the rows of elements 4i .. 4i + 3 and of their
+// neighbours' in different banks.
+__host__ __device__ __forceinline__ int squares_stride(int K) { return (((K >> 3) + 3) & ~3) + 4; }
+
+// A thread holds kAqVec 16-byte pieces of the row in registers (launch_act_quant picks threads and pieces by K; longer rows
+// go through shared memory).
+template <int kAqThreads, int kAqVec>
+__global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
     const float* x, const float* __restrict__ norm_w, int do_norm, float eps, int K, int x_stride,
     uint32_t* words, float* inv, int8_t* a_out, int* sum_out, int use_pdl) {
     extern __shared__ __align__(16) float s_y[];   // K floats (or eight padded rows of K/8 squares) + 32 scratch
-    float* s_f = s_y + K + 64;
+    const int stride = squares_stride(K);
+    float* s_f = s_y + (8 * stride > K ? 8 * stride : K);
     const int tid = threadIdx.x, seq = blockIdx.x;
     // Let the GEMM that consumes this kernel's output start at once: its prologue (tensor-memory allocation, the first
     // weight copies, expanding the first weight chunks) depends on nothing here and takes as long as this whole kernel;
@@ -85,7 +92,7 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
     // The whole row in registers as 16-byte loads, all in flight at once; shared memory is only touched where another
     // thread needs the value (the sum of squares in reference order, the packed fragments of the mma.sync path), instead
     // of four passes over a staged copy.
-    const bool vec = (K & 3) == 0 && K <= 4 * kAqVec * kNqThreads && (x_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+    const bool vec = (K & 3) == 0 && K <= 4 * kAqVec * kAqThreads && (x_stride & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
                      (!norm_w || (reinterpret_cast<uintptr_t>(norm_w) & 15) == 0) && (!a_out || (reinterpret_cast<uintptr_t>(a_out) & 3) == 0);
     if (vec) {
         const int k4 = K >> 2;
@@ -94,30 +101,26 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
         if (has_w) {                                    // model constants: no need to wait for the previous kernel
 #pragma unroll
             for (int r = 0; r < kAqVec; ++r) {
-                const int i = tid + r * kNqThreads;
+                const int i = tid + r * kAqThreads;
                 w4[r] = i < k4 ? __ldg(reinterpret_cast<const float4*>(norm_w) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
+        const bool chains = (K & 31) == 0;
         if (use_pdl) pdl_wait();
         AQT(1);
 #pragma unroll
         for (int r = 0; r < kAqVec; ++r) {
-            const int i = tid + r * kNqThreads;
+            const int i = tid + r * kAqThreads;
             v[r] = i < k4 ? __ldcg(reinterpret_cast<const float4*>(xs) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         float m = 0.0f;
         if (do_norm) {
             float ss;
-            if ((K & 7) == 0) {
-                // Squares from every thread, stored chain-major (lane j's x[j]^2, x[j+8]^2, ... contiguous, rows padded so
-                // that the eight lanes' 16-byte loads fall in different banks); the eight chains of the reference's order
-                // then cost one load per four adds and one add per element. The chain shares its SM with the
-                // consuming GEMM's first round of weight expansion, and every instruction it does not have to issue is
-                // one it does not have to queue for (load + square + add per element ran at 10.6 cycles per step there).
-                const int rows = K >> 3, stride = ((rows + 3) & ~3) + 4;
+            if (chains) {
+                // squares chain-major (element e in row e & 7, column e >> 3); a lane a chain
 #pragma unroll
                 for (int r = 0; r < kAqVec; ++r) {
-                    const int i = tid + r * kNqThreads;
+                    const int i = tid + r * kAqThreads;
                     if (i < k4) {
                         float* d = s_y + (4 * (i & 1)) * stride + (i >> 1);      // element 4i + c: row (4i + c) & 7, column (4i + c) >> 3
                         d[0] = __fmul_rn(v[r].x, v[r].x);
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
                 }
                 __syncthreads();
                 AQT(2);
-                if (tid < 8) s_f[tid] = sequential_sum(s_y + tid * stride, rows);
+                if (tid < 8) s_f[tid] = sequential_sum(s_y + tid * stride, K >> 3);
                 __syncthreads();
                 ss = s_f[0];
 #pragma unroll
@@ -136,7 +139,7 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
             } else {
 #pragma unroll
                 for (int r = 0; r < kAqVec; ++r) {
-                    const int i = tid + r * kNqThreads;
+                    const int i = tid + r * kAqThreads;
                     if (i < k4) reinterpret_cast<float4*>(s_y)[i] = v[r];
                 }
                 __syncthreads();
@@ -161,12 +164,12 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
             __syncthreads();
 #pragma unroll
             for (int r = 0; r < kAqVec; ++r) {
-                const int i = tid + r * kNqThreads;
+                const int i = tid + r * kAqThreads;
                 if (i < k4) reinterpret_cast<float4*>(s_y)[i] = v[r];
             }
             __syncthreads();
             const int nsets = ((K >> 1) + 15) / 16;
-            for (int wd = tid; wd < nsets * 8; wd += kNqThreads) {
+            for (int wd = tid; wd < nsets * 8; wd += kAqThreads) {
                 const int s = wd >> 3, tt = (wd >> 1) & 3, odd = wd & 1;
                 uint32_t word = 0;
 #pragma unroll
@@ -182,7 +185,7 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
             int part = 0;
 #pragma unroll
             for (int r = 0; r < kAqVec; ++r) {
-                const int i = tid + r * kNqThreads;
+                const int i = tid + r * kAqThreads;
                 const int q0 = (int)roundf(v[r].x * to_q), q1 = (int)roundf(v[r].y * to_q), q2 = (int)roundf(v[r].z * to_q), q3 = (int)roundf(v[r].w * to_q);
                 if (i < k4) {
                     if (a_out)
@@ -207,24 +210,24 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
     }
     // rows that are longer, or not aligned for 16-byte loads: element by element through shared memory
     if (use_pdl) pdl_wait();
-    for (int i = tid; i < K; i += kNqThreads) s_y[i] = __ldcg(xs + i);
+    for (int i = tid; i < K; i += kAqThreads) s_y[i] = __ldcg(xs + i);
     __syncthreads();
     float m = 0.0f;
     if (do_norm) {
         const float ss = sumsq_reference_order(s_y, K, s_f);
         const float inv_rms = rms_inv(ss, K, eps);
-        for (int i = tid; i < K; i += kNqThreads) {
+        for (int i = tid; i < K; i += kAqThreads) {
             const float y = rms_apply(s_y[i], inv_rms, norm_w, i);
             s_y[i] = y;
             m = fmaxf(m, fabsf(y));
         }
     } else {
-        for (int i = tid; i < K; i += kNqThreads) m = fmaxf(m, fabsf(s_y[i]));
+        for (int i = tid; i < K; i += kAqThreads) m = fmaxf(m, fabsf(s_y[i]));
     }
     m = fmaxf(block_max_nonneg(m, s_f), 1e-6f);      // TenzoEngine.cpp:28-32
     const float to_q = 31.0f / m;             // :34
     const int nsets = ((K >> 1) + 15) / 16;
-    for (int wd = tid; words && wd < nsets * 8; wd += kNqThreads) {
+    for (int wd = tid; words && wd < nsets * 8; wd += kAqThreads) {
         const int s = wd >> 3, tt = (wd >> 1) & 3, odd = wd & 1;
         uint32_t word = 0;
 #pragma unroll
@@ -238,7 +241,7 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
     if (tid == 0) inv[seq] = m / 31.0f;       // :35
     if (a_out || sum_out) {
         int part = 0;
-        for (int i = tid; i < K; i += kNqThreads) {
+        for (int i = tid; i < K; i += kAqThreads) {
             const int q = (int)roundf(s_y[i] * to_q);
             if (a_out) a_out[(size_t)seq * K + i] = (int8_t)q;
             part += q;
@@ -258,14 +261,19 @@ __global__ void __launch_bounds__(kNqThreads) act_quant_kernel(
 
 cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, float eps, int K, int batch, int x_stride,
                              uint32_t* words, float* inv, int8_t* a_out, int* sum_out, int use_pdl, cudaStream_t st) {
-    const size_t smem = (size_t)(K + 96) * sizeof(float);
+    const int rows = 8 * squares_stride(K);
+    const size_t smem = (size_t)((rows > K ? rows : K) + 32) * sizeof(float);
+    // 16-byte pieces a thread: as few as the row needs (registers: 1536 rows of 2560 in 21 us with seven, 13 with three), 512
+    // threads for rows above 7168 (14336 went through shared memory element by element: 17 us, now 10)
+    auto kernel = K <= 3072 ? act_quant_kernel<256, 3> : K <= 4096 ? act_quant_kernel<256, 4> : K <= 7168 ? act_quant_kernel<256, 7> : act_quant_kernel<512, 7>;
+    const int threads = K <= 7168 ? 256 : 512;
     if (smem > 48 * 1024) {
-        cudaError_t ea = cudaFuncSetAttribute(act_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+        cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
         if (ea != cudaSuccess) return ea;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)batch, 1, 1);
-    cfg.blockDim = dim3(kNqThreads, 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -273,7 +281,7 @@ cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, f
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, act_quant_kernel, x, norm_w, do_norm, eps, K, x_stride, words, inv, a_out, sum_out, use_pdl);
+    return cudaLaunchKernelEx(&cfg, kernel, x, norm_w, do_norm, eps, K, x_stride, words, inv, a_out, sum_out, use_pdl);
 }
 
 }  // namespace tz
