@@ -390,8 +390,6 @@ struct LightRing {
     static constexpr int bytes = kValueStages * 4 * (v_floats + w_floats);
 };
 
-__device__ __forceinline__ void named_barrier_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
-
 // A sign-extended byte, converted as a 32-bit integer: that conversion issues like an FMA (one cycle), the one from a byte
 // goes through the special-function pipe (eight), which is what the compiler takes when it knows the range.
 __device__ __forceinline__ int byte_at(const int8_t* p) {

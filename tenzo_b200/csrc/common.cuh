@@ -38,14 +38,16 @@ __device__ __forceinline__ uint4 ld_cg_u4(const void* p) { return __ldcg(reinter
 // Ask L2 to fetch [base, base+bytes) ahead of use: the kernels of a decode step run one after another
 // on data-dependent vectors, so each kernel requests the NEXT kernel's weights while it works and
 // HBM keeps streaming across kernel boundaries. Work is spread over the whole grid, one line per thread.
-__device__ __forceinline__ void l2_prefetch_slice(const void* base, size_t bytes) {
+// (tid of n_threads in the CTA take part.)
+__device__ __forceinline__ void l2_prefetch_workers(const void* base, size_t bytes, int tid, int n_threads) {
     if (!base) return;
     const size_t n_lines = (bytes + 127) / 128;
     const size_t cta = blockIdx.x + (size_t)gridDim.x * (blockIdx.y + (size_t)gridDim.y * blockIdx.z);
-    const size_t n_threads = (size_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x;
-    for (size_t c = cta * blockDim.x + threadIdx.x; c < n_lines; c += n_threads)
+    const size_t all = (size_t)gridDim.x * gridDim.y * gridDim.z * n_threads;
+    for (size_t c = cta * n_threads + tid; c < n_lines; c += all)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(base) + c * 128));
 }
+__device__ __forceinline__ void l2_prefetch_slice(const void* base, size_t bytes) { l2_prefetch_workers(base, bytes, threadIdx.x, blockDim.x); }
 
 // ---- bulk asynchronous copy (TMA, 1-D) global -> shared with mbarrier completion ---------------------
 // A bulk copy keeps tens of kilobytes in flight per SM from a single instruction; ordinary loads
@@ -79,6 +81,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
 
 // Barrier among `count` threads (a multiple of 32) of the CTA; id 1..15 (0 is __syncthreads).
 __device__ __forceinline__ void named_barrier_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
+
+__device__ __forceinline__ void named_barrier_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 
 // One non-blocking look at phase `parity` of an mbarrier.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, unsigned parity) {

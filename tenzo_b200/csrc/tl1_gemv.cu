@@ -39,7 +39,6 @@
 //     batch > 1: act_quant_kernel (norm_quant.cu) has written packed int8 activations to a
 //     workspace; CTAs stage their K range for 8 or 32 sequences and reuse every weight word for all.
 #include <cooperative_groups.h>
-#include <type_traits>
 
 #include "common.cuh"
 #include "attn_common.cuh"
@@ -108,10 +107,6 @@ constexpr int kChunks = TZ_GEMV_CHUNKS;
 
 __device__ int g_tl1_timeouts = 0; // set when a bounded mbarrier wait gave up (the result of that launch is invalid)
 
-// One sequence, 4096 < K <= 8192: a thread owns up to four 16-byte pieces of the input vector and parks their norm weights in
-// a private shared-memory slot while it waits (see the prologue): [4][threads] float4.
-__host__ __device__ constexpr int own_park_floats(int K) { return (K > 2 * 4 * kFusedWarps * 32 && K <= 4 * 4 * kFusedWarps * 32) ? 4 * kFusedWarps * 32 * 4 : 0; }
-
 template <int NT, bool FUSED>
 struct GemvSmem {
     static constexpr int SL = FUSED ? 1 : 8 * NT;                       // sequences per CTA
@@ -119,7 +114,7 @@ struct GemvSmem {
     //               | s_b[sets*SL*8] | weights[nb_cta*sets*128] | (fused) x[K]
     static __host__ __device__ int head_words() { return (128 * SL + 2 * SL + 32 + 2 + 4 * kChunks + 3) & ~3; }
     static __host__ __device__ size_t bytes(int sets_per_cta, int K, int nb_cta) {
-        return (size_t)(head_words() + sets_per_cta * SL * 8 + nb_cta * sets_per_cta * 128 + (FUSED ? K + 64 + own_park_floats(K) : 0)) * 4;   // x, or its squares in padded chain-major rows (+ parked norm weights)
+        return (size_t)(head_words() + sets_per_cta * SL * 8 + nb_cta * sets_per_cta * 128 + (FUSED ? K : 0)) * 4;
     }
 };
 
@@ -186,32 +181,7 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
     float wreg[kWRegs];
     const bool has_w = FUSED && a.do_norm && a.norm_w;
     const bool w_in_regs = has_w && a.K <= kWRegs * kGemvThreads;
-    // Prologue form for K a multiple of 32 up to 8192 with 16-byte aligned vectors: every thread OWNS the elements it loads
-    // (16-byte pieces f = tid, tid + threads, ...; elements 4f..4f+3) and keeps them in registers from the load to the
-    // quantised bytes, which it stores straight into the packed activation words: no shared-memory round trip for the
-    // normalised vector and no second pass over it. Up to two pieces per thread (K <= 4096) their norm weights wait in
-    // registers too; with up to four, the thread parks the weights in a shared-memory slot of its own before the wait and
-    // takes them back after the sum of squares (sixteen more live registers would not fit the 64 that two CTAs per SM
-    // leave a thread).
-    const int n_pieces = a.K >> 2;
-    const bool own_ok = FUSED && (a.K & 31) == 0 &&
-                        ((reinterpret_cast<uintptr_t>(a.x + (size_t)seq0 * a.x_stride) | (has_w ? reinterpret_cast<uintptr_t>(a.norm_w) : 0)) & 15) == 0;
-    const int own_p = !own_ok ? 0 : n_pieces <= 2 * kGemvThreads ? 2 : n_pieces <= 4 * kGemvThreads ? 4 : 0;
-    float4* s_w4 = reinterpret_cast<float4*>(s_x + a.K + 64);          // [4][threads], own_p == 4 only
-    if (own_p == 2 && has_w) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int f = tid + j * kGemvThreads;
-            const float4 w4 = f < n_pieces ? __ldg(reinterpret_cast<const float4*>(a.norm_w) + f) : make_float4(0.f, 0.f, 0.f, 0.f);
-            wreg[4 * j] = w4.x; wreg[4 * j + 1] = w4.y; wreg[4 * j + 2] = w4.z; wreg[4 * j + 3] = w4.w;
-        }
-    } else if (own_p == 4 && has_w) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int f = tid + j * kGemvThreads;
-            if (f < n_pieces) s_w4[j * kGemvThreads + tid] = __ldg(reinterpret_cast<const float4*>(a.norm_w) + f);
-        }
-    } else if (own_p == 0 && w_in_regs) {
+    if (w_in_regs) {
 #pragma unroll
         for (int r = 0; r < kWRegs; ++r) {
             const int i = tid + r * kGemvThreads;
@@ -231,112 +201,8 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
     if (FUSED && a.epilogue == TENZO_EPI_RESIDUAL && split == 0 && tid < 64)
         resid_v = __ldcg(a.resid + (size_t)seq0 * a.out_stride + unit * 64 + tid);
 
-    auto own_prologue = [&](auto pieces_c) {
-        constexpr int P = decltype(pieces_c)::value;      // pieces per thread
-        // ---- RMSNorm + absmax(31) quantiser, recomputed identically by every CTA; owned elements (see above) --------
-        const float4* x4 = reinterpret_cast<const float4*>(a.x + (size_t)seq0 * a.x_stride);
-        float xv[4 * P];
-#pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const int f = tid + j * kGemvThreads;
-            const float4 v = f < n_pieces ? __ldcg(x4 + f) : make_float4(0.f, 0.f, 0.f, 0.f);
-            xv[4 * j] = v.x; xv[4 * j + 1] = v.y; xv[4 * j + 2] = v.z; xv[4 * j + 3] = v.w;
-        }
-        float m = 0.0f;
-        if (a.do_norm) {
-            // squares chain-major (element e in row e & 7, column e >> 3) in padded rows, 16-byte aligned and four banks
-            // apart: the lane of chain c then reads four of its elements per load
-            const int stride = (((a.K >> 3) + 3) & ~3) + 4;
-#pragma unroll
-            for (int j = 0; j < P; ++j) {
-                const int f = tid + j * kGemvThreads;
-                if (f < n_pieces) {
-                    float* d = s_x + (4 * (f & 1)) * stride + (f >> 1);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) d[k * stride] = __fmul_rn(xv[4 * j + k], xv[4 * j + k]);
-                }
-            }
-            __syncthreads();
-            TZ_STAMP(8);
-            if (tid < 8) {
-                // eight elements requested while the previous eight are added (two registers sets of two loads)
-                const float4* p = reinterpret_cast<const float4*>(s_x + tid * stride);
-                const int n4 = a.K >> 5;                                  // 16-byte pieces per chain
-                float sum = 0.0f;
-                auto add4 = [&](const float4& v) {
-                    sum = __fadd_rn(sum, v.x); sum = __fadd_rn(sum, v.y); sum = __fadd_rn(sum, v.z); sum = __fadd_rn(sum, v.w);
-                };
-                float4 a0 = p[0], a1 = n4 > 1 ? p[1] : make_float4(0.f, 0.f, 0.f, 0.f), b0, b1;
-                int i = 0;
-                for (; i + 4 <= n4; i += 4) {
-                    b0 = p[i + 2]; b1 = p[i + 3];
-                    add4(a0); add4(a1);
-                    if (i + 6 <= n4) { a0 = p[i + 4]; a1 = p[i + 5]; } else if (i + 5 <= n4) { a0 = p[i + 4]; }
-                    add4(b0); add4(b1);
-                }
-                for (; i < n4; ++i) add4(p[i]);                           // at most three pieces (read again: rare shapes)
-                s_f[tid] = sum;
-            }
-            __syncthreads();
-            float ss = s_f[0];
-#pragma unroll
-            for (int j = 1; j < 8; ++j) ss = __fadd_rn(ss, s_f[j]);     // the eight lanes left to right (common.cuh)
-            TZ_STAMP(9);
-            const float inv_rms = rms_inv(ss, a.K, a.eps);
-#pragma unroll
-            for (int r = 0; r < 4 * P; ++r) {
-                float y = xv[r] * inv_rms;                              // x * inv_rms * w, left to right (:158)
-                if (has_w) {
-                    if constexpr (P == 2) {
-                        y = y * wreg[r];
-                    } else {                                                // parked before the wait (same thread, same slot)
-                        const float* wp = reinterpret_cast<const float*>(s_w4 + (r >> 2) * kGemvThreads + tid);
-                        if (tid + (r >> 2) * kGemvThreads < n_pieces) y = y * wp[r & 3];
-                    }
-                }
-                xv[r] = y;
-                m = fmaxf(m, fabsf(y));                                 // slots beyond K hold zeros
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < 4 * P; ++r) m = fmaxf(m, fabsf(xv[r]));
-        }
-        TZ_STAMP(10);
-        m = fmaxf(block_max_nonneg(m, s_f), 1e-6f); // TenzoEngine.cpp:28-32 (m: running maximum of |y| from 0)
-        TZ_STAMP(11);
-        const float to_q = 31.0f / m;               // :34
-        if (tid == 0) s_inv[0] = m / 31.0f;         // :35
-        const bool parity_out = a.a_out && blockIdx.x == 0;
-        uint8_t* s_b8 = reinterpret_cast<uint8_t*>(s_b);
-        int sa = 0;
-#pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const int f = tid + j * kGemvThreads, s = f >> 3, i = (f >> 1) & 3;     // element 4f + k: set, byte of its word
-            if (f < n_pieces) {
-                const bool mine = s >= s_begin && s < s_end;                        // this CTA's K range
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const int q = (int)roundf(xv[4 * j + k] * to_q);                // :41-42, half away from zero
-                    // word (set, column c = 4 (f & 1) + k) holds its elements 8 i + c, i = 0..3; even columns carry the factor 4
-                    if (mine) {
-                        s_b8[(((s - s_begin) * 8 + 4 * (f & 1) + k) << 2) + i] = (uint8_t)(int8_t)((k & 1) ? q : 4 * q);
-                        sa += q;
-                    }
-                    if (parity_out) a.a_out[(size_t)seq0 * a.K + 4 * f + k] = (int8_t)q;
-                }
-            }
-        }
-        sa = warp_sum_i(sa);
-        if (lane == 0 && sa) atomicAdd(&s_sa4[0], 4 * sa);
-        if (a.inv_out && blockIdx.x == 0 && tid == 0) a.inv_out[seq0] = m / 31.0f;
-        TZ_STAMP(12);
-    };
-    if (own_p == 2) {
-        own_prologue(std::integral_constant<int, 2>{});
-    } else if (own_p == 4) {
-        own_prologue(std::integral_constant<int, 4>{});
-    } else if (FUSED) {
-        // ---- the same for any other K: x staged in shared memory, two passes over it ----------------
+    if (FUSED) {
+        // ---- RMSNorm + absmax(31) quantiser, recomputed identically by every CTA: x staged in shared memory, two passes over it ----------------
         const float* x = a.x + (size_t)seq0 * a.x_stride;
         const bool vec = ((a.K & 3) == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
         if (vec) {
@@ -519,6 +385,353 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
     TZ_TRACE_FLUSH;
 }
 
+// ---- one sequence, K a multiple of 32 up to 8192, 16-byte aligned vectors -----------------------------------------------------
+// The product of tl1_mma_kernel<1, true> with everything that can be taken off the path between the input vector and it.
+//   * The sum of squares. In the reference's order that is eight chains of K/8 dependent additions (2 600 cycles at K = 2560,
+//     6 300 at 6912 in place), and the quantiser needs 1 / rms from it. But y * (31 / max|y|) hardly depends on the last
+//     bits of 1 / rms: so the activations are quantised with a sum in any order, the product runs on them, and a warp of its
+//     own adds up the chains meanwhile. Then every thread checks its elements with the exact 1 / rms: if each quantised
+//     value lies less than half a unit from the exact quotient and no |y| exceeds the presumed maximum, the integers are
+//     the reference's, and only the scale is taken from the exact values; else (about one product in two hundred: some
+//     quotient within 1e-6 of a half) the activations are quantised again, as the reference does it, and the product
+//     repeated. Same results either way, bit for bit. What the check covers need not be exact before it: the presumed
+//     1 / rms and 31 / max are approximate reciprocals, the rounding is an addition of 1.5 * 2^23.
+//   * Cluster meetings. A CTA takes half a 64-row block (16 of the 32 bytes of each column pair: rows c and c + 32) over the
+//     whole of K instead of a block over half of K; with two blocks a CTA (GLU) and enough of them, whole blocks.
+// Threads 32-543 own 16-byte pieces of x (piece f = t, t + 512, ...: elements 4f .. 4f + 3) from the load to the packed bytes;
+// x also lies in shared memory by chains, which the check reads again. The chain warp is warp 0: the scheduler prefers it.
+constexpr int kOneWorkers = kFusedWarps * 32, kOneThreads = kOneWorkers + 32;
+
+struct OneSmem {
+    // 32-bit words: s_d[128] | s_f[64] | s_b[sets * 8] | x by chains [8][stride] | weights [nb_cta][K/2 column pairs][4 HB words]
+    static constexpr int head_words = 128 + 64;
+    static __host__ __device__ int stride(int K) { return (K >> 3) + 4; }        // rows 16-byte aligned; elements 4f .. 4f + 3 and their neighbours' in different banks
+    static size_t bytes(int K, int nb_cta, int hb) { return (size_t)(head_words + (K >> 2) + 8 * stride(K) + nb_cta * (K >> 1) * 4 * hb) * 4; }
+};
+
+// Barrier of the 512 workers that also ors a flag.
+__device__ __forceinline__ bool workers_any(bool v) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"(v ? 1u : 0u), "n"(kOneWorkers) : "memory");
+    return r != 0;
+}
+
+template <int P, int HB>      // pieces a worker owns at most; halves of a row block a CTA takes
+__global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunch L) {
+    const tenzo_tl1_gemv_args& a = L.a;
+    extern __shared__ __align__(16) uint32_t smem[];
+    constexpr int kRows = 32 * HB;                                   // rows of a block in this CTA
+    int* s_d = reinterpret_cast<int*>(smem);                         // [nb_cta][kRows] accumulators: low-nibble rows x4, high-nibble rows x64
+    float* s_f = reinterpret_cast<float*>(smem + 128);               // [0,16) partial sums, [16,32) maxima, 32: 1/rms, 34-35: x and w of the maximum
+    int* s_sa = reinterpret_cast<int*>(s_f + 36);                    // sum of the activations
+    uint32_t* s_b = smem + OneSmem::head_words;                      // [sets][4 t][2] packed activations
+    float* s_x = reinterpret_cast<float*>(s_b + (a.K >> 2));         // [8][stride]
+    const int stride = OneSmem::stride(a.K), n_pieces = a.K >> 2, kh = a.K >> 1, n_sets = a.K >> 5;
+    unsigned char* s_wt = reinterpret_cast<unsigned char*>(s_x + 8 * stride);      // [nb_cta][kh][16 HB]
+    const bool glu = a.epilogue == TENZO_EPI_RELU2_GLU;
+    const int nb_cta = glu ? 2 : 1;
+    const int unit = HB == 2 ? blockIdx.x : blockIdx.x >> 1, half = HB == 2 ? 0 : blockIdx.x & 1;
+    const int lane = threadIdx.x & 31;
+
+    if (threadIdx.x < 32) {
+        // ---- the chain warp ----------------------------------------------------------------------------------------------------
+        if (a.use_pdl) pdl_wait();
+        if (!a.do_norm) return;
+        named_barrier_sync(3, kOneThreads);                          // x is in place
+        float sum = 0.0f;
+        if (lane < 8) {
+            const float4* p = reinterpret_cast<const float4*>(s_x + lane * stride);
+            const int n4 = a.K >> 5;
+            auto add4 = [&](const float4& v) {
+                sum = __fadd_rn(sum, __fmul_rn(v.x, v.x));
+                sum = __fadd_rn(sum, __fmul_rn(v.y, v.y));
+                sum = __fadd_rn(sum, __fmul_rn(v.z, v.z));
+                sum = __fadd_rn(sum, __fmul_rn(v.w, v.w));
+            };
+            int j = 0;
+#pragma unroll 1
+            for (; j + 8 <= n4; j += 8) {                            // eight loads, then their 32 squares and additions
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = p[j + u];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) add4(v[u]);
+            }
+#pragma unroll 1
+            for (; j < n4; ++j) add4(p[j]);
+        }
+        float ss = __shfl_sync(0xffffffffu, sum, 0);
+#pragma unroll
+        for (int j = 1; j < 8; ++j) ss = __fadd_rn(ss, __shfl_sync(0xffffffffu, sum, j));      // the eight lanes left to right (common.cuh)
+        if (lane == 0) s_f[32] = rms_inv(ss, a.K, a.eps);
+        named_barrier_arrive(4, kOneThreads);
+        return;
+    }
+
+    // ---- before the producer has finished: this CTA's weights, the next kernel's, the norm weights --------------------------------
+    const int tid = threadIdx.x - 32, warp = tid >> 5;
+    for (int bk = 0; bk < nb_cta; ++bk) {
+        const uint8_t* src = a.w + (size_t)(bk ? unit + L.units : unit) * kh * 32 + 16 * half;
+        for (int i = tid; i < kh * HB; i += kOneWorkers) {           // 16-byte pieces: HB a column pair
+            const uint8_t* p = HB == 2 ? src + (size_t)i * 16 : src + (size_t)i * 32;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(s_wt + ((size_t)bk * kh * HB + i) * 16)), "l"(p) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    l2_prefetch_workers(a.prefetch, a.prefetch_bytes, tid, kOneWorkers);
+    if (tid < 128) s_d[tid] = 0;
+    if (tid == 0) *s_sa = 0;
+    const bool has_w = a.do_norm && a.norm_w;
+    const float4* w4 = reinterpret_cast<const float4*>(a.norm_w);
+    auto load_w = [&](int j) {
+        const int f = tid + j * kOneWorkers;
+        return has_w && f < n_pieces ? __ldg(w4 + f) : make_float4(1.f, 1.f, 1.f, 1.f);
+    };
+    float4 wr[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) wr[j] = load_w(j);                   // model constants; four pieces: read again (from L1) for the check
+    if (a.use_pdl) {
+        pdl_wait();
+        pdl_launch_dependents();                                     // the next kernel's CTAs may come in and fetch their weights from here on
+    }
+    const int my_row = tid & (kRows - 1), out_row = unit * 64 + (my_row < kRows / 2 ? 16 * half + my_row : 32 + 16 * half + my_row - kRows / 2);
+    float resid_v = 0.0f;
+    if (a.epilogue == TENZO_EPI_RESIDUAL && tid < kRows) resid_v = __ldcg(a.resid + out_row);
+
+    auto normed = [&](float x, float inv_rms, float w) {             // x * inv_rms * w, left to right (:158)
+        const float y = x * inv_rms;
+        return has_w ? y * w : y;
+    };
+    auto x_of = [&](int f, int k) { return s_x[(4 * (f & 1) + k) * stride + (f >> 1)]; };
+    auto workers_max = [&](float m) {                                // maximum over the workers of values >= 0
+        m = warp_max_nonneg(m);
+        if (lane == 0) s_f[16 + warp] = m;
+        named_barrier_sync(1, kOneWorkers);
+        return warp_max_nonneg(s_f[16 + (lane & 15)]);
+    };
+    // Element 4f + k goes to byte (f >> 1) & 3 of word (set f >> 3, column 4 (f & 1) + k); even columns carry the factor 4.
+    uint8_t* s_b8 = reinterpret_cast<uint8_t*>(s_b);
+    auto put = [&](int f, int k, int q) { s_b8[(((f >> 3) * 8 + 4 * (f & 1) + k) << 2) + ((f >> 1) & 3)] = (uint8_t)((k & 1) ? q : 4 * q); };
+    float y[4 * P];                                                  // the vector, normalised, then the quantised values
+    auto exact_quantise = [&](float m) {                             // as the reference does it (:28-42)
+        const float to_q = 31.0f / fmaxf(m, 1e-6f);
+        int sa = 0;
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const int f = tid + j * kOneWorkers;
+            if (f < n_pieces)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    y[4 * j + k] = roundf(y[4 * j + k] * to_q);      // half away from zero
+                    put(f, k, (int)y[4 * j + k]);
+                    sa += (int)y[4 * j + k];
+                }
+        }
+        sa = warp_sum_i(sa);
+        if (lane == 0 && sa) atomicAdd(s_sa, sa);
+    };
+
+    const float4* x4 = reinterpret_cast<const float4*>(a.x);
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const int f = tid + j * kOneWorkers;
+        const float4 v = f < n_pieces ? __ldcg(x4 + f) : make_float4(0.f, 0.f, 0.f, 0.f);
+        y[4 * j] = v.x; y[4 * j + 1] = v.y; y[4 * j + 2] = v.z; y[4 * j + 3] = v.w;
+    }
+    float m = 0.0f;
+    if (a.do_norm) {
+        float part = 0.0f;
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const int f = tid + j * kOneWorkers;
+            if (f < n_pieces) {
+                float* d = s_x + (4 * (f & 1)) * stride + (f >> 1);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    d[k * stride] = y[4 * j + k];
+                    part = __fmaf_rn(y[4 * j + k], y[4 * j + k], part);
+                }
+            }
+        }
+        part = warp_sum(part);
+        if (lane == 0) s_f[warp] = part;
+        named_barrier_sync(3, kOneThreads);
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = reinterpret_cast<const float4*>(s_f)[j];
+            ss += (v.x + v.y) + (v.z + v.w);
+        }
+        const float inv_rms = rsqrtf(ss * (1.0f / (float)a.K) + a.eps);      // presumed
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const float w[4] = {wr[j].x, wr[j].y, wr[j].z, wr[j].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                y[4 * j + k] = normed(y[4 * j + k], inv_rms, w[k]);
+                m = fmaxf(m, fabsf(y[4 * j + k]));                   // slots beyond K hold zeros
+            }
+        }
+        const float m_own = m;
+        m = workers_max(m);
+        if (m_own == m) {                                            // whose element it is (any of equal ones)
+#pragma unroll
+            for (int j = 0; j < P; ++j) {
+                const float w[4] = {wr[j].x, wr[j].y, wr[j].z, wr[j].w};
+                const int f = tid + j * kOneWorkers;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (f < n_pieces && fabsf(y[4 * j + k]) == m) *reinterpret_cast<float2*>(s_f + 34) = make_float2(x_of(f, k), w[k]);
+            }
+        }
+        const float to_q = __fdividef(31.0f, fmaxf(m, 1e-6f));
+        constexpr float kRound = 12582912.0f;                        // 1.5 * 2^23: v + kRound holds round(v) in its low bits
+        int sa = 0;
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const int f = tid + j * kOneWorkers;
+            if (f < n_pieces)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float r = __fmaf_rn(y[4 * j + k], to_q, kRound);
+                    const int q = __float_as_int(r) - __float_as_int(kRound);
+                    y[4 * j + k] = r - kRound;
+                    put(f, k, q);
+                    sa += q;
+                }
+        }
+        sa = warp_sum_i(sa);
+        if (lane == 0 && sa) atomicAdd(s_sa, sa);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 4 * P; ++r) m = fmaxf(m, fabsf(y[r]));
+        m = workers_max(m);
+        exact_quantise(m);
+    }
+
+    const int g = lane >> 2, t4 = lane & 3;
+    const int wb = kFusedWarps / nb_cta, my_blk = glu ? (warp & 1) : 0, wi = glu ? (warp >> 1) : warp;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll 1
+    for (bool checked = !a.do_norm;;) {
+        named_barrier_sync(1, kOneWorkers);                          // packed words and weights are in place
+        // Sets of 16 column pairs. Lane (g, t4) takes bytes 2 HB g .. of column pairs 16 s + 4 i + t4, i = 0..3; a 4 x 4
+        // byte transpose gives T[j], byte row 2 HB g + j at the four column pairs; four masks of it are the A fragments (top of file).
+        int acc[2 * HB][4];
+#pragma unroll
+        for (int j = 0; j < 2 * HB; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[j][e] = 0;
+        const unsigned char* wt = s_wt + ((size_t)my_blk * kh + 16 * wi + t4) * (16 * HB) + 2 * HB * g;
+        const uint32_t* bp = s_b + wi * 8 + t4 * 2;
+#pragma unroll 2
+        for (int s = wi; s < n_sets; s += wb, wt += 256 * HB * wb, bp += 8 * wb) {
+            uint32_t W[4], T[2 * HB];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if constexpr (HB == 2) W[i] = *reinterpret_cast<const uint32_t*>(wt + 4 * i * 32);
+                else W[i] = *reinterpret_cast<const uint16_t*>(wt + 4 * i * 16);
+            }
+            const uint32_t p0 = prmt(W[0], W[1], 0x5140u), p1 = prmt(W[2], W[3], 0x5140u);
+            T[0] = prmt(p0, p1, 0x5410u);
+            T[1] = prmt(p0, p1, 0x7632u);
+            if constexpr (HB == 2) {
+                const uint32_t p2 = prmt(W[0], W[1], 0x7362u), p3 = prmt(W[2], W[3], 0x7362u);
+                T[2] = prmt(p2, p3, 0x5410u);
+                T[3] = prmt(p2, p3, 0x7632u);
+            }
+            uint2 b = make_uint2(0, 0);
+            if (g == 0) b = *reinterpret_cast<const uint2*>(bp);
+#pragma unroll
+            for (int j = 0; j < 2 * HB; ++j)
+                mma_u8s8(acc[j], T[j] & 0x03030303u, T[j] & 0x30303030u, T[j] & 0x0C0C0C0Cu, T[j] & 0xC0C0C0C0u, b.x, b.y);
+        }
+        if (t4 == 0) {                                               // column 0 of D: the warps of a block meet
+#pragma unroll
+            for (int j = 0; j < 2 * HB; ++j) {
+                atomicAdd(&s_d[my_blk * kRows + 2 * HB * g + j], acc[j][0]);                   // x4
+                atomicAdd(&s_d[my_blk * kRows + kRows / 2 + 2 * HB * g + j], acc[j][2]);       // x64
+            }
+        }
+        if (checked) {
+            named_barrier_sync(1, kOneWorkers);
+            break;
+        }
+        // ---- the exact 1 / rms is known by now (or soon): do the integers stand? --------------------------------------------------
+        float4 wc[P];
+#pragma unroll
+        for (int j = 0; j < P; ++j) wc[j] = P == 2 ? wr[j] : load_w(j);
+        named_barrier_sync(4, kOneThreads);
+        const float inv_rms = s_f[32];
+        const float2 top = *reinterpret_cast<const float2*>(s_f + 34);
+        const float m_top = fabsf(normed(top.x, inv_rms, top.y)), to_q = 31.0f / fmaxf(m_top, 1e-6f);
+        bool good = true;
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const float w[4] = {wc[j].x, wc[j].y, wc[j].z, wc[j].w};
+            const int f = tid + j * kOneWorkers;
+            if (f < n_pieces)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float v = normed(x_of(f, k), inv_rms, w[k]);
+                    good = good && fabsf(v) <= m_top && fabsf(v * to_q - y[4 * j + k]) < 0.5f;
+                }
+        }
+        m = m_top;
+        if (!workers_any(!good)) break;                              // (also: every warp's sums are in s_d)
+        float mm = 0.0f;
+#pragma unroll
+        for (int j = 0; j < P; ++j) {
+            const float w[4] = {wc[j].x, wc[j].y, wc[j].z, wc[j].w};
+            const int f = tid + j * kOneWorkers;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                y[4 * j + k] = f < n_pieces ? normed(x_of(f, k), inv_rms, w[k]) : 0.0f;
+                mm = fmaxf(mm, fabsf(y[4 * j + k]));
+            }
+        }
+        if (tid < 128) s_d[tid] = 0;
+        if (tid == 0) *s_sa = 0;
+        m = workers_max(mm);                                         // (its barrier also: the zeroes are in place)
+        exact_quantise(m);
+        checked = true;
+    }
+    const float inv_act = fmaxf(m, 1e-6f) / 31.0f;                   // :35
+    if (blockIdx.x == 0) {                                           // parity-check outputs
+        if (a.inv_out && tid == 0) a.inv_out[0] = inv_act;
+        if (a.a_out)
+#pragma unroll
+            for (int j = 0; j < P; ++j) {
+                const int f = tid + j * kOneWorkers;
+                if (f < n_pieces)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) a.a_out[4 * f + k] = (int8_t)(int)y[4 * j + k];
+            }
+    }
+    if (tid < kRows) {
+        const int sum_a = *s_sa;
+        float v[2];
+#pragma unroll
+        for (int bk = 0; bk < 2; ++bk) {
+            if (bk >= nb_cta) break;
+            const int raw = s_d[bk * kRows + tid];
+            const int accv = (tid < kRows / 2 ? (raw >> 2) : (raw >> 6)) - sum_a;
+            if (a.acc_out) a.acc_out[out_row + (bk ? L.units * 64 : 0)] = accv;
+            v[bk] = (float)accv * (inv_act * seg_scale_for(a, bk ? unit + L.units : unit));   // :1554, :118
+        }
+        float* o = a.out + out_row;
+        if (a.epilogue == TENZO_EPI_STORE) {
+            *o = v[0];
+        } else if (a.epilogue == TENZO_EPI_RESIDUAL) {
+            *o = resid_v + v[0];                                       // :1590
+        } else {
+            const float rl = fmaxf(0.0f, v[0]);
+            *o = (rl * rl) * v[1];                                     // :1618-1619
+        }
+    }
+}
+
 // Cluster size along K: 1, 2, 4 or 8. Enough CTAs to put one on every SM, few enough sets per warp
 // that a warp's loads are all in flight at once, a K range whose packed activations fit in shared
 // memory, never more CTAs than sets.
@@ -580,6 +793,34 @@ static cudaError_t launch_gemv(const GemvLaunch& L, cudaStream_t st) {
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     return cudaLaunchKernelEx(&cfg, tl1_mma_kernel<NT, FUSED>, L);
+}
+
+static bool tl1_one_applicable(const tenzo_tl1_gemv_args& a) {
+    const bool w = a.do_norm && a.norm_w;
+    return a.batch == 1 && a.K % 32 == 0 && a.K <= 8192 && ((reinterpret_cast<uintptr_t>(a.x) | (w ? reinterpret_cast<uintptr_t>(a.norm_w) : 0)) & 15) == 0;
+}
+
+static cudaError_t launch_tl1_one(const GemvLaunch& L, cudaStream_t st) {
+    const tenzo_tl1_gemv_args& a = L.a;
+    const int nb_cta = a.epilogue == TENZO_EPI_RELU2_GLU ? 2 : 1;
+    // Half blocks double the CTAs and halve their loops; whole blocks where their number comes near the SMs' already and two
+    // such CTAs fit an SM (the next kernel's come in beside this one's).
+    const int hb = L.units >= 100 && L.units <= 148 && OneSmem::bytes(a.K, nb_cta, 2) <= 110 * 1024 ? 2 : 1;
+    const size_t smem = OneSmem::bytes(a.K, nb_cta, hb);
+    auto kernel = a.K <= 8 * kOneWorkers ? (hb == 2 ? tl1_one_kernel<2, 2> : tl1_one_kernel<2, 1>) : (hb == 2 ? tl1_one_kernel<4, 2> : tl1_one_kernel<4, 1>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(L.units * (3 - hb)), 1, 1);
+    cfg.blockDim = dim3(kOneThreads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.use_pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, L);
 }
 
 }  // namespace tz
@@ -662,7 +903,7 @@ extern "C" int tenzo_cuda_tl1_gemv(const tenzo_tl1_gemv_args* args, void* stream
     L.act_inv = nullptr;
     cudaError_t e;
     if (a.batch == 1) {
-        e = launch_gemv<1, true>(L, st);
+        e = tl1_one_applicable(a) ? launch_tl1_one(L, st) : launch_gemv<1, true>(L, st);
     } else {
         uint32_t* words = static_cast<uint32_t*>(a.workspace);
         const size_t act_bytes = (((size_t)a.batch * L.nsets * 32 > (size_t)a.batch * a.K ? (size_t)a.batch * L.nsets * 32 : (size_t)a.batch * a.K) + 15) & ~(size_t)15;
