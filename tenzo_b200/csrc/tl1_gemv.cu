@@ -39,6 +39,7 @@
 //     batch > 1: act_quant_kernel (norm_quant.cu) has written packed int8 activations to a
 //     workspace; CTAs stage their K range for 8 or 32 sequences and reuse every weight word for all.
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "common.cuh"
 #include "attn_common.cuh"
@@ -68,7 +69,7 @@ __device__ __forceinline__ float seg_scale_for(const tenzo_tl1_gemv_args& a, int
 }
 
 __device__ __forceinline__ void mma_u8s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -388,24 +389,30 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
 // ---- one sequence, K a multiple of 32 up to 8192, 16-byte aligned vectors -----------------------------------------------------
 // The product of tl1_mma_kernel<1, true> with everything that can be taken off the path between the input vector and it.
 //   * The sum of squares. In the reference's order that is eight chains of K/8 dependent additions (2 600 cycles at K = 2560,
-//     6 300 at 6912 in place), and the quantiser needs 1 / rms from it. But y * (31 / max|y|) hardly depends on the last
-//     bits of 1 / rms: so the activations are quantised with a sum in any order, the product runs on them, and a warp of its
-//     own adds up the chains meanwhile. Then every thread checks its elements with the exact 1 / rms: if each quantised
-//     value lies less than half a unit from the exact quotient and no |y| exceeds the presumed maximum, the integers are
-//     the reference's, and only the scale is taken from the exact values; else (about one product in two hundred: some
-//     quotient within 1e-6 of a half) the activations are quantised again, as the reference does it, and the product
-//     repeated. Same results either way, bit for bit. What the check covers need not be exact before it: the presumed
-//     1 / rms and 31 / max are approximate reciprocals, the rounding is an addition of 1.5 * 2^23.
+//     6 300 at 6912 in place), and the quantiser needs 1 / rms from it. But (x / rms * w) * (31 / max|x / rms * w|) depends
+//     on 1 / rms in its last bits only: so x * w is quantised as it is, the product runs on that, and a warp of its own adds
+//     up the chains meanwhile. Then every thread checks its elements with the exact 1 / rms: if each quantised value lies
+//     less than half a unit from the exact quotient and no |y| exceeds that of the presumed maximum, the integers are the
+//     reference's, and only the scale is taken from the exact values; else (about one product in two hundred: some quotient
+//     within 1e-6 of a half) the activations are quantised again, as the reference does it, and the product repeated. Same
+//     results either way, bit for bit. What the check covers need not be exact before it: 31 / max is an approximate
+//     quotient, the rounding is an addition of 1.5 * 2^23.
 //   * Cluster meetings. A CTA takes half a 64-row block (16 of the 32 bytes of each column pair: rows c and c + 32) over the
 //     whole of K instead of a block over half of K; with two blocks a CTA (GLU) and enough of them, whole blocks.
-// Threads 32-543 own 16-byte pieces of x (piece f = t, t + 512, ...: elements 4f .. 4f + 3) from the load to the packed bytes;
-// x also lies in shared memory by chains, which the check reads again. The chain warp is warp 0: the scheduler prefers it.
+//   * Byte shuffling. A weight word goes into the tensor core as it lies in memory, four rows of one column pair, masked but not
+//     transposed: its bytes are the k index there, and column n of B has the activation in byte n and zeroes elsewhere, so
+//     that column n of D is row n of the word.
+// A worker owns 16-byte pieces of x (piece f = t, t + 512, ...: elements 4f .. 4f + 3) from the load to the packed bytes.
+// The chain warp is warp 0: the scheduler prefers it.
+// What bounds it: latency. Of the 2.9 us of a K = 2560 product 0.5 us are the load of x, 0.2 the maximum, 0.6 the quantiser, 0.7
+// the product, 0.8 the rest of the chain and the check. In a decode step (launches overlapped) 3840 x 2560 4.8 -> 4.3 us,
+// 2560 x 2560 4.9 -> 3.9, gate|up 13824 x 2560 6.1 -> 5.2, 2560 x 6912 8.8 -> 7.2, against the kernel above.
 constexpr int kOneWorkers = kFusedWarps * 32, kOneThreads = kOneWorkers + 32;
 
 struct OneSmem {
-    // 32-bit words: s_d[128] | s_f[64] | s_b[sets * 8] | x by chains [8][stride] | weights [nb_cta][K/2 column pairs][4 HB words]
+    // 32-bit words: s_d[128] | s_f[64] | s_b[sets * 8] | squares by chains [8][stride] | weights [nb_cta][K/2 column pairs][4 HB words]
     static constexpr int head_words = 128 + 64;
-    static __host__ __device__ int stride(int K) { return (K >> 3) + 4; }        // rows 16-byte aligned; elements 4f .. 4f + 3 and their neighbours' in different banks
+    static __host__ __device__ int stride(int K) { return (K >> 3) | 4; }        // an odd number of 16-byte pieces: eight rows' pieces in different banks
     static size_t bytes(int K, int nb_cta, int hb) { return (size_t)(head_words + (K >> 2) + 8 * stride(K) + nb_cta * (K >> 1) * 4 * hb) * 4; }
 };
 
@@ -423,12 +430,13 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
     extern __shared__ __align__(16) uint32_t smem[];
     constexpr int kRows = 32 * HB;                                   // rows of a block in this CTA
     int* s_d = reinterpret_cast<int*>(smem);                         // [nb_cta][kRows] accumulators: low-nibble rows x4, high-nibble rows x64
-    float* s_f = reinterpret_cast<float*>(smem + 128);               // [0,16) partial sums, [16,32) maxima, 32: 1/rms, 34-35: x and w of the maximum
+    float* s_f = reinterpret_cast<float*>(smem + 128);               // [0,16) maxima, 32: 1/rms
     int* s_sa = reinterpret_cast<int*>(s_f + 36);                    // sum of the activations
-    uint32_t* s_b = smem + OneSmem::head_words;                      // [sets][4 t][2] packed activations
-    float* s_x = reinterpret_cast<float*>(s_b + (a.K >> 2));         // [8][stride]
+    int* s_top = s_sa + 1;                                           // element of the presumed maximum
+    uint32_t* s_b = smem + OneSmem::head_words;                      // [sets][8]: word c of set b holds activations 32 b + c + 8 j as bytes j, even c times 4
+    float* s_sq = reinterpret_cast<float*>(s_b + (a.K >> 2));        // [8][stride]
     const int stride = OneSmem::stride(a.K), n_pieces = a.K >> 2, kh = a.K >> 1, n_sets = a.K >> 5;
-    unsigned char* s_wt = reinterpret_cast<unsigned char*>(s_x + 8 * stride);      // [nb_cta][kh][16 HB]
+    unsigned char* s_wt = reinterpret_cast<unsigned char*>(s_sq + 8 * stride);     // [nb_cta][kh][16 HB]
     const bool glu = a.epilogue == TENZO_EPI_RELU2_GLU;
     const int nb_cta = glu ? 2 : 1;
     const int unit = HB == 2 ? blockIdx.x : blockIdx.x >> 1, half = HB == 2 ? 0 : blockIdx.x & 1;
@@ -438,20 +446,20 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
         // ---- the chain warp ----------------------------------------------------------------------------------------------------
         if (a.use_pdl) pdl_wait();
         if (!a.do_norm) return;
-        named_barrier_sync(3, kOneThreads);                          // x is in place
+        named_barrier_sync(3, kOneThreads);                          // the squares are in place
         float sum = 0.0f;
         if (lane < 8) {
-            const float4* p = reinterpret_cast<const float4*>(s_x + lane * stride);
+            const float4* p = reinterpret_cast<const float4*>(s_sq + lane * stride);
             const int n4 = a.K >> 5;
             auto add4 = [&](const float4& v) {
-                sum = __fadd_rn(sum, __fmul_rn(v.x, v.x));
-                sum = __fadd_rn(sum, __fmul_rn(v.y, v.y));
-                sum = __fadd_rn(sum, __fmul_rn(v.z, v.z));
-                sum = __fadd_rn(sum, __fmul_rn(v.w, v.w));
+                sum = __fadd_rn(sum, v.x);
+                sum = __fadd_rn(sum, v.y);
+                sum = __fadd_rn(sum, v.z);
+                sum = __fadd_rn(sum, v.w);
             };
             int j = 0;
 #pragma unroll 1
-            for (; j + 8 <= n4; j += 8) {                            // eight loads, then their 32 squares and additions
+            for (; j + 8 <= n4; j += 8) {                            // eight loads, then their 32 additions
                 float4 v[8];
 #pragma unroll
                 for (int u = 0; u < 8; ++u) v[u] = p[j + u];
@@ -481,20 +489,25 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
     asm volatile("cp.async.commit_group;" ::: "memory");
     l2_prefetch_workers(a.prefetch, a.prefetch_bytes, tid, kOneWorkers);
     if (tid < 128) s_d[tid] = 0;
-    if (tid == 0) *s_sa = 0;
+    if (tid == 0) *s_sa = *s_top = 0;
     const bool has_w = a.do_norm && a.norm_w;
-    const float4* w4 = reinterpret_cast<const float4*>(a.norm_w);
-    auto load_w = [&](int j) {
+    constexpr bool kKeep = P <= 2;                                   // w and the result stay in registers for the check, else they are read again
+    // Pieces beyond the vector read its first one: a load under a condition would be waited for before the next.
+    auto load_w = [&](int j, float (&w)[4]) {
         const int f = tid + j * kOneWorkers;
-        return has_w && f < n_pieces ? __ldg(w4 + f) : make_float4(1.f, 1.f, 1.f, 1.f);
+        const float4 v = has_w ? __ldg(reinterpret_cast<const float4*>(a.norm_w) + (f < n_pieces ? f : 0)) : make_float4(1.f, 1.f, 1.f, 1.f);
+        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
     };
-    float4 wr[P];
+    auto load_x = [&](int j, float (&x)[4]) {
+        const int f = tid + j * kOneWorkers;
+        const float4 v = __ldcg(reinterpret_cast<const float4*>(a.x) + (f < n_pieces ? f : 0));
+        x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    };
+    float xr[P][4], wr[P][4];
 #pragma unroll
-    for (int j = 0; j < P; ++j) wr[j] = load_w(j);                   // model constants; four pieces: read again (from L1) for the check
-    if (a.use_pdl) {
-        pdl_wait();
-        pdl_launch_dependents();                                     // the next kernel's CTAs may come in and fetch their weights from here on
-    }
+    for (int j = 0; j < P; ++j)
+        load_w(j, wr[j]);                                            // model constants
+    if (a.use_pdl) pdl_wait();
     const int my_row = tid & (kRows - 1), out_row = unit * 64 + (my_row < kRows / 2 ? 16 * half + my_row : 32 + 16 * half + my_row - kRows / 2);
     float resid_v = 0.0f;
     if (a.epilogue == TENZO_EPI_RESIDUAL && tid < kRows) resid_v = __ldcg(a.resid + out_row);
@@ -503,155 +516,181 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
         const float y = x * inv_rms;
         return has_w ? y * w : y;
     };
-    auto x_of = [&](int f, int k) { return s_x[(4 * (f & 1) + k) * stride + (f >> 1)]; };
     auto workers_max = [&](float m) {                                // maximum over the workers of values >= 0
         m = warp_max_nonneg(m);
-        if (lane == 0) s_f[16 + warp] = m;
+        if (lane == 0) s_f[warp] = m;
         named_barrier_sync(1, kOneWorkers);
-        return warp_max_nonneg(s_f[16 + (lane & 15)]);
+        return warp_max_nonneg(s_f[lane & 15]);
     };
-    // Element 4f + k goes to byte (f >> 1) & 3 of word (set f >> 3, column 4 (f & 1) + k); even columns carry the factor 4.
-    uint8_t* s_b8 = reinterpret_cast<uint8_t*>(s_b);
-    auto put = [&](int f, int k, int q) { s_b8[(((f >> 3) * 8 + 4 * (f & 1) + k) << 2) + ((f >> 1) & 3)] = (uint8_t)((k & 1) ? q : 4 * q); };
-    float y[4 * P];                                                  // the vector, normalised, then the quantised values
-    auto exact_quantise = [&](float m) {                             // as the reference does it (:28-42)
+    constexpr float kRound = 12582912.0f;                            // 1.5 * 2^23: v + kRound holds round(v) in its low bits
+    float r[kKeep ? P : 1][4];                                       // kRound + the quantised values
+    // Element 4f + k goes to byte (f >> 1) & 3 of word (set f >> 3, c = 4 (f & 1) + k); even columns carry the factor 4.
+    uint8_t* s_b8 = reinterpret_cast<uint8_t*>(s_b) + ((tid >> 3) * 8 + 4 * (tid & 1)) * 4 + ((tid >> 1) & 3);
+    auto put = [&](int j, const float (&v)[4]) {                     // takes kRound + the values, returns their sum
+        const uint32_t q0 = __float_as_uint(v[0]), q1 = __float_as_uint(v[1]), q2 = __float_as_uint(v[2]), q3 = __float_as_uint(v[3]);
+        uint8_t* d = s_b8 + j * (4 * kOneWorkers);
+        d[0] = (uint8_t)(q0 << 2);
+        d[4] = (uint8_t)q1;
+        d[8] = (uint8_t)(q2 << 2);
+        d[12] = (uint8_t)q3;
+        if constexpr (kKeep)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[j][k] = v[k];
+        return (int)(q0 + q1 + q2 + q3 - 4u * __float_as_uint(kRound));
+    };
+    auto quantised = [&](int j, float (&q)[4]) {
+        if constexpr (kKeep) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = r[j][k] - kRound;
+        } else {
+            const uint4 u = *reinterpret_cast<const uint4*>(s_b + (tid >> 3) * 8 + 4 * (tid & 1) + j * kOneWorkers);
+            const uint32_t sel = 0x7540u + ((tid >> 1) & 3);         // the thread's byte of a word, as a float: 2^23 + 128 + the signed byte
+            auto byte_of = [&](uint32_t v) { return __uint_as_float(prmt(v ^ 0x80808080u, 0x4B000000u, sel)); };
+            q[0] = __fmaf_rn(byte_of(u.x), 0.25f, -2097184.0f);
+            q[1] = byte_of(u.y) - 8388736.0f;
+            q[2] = __fmaf_rn(byte_of(u.z), 0.25f, -2097184.0f);
+            q[3] = byte_of(u.w) - 8388736.0f;
+        }
+    };
+    auto add_sa = [&](int sa) {
+        sa = warp_sum_i(sa);
+        if (lane == 0 && sa) atomicAdd(s_sa, sa);
+    };
+    // As the reference does it (:28-42): this thread's values, their maximum over the vector m.
+    auto exact_quantise = [&](float m, auto value) {
         const float to_q = 31.0f / fmaxf(m, 1e-6f);
         int sa = 0;
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const int f = tid + j * kOneWorkers;
-            if (f < n_pieces)
+        for (int j = 0; j < P; ++j)
+            if (tid + j * kOneWorkers < n_pieces) {
+                float v[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    y[4 * j + k] = roundf(y[4 * j + k] * to_q);      // half away from zero
-                    put(f, k, (int)y[4 * j + k]);
-                    sa += (int)y[4 * j + k];
-                }
-        }
-        sa = warp_sum_i(sa);
-        if (lane == 0 && sa) atomicAdd(s_sa, sa);
+                for (int k = 0; k < 4; ++k) v[k] = roundf(value(j, k) * to_q) + kRound;      // half away from zero
+                sa += put(j, v);
+            }
+        add_sa(sa);
     };
 
-    const float4* x4 = reinterpret_cast<const float4*>(a.x);
 #pragma unroll
-    for (int j = 0; j < P; ++j) {
-        const int f = tid + j * kOneWorkers;
-        const float4 v = f < n_pieces ? __ldcg(x4 + f) : make_float4(0.f, 0.f, 0.f, 0.f);
-        y[4 * j] = v.x; y[4 * j + 1] = v.y; y[4 * j + 2] = v.z; y[4 * j + 3] = v.w;
-    }
+    for (int j = 0; j < P; ++j)
+        load_x(j, xr[j]);
     float m = 0.0f;
     if (a.do_norm) {
-        float part = 0.0f;
+        auto z = [&](int j, int k) { return xr[j][k] * wr[j][k]; };
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const int f = tid + j * kOneWorkers;
-            if (f < n_pieces) {
-                float* d = s_x + (4 * (f & 1)) * stride + (f >> 1);
+        for (int j = 0; j < P; ++j)
+            if (tid + j * kOneWorkers < n_pieces) {
+                const int f = tid + j * kOneWorkers;
+                float* d = s_sq + (4 * (f & 1)) * stride + (f >> 1);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    d[k * stride] = y[4 * j + k];
-                    part = __fmaf_rn(y[4 * j + k], y[4 * j + k], part);
+                    d[k * stride] = __fmul_rn(xr[j][k], xr[j][k]);
+                    m = fmaxf(m, fabsf(z(j, k)));
                 }
             }
-        }
-        part = warp_sum(part);
-        if (lane == 0) s_f[warp] = part;
-        named_barrier_sync(3, kOneThreads);
-        float ss = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 v = reinterpret_cast<const float4*>(s_f)[j];
-            ss += (v.x + v.y) + (v.z + v.w);
-        }
-        const float inv_rms = rsqrtf(ss * (1.0f / (float)a.K) + a.eps);      // presumed
-#pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const float w[4] = {wr[j].x, wr[j].y, wr[j].z, wr[j].w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                y[4 * j + k] = normed(y[4 * j + k], inv_rms, w[k]);
-                m = fmaxf(m, fabsf(y[4 * j + k]));                   // slots beyond K hold zeros
-            }
-        }
         const float m_own = m;
-        m = workers_max(m);
+        m = warp_max_nonneg(m);
+        if (lane == 0) s_f[warp] = m;
+        if (a.use_pdl) pdl_launch_dependents();                      // x is here: the next kernel's CTAs may come in and ask for their weights
+        named_barrier_sync(3, kOneThreads);
+        m = warp_max_nonneg(s_f[lane & 15]);
+        // The products x * w again rather than kept: they would take the registers that hold w.
+        auto forget = [&] {
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) asm volatile("" : "+f"(wr[j][k]));
+        };
+        forget();
         if (m_own == m) {                                            // whose element it is (any of equal ones)
 #pragma unroll
-            for (int j = 0; j < P; ++j) {
-                const float w[4] = {wr[j].x, wr[j].y, wr[j].z, wr[j].w};
-                const int f = tid + j * kOneWorkers;
+            for (int j = 0; j < P; ++j)
+                if (tid + j * kOneWorkers < n_pieces)
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (f < n_pieces && fabsf(y[4 * j + k]) == m) *reinterpret_cast<float2*>(s_f + 34) = make_float2(x_of(f, k), w[k]);
-            }
+                    for (int k = 0; k < 4; ++k)
+                        if (fabsf(z(j, k)) == m) *s_top = 4 * (tid + j * kOneWorkers) + k;
         }
-        const float to_q = __fdividef(31.0f, fmaxf(m, 1e-6f));
-        constexpr float kRound = 12582912.0f;                        // 1.5 * 2^23: v + kRound holds round(v) in its low bits
+        forget();
+        const float to_q = __fdividef(31.0f, fmaxf(m, 1e-30f));
         int sa = 0;
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const int f = tid + j * kOneWorkers;
-            if (f < n_pieces)
+        for (int j = 0; j < P; ++j)
+            if (tid + j * kOneWorkers < n_pieces) {
+                float v[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float r = __fmaf_rn(y[4 * j + k], to_q, kRound);
-                    const int q = __float_as_int(r) - __float_as_int(kRound);
-                    y[4 * j + k] = r - kRound;
-                    put(f, k, q);
-                    sa += q;
-                }
-        }
-        sa = warp_sum_i(sa);
-        if (lane == 0 && sa) atomicAdd(s_sa, sa);
+                for (int k = 0; k < 4; ++k) v[k] = __fmaf_rn(z(j, k), to_q, kRound);
+                sa += put(j, v);
+            }
+        add_sa(sa);
     } else {
 #pragma unroll
-        for (int r = 0; r < 4 * P; ++r) m = fmaxf(m, fabsf(y[r]));
+        for (int j = 0; j < P; ++j)
+            if (tid + j * kOneWorkers < n_pieces)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) m = fmaxf(m, fabsf(xr[j][k]));
+        if (a.use_pdl) pdl_launch_dependents();
         m = workers_max(m);
-        exact_quantise(m);
+        exact_quantise(m, [&](int j, int k) { return xr[j][k]; });
     }
 
     const int g = lane >> 2, t4 = lane & 3;
-    const int wb = kFusedWarps / nb_cta, my_blk = glu ? (warp & 1) : 0, wi = glu ? (warp >> 1) : warp;
+    // Weight word i of this lane: column pair 4 i + t4 of the set, or (halves) 4 (2 i + (g >> 2)) + t4; B has the activation of
+    // that pair in byte g & 3: byte i (2 i + (g >> 2)) of the packed words.
+    constexpr int kWords = 2 * HB;
+    const uint32_t sel0 = (0x4444u & ~(0xfu << (4 * (g & 3)))) | ((HB == 2 ? 0u : (uint32_t)(g >> 2)) << (4 * (g & 3)));
+    const uint32_t sel_step = (HB == 2 ? 1u : 2u) << (4 * (g & 3));
+    const uint32_t w_off = HB == 2 ? t4 * 32 + 4 * g : (4 * (g >> 2) + t4) * 16 + 4 * (g & 3);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll 1
     for (bool checked = !a.do_norm;;) {
         named_barrier_sync(1, kOneWorkers);                          // packed words and weights are in place
-        // Sets of 16 column pairs. Lane (g, t4) takes bytes 2 HB g .. of column pairs 16 s + 4 i + t4, i = 0..3; a 4 x 4
-        // byte transpose gives T[j], byte row 2 HB g + j at the four column pairs; four masks of it are the A fragments (top of file).
-        int acc[2 * HB][4];
-#pragma unroll
-        for (int j = 0; j < 2 * HB; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[j][e] = 0;
-        const unsigned char* wt = s_wt + ((size_t)my_blk * kh + 16 * wi + t4) * (16 * HB) + 2 * HB * g;
-        const uint32_t* bp = s_b + wi * 8 + t4 * 2;
-#pragma unroll 2
-        for (int s = wi; s < n_sets; s += wb, wt += 256 * HB * wb, bp += 8 * wb) {
-            uint32_t W[4], T[2 * HB];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if constexpr (HB == 2) W[i] = *reinterpret_cast<const uint32_t*>(wt + 4 * i * 32);
-                else W[i] = *reinterpret_cast<const uint16_t*>(wt + 4 * i * 16);
-            }
-            const uint32_t p0 = prmt(W[0], W[1], 0x5140u), p1 = prmt(W[2], W[3], 0x5140u);
-            T[0] = prmt(p0, p1, 0x5410u);
-            T[1] = prmt(p0, p1, 0x7632u);
-            if constexpr (HB == 2) {
-                const uint32_t p2 = prmt(W[0], W[1], 0x7362u), p3 = prmt(W[2], W[3], 0x7362u);
-                T[2] = prmt(p2, p3, 0x5410u);
-                T[3] = prmt(p2, p3, 0x7632u);
-            }
-            uint2 b = make_uint2(0, 0);
-            if (g == 0) b = *reinterpret_cast<const uint2*>(bp);
-#pragma unroll
-            for (int j = 0; j < 2 * HB; ++j)
-                mma_u8s8(acc[j], T[j] & 0x03030303u, T[j] & 0x30303030u, T[j] & 0x0C0C0C0Cu, T[j] & 0xC0C0C0C0u, b.x, b.y);
+        float top_x = 0.0f, top_w = 1.0f;
+        if (!checked) {
+            top_x = __ldcg(a.x + *s_top);
+            if (has_w) top_w = __ldg(a.norm_w + *s_top);
         }
-        if (t4 == 0) {                                               // column 0 of D: the warps of a block meet
+        int acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+        auto product = [&](auto blocks) {
+            constexpr int NB = decltype(blocks)::value;
+            // One block: the warps of the chain's scheduler stay out of the way, the chain is what the CTA waits for then (two
+            // blocks: the product is). Down at K = 6912 7.6 -> 7.2 us.
+            const int pw = NB == 2 ? kFusedWarps : kFusedWarps * 3 / 4, pi = NB == 2 ? warp : warp - (warp >> 2);
+            if (NB == 1 && (warp & 3) == 3) return;
+            const unsigned char* wt = s_wt + (size_t)pi * (256 * HB) + w_off;
+            const size_t blk = (size_t)kh * (16 * HB);
+            const uint2* bp = reinterpret_cast<const uint2*>(s_b + pi * 8) + t4;
+#pragma unroll 2
+            for (int s = pi; s < n_sets; s += pw, wt += 256 * HB * pw, bp += 4 * pw) {
+                uint32_t W[NB][kWords];
+                const uint2 b = *bp;
 #pragma unroll
-            for (int j = 0; j < 2 * HB; ++j) {
-                atomicAdd(&s_d[my_blk * kRows + 2 * HB * g + j], acc[j][0]);                   // x4
-                atomicAdd(&s_d[my_blk * kRows + kRows / 2 + 2 * HB * g + j], acc[j][2]);       // x64
+                for (int bk = 0; bk < NB; ++bk)
+#pragma unroll
+                    for (int i = 0; i < kWords; ++i) W[bk][i] = *reinterpret_cast<const uint32_t*>(wt + bk * blk + 128 * i);
+#pragma unroll
+                for (int i = 0; i < kWords; ++i) {
+                    const uint32_t be = prmt(b.x, 0u, sel0 + i * sel_step), bo = prmt(b.y, 0u, sel0 + i * sel_step);
+#pragma unroll
+                    for (int bk = 0; bk < NB; ++bk) {
+                        const uint32_t w = W[bk][i];
+                        mma_u8s8(acc[bk], w & 0x03030303u, w & 0x30303030u, w & 0x0C0C0C0Cu, w & 0xC0C0C0C0u, be, bo);
+                    }
+                }
+            }
+        };
+        if (glu) product(std::integral_constant<int, 2>{});
+        else product(std::integral_constant<int, 1>{});
+        // D: rows g (low nibbles) and g + 8 (high ones), columns 2 t4, 2 t4 + 1: byte rows 4 g + column; of halves, columns 4-7
+        // belong to the words of lanes g >= 4 and the other columns to those below. The warps meet.
+        if (HB == 2 ? t4 < 2 : (t4 >> 1) == (g >> 2)) {
+            int* d = s_d + 4 * (HB == 2 ? g : g & 3) + 2 * (t4 & 1);
+#pragma unroll
+            for (int bk = 0; bk < 2; ++bk, d += kRows) {
+                if (bk >= nb_cta) break;
+                atomicAdd(d, acc[bk][0]);                            // x4
+                atomicAdd(d + 1, acc[bk][1]);
+                atomicAdd(d + kRows / 2, acc[bk][2]);                // x64
+                atomicAdd(d + kRows / 2 + 1, acc[bk][3]);
             }
         }
         if (checked) {
@@ -659,42 +698,38 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
             break;
         }
         // ---- the exact 1 / rms is known by now (or soon): do the integers stand? --------------------------------------------------
-        float4 wc[P];
+        if constexpr (!kKeep)
 #pragma unroll
-        for (int j = 0; j < P; ++j) wc[j] = P == 2 ? wr[j] : load_w(j);
+            for (int j = 0; j < P; ++j) load_w(j, wr[j]);
         named_barrier_sync(4, kOneThreads);
-        const float inv_rms = s_f[32];
-        const float2 top = *reinterpret_cast<const float2*>(s_f + 34);
-        const float m_top = fabsf(normed(top.x, inv_rms, top.y)), to_q = 31.0f / fmaxf(m_top, 1e-6f);
+        float inv_rms = s_f[32];
+        const float m_top = fabsf(normed(top_x, inv_rms, top_w)), to_q = 31.0f / fmaxf(m_top, 1e-6f);
         bool good = true;
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const float w[4] = {wc[j].x, wc[j].y, wc[j].z, wc[j].w};
-            const int f = tid + j * kOneWorkers;
-            if (f < n_pieces)
+        for (int j = 0; j < P; ++j)
+            if (tid + j * kOneWorkers < n_pieces) {
+                float q[4];
+                quantised(j, q);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const float v = normed(x_of(f, k), inv_rms, w[k]);
-                    good = good && fabsf(v) <= m_top && fabsf(v * to_q - y[4 * j + k]) < 0.5f;
+                    const float v = normed(xr[j][k], inv_rms, wr[j][k]);
+                    good = good && fabsf(v) <= m_top && fabsf(v * to_q - q[k]) < 0.5f;
                 }
-        }
+            }
         m = m_top;
         if (!workers_any(!good)) break;                              // (also: every warp's sums are in s_d)
+        asm volatile("" : "+f"(inv_rms));                            // (the check's values again, not kept: registers)
         float mm = 0.0f;
 #pragma unroll
-        for (int j = 0; j < P; ++j) {
-            const float w[4] = {wc[j].x, wc[j].y, wc[j].z, wc[j].w};
-            const int f = tid + j * kOneWorkers;
+        for (int j = 0; j < P; ++j)
+            if (tid + j * kOneWorkers < n_pieces)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                y[4 * j + k] = f < n_pieces ? normed(x_of(f, k), inv_rms, w[k]) : 0.0f;
-                mm = fmaxf(mm, fabsf(y[4 * j + k]));
-            }
-        }
+                for (int k = 0; k < 4; ++k) mm = fmaxf(mm, fabsf(normed(xr[j][k], inv_rms, wr[j][k])));
         if (tid < 128) s_d[tid] = 0;
         if (tid == 0) *s_sa = 0;
         m = workers_max(mm);                                         // (its barrier also: the zeroes are in place)
-        exact_quantise(m);
+        asm volatile("" : "+f"(inv_rms));
+        exact_quantise(m, [&](int j, int k) { return normed(xr[j][k], inv_rms, wr[j][k]); });
         checked = true;
     }
     const float inv_act = fmaxf(m, 1e-6f) / 31.0f;                   // :35
@@ -702,12 +737,13 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
         if (a.inv_out && tid == 0) a.inv_out[0] = inv_act;
         if (a.a_out)
 #pragma unroll
-            for (int j = 0; j < P; ++j) {
-                const int f = tid + j * kOneWorkers;
-                if (f < n_pieces)
+            for (int j = 0; j < P; ++j)
+                if (tid + j * kOneWorkers < n_pieces) {
+                    float q[4];
+                    quantised(j, q);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) a.a_out[4 * f + k] = (int8_t)(int)y[4 * j + k];
-            }
+                    for (int k = 0; k < 4; ++k) a.a_out[4 * (tid + j * kOneWorkers) + k] = (int8_t)(int)q[k];
+                }
     }
     if (tid < kRows) {
         const int sum_a = *s_sa;

@@ -1,5 +1,5 @@
-"""Where the tensor-core paths begin (two sequences for the LM head, nine for TL1 products), and the cluster form of the
-sampler's candidate selection, against the one-sequence kernels and numpy."""
+"""The one-sequence TL1 product against the batched one, where the tensor-core paths begin (two sequences for the LM head, nine
+for TL1 products) against the one-sequence kernels, and the cluster form of the sampler's candidate selection against numpy."""
 import numpy as np
 import pytest
 import torch
@@ -35,6 +35,29 @@ def test_tl1_product_of_a_few_sequences_matches_one_at_a_time(cuda_lib, N, K, B)
     many = run(x, res)
     for b in range(B):
         assert np.array_equal(many[b], run(x[b:b + 1].contiguous(), res[b:b + 1].contiguous())[0])
+    assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
+
+
+@pytest.mark.parametrize("what", ["normal", "halves", "zeros", "tiny", "plain"])
+@pytest.mark.parametrize("N,K", [(128, 32), (64, 64), (12800, 128), (192, 2592), (128, 4128), (128, 6912), (128, 8192)])
+def test_tl1_product_of_one_sequence_matches_the_batched_kernel(cuda_lib, N, K, what):
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([84, N, K])
+    x, nw = rng.standard_normal((1, K)).astype(np.float32), (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    if what == "halves":                             # quotients on the rounding boundary: the presumed integers do not stand
+        x[0] = ((rng.integers(-31, 31, K) + 0.5) / 31).astype(np.float32)
+        x[0, K // 3], nw[:] = 1.0, 1.0
+    x *= {"zeros": 0.0, "tiny": 1e-20}.get(what, 1.0)
+    w, n_blocks, norm = dev(synth.random_tl1_packed(rng, N, K)), N // 64, what != "plain"
+    two = lambda a: dev(np.concatenate([a, a[:, ::-1]]))
+    for epi in [kernels.EPI_STORE, kernels.EPI_RESIDUAL] + ([kernels.EPI_RELU2_GLU] if n_blocks % 2 == 0 else []):
+        glu, res = epi == kernels.EPI_RELU2_GLU, rng.standard_normal((1, N)).astype(np.float32)
+        args = (w, n_blocks, K, [0.02, 0.03] if glu else [0.02], [n_blocks // 2, n_blocks] if glu else None)
+        kw = dict(epilogue=epi, norm_w=dev(nw) if norm else None, do_norm=norm)
+        resid = epi == kernels.EPI_RESIDUAL
+        one = kernels.tl1_gemv(dev(x), *args, resid=dev(res) if resid else None, **kw)["out"]
+        many = kernels.tl1_gemv(two(x), *args, resid=two(res) if resid else None, **kw)["out"]
+        assert np.array_equal(host(one)[0], host(many)[0])
     assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
 
 
