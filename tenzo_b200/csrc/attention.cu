@@ -136,7 +136,8 @@ __global__ void __launch_bounds__(TILED ? kTileThreads : kAttnThreads) attn_kern
     // their round trips overlap the producer's tail. (Callers that launch with use_pdl directly behind a kernel that
     // writes the position, the tables or cache rows below it must not: include/tenzo_kernels.h says so.)
     constexpr bool kEarly = !TILED && !PAGED;
-    if (!kEarly && a.use_pdl) pdl_wait();
+    // Without an append the last rows come from a kernel of this step (a prompt's own keys): the wait comes first then.
+    if (a.use_pdl && (!kEarly || !a.append)) pdl_wait();
     TZ_PH_DECL;
     const int pos = __ldcg(a.pos + seq);
     // max_len sizes the score vectors and the staged block table: a position outside [0, max_len) would write past

@@ -85,7 +85,11 @@ __global__ void record_tokens_kernel(const int* next, int* history, int step, in
 __global__ void __launch_bounds__(64) kv_append_rows_kernel(const float* qkv, int row_stride, int q_dim, int kv_dim, int n_kv, int pos0,
                                                             const float* rope_cos, const float* rope_sin, int8_t* cache_k, int8_t* cache_v,
                                                             float* scale_k, float* scale_v, size_t layer_row_base, int max_seq,
-                                                            const int* table, int n_layers, int layer) {
+                                                            const int* table, int n_layers, int layer, int use_pdl) {
+    if (use_pdl) {                            // a few hundred bytes of work a block: resident early, and so are its readers
+        tz::pdl_wait();
+        tz::pdl_launch_dependents();
+    }
     const int token = blockIdx.x, kvh = blockIdx.y, is_v = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pos = pos0 + token;
     const float* src = qkv + (size_t)token * row_stride + q_dim + (is_v ? kv_dim : 0) + kvh * 128;
@@ -554,24 +558,33 @@ void Engine::prefill_chunk(const int* tokens, int M) {
     TZ_KERNEL(tenzo_cuda_embedding_i8(lm_w, lm_scales, h, pf_tokens, M, pf_x, h, V, stream));
     launches += 1;
     const int gemv_kernels = M > 1 ? 2 : 1;
-    const int max_len = bucket_for(pos0 + M, cfg.max_seq_len);
+    const int max_len = pos0 + M;          // no graph is kept here, so no bucket: score passes and spans follow the prompt
     for (int l = 0; l < L; ++l) {
         const LayerDev& d = layers[l];
         if (!d.set) throw std::runtime_error("layer weights were never set");
         tenzo_tl1_gemv_args g;
         std::memset(&g, 0, sizeof g);
-        g.do_norm = 1; g.eps = 1e-5f; g.batch = M; g.workspace = pf_ws; g.use_pdl = 0;
+        g.do_norm = 1; g.eps = 1e-5f; g.batch = M; g.workspace = pf_ws; g.use_pdl = use_pdl;
         g.x = pf_x; g.x_stride = h; g.norm_w = d.in_norm; g.w = d.qkv; g.K = h;
         g.n_blocks = (qd + 2 * kvd) / 64;
         g.seg_end[0] = qd / 64; g.seg_end[1] = (qd + kvd) / 64; g.seg_end[2] = g.n_blocks;
         g.seg_scale[0] = d.s_q; g.seg_scale[1] = d.s_k; g.seg_scale[2] = d.s_v;
         g.epilogue = TENZO_EPI_STORE; g.out = pf_qkv; g.out_stride = qd + 2 * kvd;
+        g.prefetch = d.o; g.prefetch_bytes = (size_t)h * h / 4;
         TZ_KERNEL(tenzo_cuda_tl1_gemv(&g, stream));
         const size_t layer_row_base = (size_t)l * cfg.num_kv_heads * cfg.max_seq_len;
-        kv_append_rows_kernel<<<dim3((unsigned)M, (unsigned)cfg.num_kv_heads), 64, 0, stream>>>(
-            pf_qkv, qd + 2 * kvd, qd, kvd, cfg.num_kv_heads, pos0, rope_cos, rope_sin, cache_k, cache_v, scale_k, scale_v, layer_row_base,
-            cfg.max_seq_len, paged ? d_table : nullptr, L, l);
-        TZ_CUDA(cudaGetLastError());
+        cudaLaunchConfig_t cfg_append = {};
+        cfg_append.gridDim = dim3((unsigned)M, (unsigned)cfg.num_kv_heads);
+        cfg_append.blockDim = dim3(64);
+        cfg_append.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg_append.attrs = attr;
+        cfg_append.numAttrs = use_pdl ? 1 : 0;
+        TZ_CUDA(cudaLaunchKernelEx(&cfg_append, kv_append_rows_kernel, (const float*)pf_qkv, qd + 2 * kvd, qd, kvd, cfg.num_kv_heads, pos0,
+                                   (const float*)rope_cos, (const float*)rope_sin, cache_k, cache_v, scale_k, scale_v, layer_row_base,
+                                   cfg.max_seq_len, (const int*)(paged ? d_table : nullptr), L, l, (int)use_pdl));
         tenzo_attention_args a;
         std::memset(&a, 0, sizeof a);
         a.q = pf_qkv; a.out = pf_attn; a.q_stride = a.kv_stride = qd + 2 * kvd;
@@ -579,13 +592,16 @@ void Engine::prefill_chunk(const int* tokens, int M) {
         a.seq_stride_kv = 0; a.seq_stride_sc = 0;          // every query row reads the one sequence's cache
         a.pos = pf_pos; a.rope_cos = rope_cos; a.rope_sin = rope_sin;
         a.layer = l; a.n_q = cfg.num_q_heads; a.n_kv = cfg.num_kv_heads; a.head_dim = 128;
-        a.max_seq = cfg.max_seq_len; a.batch = M; a.max_len = max_len; a.append = 0;
+        a.max_seq = cfg.max_seq_len; a.batch = M; a.max_len = max_len; a.append = 0; a.use_pdl = use_pdl;
         a.workspace = pf_attn_ws; a.workspace_bytes = pf_attn_ws_bytes;
         if (paged) { a.block_table = d_table; a.table_stride = 0; a.n_layers = L; a.n_pool_blocks = total_blocks; }      // every query row reads sequence 0's table
         TZ_KERNEL(tenzo_cuda_attention_int8(&a, stream));
         g.x = pf_attn; g.x_stride = qd; g.norm_w = d.attn_sub_norm; g.w = d.o; g.K = h;
         g.n_blocks = h / 64; g.seg_end[0] = g.seg_end[1] = g.seg_end[2] = g.n_blocks; g.seg_scale[0] = d.s_o;
         g.epilogue = TENZO_EPI_RESIDUAL; g.resid = pf_x; g.out = pf_h1; g.out_stride = h;
+        const LayerDev* nxt = l + 1 < L ? &layers[l + 1] : nullptr;
+        if (d.has_mlp) { g.prefetch = d.gateup; g.prefetch_bytes = (size_t)2 * ffn * h / 4; }
+        else { g.prefetch = nxt ? nxt->qkv : nullptr; g.prefetch_bytes = (size_t)(qd + 2 * kvd) * h / 4; }
         TZ_KERNEL(tenzo_cuda_tl1_gemv(&g, stream));
         launches += 2 * gemv_kernels + 1 + attn_kernels(a);
         if (d.has_mlp) {
@@ -593,10 +609,12 @@ void Engine::prefill_chunk(const int* tokens, int M) {
             g.n_blocks = 2 * ffn / 64; g.seg_end[0] = ffn / 64; g.seg_end[1] = g.seg_end[2] = g.n_blocks;
             g.seg_scale[0] = d.s_gate; g.seg_scale[1] = d.s_up;
             g.epilogue = TENZO_EPI_RELU2_GLU; g.resid = nullptr; g.out = pf_act; g.out_stride = ffn;
+            g.prefetch = d.down; g.prefetch_bytes = (size_t)h * ffn / 4;
             TZ_KERNEL(tenzo_cuda_tl1_gemv(&g, stream));
             g.x = pf_act; g.x_stride = ffn; g.norm_w = d.ffn_sub_norm; g.w = d.down; g.K = ffn;
             g.n_blocks = h / 64; g.seg_end[0] = g.seg_end[1] = g.seg_end[2] = g.n_blocks; g.seg_scale[0] = d.s_down;
             g.epilogue = TENZO_EPI_RESIDUAL; g.resid = pf_h1; g.out = pf_x; g.out_stride = h;
+            g.prefetch = nxt ? nxt->qkv : nullptr; g.prefetch_bytes = (size_t)(qd + 2 * kvd) * h / 4;
             TZ_KERNEL(tenzo_cuda_tl1_gemv(&g, stream));
             launches += 2 * gemv_kernels;
         } else {
