@@ -278,11 +278,17 @@ __global__ void __launch_bounds__(kScoreWarps * 32, 2) split_scores_kernel(const
 // Scores -> exponentials (in place) and 1 / sum, for HS heads of an item per CTA. Chunks of keys go through two
 // shared-memory buffers: while HS warps add up one chunk, each a head in key order, the others evaluate the next. Many
 // items: four heads a CTA and small chunks, so that all CTAs are resident at once; few: one head, long chunks (fewer sums).
-template <int HS> struct SoftShape { static constexpr int eval = HS == 1 ? 512 : 256, threads = eval + 32 * HS, chunk = 4096 / HS; };
-template <int GH, int HS, bool PAGED>
-__global__ void __launch_bounds__(SoftShape<HS>::threads, HS == 1 ? 2 : 3) split_softmax_kernel(const SplitLaunch L) {
+// MANY: more items than three CTAs an SM hold. The summing warps are what an item takes its time for, so half the evaluating
+// threads and five CTAs an SM then (a prompt of 1536 rows: 27.75 -> 27.05 ms in all, 640 items of 4096 keys 40 -> 37 us; but
+// 320 items of 8192 keys 49 -> 55).
+template <int HS, bool MANY> struct SoftShape {
+    static constexpr int eval = HS == 1 ? 512 : MANY ? 128 : 256, threads = eval + 32 * HS, chunk = 4096 / HS;
+    static constexpr int resident = HS == 1 ? 2 : MANY ? 5 : 3;
+};
+template <int GH, int HS, bool PAGED, bool MANY>
+__global__ void __launch_bounds__(SoftShape<HS, MANY>::threads, SoftShape<HS, MANY>::resident) split_softmax_kernel(const SplitLaunch L) {
     const tenzo_attention_args& a = L.a;
-    constexpr int kEval = SoftShape<HS>::eval, kSoftChunk = SoftShape<HS>::chunk;
+    constexpr int kEval = SoftShape<HS, MANY>::eval, kSoftChunk = SoftShape<HS, MANY>::chunk;
     extern __shared__ __align__(16) float s_e[];       // [2][HS][padded chunk]
     __shared__ float s_max[HS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sw = warp - kEval / 32;   // sw >= 0: summing warp of head sw
@@ -794,13 +800,14 @@ static cudaError_t launch_values(const SplitLaunch& L, int heavy, int items, cud
     return split_launch(split_values_kernel<GH, GV, PAGED>, dim3((unsigned)blocks), kValueThreads, smem, st, L.a.use_pdl != 0, L, heavy);
 }
 
-template <int GH, int HS, bool PAGED>
+template <int GH, int HS, bool PAGED, bool MANY = false>
 static cudaError_t launch_softmax(const SplitLaunch& L, long long items, cudaStream_t st) {
-    const int chunk = L.tp < SoftShape<HS>::chunk ? L.tp : SoftShape<HS>::chunk;
+    using Shape = SoftShape<HS, MANY>;
+    const int chunk = L.tp < Shape::chunk ? L.tp : Shape::chunk;
     const size_t smem = (size_t)2 * HS * ordered_sum_padded(chunk) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(split_softmax_kernel<GH, HS, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(split_softmax_kernel<GH, HS, PAGED, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return split_launch(split_softmax_kernel<GH, HS, PAGED>, dim3((unsigned)(items * (GH / HS))), SoftShape<HS>::threads, smem, st, L.a.use_pdl != 0, L);
+    return split_launch(split_softmax_kernel<GH, HS, PAGED, MANY>, dim3((unsigned)(items * (GH / HS))), Shape::threads, smem, st, L.a.use_pdl != 0, L);
 }
 
 template <int GH, bool PAGED>
@@ -813,7 +820,8 @@ static cudaError_t split_pass(const SplitLaunch& L, int n_seq, cudaStream_t st) 
     e = split_launch(split_scores_kernel<GH, PAGED>, dim3((unsigned)L.n_spans, (unsigned)L.groups, (unsigned)n_seq), kScoreWarps * 32, smem, st, L.a.use_pdl != 0, L, km);
     if (e != cudaSuccess) return e;
     const long long items = (long long)n_seq * L.groups;
-    e = GH == 1 || items >= 148 ? launch_softmax<GH, GH, PAGED>(L, items, st) : launch_softmax<GH, 1, PAGED>(L, items, st);
+    if (GH > 1 && items > 3 * 148) e = launch_softmax<GH, GH, PAGED, GH != 1>(L, items, st);
+    else e = GH == 1 || items >= 148 ? launch_softmax<GH, GH, PAGED>(L, items, st) : launch_softmax<GH, 1, PAGED>(L, items, st);
     if (e != cudaSuccess) return e;
     const ValueSplit v = pick_values(items, GH);
     return v.gv == GH ? launch_values<GH, GH, PAGED>(L, v.heavy, (int)items, st) : launch_values<GH, 1, PAGED>(L, v.heavy, (int)items, st);
@@ -831,11 +839,14 @@ int attn_split_kernels(const tenzo_attention_args& a) {
     return 3 * ((a.batch + per_pass - 1) / per_pass);
 }
 
-// With heads for every SM the three kernels win from about 256 keys on (12 x 1500 keys, 20/5 heads: 34 us against 50 in one
-// kernel; 12 x 200: 15 against 14), with fewer from about 1000 (one sequence of 1024 keys: 17.5 us against 19, of 512: 15
-// against 10, of 6003: 48 against 98). max_len is an upper bound that callers round up, so the line lies one step further.
+// With heads for nearly two CTAs an SM the three kernels win at any length (20/5 heads, 16 x 16 keys: 10.5 us against 13.2 in
+// one kernel, 64 x 64: 18.5 and 25.8, 256 x 256: 60 and 111; 32/8 heads alike), with heads for every SM from about 256 keys on
+// (8 x 128: 12.1 and 10.5; 12 x 1500: 34 and 50), with fewer from about 1000 (one sequence of 1024 keys: 17.5 us against 19,
+// of 512: 15 against 10, of 6003: 48 against 98). max_len is an upper bound that callers round up, so these lines lie one
+// step further.
 bool attn_split_preferred(const tenzo_attention_args& a) {
-    return a.max_len > ((long long)a.batch * a.n_q >= 148 ? 256 : 1024);
+    const long long heads = (long long)a.batch * a.n_q;
+    return heads >= 256 || a.max_len > (heads >= 148 ? 256 : 1024);
 }
 
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st) {

@@ -269,7 +269,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-    if (a.use_pdl) pdl_launch_dependents();
     if (tid == 0) UT(1);
     bool timed_out = false, epi_ok = false;
     const int mma_t = warp == 1 ? 0 : warp - (1 + 4 * kExpandGroups);        // issuing thread 0..3: warp 1 and the three warps after the expand warps
@@ -284,7 +283,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             }
         } else {
             // ---- per-sequence epilogue operands (quantiser outputs) ---------------------------------------
-            if (a.use_pdl) pdl_wait();
+            if (a.use_pdl) {
+                pdl_wait();
+                pdl_launch_dependents();                         // after the own wait: see act_quant_kernel
+            }
             for (int i = lane - 1; i < N; i += 31) {
                 const int seq = seq0 + i;
                 s_inv[i] = seq < a.batch ? __ldcg(L.inv + seq) : 0.0f;
