@@ -29,6 +29,7 @@
 #include "../../include/tenzo.h"
 #include "../../include/tenzo_ext.h"
 #include "common.cuh"
+#include "lm_head.cuh"
 #include "../../include/tenzo_kernels.h"
 #include "engine.h"
 #include "sampler.h"
@@ -61,7 +62,8 @@ void set_error(const std::string& m) { g_last_error = m; }
         if (_r < 0) throw std::runtime_error(std::string(#expr) + " rejected its arguments");   \
     } while (0)
 
-__global__ void advance_kernel(int* pos, int* tokens, const int* next, int batch, int feed_back, int vocab) {
+__global__ void advance_kernel(int* pos, int* tokens, const int* next, int batch, int feed_back, int vocab, int use_pdl) {
+    if (use_pdl) tz::pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < batch) {
         pos[i] += 1;
@@ -489,7 +491,7 @@ void Engine::enqueue_layer(int l, int max_len, bool gemv_only) {
         g.n_blocks = h / 64; g.seg_end[0] = g.seg_end[1] = g.seg_end[2] = g.n_blocks; g.seg_scale[0] = d.s_down;
         g.epilogue = TENZO_EPI_RESIDUAL; g.resid = b_h1; g.out = b_x; g.out_stride = h;
         if (nxt) { g.prefetch = nxt->qkv; g.prefetch_bytes = (size_t)(qd + 2 * kvd) * h / 4; }
-        else { g.prefetch = lm_w; g.prefetch_bytes = (size_t)64 << 20; if ((size_t)V * h < g.prefetch_bytes) g.prefetch_bytes = (size_t)V * h; }
+        else { g.prefetch = lm_w; g.prefetch_bytes = tz::kLmPrefetchBefore; if ((size_t)V * h < g.prefetch_bytes) g.prefetch_bytes = (size_t)V * h; }
         TZ_KERNEL(tenzo_cuda_tl1_gemv(&g, stream));
         launches += 2 * gemv_kernels;
     } else {
@@ -507,8 +509,16 @@ void Engine::enqueue_step(bool with_logits, bool feed_back, int max_len) {
                                         d_next, lm_scratch, use_pdl, stream));
         launches += batch >= 2 && h % 128 == 0 ? 3 : 2;   // (quantiser +) LM head + argmax finish
     }
-    advance_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(d_pos, d_tokens, d_next, batch, feed_back ? 1 : 0, V);
-    TZ_CUDA(cudaGetLastError());
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)(batch + 127) / 128);
+    c.blockDim = dim3(128);
+    c.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = attr;
+    c.numAttrs = use_pdl ? 1 : 0;
+    TZ_CUDA(cudaLaunchKernelEx(&c, advance_kernel, d_pos, d_tokens, (const int*)d_next, batch, feed_back ? 1 : 0, V, (int)use_pdl));
     launches += 1;
 }
 

@@ -67,10 +67,49 @@ __global__ void __launch_bounds__(kLmThreads, NS == 1 ? 4 : 0) lm_head_kernel(
     const int nvec = hidden >> 4;                                     // 16-byte pieces per row
     const bool vec_ok = (hidden & 15) == 0;
 
+    if constexpr (NS == 1) {
+        const size_t table = (size_t)vocab * hidden;
+        if (use_pdl && table > kLmPrefetchBefore)
+            l2_prefetch_slice(w + kLmPrefetchBefore, table - kLmPrefetchBefore < kLmPrefetchMore ? table - kLmPrefetchBefore : kLmPrefetchMore);
+    }
     if (use_pdl) pdl_wait();
 
-    // ---- prologue: final RMSNorm + absmax(127) quantiser (:1638, :1666-1678), one warp per sequence
-    for (int n = warp; n < NS; n += kLmWarps) {
+    // ---- prologue: final RMSNorm + absmax(127) quantiser (:1638, :1666-1678): one warp per sequence, or all of them for the one
+    // there is (a warp alone took 5 us for 2560 elements, a tenth of the kernel, with the memory idle)
+    if constexpr (NS == 1) {
+        __shared__ float s_red[kLmWarps + 1];
+        const float* xs = x + (size_t)seq0 * x_stride;
+        float m = 0.0f;
+        for (int i = tid; i < hidden; i += kLmThreads) {
+            const float v = __ldcg(xs + i);
+            s_y[i] = v;
+            if (!do_norm) m = fmaxf(m, fabsf(v));
+        }
+        __syncthreads();
+        if (do_norm) {
+            if (warp == 0) {
+                const float inv = rms_inv(warp_sumsq_reference_order(s_y, hidden, lane), hidden, eps);
+                if (lane == 0) s_red[kLmWarps] = inv;
+            }
+            __syncthreads();
+            const float inv_rms = s_red[kLmWarps];
+            for (int i = tid; i < hidden; i += kLmThreads) {
+                const float v = rms_apply(s_y[i], inv_rms, norm_w, i);
+                s_y[i] = v;
+                m = fmaxf(m, fabsf(v));
+            }
+        }
+        m = warp_max(m);
+        if (lane == 0) s_red[warp] = m;
+        __syncthreads();
+        m = fmaxf(warp_max(s_red[lane & (kLmWarps - 1)]), 1e-8f);
+        const float sx = m / 127.0f;                                  // :1671
+        const float inv_s = 1.0f / sx;                                // :1672
+        for (int i = tid; i < hpad; i += kLmThreads)
+            s_x8[i] = i < hidden ? (int8_t)(int)fminf(fmaxf(roundf(s_y[i] * inv_s), -128.0f), 127.0f) : (int8_t)0;
+        if (tid == 0) s_sx[0] = sx;
+    }
+    for (int n = warp; NS > 1 && n < NS; n += kLmWarps) {
         float* y = s_y + (size_t)n * hidden;
         int8_t* x8 = s_x8 + (size_t)n * hpad;
         if (seq0 + n >= batch) {
@@ -179,12 +218,17 @@ __global__ void __launch_bounds__(kLmThreads, NS == 1 ? 4 : 0) lm_head_kernel(
     }
 }
 
-__global__ void __launch_bounds__(256) argmax_finish_kernel(const LmBest* cta_best, int n, int* argmax_out) {
+__global__ void __launch_bounds__(256) argmax_finish_kernel(const LmBest* cta_best, int n, int* argmax_out, int use_pdl) {
     __shared__ LmBest s[256];
+    if (use_pdl) {
+        pdl_wait();
+        pdl_launch_dependents();
+    }
     const int seq = blockIdx.x, tid = threadIdx.x;
     LmBest b = {-INFINITY, 0x7fffffff};
     for (int i = tid; i < n; i += 256) {
-        const LmBest c = cta_best[(size_t)seq * n + i];
+        const LmBest* p = cta_best + (size_t)seq * n + i;
+        const LmBest c = {__ldcg(&p->val), __ldcg(&p->idx)};
         if (better(c.val, c.idx, b.val, b.idx)) b = c;
     }
     s[tid] = b;
@@ -197,15 +241,41 @@ __global__ void __launch_bounds__(256) argmax_finish_kernel(const LmBest* cta_be
     if (tid == 0) argmax_out[seq] = s[0].idx == 0x7fffffff ? 0 : s[0].idx;
 }
 
+static cudaError_t launch_argmax_finish(const LmBest* cand, int n, int* argmax_out, int batch, int use_pdl, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)batch);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = use_pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, argmax_finish_kernel, cand, n, argmax_out, use_pdl);
+}
+
 // vocab > 0: ids outside [0, vocab) are read as row 0 instead of reaching past the table.
 __global__ void embedding_i8_kernel(const int8_t* __restrict__ w, const float* __restrict__ row_scales, int hidden,
                                     const int* __restrict__ tokens, float* x, int x_stride, int vocab) {
     const int seq = blockIdx.x;
+    pdl_launch_dependents();                  // a launch behind this one that allows it: its weights come in meanwhile
     int tok = tokens[seq];
     if (vocab > 0 && (tok < 0 || tok >= vocab)) tok = 0;
     const int8_t* row = w + (size_t)tok * hidden;
     const float s = row_scales[tok];
-    for (int i = threadIdx.x; i < hidden; i += blockDim.x) x[(size_t)seq * x_stride + i] = (float)row[i] * s;   // :1313
+    float* o = x + (size_t)seq * x_stride;
+    if ((hidden & 3) == 0 && (reinterpret_cast<uintptr_t>(w) & 3) == 0) {     // four columns a load: one or two rounds
+#pragma unroll 4
+        for (int p = threadIdx.x; p < hidden >> 2; p += blockDim.x) {
+            const char4 v = reinterpret_cast<const char4*>(row)[p];
+            o[4 * p] = (float)v.x * s;                                        // :1313
+            o[4 * p + 1] = (float)v.y * s;
+            o[4 * p + 2] = (float)v.z * s;
+            o[4 * p + 3] = (float)v.w * s;
+        }
+        return;
+    }
+    for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = (float)row[i] * s;
 }
 
 __global__ void tl1_pack_rows2bit_kernel(const uint8_t* __restrict__ raw, int N, int K, uint8_t* packed) {
@@ -262,8 +332,7 @@ static int lm_head_launch(const float* x, const float* norm_w, int do_norm, floa
         rc = launch_lm_head_umma(q8, sx, w, row_scales, vocab, hidden, batch, logits, acc_out, argmax_out ? cand : nullptr, use_pdl, st);
         if (rc) return rc;
         if (argmax_out) {
-            argmax_finish_kernel<<<batch, 256, 0, st>>>(cand, n_tiles, argmax_out);
-            if (cudaGetLastError() != cudaSuccess) return (int)cudaErrorLaunchFailure;
+            if (launch_argmax_finish(cand, n_tiles, argmax_out, batch, use_pdl, st) != cudaSuccess) return (int)cudaErrorLaunchFailure;
         }
         return 0;
     }
@@ -292,8 +361,7 @@ static int lm_head_launch(const float* x, const float* norm_w, int do_norm, floa
                                                batch, logits, acc_out, static_cast<LmBest*>(scratch), use_pdl);
     if (e != cudaSuccess) return (int)e;
     if (argmax_out) {
-        argmax_finish_kernel<<<batch, 256, 0, st>>>(static_cast<const LmBest*>(scratch), kLmCtas, argmax_out);
-        e = cudaGetLastError();
+        e = launch_argmax_finish(static_cast<const LmBest*>(scratch), kLmCtas, argmax_out, batch, use_pdl, st);
     }
     return e == cudaSuccess ? 0 : (int)e;
 }

@@ -12,6 +12,10 @@ __device__ __forceinline__ bool better(float v, int i, float bv, int bi) {
     return v > bv || (v == bv && i < bi);
 }
 
+// The layer before the LM head asks for this much of the table; the one-sequence kernel asks for the next piece while its
+// own activations are being prepared (together they stay below the 126 MB of L2).
+constexpr size_t kLmPrefetchBefore = (size_t)64 << 20, kLmPrefetchMore = (size_t)24 << 20;
+
 constexpr int kLmuMaxTiles = 2048;   // 128-row vocabulary tiles the tensor-core path's scratch is sized for (vocab <= 262144)
 
 }  // namespace tz
