@@ -844,8 +844,10 @@ static cudaError_t launch_tl1_one(const GemvLaunch& L, cudaStream_t st) {
     const int hb = L.units >= 100 && L.units <= 148 && OneSmem::bytes(a.K, nb_cta, 2) <= 110 * 1024 ? 2 : 1;
     const size_t smem = OneSmem::bytes(a.K, nb_cta, hb);
     auto kernel = a.K <= 8 * kOneWorkers ? (hb == 2 ? tl1_one_kernel<2, 2> : tl1_one_kernel<2, 1>) : (hb == 2 ? tl1_one_kernel<4, 2> : tl1_one_kernel<4, 1>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(L.units * (3 - hb)), 1, 1);
     cfg.blockDim = dim3(kOneThreads, 1, 1);

@@ -7,12 +7,15 @@ eager/PyTorch fallback.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import torch
 
 from . import abi, load_library
 
 EPI_STORE, EPI_RESIDUAL, EPI_RELU2_GLU = 0, 1, 2
+_TL1_ARGS = struct.Struct("@PPifPii3i3fiPPPPPiiiPNPi0P")       # abi.Tl1GemvArgs
+assert _TL1_ARGS.size == C.sizeof(abi.Tl1GemvArgs)
 
 
 def _stream() -> int:
@@ -51,24 +54,16 @@ def tl1_gemv(x: torch.Tensor, w: torch.Tensor, n_blocks: int, K: int, scales, se
     acc = torch.empty(batch, n_blocks * 64, dtype=torch.int32, device=x.device) if want_acc else None
     a8 = torch.empty(batch, K, dtype=torch.int8, device=x.device) if want_act else None
     inv = torch.empty(batch, dtype=torch.float32, device=x.device) if want_act else None
-    scales = list(scales) + [0.0] * (3 - len(scales))
-    seg_ends = list(seg_ends) if seg_ends is not None else [n_blocks] * 3
-    seg_ends = seg_ends + [n_blocks] * (3 - len(seg_ends))
-    g = abi.Tl1GemvArgs()
-    g.x, g.norm_w, g.do_norm, g.eps = _ptr(x), _ptr(norm_w), int(do_norm), eps
-    g.w, g.n_blocks, g.K = _ptr(w), n_blocks, K
-    g.seg_end = (C.c_int * 3)(*seg_ends)
-    g.seg_scale = (C.c_float * 3)(*scales)
-    g.epilogue, g.resid, g.out = epilogue, _ptr(resid), _ptr(out)
-    g.acc_out, g.a_out, g.inv_out = _ptr(acc), _ptr(a8), _ptr(inv)
-    g.batch, g.x_stride, g.out_stride = batch, x.stride(0), out.stride(0)
+    scales = (*scales, 0.0, 0.0, 0.0)[:max(3, len(scales))]
+    seg_ends = (n_blocks,) * 3 if seg_ends is None else (*seg_ends, n_blocks, n_blocks, n_blocks)[:max(3, len(seg_ends))]
     ws = workspace
     if batch > 1 and ws is None:
         ws = torch.empty(lib.tenzo_cuda_tl1_gemv_workspace_bytes(batch, K), dtype=torch.uint8, device=x.device)
-    g.workspace, g.use_pdl = _ptr(ws), int(use_pdl)
-    if prefetch is not None:
-        g.prefetch, g.prefetch_bytes = _ptr(prefetch), prefetch.numel() * prefetch.element_size()
-    _ok(lib.tenzo_cuda_tl1_gemv(C.byref(g), _stream()), "tenzo_cuda_tl1_gemv")
+    # Packed in one go: a one-sequence call is bound by this function, not by its kernel (22 attribute assignments take 2.2 us).
+    g = _TL1_ARGS.pack(_ptr(x), _ptr(norm_w) or 0, do_norm, eps, _ptr(w) or 0, n_blocks, K, *seg_ends, *scales, epilogue, _ptr(resid) or 0, _ptr(out),
+                       _ptr(acc) or 0, _ptr(a8) or 0, _ptr(inv) or 0, batch, x.stride(0), out.stride(0), _ptr(prefetch) or 0,
+                       0 if prefetch is None else prefetch.numel() * prefetch.element_size(), _ptr(ws) or 0, use_pdl)
+    _ok(lib.tenzo_cuda_tl1_gemv(g, _stream()), "tenzo_cuda_tl1_gemv")
     return dict(out=out, acc=acc, a=a8, inv=inv)
 
 
