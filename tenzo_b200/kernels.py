@@ -19,7 +19,7 @@ assert _TL1_ARGS.size == C.sizeof(abi.Tl1GemvArgs)
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())      # the handle alone, without a Stream object
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
