@@ -77,7 +77,7 @@ def run_gemv(args):
         "data": "synthetic", "config": {"workload": f"gemv: TL1 bitlinear {N}x{K}, batch 1, {n_mat} distinct matrices per step "
                                                     f"({n_mat * N * K // 4 / 1e6:.0f} MB > L2), one graph per step", "pdl": int(args.pdl)},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "kernel": "tl1_mma_kernel", "achieved": gbs, "peak": peak[0], "peak_source": peak[1], "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": "tl1_one_kernel", "achieved": gbs, "peak": peak[0], "peak_source": peak[1], "unit": "GB/s",
                      "frac": gbs / peak[0], "traffic": 4482816.0, "traffic_source": "ncu dram__bytes_read+write per launch of this workload run with "
                      "--no-prefetch; with the next-matrix L2 prefetch on, ncu's cache flush between replays counts that matrix twice (8.9 MB)",
                      "bytes_per_launch": bytes_per, "us_per_launch": ms * 1e3 / launches},
@@ -327,7 +327,7 @@ def run_attn(args):
         "config": {"workload": f"attn: fused INT8-KV GQA decode attention, batch {B}, {nq}q/{nkv}kv heads, context {T}",
                    "l2": f"KV {bytes_per / 1e6:.0f} MB per step, larger than L2"},
         "gpu_launches": args.steps,
-        "roofline": {"bound": "hbm", "kernel": "attn_kernel", "achieved": gbs, "peak": peak[0], "peak_source": peak[1], "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": "split_scores, split_softmax and split_values kernels", "achieved": gbs, "peak": peak[0], "peak_source": peak[1], "unit": "GB/s",
                      "frac": gbs / peak[0], "traffic": bytes_per * (265.2 / 259.5),
                      "traffic_source": "ncu at 24 sequences: 260.2 MB read + 5.0 MB written for 259.5 MB algorithmic, scaled by the sequence count",
                      "bytes_per_launch": bytes_per, "us_per_launch": ms * 1e3},
