@@ -396,7 +396,8 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
 //     reference's, and only the scale is taken from the exact values; else (about one product in two hundred: some quotient
 //     within 1e-6 of a half) the activations are quantised again, as the reference does it, and the product repeated. Same
 //     results either way, bit for bit. What the check covers need not be exact before it: 31 / max is an approximate
-//     quotient, the rounding is an addition of 1.5 * 2^23.
+//     quotient, the rounding is an addition of 1.5 * 2^23. Nor need it be a number: a NaN or an overflow in x * w fails the
+//     check (the exact value is a NaN too, or the presumed integer is none of +-31 where that of the maximum has to be).
 //   * Cluster meetings. A CTA takes half a 64-row block (16 of the 32 bytes of each column pair: rows c and c + 32) over the
 //     whole of K instead of a block over half of K; with two blocks a CTA (GLU) and enough of them, whole blocks.
 //   * Byte shuffling. A weight word goes into the tensor core as it lies in memory, four rows of one column pair, masked but not
@@ -556,7 +557,9 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
         sa = warp_sum_i(sa);
         if (lane == 0 && sa) atomicAdd(s_sa, sa);
     };
-    // As the reference does it (:28-42): this thread's values, their maximum over the vector m.
+    // As the reference does it (:28-42): this thread's values, their maximum over the vector m. What is no number (a NaN element,
+    // or an infinite one, whose quotient is one) becomes the integer 0, as in the conversion of the other kernels; the rest lies
+    // within +-31.
     auto exact_quantise = [&](float m, auto value) {
         const float to_q = 31.0f / fmaxf(m, 1e-6f);
         int sa = 0;
@@ -565,7 +568,10 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
             if (tid + j * kOneWorkers < n_pieces) {
                 float v[4];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) v[k] = roundf(value(j, k) * to_q) + kRound;      // half away from zero
+                for (int k = 0; k < 4; ++k) {
+                    const float y = value(j, k) * to_q;
+                    v[k] = y == y ? roundf(y) + kRound : kRound;     // half away from zero
+                }
                 sa += put(j, v);
             }
         add_sa(sa);

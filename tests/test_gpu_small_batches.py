@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 from gpu_helpers import dev, host
-from helpers import synth
+from helpers import ora, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -58,6 +58,41 @@ def test_tl1_product_of_one_sequence_matches_the_batched_kernel(cuda_lib, N, K, 
         one = kernels.tl1_gemv(dev(x), *args, resid=dev(res) if resid else None, **kw)["out"]
         many = kernels.tl1_gemv(two(x), *args, resid=two(res) if resid else None, **kw)["out"]
         assert np.array_equal(host(one)[0], host(many)[0])
+    assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
+
+
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("what", ["nan", "inf", "all nan", "nan weight", "inf weight", "overflow"])
+@pytest.mark.parametrize("N,K", [(128, 64), (12800, 128), (192, 2592), (128, 6912)])
+def test_tl1_product_of_one_sequence_with_non_finite_activations(cuda_lib, N, K, what, norm):
+    """An element that is no number becomes the integer 0 (the CPU engine's conversion), so it must not reach the sum of the
+    activations either: integers, scale, accumulators and outputs equal those of the batched kernel, and the oracle's where the
+    vector goes into the quantiser as it is."""
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([85, N, K])
+    x, nw = rng.standard_normal((1, K)).astype(np.float32), (1 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    at = [0, K // 3, K - 1]
+    if what in ("nan", "inf"):
+        x[0, at] = [np.nan, np.nan, -np.nan] if what == "nan" else [np.inf, 1.0, -np.inf]
+    elif what == "all nan":
+        x[0] = np.nan
+    elif what == "overflow":                         # x * w overflows before it is divided by the root mean square
+        x[0, at], nw[at] = np.float32(1e18), np.float32(1e30)
+    else:
+        nw[at] = np.nan if what == "nan weight" else np.inf
+    w = dev(synth.random_tl1_packed(rng, N, K))
+    for epi in (kernels.EPI_STORE, kernels.EPI_RELU2_GLU):
+        args = (w, N // 64, K, [0.02, 0.03], [N // 128, N // 64])
+        kw = dict(epilogue=epi, norm_w=dev(nw) if norm else None, do_norm=norm, want_acc=True, want_act=True)
+        if epi == kernels.EPI_RELU2_GLU and N // 64 % 2:
+            continue
+        one, two = (kernels.tl1_gemv(dev(v), *args, **kw) for v in (x, np.concatenate([x, x[:, ::-1]])))
+        for k in ("a", "inv", "acc", "out"):
+            assert np.array_equal(host(one[k])[0], host(two[k])[0], equal_nan=True), f"{k} differs from the batched kernel's"
+        if not norm:
+            a = np.zeros(K, np.int8)
+            inv = ora.load_oracle().ora_act_quant31(ora.ptr(x[0], ora.c_f32p), K, ora.ptr(a, ora.c_i8p))
+            assert np.array_equal(host(one["a"])[0], a) and host(one["inv"])[0] == np.float32(inv)
     assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
 
 
