@@ -33,6 +33,7 @@
 
 #include "attn_common.cuh"
 #include "common.cuh"
+#include "umma.cuh"
 #include "../../include/tenzo_kernels.h"
 
 namespace tz {
@@ -594,36 +595,11 @@ __global__ void __launch_bounds__(TILED ? kTileThreads : kAttnThreads) attn_kern
 // The K cache as a 3-D byte tensor {128, rows per sequence, sequences} for the scoring warps' tile loads.
 // Block pools (paged): a 2-D byte matrix {128, every row of the pool}, read in boxes of one block slice (16 rows).
 static int make_k_tensor_map(const tenzo_attention_args& a, CUtensorMap* out, bool paged) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn)
-            return -4;
-        encode = reinterpret_cast<EncodeFn>(fn);
-    }
-    if (paged) {
-        const cuuint64_t rows = (cuuint64_t)a.n_pool_blocks * a.n_layers * a.n_kv * 16;
-        const cuuint64_t dims[2] = {(cuuint64_t)kHd, rows};
-        const cuuint64_t strides[1] = {(cuuint64_t)kHd};
-        const cuuint32_t box[2] = {(cuuint32_t)kHd, 16u};
-        const cuuint32_t estr[2] = {1u, 1u};
-        const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a.cache_k, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        return r == CUDA_SUCCESS ? 0 : -4;
-    }
+    if (paged)
+        return encode_2d(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.cache_k, kHd, (uint64_t)a.n_pool_blocks * a.n_layers * a.n_kv * 16, kHd, kHd, 16u, CU_TENSOR_MAP_SWIZZLE_128B);
     // rows reachable from the layers up to this one; tiles that run past them are zero-filled and their keys are never used
-    const cuuint64_t rows = (cuuint64_t)(a.layer + 1) * a.n_kv * a.max_seq;
-    const cuuint64_t dims[3] = {(cuuint64_t)kHd, rows, (cuuint64_t)a.batch};
-    const cuuint64_t strides[2] = {(cuuint64_t)kHd, (cuuint64_t)a.seq_stride_kv};
-    const cuuint32_t box[3] = {(cuuint32_t)kHd, (cuuint32_t)kTileKeys, 1u};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a.cache_k, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : -4;
+    const uint64_t rows = (uint64_t)(a.layer + 1) * a.n_kv * a.max_seq;
+    return encode_3d_bytes(out, a.cache_k, kHd, rows, (uint64_t)a.batch, (uint64_t)a.seq_stride_kv, kHd, (uint32_t)kTileKeys, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int GH, bool TILED, bool PAGED = false>

@@ -30,6 +30,7 @@
 
 #include "attn_common.cuh"
 #include "common.cuh"
+#include "umma.cuh"
 #include "../../include/tenzo_kernels.h"
 
 namespace tz {
@@ -391,27 +392,10 @@ __global__ void __launch_bounds__(128) attn_fast_merge_kernel(const FaLaunch L) 
 }
 
 static int fa_tensor_map(const tenzo_attention_args& a, const int8_t* base, CUtensorMap* out) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess || !fn)
-            return -4;
-        encode = reinterpret_cast<EncodeFn>(fn);
-    }
     // rows reachable from the layers up to this one; tiles that run past them are zero-filled and their keys masked
-    const cuuint64_t rows = (cuuint64_t)(a.layer + 1) * a.n_kv * a.max_seq;
-    const cuuint64_t dims[3] = {(cuuint64_t)kHd, rows, (cuuint64_t)a.batch};
-    const cuuint64_t strides[2] = {(cuuint64_t)kHd, (cuuint64_t)(a.batch > 1 ? a.seq_stride_kv : (size_t)rows * kHd)};
-    const cuuint32_t box[3] = {(cuuint32_t)kHd, (cuuint32_t)kFaBlk, 1u};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(base), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : -4;
+    const uint64_t rows = (uint64_t)(a.layer + 1) * a.n_kv * a.max_seq;
+    return encode_3d_bytes(out, base, kHd, rows, (uint64_t)a.batch, a.batch > 1 ? (uint64_t)a.seq_stride_kv : rows * kHd, kHd, (uint32_t)kFaBlk,
+                           CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 static size_t fa_smem_bytes() {

@@ -1,4 +1,4 @@
-// Pieces shared by the tcgen05 kernels (tl1_umma.cu, lm_head_umma.cu): mbarrier / proxy / tensor-memory
+// Pieces shared by the tcgen05 kernels (tl1_umma.cu, lm_head_umma.cu) and, the last, by the attention kernels: mbarrier / proxy / tensor-memory
 // helpers, the shared-memory operand descriptor for K-major tiles with the 128-byte swizzle, the
 // kind::i8 MMA issue, and the host-side tensor-map encoder (driver entry point fetched through the
 // runtime, so the library does not link against libcuda).
@@ -77,32 +77,39 @@ static inline TensorMapEncodeFn tensor_map_encoder() {
     return encode;
 }
 
+// One tensor map of `rank` dimensions. The encoder wants a current context, and a host thread that has made no runtime call
+// yet has none: cudaSetDevice makes the device's primary context the thread's (also while a stream is captured).
+static inline int encode_tensor_map(CUtensorMap* out, CUtensorMapDataType type, cuuint32_t rank, const void* base, const cuuint64_t* dims,
+                                    const cuuint64_t* strides, const cuuint32_t* box, CUtensorMapSwizzle swizzle) {
+    const TensorMapEncodeFn encode = tensor_map_encoder();
+    if (!encode) return -4;
+    const cuuint32_t estr[3] = {1u, 1u, 1u};
+    auto run = [&] {
+        return encode(out, type, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    if (run() == CUDA_SUCCESS) return 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return -4;
+    return run() == CUDA_SUCCESS ? 0 : -4;
+}
+
 // 2-D row-major tensor map: `inner` elements per row, `rows` rows `row_stride_bytes` apart, box {box_inner, box_rows}.
 static inline int encode_2d(CUtensorMap* out, CUtensorMapDataType type, const void* base, uint64_t inner, uint64_t rows, uint64_t row_stride_bytes,
                      uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
-    const TensorMapEncodeFn encode = tensor_map_encoder();
-    if (!encode) return -4;
     const cuuint64_t dims[2] = {inner, rows};
     const cuuint64_t strides[1] = {row_stride_bytes};
     const cuuint32_t box[2] = {box_inner, box_rows};
-    const cuuint32_t estr[2] = {1u, 1u};
-    const CUresult r = encode(out, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : -4;
+    return encode_tensor_map(out, type, 2, base, dims, strides, box, swizzle);
 }
 
 // 3-D byte tensor {inner, rows, planes}, rows `inner` bytes apart, planes `plane_stride` bytes apart, box {box_inner, box_rows, 1}.
 static inline int encode_3d_bytes(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t planes, uint64_t plane_stride,
                                   uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
-    const TensorMapEncodeFn encode = tensor_map_encoder();
-    if (!encode) return -4;
     const cuuint64_t dims[3] = {inner, rows, planes};
     const cuuint64_t strides[2] = {inner, plane_stride};
     const cuuint32_t box[3] = {box_inner, box_rows, 1u};
-    const cuuint32_t estr[3] = {1u, 1u, 1u};
-    const CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : -4;
+    return encode_tensor_map(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, base, dims, strides, box, swizzle);
 }
 
 }  // namespace tz
