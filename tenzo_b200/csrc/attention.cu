@@ -610,7 +610,7 @@ static int launch_attn(const AttnLaunch& L, cudaStream_t st) {
         if (int rc = make_k_tensor_map(L.a, &kmap, PAGED)) return rc;
     const size_t smem = (TILED ? AttnSmem<GH>::bytes_tiled(L.a.max_len, L.n_tile_warps) : AttnSmem<GH>::bytes(L.a.max_len)) +
                         (PAGED ? AttnSmem<GH>::table_bytes(L.a.max_len) : 0);
-    cudaError_t e = cudaFuncSetAttribute(attn_kernel<GH, TILED, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(attn_kernel<GH, TILED, PAGED>, kMaxSmem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(L.a.n_q / GH), (unsigned)L.a.batch, 1);

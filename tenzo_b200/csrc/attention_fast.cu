@@ -439,7 +439,7 @@ static cudaError_t fa_launch_ex(void (*kernel)(KArgs...), dim3 grid, dim3 block,
 template <int G>
 static int fa_launch(const FaLaunch& L, const CUtensorMap& km, const CUtensorMap& vm, cudaStream_t st) {
     const size_t smem = fa_smem_bytes();
-    cudaError_t e = cudaFuncSetAttribute(attn_fast_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(attn_fast_kernel<G>, smem);
     if (e != cudaSuccess) return (int)e;
     e = fa_launch_ex(attn_fast_kernel<G>, dim3((unsigned)L.n_splits, (unsigned)L.a.n_kv, (unsigned)L.a.batch), dim3(kFaThreads), smem, st, L.a.use_pdl != 0, L, km, vm);
     return e == cudaSuccess ? 0 : (int)e;

@@ -794,7 +794,7 @@ template <int GH, int GV, bool PAGED>
 static cudaError_t launch_values(const SplitLaunch& L, int heavy, int items, cudaStream_t st) {
     const int smem = heavy ? HeavyRing<GH>::bytes : LightRing<GV>::bytes;
     static_assert(HeavyRing<GH>::bytes >= LightRing<GV>::bytes, "");
-    cudaError_t e = cudaFuncSetAttribute(split_values_kernel<GH, GV, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, HeavyRing<GH>::bytes);
+    cudaError_t e = allow_smem(split_values_kernel<GH, GV, PAGED>, HeavyRing<GH>::bytes);
     if (e != cudaSuccess) return e;
     const int blocks = (heavy + 1) / 2 + (items - heavy) * (GH / GV) * 4;
     return split_launch(split_values_kernel<GH, GV, PAGED>, dim3((unsigned)blocks), kValueThreads, smem, st, L.a.use_pdl != 0, L, heavy);
@@ -805,8 +805,7 @@ static cudaError_t launch_softmax(const SplitLaunch& L, long long items, cudaStr
     using Shape = SoftShape<HS, MANY>;
     const int chunk = L.tp < Shape::chunk ? L.tp : Shape::chunk;
     const size_t smem = (size_t)2 * HS * ordered_sum_padded(chunk) * sizeof(float);
-    cudaError_t e = cudaFuncSetAttribute(split_softmax_kernel<GH, HS, PAGED, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    static_assert(2 * HS * ordered_sum_padded(Shape::chunk) * sizeof(float) <= 47 * 1024, "more than a kernel may have without asking");
     return split_launch(split_softmax_kernel<GH, HS, PAGED, MANY>, dim3((unsigned)(items * (GH / HS))), Shape::threads, smem, st, L.a.use_pdl != 0, L);
 }
 
@@ -815,7 +814,7 @@ static cudaError_t split_pass(const SplitLaunch& L, int n_seq, cudaStream_t st) 
     CUtensorMap km;
     if (k_tensor_map(L, &km)) return cudaErrorInvalidValue;
     const size_t smem = 1024 + (size_t)kScoreWarps * kSpTileBytes;
-    cudaError_t e = cudaFuncSetAttribute(split_scores_kernel<GH, PAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(split_scores_kernel<GH, PAGED>, smem);
     if (e != cudaSuccess) return e;
     e = split_launch(split_scores_kernel<GH, PAGED>, dim3((unsigned)L.n_spans, (unsigned)L.groups, (unsigned)n_seq), kScoreWarps * 32, smem, st, L.a.use_pdl != 0, L, km);
     if (e != cudaSuccess) return e;

@@ -12,6 +12,16 @@ namespace tz {
 
 constexpr int kWarp = 32;
 
+// The dynamic shared memory that launches of a kernel may ask for is an attribute of the kernel on its device, not of a launch,
+// and every host thread sets the same one. So it is always set to the most that any launch of the kernel asks for: a limit of
+// the call's own size would be lowered by another thread's smaller call between the setting and the launch, which is then
+// refused. (Set at each call and not once: it is gone after a device reset, and another device has its own.)
+constexpr size_t kMaxSmem = 227 * 1024;        // static and dynamic together
+template <typename Kernel>
+inline cudaError_t allow_smem(Kernel* kernel, size_t most) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // dp4a with unsigned bytes in `a` and signed bytes in `b` (PTX dp4a.u32.s32), accumulating in s32.
 __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
     int d;

@@ -1057,12 +1057,8 @@ bool pc_plan(int h, int qd, int kvd, int ffn, int n_q, int n_kv, int V, int n_la
 }
 
 cudaError_t pc_launch(const PcParams& p, int grid, cudaStream_t st) {
-    static int attr_bytes = 0;
-    if (p.plan.total_bytes > attr_bytes) {
-        cudaError_t e = cudaFuncSetAttribute(decode_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return e;
-        attr_bytes = 227 * 1024;
-    }
+    cudaError_t e = allow_smem(decode_persistent_kernel, kMaxSmem);
+    if (e != cudaSuccess) return e;
     void* args[] = {const_cast<PcParams*>(&p)};
     return cudaLaunchCooperativeKernel((const void*)decode_persistent_kernel, dim3((unsigned)grid), dim3(kPcBlock), args,
                                        (size_t)p.plan.total_bytes, st);

@@ -338,11 +338,11 @@ static int lm_head_launch(const float* x, const float* norm_w, int do_norm, floa
     }
     const size_t hpad = ((size_t)hidden + 15) & ~(size_t)15;
     auto smem_for = [&](int ns) { return (size_t)ns * hidden * sizeof(float) + 8 * sizeof(float) + (size_t)kLmWarps * ns * sizeof(LmBest) + ns * hpad + 16; };
-    const bool eight = allow_batched && batch > 1 && smem_for(8) <= 200 * 1024;   // eight sequences share each row read
+    constexpr size_t kMostSmem = 200 * 1024;
+    const bool eight = allow_batched && batch > 1 && smem_for(8) <= kMostSmem;    // eight sequences share each row read
     const size_t smem = smem_for(eight ? 8 : 1);
     if (smem > 48 * 1024) {
-        cudaError_t ea = eight ? cudaFuncSetAttribute(lm_head_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                               : cudaFuncSetAttribute(lm_head_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t ea = eight ? allow_smem(lm_head_kernel<8>, kMostSmem) : allow_smem(lm_head_kernel<1>, kMostSmem);
         if (ea != cudaSuccess) return (int)ea;
     }
     cudaLaunchConfig_t cfg = {};

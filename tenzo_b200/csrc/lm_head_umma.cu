@@ -210,7 +210,7 @@ int launch_lm_head_umma(const int8_t* q8, const float* sx, const int8_t* w, cons
     if (int rc = encode_2d(&omap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, obase, (uint64_t)vocab, (uint64_t)batch, (uint64_t)vocab * 4, kLmuRows,
                            (uint32_t)L.n_box, CU_TENSOR_MAP_SWIZZLE_NONE)) return rc;
     const size_t smem = LmUmmaSmem::bytes(L.n_box);
-    cudaError_t e = cudaFuncSetAttribute(lm_head_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(lm_head_umma_kernel, LmUmmaSmem::bytes(kLmuMaxN));
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)L.n_tiles, (unsigned)((batch + kLmuMaxN - 1) / kLmuMaxN), 1);

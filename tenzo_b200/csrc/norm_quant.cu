@@ -271,7 +271,7 @@ cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, f
     auto kernel = K <= 3072 ? act_quant_kernel<256, 3> : K <= 4096 ? act_quant_kernel<256, 4> : K <= 7168 ? act_quant_kernel<256, 7> : act_quant_kernel<512, 7>;
     const int threads = K <= 7168 ? 256 : 512;
     if (smem > 48 * 1024) {
-        cudaError_t ea = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+        cudaError_t ea = allow_smem(kernel, 96 * 1024);
         if (ea != cudaSuccess) return ea;
     }
     cudaLaunchConfig_t cfg = {};
@@ -302,7 +302,7 @@ extern "C" int tenzo_cuda_rmsnorm_quant(const float* x, const float* norm_w, int
     if (dim > 16384) return -5;
     const size_t smem = (size_t)(dim + 32) * sizeof(float);
     if (smem > 48 * 1024) {
-        cudaError_t ea = cudaFuncSetAttribute(tz::rmsnorm_quant_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+        cudaError_t ea = tz::allow_smem(tz::rmsnorm_quant_kernel, 80 * 1024);
         if (ea != cudaSuccess) return (int)ea;
     }
     tz::rmsnorm_quant_kernel<<<batch, tz::kNqThreads, smem, static_cast<cudaStream_t>(stream)>>>(

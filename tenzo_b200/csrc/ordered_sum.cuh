@@ -20,11 +20,11 @@ namespace tz {
 // `e` is in shared memory, 16-byte aligned, and readable up to ordered_sum_padded(n) floats, zeros beyond n. All 32 lanes
 // call it with the same arguments and get the same result.
 constexpr int kOrderedHead = 64;
-__host__ __device__ __forceinline__ int ordered_sum_segment(int n) {          // elements a lane takes behind the head: whole 16-byte pieces, an odd number of them (no bank conflicts)
+__host__ __device__ constexpr int ordered_sum_segment(int n) {          // elements a lane takes behind the head: whole 16-byte pieces, an odd number of them (no bank conflicts)
     const int pieces = n > kOrderedHead ? (n - kOrderedHead + 127) >> 7 : 1;
     return 4 * (pieces | 1);
 }
-__host__ __device__ __forceinline__ int ordered_sum_padded(int n) { return kOrderedHead + 32 * ordered_sum_segment(n); }
+__host__ __device__ constexpr int ordered_sum_padded(int n) { return kOrderedHead + 32 * ordered_sum_segment(n); }
 
 // The plain loop over n values (n a multiple of 4): eight 16-byte loads, then their 32 additions. Loading the next batch during
 // the additions is slower: a wait for one batch then also waits for the loads of the next.

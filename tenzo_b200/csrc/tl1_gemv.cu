@@ -409,12 +409,14 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
 // the product, 0.8 the rest of the chain and the check. In a decode step (launches overlapped) 3840 x 2560 4.8 -> 4.3 us,
 // 2560 x 2560 4.9 -> 3.9, gate|up 13824 x 2560 6.1 -> 5.2, 2560 x 6912 8.8 -> 7.2, against the kernel above.
 constexpr int kOneWorkers = kFusedWarps * 32, kOneThreads = kOneWorkers + 32;
+constexpr int kOneMaxK = 8192;
 
 struct OneSmem {
     // 32-bit words: s_d[128] | s_f[64] | s_b[sets * 8] | squares by chains [8][stride] | weights [nb_cta][K/2 column pairs][4 HB words]
     static constexpr int head_words = 128 + 64;
-    static __host__ __device__ int stride(int K) { return (K >> 3) | 4; }        // an odd number of 16-byte pieces: eight rows' pieces in different banks
-    static size_t bytes(int K, int nb_cta, int hb) { return (size_t)(head_words + (K >> 2) + 8 * stride(K) + nb_cta * (K >> 1) * 4 * hb) * 4; }
+    static __host__ __device__ constexpr int stride(int K) { return (K >> 3) | 4; }        // an odd number of 16-byte pieces: eight rows' pieces in different banks
+    static constexpr size_t bytes(int K, int nb_cta, int hb) { return (size_t)(head_words + (K >> 2) + 8 * stride(K) + nb_cta * (K >> 1) * 4 * hb) * 4; }
+    static constexpr size_t most() { return bytes(kOneMaxK, 2, 1); }             // two whole blocks a CTA only up to 110 KB (launch_tl1_one)
 };
 
 // Barrier of the 512 workers that also ors a flag.
@@ -808,9 +810,10 @@ static cudaError_t launch_gemv(const GemvLaunch& L, cudaStream_t st) {
     const tenzo_tl1_gemv_args& a = L.a;
     const int sets_per_cta = (L.nsets + L.ksplit - 1) / L.ksplit + 1;
     const size_t smem = Lay::bytes(sets_per_cta, a.K, a.epilogue == TENZO_EPI_RELU2_GLU ? 2 : 1);
-    if (smem > 220 * 1024) return cudaErrorInvalidValue;
+    constexpr size_t kMostSmem = 220 * 1024;
+    if (smem > kMostSmem) return cudaErrorInvalidValue;
     if (smem > 48 * 1024) {
-        cudaError_t ea = cudaFuncSetAttribute(tl1_mma_kernel<NT, FUSED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t ea = allow_smem(tl1_mma_kernel<NT, FUSED>, kMostSmem);
         if (ea != cudaSuccess) return ea;
     }
     cudaLaunchConfig_t cfg = {};
@@ -839,7 +842,7 @@ static cudaError_t launch_gemv(const GemvLaunch& L, cudaStream_t st) {
 
 static bool tl1_one_applicable(const tenzo_tl1_gemv_args& a) {
     const bool w = a.do_norm && a.norm_w;
-    return a.batch == 1 && a.K % 32 == 0 && a.K <= 8192 && ((reinterpret_cast<uintptr_t>(a.x) | (w ? reinterpret_cast<uintptr_t>(a.norm_w) : 0)) & 15) == 0;
+    return a.batch == 1 && a.K % 32 == 0 && a.K <= kOneMaxK && ((reinterpret_cast<uintptr_t>(a.x) | (w ? reinterpret_cast<uintptr_t>(a.norm_w) : 0)) & 15) == 0;
 }
 
 static cudaError_t launch_tl1_one(const GemvLaunch& L, cudaStream_t st) {
@@ -851,7 +854,7 @@ static cudaError_t launch_tl1_one(const GemvLaunch& L, cudaStream_t st) {
     const size_t smem = OneSmem::bytes(a.K, nb_cta, hb);
     auto kernel = a.K <= 8 * kOneWorkers ? (hb == 2 ? tl1_one_kernel<2, 2> : tl1_one_kernel<2, 1>) : (hb == 2 ? tl1_one_kernel<4, 2> : tl1_one_kernel<4, 1>);
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(kernel, OneSmem::most());
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};

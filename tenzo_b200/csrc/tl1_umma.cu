@@ -599,7 +599,7 @@ int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float*
     Kernel kernel = a.epilogue == TENZO_EPI_RELU2_GLU   ? (cl ? tl1_umma_kernel<TENZO_EPI_RELU2_GLU, true> : tl1_umma_kernel<TENZO_EPI_RELU2_GLU, false>)
                     : a.epilogue == TENZO_EPI_RESIDUAL ? (cl ? tl1_umma_kernel<TENZO_EPI_RESIDUAL, true> : tl1_umma_kernel<TENZO_EPI_RESIDUAL, false>)
                                                        : (cl ? tl1_umma_kernel<TENZO_EPI_STORE, true> : tl1_umma_kernel<TENZO_EPI_STORE, false>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kernel, kMaxSmem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)L.units, (unsigned)seq_tiles, (unsigned)L.ksplit);

@@ -1,4 +1,5 @@
-"""Per-kernel calls from host threads: from a thread that has made no CUDA call yet."""
+"""Per-kernel calls from host threads: from a thread that has made no CUDA call yet, and of different sizes from two threads side
+by side (a call's dynamic shared memory lies under a limit that is an attribute of the kernel, not of the launch)."""
 import ctypes as C
 import threading
 
@@ -101,3 +102,14 @@ def test_first_cuda_call_of_a_thread(cuda_lib, name):
         call.out.zero_()
         assert in_threads([call], 1) == [0]
         assert torch.equal(call.out, want)
+
+
+@pytest.mark.parametrize("name", PAIRS)
+def test_two_threads_with_different_sizes(cuda_lib, name):
+    calls = PAIRS[name](cuda_lib)
+    assert [c(torch.cuda.current_stream()) for c in calls] == [0, 0]
+    torch.cuda.synchronize()
+    want = [c.out.clone() for c in calls]
+    assert in_threads(calls, 4000) == [0, 0]
+    for c, w in zip(calls, want):
+        assert torch.equal(c.out, w)
