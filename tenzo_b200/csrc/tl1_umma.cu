@@ -555,14 +555,15 @@ bool tl1_umma_applicable(const tenzo_tl1_gemv_args& a) {
 // CTAs of a cluster that split one tile's K range: doubled while the grid still fits the SMs (one CTA per SM) and
 // every CTA keeps at least four 128-byte chunks. TENZO_UMMA_KSPLIT = 1, 2, 4 or 8 overrides the choice (measurement aid).
 static int pick_umma_ksplit(int ctas, int n_chunks) {
-    static int n_sm = 0, forced = -1;
-    if (forced < 0) {
+    static const int forced = [] {
         const char* e = std::getenv("TENZO_UMMA_KSPLIT");
         const int v = e ? std::atoi(e) : 0;
-        forced = (v == 1 || v == 2 || v == 4 || v == 8) ? v : 0;
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n_sm <= 0) n_sm = 148;
-    }
+        return v == 1 || v == 2 || v == 4 || v == 8 ? v : 0;
+    }();
+    static const int n_sm = [] {                             // (both set by one thread while others wait)
+        int dev = 0, n = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
+    }();
     if (forced) return forced <= n_chunks ? forced : 1;
     int k = 1;
     while (k < 8 && ctas * k * 2 <= n_sm && n_chunks / (k * 2) >= 4) k *= 2;

@@ -108,6 +108,18 @@ def test_kernel_entry_points_reject_bad_arguments_without_a_device(lib):
     assert lib.tenzo_cuda_attention_heads_per_cta(1, 20, 5, 256) == 1 and lib.tenzo_cuda_attention_heads_per_cta(64, 20, 5, 8192) == 4
 
 
+def test_tensor_core_cluster_size_from_many_threads_at_once():
+    """The first calls of a process, from several threads at once, see the same machine as later ones."""
+    import subprocess
+    import sys
+    code = ("import threading; from tenzo_b200 import load_library; L = load_library(); n = 8; got = [0] * n; start = threading.Barrier(n)\n"
+            "def work(i): start.wait(); got[i] = L.tenzo_cuda_tl1_gemm_ksplit(40, 2560, 64, 1)\n"
+            "ts = [threading.Thread(target=work, args=(i,)) for i in range(n)]; [t.start() for t in ts]; [t.join() for t in ts]; print(got)")
+    for _ in range(3):
+        r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, check=True)
+        assert r.stdout.split("\n")[0] == str([4] * 8)
+
+
 def test_tensor_core_gemm_layout_invariants(lib):
     """What the batched GEMM's hand-offs rely on, for every batch it can be given: the ring has a multiple of four slots
     (slot s then always belongs to expand group s % 4 and issuing thread s % 4, so each barrier's phases are seen in order
