@@ -150,7 +150,7 @@ def declare_ext_abi(L):
 
 def declare_kernel_abi(L):
     vp, i32, f32, sz = C.c_void_p, C.c_int, C.c_float, C.c_size_t
-    L.tenzo_cuda_tl1_gemv.restype, L.tenzo_cuda_tl1_gemv.argtypes = i32, [vp, vp]      # Tl1GemvArgs by reference, or its bytes
+    L.tenzo_cuda_tl1_gemv.restype, L.tenzo_cuda_tl1_gemv.argtypes = i32, [C.POINTER(Tl1GemvArgs), vp]
     L.tenzo_cuda_tl1_gemv_ksplit.restype, L.tenzo_cuda_tl1_gemv_ksplit.argtypes = i32, [i32, i32, i32]
     L.tenzo_cuda_tl1_gemm_ksplit.restype, L.tenzo_cuda_tl1_gemm_ksplit.argtypes = i32, [i32, i32, i32, i32]
     L.tenzo_cuda_tl1_gemm_layout.restype = i32

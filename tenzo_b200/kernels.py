@@ -7,6 +7,7 @@ eager/PyTorch fallback.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import struct
 
 import torch
@@ -16,6 +17,15 @@ from . import abi, load_library
 EPI_STORE, EPI_RESIDUAL, EPI_RELU2_GLU = 0, 1, 2
 _TL1_ARGS = struct.Struct("@PPifPii3i3fiPPPPPiiiPNPi0P")       # abi.Tl1GemvArgs
 assert _TL1_ARGS.size == C.sizeof(abi.Tl1GemvArgs)
+
+
+@functools.cache
+def _tl1_gemv_packed():
+    """tenzo_cuda_tl1_gemv for this module: a prototype of its own, which takes the bytes of _TL1_ARGS and no other object. The
+    library's shared one (abi.py) takes an abi.Tl1GemvArgs."""
+    fn = load_library()["tenzo_cuda_tl1_gemv"]
+    fn.restype, fn.argtypes = C.c_int, [C.c_char_p, C.c_void_p]
+    return fn
 
 
 def _stream() -> int:
@@ -63,7 +73,7 @@ def tl1_gemv(x: torch.Tensor, w: torch.Tensor, n_blocks: int, K: int, scales, se
     g = _TL1_ARGS.pack(_ptr(x), _ptr(norm_w) or 0, do_norm, eps, _ptr(w) or 0, n_blocks, K, *seg_ends, *scales, epilogue, _ptr(resid) or 0, _ptr(out),
                        _ptr(acc) or 0, _ptr(a8) or 0, _ptr(inv) or 0, batch, x.stride(0), out.stride(0), _ptr(prefetch) or 0,
                        0 if prefetch is None else prefetch.numel() * prefetch.element_size(), _ptr(ws) or 0, use_pdl)
-    _ok(lib.tenzo_cuda_tl1_gemv(g, _stream()), "tenzo_cuda_tl1_gemv")
+    _ok(_tl1_gemv_packed()(g, _stream()), "tenzo_cuda_tl1_gemv")
     return dict(out=out, acc=acc, a=a8, inv=inv)
 
 

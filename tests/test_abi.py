@@ -108,6 +108,24 @@ def test_kernel_entry_points_reject_bad_arguments_without_a_device(lib):
     assert lib.tenzo_cuda_attention_heads_per_cta(1, 20, 5, 256) == 1 and lib.tenzo_cuda_attention_heads_per_cta(64, 20, 5, 8192) == 4
 
 
+def test_kernel_entry_points_refuse_another_struct(lib):
+    for fn, other in ((lib.tenzo_cuda_tl1_gemv, abi.AttentionArgs), (lib.tenzo_cuda_attention_int8, abi.Tl1GemvArgs)):
+        for arg in (C.byref(other()), bytes(C.sizeof(abi.Tl1GemvArgs)), 8):
+            with pytest.raises(C.ArgumentError):
+                fn(arg, None)
+
+
+def test_packed_product_arguments_are_the_struct():
+    from tenzo_b200 import kernels
+    values = [float(i) if f in "f" else i for i, f in enumerate("PPifPiiiiifffiPPPPPiiiPNPi", 1)]
+    g = abi.Tl1GemvArgs.from_buffer_copy(kernels._TL1_ARGS.pack(*values))
+    got = []
+    for name, _ in abi.Tl1GemvArgs._fields_:
+        v = getattr(g, name)
+        got += list(v) if isinstance(v, C.Array) else [v.value if hasattr(v, "value") else v]
+    assert got == values
+
+
 def test_tensor_core_cluster_size_from_many_threads_at_once():
     """The first calls of a process, from several threads at once, see the same machine as later ones."""
     import subprocess
