@@ -29,7 +29,8 @@ def _tl1_gemv_packed():
 
 
 def _stream() -> int:
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())      # the handle alone, without a Stream object
+    # (0.75 us; torch.cuda.current_stream().cuda_stream gives the same handle by way of a Python object, in 3.3)
+    return torch.accelerator.current_stream().native_handle
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:

@@ -113,3 +113,12 @@ def test_two_threads_with_different_sizes(cuda_lib, name):
     assert in_threads(calls, 4000) == [0, 0]
     for c, w in zip(calls, want):
         assert torch.equal(c.out, w)
+
+
+def test_calls_go_to_the_current_stream(cuda_lib):
+    from tenzo_b200 import kernels
+    side = torch.cuda.Stream()
+    assert kernels._stream() == torch.cuda.current_stream().cuda_stream
+    with torch.cuda.stream(side):
+        assert kernels._stream() == side.cuda_stream
+    assert kernels._stream() == torch.cuda.current_stream().cuda_stream
