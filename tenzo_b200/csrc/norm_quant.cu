@@ -101,6 +101,9 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
                 w4[r] = i < k4 ? __ldg(reinterpret_cast<const float4*>(norm_w) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
+        // Chains of whole 16-byte pieces. For the other multiples of eight they gain nothing: the elements behind the last piece are
+        // added load by load (quantiser and product of 128 rows, in place and by chains: K = 2568 8.66 and 8.74 us at two sequences,
+        // 21.1 and 21.3 at 256; K = 6920 11.40 and 11.19, 28.37 and 28.30; K = 14344 17.53 and 17.51, 45.77 and 45.82).
         const bool chains = (K & 31) == 0;
         // The GEMM that consumes this kernel's output starts now: its prologue (tensor-memory allocation, the first weight
         // copies, expanding the first chunks) takes as long as the rest of this kernel; it waits for this grid before it
