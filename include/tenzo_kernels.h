@@ -87,6 +87,10 @@ TENZO_API size_t tenzo_cuda_tl1_gemv_workspace_bytes(int batch, int K);
  * since the last call gave up waiting — its output is then invalid; 0 otherwise; -1 if the query failed.
  * Synchronises with the device. */
 TENZO_API int tenzo_cuda_tl1_gemv_take_timeouts(void);
+/* One sequence: how many products since the last call were multiplied twice, because the integers presumed before the exact
+ * root mean square was known did not stand (same results either way; one product in 200 to 600, and vectors whose
+ * largest normalised magnitude is under the quantiser's floor of 1e-6 without being zero). -1 if the query failed. Synchronises with the device. */
+TENZO_API int tenzo_cuda_tl1_gemv_take_repeats(void);
 /* Test aid: launches a tiny kernel whose wait on a copy that is never issued runs out (after 2^8 polls), so that the flag
  * above is raised exactly as a real give-up raises it, without any fault or hang (the kernel finishes normally). Lets a
  * host exercise its own handling of the failure: the next tenzo_cuda_tl1_gemv_take_timeouts() returns 1, and an engine

@@ -50,7 +50,9 @@ def test_tl1_product_of_one_sequence_matches_the_batched_kernel(cuda_lib, N, K, 
     x *= {"zeros": 0.0, "tiny": 1e-20}.get(what, 1.0)
     w, n_blocks, norm = dev(synth.random_tl1_packed(rng, N, K)), N // 64, what != "plain"
     two = lambda a: dev(np.concatenate([a, a[:, ::-1]]))
-    for epi in [kernels.EPI_STORE, kernels.EPI_RESIDUAL] + ([kernels.EPI_RELU2_GLU] if n_blocks % 2 == 0 else []):
+    epilogues = [kernels.EPI_STORE, kernels.EPI_RESIDUAL] + ([kernels.EPI_RELU2_GLU] if n_blocks % 2 == 0 else [])
+    assert cuda_lib.tenzo_cuda_tl1_gemv_take_repeats() >= 0
+    for epi in epilogues:
         glu, res = epi == kernels.EPI_RELU2_GLU, rng.standard_normal((1, N)).astype(np.float32)
         args = (w, n_blocks, K, [0.02, 0.03] if glu else [0.02], [n_blocks // 2, n_blocks] if glu else None)
         kw = dict(epilogue=epi, norm_w=dev(nw) if norm else None, do_norm=norm)
@@ -58,6 +60,8 @@ def test_tl1_product_of_one_sequence_matches_the_batched_kernel(cuda_lib, N, K, 
         one = kernels.tl1_gemv(dev(x), *args, resid=dev(res) if resid else None, **kw)["out"]
         many = kernels.tl1_gemv(two(x), *args, resid=two(res) if resid else None, **kw)["out"]
         assert np.array_equal(host(one)[0], host(many)[0])
+    repeats = cuda_lib.tenzo_cuda_tl1_gemv_take_repeats()
+    assert repeats in {"normal": range(len(epilogues) + 1), "plain": [0], "zeros": [0]}.get(what, [len(epilogues)])     # halves, tiny: each time
     assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
 
 
