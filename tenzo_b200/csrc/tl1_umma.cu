@@ -652,7 +652,7 @@ extern "C" __attribute__((visibility("default"))) int tenzo_trace_umma_chunks(lo
 #endif
 
 extern "C" int tenzo_cuda_tl1_gemm_layout(int batch, int* slots, int* weight_groups, size_t* smem_bytes, size_t* epilogue_bytes) {
-    if (batch < 16) return -1;
+    if (batch < tz::kUmmaMinBatch) return -1;                    // the tensor-core path does not apply
     const int per_cta = batch < tz::kMaxN ? batch : tz::kMaxN, n_box = (per_cta + 15) & ~15;
     if (slots) *slots = tz::UmmaSmem::slots_for(n_box);
     if (weight_groups) *weight_groups = tz::UmmaSmem::pgroups_for(n_box);

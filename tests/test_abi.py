@@ -144,7 +144,7 @@ def test_tensor_core_gemm_layout_invariants(lib):
     by one waiter - a parity wait cannot tell phase k from phase k - 2), at least four of them, the A slots fit in tensor
     memory beside the accumulators, everything fits in an SM's shared memory, and the two rings can hold what the
     epilogue assembles in them."""
-    for batch in list(range(16, 273)) + [300, 1000, 4096]:
+    for batch in list(range(9, 273)) + [300, 1000, 4096]:
         slots, groups, smem, epi = C.c_int(), C.c_int(), C.c_size_t(), C.c_size_t()
         assert lib.tenzo_cuda_tl1_gemm_layout(batch, C.byref(slots), C.byref(groups), C.byref(smem), C.byref(epi)) == 0
         n_box = (min(batch, 256) + 15) // 16 * 16
@@ -155,7 +155,7 @@ def test_tensor_core_gemm_layout_invariants(lib):
         rings = slots.value * n_box * 128 + groups.value * 8 * 4096
         assert rings + 1024 < smem.value                 # plus alignment slack, barriers, per-sequence operands
         assert epi.value <= rings, (batch, epi.value, rings)
-    assert lib.tenzo_cuda_tl1_gemm_layout(15, None, None, None, None) == -1
+    assert lib.tenzo_cuda_tl1_gemm_layout(8, None, None, None, None) == -1
 
 
 def test_engine_creation_fails_loudly_without_a_gpu(lib):

@@ -319,7 +319,7 @@ def test_load_model_from_files_matches_the_cpu_engine(tmp_path, with_manifest):
 def test_chunked_prefill_equals_token_by_token(cuda_lib):
     """tenzo_ext_prefill_chunk (prompt rows through the GEMM path, K/V appended, causal attention as independent queries)
     leaves the same KV cache bytes and scales as token-by-token prefill and the same greedy continuation, which is also
-    the CPU engine's. Chunks of 1, 15 (per-sequence kernels), 16+ (tensor cores) and a chunk that starts mid-sequence."""
+    the CPU engine's. Chunks of 1 (one-sequence kernels), of nine and more (tensor cores) and a chunk that starts mid-sequence."""
     cfg = dict(synth.TINY, hidden_size=512, num_q_heads=4, num_kv_heads=2, ffn_dim=768, num_layers=2, vocab_size=2048, max_seq_len=400)
     m = synth.SyntheticModel(cfg, seed=41)
     prompt = synth.prompt_tokens(12, 301, cfg["vocab_size"])

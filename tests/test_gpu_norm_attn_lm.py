@@ -228,7 +228,7 @@ def test_full_vocab_lm_head_properties(cuda_lib):
 
 @pytest.mark.parametrize("V,H,B", [(5000, 256, 16), (1028, 128, 40), (128256, 2560, 64), (32000, 4096, 300)])
 def test_lm_head_tensor_core_path_matches_single_sequence_path(cuda_lib, V, H, B):
-    """16 or more sequences run on tcgen05: logits, accumulators and argmax (with duplicated best rows, so the
+    """Two or more sequences run on tcgen05: logits, accumulators and argmax (with duplicated best rows, so the
     first-maximum rule matters) equal the one-sequence kernel's, which the tests above pin to the reference."""
     from tenzo_b200 import kernels
     rng = np.random.default_rng([55, V, H, B])

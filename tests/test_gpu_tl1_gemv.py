@@ -153,7 +153,7 @@ def test_argument_errors(cuda_lib):
 
 @pytest.mark.parametrize("N,K,batch", [(128, 128, 16), (192, 256, 40), (640, 2560, 64), (2560, 6912, 256), (256, 384, 300), (128, 16384, 17)])
 def test_tensor_core_path_bit_exact(cuda_lib, N, K, batch):
-    """16 or more sequences with K a multiple of 128 run on tcgen05 (codes 0..2 as u8, activations s8,
+    """Nine or more sequences with K a multiple of 128 run on tcgen05 (codes 0..2 as u8, activations s8,
     int32 accumulators in tensor memory): accumulators, quantised activations and outputs equal the oracle's."""
     from tenzo_b200 import kernels
     rng = np.random.default_rng([45, N, K, batch])
