@@ -401,7 +401,7 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
 //     quotient, the rounding is an addition of 1.5 * 2^23. Nor need it be a number: a NaN or an overflow in x * w fails the
 //     check (the exact value is a NaN too, or the presumed integer is none of +-31 where that of the maximum has to be).
 //   * Cluster meetings. A CTA takes half a 64-row block (16 of the 32 bytes of each column pair: rows c and c + 32) over the
-//     whole of K instead of a block over half of K; with two blocks a CTA (GLU) and enough of them, whole blocks.
+//     whole of K instead of a block over half of K; whole blocks where halves would be more than one CTA an SM.
 //   * Byte shuffling. A weight word goes into the tensor core as it lies in memory, four rows of one column pair, masked but not
 //     transposed: its bytes are the k index there, and column n of B has the activation in byte n and zeroes elsewhere, so
 //     that column n of D is row n of the word.
@@ -418,7 +418,7 @@ struct OneSmem {
     static constexpr int head_words = 128 + 64;
     static __host__ __device__ constexpr int stride(int K) { return (K >> 3) | 4; }        // an odd number of 16-byte pieces: eight rows' pieces in different banks
     static constexpr size_t bytes(int K, int nb_cta, int hb) { return (size_t)(head_words + (K >> 2) + 8 * stride(K) + nb_cta * (K >> 1) * 4 * hb) * 4; }
-    static constexpr size_t most() { return bytes(kOneMaxK, 2, 1); }             // two whole blocks a CTA only up to 110 KB (launch_tl1_one)
+    static constexpr size_t most() { return bytes(kOneMaxK, 2, 1); }             // = bytes(kOneMaxK, 1, 2); two whole blocks a CTA only where they fit it
 };
 
 // Barrier of the 512 workers that also ors a flag.
@@ -852,9 +852,12 @@ static bool tl1_one_applicable(const tenzo_tl1_gemv_args& a) {
 static cudaError_t launch_tl1_one(const GemvLaunch& L, cudaStream_t st) {
     const tenzo_tl1_gemv_args& a = L.a;
     const int nb_cta = a.epilogue == TENZO_EPI_RELU2_GLU ? 2 : 1;
-    // Half blocks double the CTAs and halve their loops; whole blocks where their number comes near the SMs' already and two
-    // such CTAs fit an SM (the next kernel's come in beside this one's).
-    const int hb = L.units >= 100 && L.units <= 148 && OneSmem::bytes(a.K, nb_cta, 2) <= 110 * 1024 ? 2 : 1;
+    // Half blocks double the CTAs and halve their loops, but every CTA quantises the whole vector: they pay while each has an SM of
+    // its own. Products back to back in a graph, overlapped, half and whole blocks in us: 2560 wide 60 units 3.93 and 4.02,
+    // 74 4.02 and 4.19, 80 4.90 and 4.35, 108 5.25 and 4.53, 148 5.79 and 4.87, 224 9.57 and 6.40; with GLU 80 6.19 and 4.87,
+    // 108 6.66 and 5.13, 224 12.9 and 7.4; 4096 wide 60 4.70 and 4.68, 96 6.2 and 5.2, 224 with GLU 18.5 and 12.4; 1280 wide
+    // 60 3.50 and 3.51, 90 4.39 and 3.76. Only at 6912 whole blocks win from 40 units on already (6.73 and 6.32).
+    const int hb = 2 * L.units > 148 && OneSmem::bytes(a.K, nb_cta, 2) <= OneSmem::most() ? 2 : 1;
     const size_t smem = OneSmem::bytes(a.K, nb_cta, hb);
     auto kernel = a.K <= 8 * kOneWorkers ? (hb == 2 ? tl1_one_kernel<2, 2> : tl1_one_kernel<2, 1>) : (hb == 2 ? tl1_one_kernel<4, 2> : tl1_one_kernel<4, 1>);
     if (smem > 48 * 1024) {

@@ -39,7 +39,8 @@ def test_tl1_product_of_a_few_sequences_matches_one_at_a_time(cuda_lib, N, K, B)
 
 
 @pytest.mark.parametrize("what", ["normal", "halves", "zeros", "tiny", "plain"])
-@pytest.mark.parametrize("N,K", [(128, 32), (64, 64), (12800, 128), (192, 2592), (128, 4128), (128, 6912), (128, 8192)])
+@pytest.mark.parametrize("N,K", [(128, 32), (64, 64), (12800, 128), (192, 2592), (128, 4128), (128, 6912), (128, 8192),
+                                 (4736, 64), (4800, 64), (9472, 2560), (9600, 4096), (4800, 4128), (9600, 6912), (4800, 8192)])     # half and whole row blocks a CTA
 def test_tl1_product_of_one_sequence_matches_the_batched_kernel(cuda_lib, N, K, what):
     from tenzo_b200 import kernels
     rng = np.random.default_rng([84, N, K])
