@@ -764,6 +764,7 @@ void Engine::decode_greedy(const int* first, int n_steps, int* out) {
     if ((size_t)n_steps * batch > history_cap) {
         if (d_history) cudaFree(d_history);
         d_history = nullptr;
+        history_cap = 0;                                  // until there is a new buffer: the allocation may fail
         TZ_CUDA(cudaMalloc((void**)&d_history, (size_t)n_steps * batch * 4));
         history_cap = (size_t)n_steps * batch;
     }
