@@ -11,9 +11,16 @@
 //            key row and 64 broadcast LDS.128 of the query per key pair;
 //   softmax  one CTA per item or head; the ordered sum of the exponentials in parallel segments (ordered_sum.cuh);
 //   values   consumer warps that own the chains of an (item, dims, heads) unit, fed by producer warps.
-// Bound: instruction issue (FFMA and its conversions issue one per cycle and scheduler; packed f32x2 FMAs take two, so
-// they gain nothing). 64 x 8192 keys, 20/5 heads: 672 us in one kernel; here 115 us scores (33 instructions a key, 73 % of
-// the issue slots), 48 us softmax, 115 us values. One sequence of 6003 keys: 98 us, now 48.
+// What bounds it. A (key, item) takes 74 warp instructions (35.6 in the scores, 9.2 in the softmax, 29.2 in the value sums; 16 + 16
+// of them are the multiply-adds whose order is fixed), so 592 schedulers need 64 us a million. 64 x 8192 keys, 20/5 heads:
+// 672 us in one kernel, here 277, 106 us a million; 1536 prompt rows 100; lengths spread over a factor of two 115 (256
+// sequences up to 4096) to 156 (32 up to 2048, 32/8 heads), equal ones of the same maximum 104 and 130. The distance to 64: the
+// three kernels follow one another without overlap (113, 48 and 134 us at 64 x 8192, each alone and cold), the softmax lasts as
+// long as its summing warps' chains (38 % of the issue slots), scores and value sums use 62 to 67 % of theirs, and the
+// last round of the value sums is as long as its longest item (they are dealt out by index). Packed f32x2 FMAs hold the
+// FMA pipe for two cycles but one issue slot: 16 of them and 16 byte permutes take 46 cycles of a scheduler, 32 plain FMAs and the
+// permutes 65, so the scores and conversions would gain by them; they are not written that way yet.
+// One sequence of 6003 keys: 98 us in one kernel, here 47 (8.6, 15.6 and 34.5 us, each alone and cold).
 // Launched back to back with programmatic serialisation but without an early trigger: kernels that let their dependents in
 // before their own wait pile up on the SMs, and a small grid is then placed on the few that have room (one sequence of
 // 6003 keys took 211 us that way).
@@ -379,9 +386,11 @@ __global__ void __launch_bounds__(SoftShape<HS, MANY>::threads, SoftShape<HS, MA
 //          consumer warps each; V bytes by bulk copy, converted by the consumers (the sign-extending byte load and a
 //          32-bit conversion a dim);
 //   light  32 dims a CTA, one consumer warp of one or all heads: for when there are fewer items than schedulers. Four producer
-//          warps convert V to floats, which leaves the consumer a load, the weights and one FMA a chain and key: 4.9 cycles
-//          a key with one head against 7.1 with the conversion in the chain's warp (the FMA latency alone is 4.5). One
+//          warps convert V to floats, which leaves the consumer a load, the weights and one FMA a chain and key. One
 //          consumer a CTA because the floats pass the shared-memory pipe twice: four of them, at 13 cycles a key, waited for it.
+//          One sequence: 8.8 cycles a key with one head (6003 to 12000 keys), twice the FMA's latency; neither side waits for the
+//          other (some 30 of 630 cycles a chunk), so the loop of the chain and the producers' conversion would both have to shorten.
+//          Attention of one sequence of 6003 keys 47 us, with the heavy shape 66.
 constexpr int kValueThreads = 192;                    // heavy: four consumer warps, one a scheduler, and two producers; light: 1 + 4
 constexpr int kValueKeys = 64, kValueStages = 3;
 template <int GV>
@@ -779,10 +788,11 @@ static cudaError_t split_launch(void (*kernel)(KArgs...), dim3 grid, int threads
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// How the value sums of `items` items are cut. Heavy items run best when each of the 592 schedulers has the same number of
-// their warps, so whole rounds of 296 items are heavy; a rest that would leave most SMs idle for a round, and a batch as
-// small as that, is light (64 x 8192 keys, 20/5 heads: 276 us all heavy, 253 with 24 of the 320 items light; 60 items of
-// 1500: 34.9 and 33.5; 100 items of 2048: 53 and 58). One head a CTA only where even then few SMs have one.
+// How the value sums of `items` items are cut. Heavy items run best when each of the 592 schedulers (148 SMs) has the same
+// number of their warps, so whole rounds of 296 items are heavy; a rest that would leave most SMs idle for a round, and a
+// batch as small as that, is light (64 x 8192 keys, 20/5 heads: 276 us all heavy, 253 with 24 of the 320 items light; 60 items of
+// 1500 36.8 all heavy and 35.7 all light, 70 items 37.5 and 36.3, 80 items 42.1 and 48.1; 100 items of 2048 54.8 and 62.3). One
+// head a CTA only where even then few SMs have one. The cut goes by the number of items, whatever their lengths.
 struct ValueSplit { int heavy, gv; };
 static ValueSplit pick_values(long long items, int gh) {
     const long long rest = items % 296;
