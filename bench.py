@@ -256,8 +256,8 @@ def gemv_stack_roofline(engine, model, iters, peak):
     sec_per_launch = ms * 1e-3 / launches
     achieved = bytes_per_launch / sec_per_launch / 1e9
     return {"bound": "hbm", "kernel": "tl1_one_kernel", "achieved": achieved, "peak": peak[0], "peak_source": peak[1],
-            "unit": "GB/s", "frac": achieved / peak[0], "traffic": 1.005 * bytes_per_launch,
-            "traffic_source": "ncu dram__bytes_read+write of the 6912x2560 launch with the next-matrix L2 prefetch off: 1.005 x algorithmic",
+            "unit": "GB/s", "frac": achieved / peak[0], "traffic": 1.002 * bytes_per_launch,
+            "traffic_source": "ncu dram__bytes_read+write of the 6912x2560 launch with the next-matrix L2 prefetch off: 1.001 to 1.002 x algorithmic",
             "bytes_per_launch": bytes_per_launch, "us_per_launch": sec_per_launch * 1e6, "launches_timed": launches}
 
 
@@ -321,8 +321,8 @@ def attention_roofline(B, ctx, steps, peak, mode=0):
     torch.cuda.empty_cache()
     return {"bound": "hbm", "kernel": "attn_fast_kernel (+ append, merge)" if mode == 1 else "split_scores, split_softmax and split_values kernels", "achieved": gbs, "peak": peak[0],
             "peak_source": peak[1], "unit": "GB/s", "frac": gbs / peak[0],
-            "traffic": bytes_per * (265.2 / 259.5) if mode == 0 else bytes_per * (265.6 / 259.5),
-            "traffic_source": "ncu at 24 sequences x 8192 keys: 1.02 x algorithmic, scaled by the keys read" if mode == 0 else
+            "traffic": bytes_per * (297.5 / 259.5) if mode == 0 else bytes_per * (265.6 / 259.5),
+            "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.6 MB read + 5.9 MB written for 259.5 MB algorithmic, scaled by the keys read" if mode == 0 else
                               "ncu at 24 sequences x 8192 keys: 259.8 MB read + 5.8 MB of partial outputs written for 259.5 MB algorithmic, scaled by the keys read",
             "bytes_per_launch": bytes_per, "us_per_launch": ms * 1e3, "launches_timed": steps,
             "l2": f"{bytes_per / 1e6:.0f} MB of KV per launch, larger than L2" if bytes_per > 130e6 else "smaller than L2: an upper bound"}
