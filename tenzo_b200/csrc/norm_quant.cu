@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(kNqThreads) rmsnorm_quant_kernel(
 // packed tensor-core B fragments tl1_mma_kernel consumes: words[seq][set][t][0] holds 4*a for the
 // even columns of column pairs 16*set + 4*i + t (byte i = 0..3), words[seq][set][t][1] the odd
 // columns unscaled; columns beyond K are zero. inv[seq] = max|y|/31. `words` may be null (tensor-core GEMM
-// path: it takes the plain int8 matrix a_out [batch][K] and sum_out[seq] = sum_k a_k instead).
+// path: it takes the int8 matrix a_mma [batch][K] and sum_out[seq] = sum_k a_k instead). a_out, where asked for: the plain
+// int8 matrix.
 #ifdef TZ_AQ_TRACE
 __device__ long long g_aq_trace[8];
 #define AQT(i) do { if (blockIdx.x == 0 && threadIdx.x == 0) g_aq_trace[i] = clock64(); } while (0)
@@ -73,12 +74,21 @@ __device__ long long g_aq_trace[8];
 // neighbours' in different banks.
 __host__ __device__ __forceinline__ int squares_stride(int K) { return (((K >> 3) + 3) & ~3) + 4; }
 
+// a_mma: every four elements 4i .. 4i + 3 are one word, the even ones times four (124 at most) in its lower half and the odd ones
+// in its upper half, for words i with bit 1 set in reversed order, and words i with bit 2 set change places in pairs:
+// the order in which tl1_umma_kernel's expanding threads come by the codes.
+__device__ __forceinline__ uint32_t mma_word(int i, int q0, int q1, int q2, int q3) {
+    const uint32_t b0 = (uint8_t)(4 * q0), b1 = (uint8_t)(4 * q2), b2 = (uint8_t)q1, b3 = (uint8_t)q3;
+    return (i >> 1) & 1 ? b1 | b0 << 8 | b3 << 16 | b2 << 24 : b0 | b1 << 8 | b2 << 16 | b3 << 24;
+}
+__device__ __forceinline__ int mma_place(int i) { return i ^ ((i >> 2) & 1); }
+
 // A thread holds kAqVec 16-byte pieces of the row in registers (launch_act_quant picks threads and pieces by K; longer rows
 // go through shared memory).
 template <int kAqThreads, int kAqVec>
 __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
     const float* x, const float* __restrict__ norm_w, int do_norm, float eps, int K, int x_stride,
-    uint32_t* words, float* inv, int8_t* a_out, int* sum_out, int use_pdl) {
+    uint32_t* words, float* inv, int8_t* a_out, int8_t* a_mma, int* sum_out, int use_pdl) {
     extern __shared__ __align__(16) float s_y[];   // K floats (or eight padded rows of K/8 squares) + 32 scratch
     const int stride = squares_stride(K);
     float* s_f = s_y + (8 * stride > K ? 8 * stride : K);
@@ -187,7 +197,7 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
                 words[(size_t)seq * nsets * 8 + wd] = word;
             }
         }
-        if (a_out || sum_out) {
+        if (a_out || a_mma || sum_out) {
             int part = 0;
 #pragma unroll
             for (int r = 0; r < kAqVec; ++r) {
@@ -197,6 +207,7 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
                     if (a_out)
                         reinterpret_cast<uint32_t*>(a_out + (size_t)seq * K)[i] =
                             (uint32_t)(uint8_t)(int8_t)q0 | ((uint32_t)(uint8_t)(int8_t)q1 << 8) | ((uint32_t)(uint8_t)(int8_t)q2 << 16) | ((uint32_t)(uint8_t)(int8_t)q3 << 24);
+                    if (a_mma) reinterpret_cast<uint32_t*>(a_mma + (size_t)seq * K)[mma_place(i)] = mma_word(i, q0, q1, q2, q3);
                     part += q0 + q1 + q2 + q3;
                 }
             }
@@ -252,6 +263,11 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
             if (a_out) a_out[(size_t)seq * K + i] = (int8_t)q;
             part += q;
         }
+        for (int i = tid; a_mma && i < K >> 2; i += kAqThreads) {
+            const float* y = s_y + 4 * i;
+            reinterpret_cast<uint32_t*>(a_mma + (size_t)seq * K)[mma_place(i)] =
+                mma_word(i, (int)roundf(y[0] * to_q), (int)roundf(y[1] * to_q), (int)roundf(y[2] * to_q), (int)roundf(y[3] * to_q));
+        }
         if (sum_out) {                        // sum_k a_k, for kernels that multiply by the unsigned codes w+1
             int* s_i = reinterpret_cast<int*>(s_f);
             __syncthreads();
@@ -266,7 +282,7 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
 }
 
 cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, float eps, int K, int batch, int x_stride,
-                             uint32_t* words, float* inv, int8_t* a_out, int* sum_out, int use_pdl, cudaStream_t st) {
+                             uint32_t* words, float* inv, int8_t* a_out, int8_t* a_mma, int* sum_out, int use_pdl, cudaStream_t st) {
     const int rows = 8 * squares_stride(K);
     const size_t smem = (size_t)((rows > K ? rows : K) + 32) * sizeof(float);
     // 16-byte pieces a thread: as few as the row needs (registers: 1536 rows of 2560 in 21 us with seven, 13 with three), 512
@@ -287,7 +303,7 @@ cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, f
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = use_pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, x, norm_w, do_norm, eps, K, x_stride, words, inv, a_out, sum_out, use_pdl);
+    return cudaLaunchKernelEx(&cfg, kernel, x, norm_w, do_norm, eps, K, x_stride, words, inv, a_out, a_mma, sum_out, use_pdl);
 }
 
 }  // namespace tz

@@ -802,7 +802,7 @@ static int pick_ksplit(int n_blocks, int K, int epilogue, int batch) {
 
 // act_quant_kernel lives in norm_quant.cu
 cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, float eps, int K, int batch, int x_stride,
-                             uint32_t* words, float* inv, int8_t* a_out, int* sum_out, int use_pdl, cudaStream_t st);
+                             uint32_t* words, float* inv, int8_t* a_out, int8_t* a_mma, int* sum_out, int use_pdl, cudaStream_t st);
 // tcgen05 GEMM for nine or more sequences (tl1_umma.cu)
 bool tl1_umma_applicable(const tenzo_tl1_gemv_args& a);
 int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float* inv, const int* sum_a, cudaStream_t st);
@@ -972,13 +972,12 @@ extern "C" int tenzo_cuda_tl1_gemv(const tenzo_tl1_gemv_args* args, void* stream
         if (tl1_umma_applicable(a)) {
             int8_t* a8 = static_cast<int8_t*>(a.workspace);
             int* sums = reinterpret_cast<int*>(inv + a.batch);
-            e = launch_act_quant(a.x, a.norm_w, a.do_norm, a.eps, a.K, a.batch, a.x_stride, nullptr, inv, a8, sums, a.use_pdl, st);
+            e = launch_act_quant(a.x, a.norm_w, a.do_norm, a.eps, a.K, a.batch, a.x_stride, nullptr, inv, a.a_out, a8, sums, a.use_pdl, st);
             if (e != cudaSuccess) return (int)e;
             if (a.inv_out && (e = cudaMemcpyAsync(a.inv_out, inv, (size_t)a.batch * sizeof(float), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return (int)e;
-            if (a.a_out && (e = cudaMemcpyAsync(a.a_out, a8, (size_t)a.batch * a.K, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return (int)e;
             return launch_tl1_umma(a, a8, inv, sums, st);
         }
-        e = launch_act_quant(a.x, a.norm_w, a.do_norm, a.eps, a.K, a.batch, a.x_stride, words, inv, a.a_out, nullptr, a.use_pdl, st);
+        e = launch_act_quant(a.x, a.norm_w, a.do_norm, a.eps, a.K, a.batch, a.x_stride, words, inv, a.a_out, nullptr, nullptr, a.use_pdl, st);
         if (e != cudaSuccess) return (int)e;
         if (a.inv_out) {
             e = cudaMemcpyAsync(a.inv_out, inv, (size_t)a.batch * sizeof(float), cudaMemcpyDeviceToDevice, st);

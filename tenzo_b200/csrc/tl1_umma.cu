@@ -5,8 +5,9 @@
 // (src/runtime/TenzoEngine.cpp:22-166 and the call shapes :1547-1628 of the reference): integer
 // accumulators are exact, so the result is bit-identical to the one-sequence path.
 //
-//   D[128 weight rows][N sequences] (int32, TMEM) += A[128][K] (u8 codes 0,1,2, TMEM) * B[K][N] (s8 activations, smem)
-//   sum_k w*a = sum_k code*a - sum_k a          (w = code - 1; the per-sequence sum comes from the quantiser)
+//   D[128 weight rows][N sequences] (int32, TMEM) += A[128][K] (u8 codes 0,1,2 times 1,4 or 16,64, TMEM) * B[K][N] (s8
+//   activations times 4,1, smem); sum_k w*a = sum_k code*a - sum_k a   (w = code - 1; the per-sequence sum comes from the
+//   quantiser)
 //
 // One CTA per 128-row tile (two 64-row TL1 blocks; for the GLU epilogue the gate block and its up block, so the
 // activation is applied inside the CTA). K is walked in 128-byte chunks through a ring of 4, 8 or 12 slots (a multiple of
@@ -138,7 +139,7 @@ struct UmmaSmem {
 // One 16-sequence block of the epilogue: r = accumulators of TMEM lane m (weight row `row`, `rr` inside its block).
 template <int EPI>
 __device__ __forceinline__ void umma_epilogue_block(const tenzo_tl1_gemv_args& a, uint32_t (&r)[16], const float* s_inv, const int* s_sum, float wscale,
-                                                    int c0, int seq0, int block, int rr, int row, bool up_half, float* s_out_cols, float* s_glu_cols, bool ok) {
+                                                    int shift, int c0, int seq0, int block, int rr, int row, bool up_half, float* s_out_cols, float* s_glu_cols, bool ok) {
     float v[16];
 #pragma unroll
     for (int i = 0; i < 16; i += 4) {
@@ -148,7 +149,7 @@ __device__ __forceinline__ void umma_epilogue_block(const tenzo_tl1_gemv_args& a
         const float i4[4] = {iv.x, iv.y, iv.z, iv.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int accv = (int)r[i + e] - s4[e];
+            const int accv = ((int)r[i + e] >> shift) - s4[e];
             r[i + e] = (uint32_t)accv;
             v[i + e] = (float)accv * (i4[e] * wscale);      // :1554, :118
         }
@@ -324,13 +325,17 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         // Quarter q = warp & 3 owns TMEM lanes 32q..32q+31 = row block q >> 1, nibble half q & 1. Thread 4g + t holds
         // lanes g + 8*jj (jj = 0..3) = rows 4g + jj of the half = the four bytes of packed word g of a column pair, and
         // the columns 8n + 2t, 8n + 2t + 1 = column pairs 16n + 4t .. 16n + 4t + 3. The four words of a (thread, n) are
-        // fetched in the order u ^ t so that a warp's request covers 32 banks; the byte permutes that transpose them
-        // take the order back (selectors chosen per thread).
+        // fetched in the order u ^ t so that a warp's request covers 32 banks. A column is made of two words: their
+        // bytes, and of each byte the even column's code in the lower half, the odd column's in the upper, where they lie
+        // (1 and 4 times the code for the nibbles of the first 32 rows, 16 and 64 times for the second; the even columns'
+        // activations carry a four, and the epilogue shifts the sums back). The order of K that comes of it is the one the
+        // quantiser writes (mma_word): one permute and one mask a column, where shifting the codes down and putting the
+        // columns in order took two to four more of a pipe that takes one in two cycles. (Quantiser and product, 12 sequences: 13824 x 2560 with
+        // GLU 15.4 -> 13.9 us, 28672 x 4096 33.1 -> 29.2; 256 sequences: 23.8 -> 22.5 and 52.7 -> 48.6.)
         const int q = warp & 3, grp = (warp - 2) >> 2;
         const int blk = q >> 1, hi = q & 1, g = lane >> 2, t = lane & 3;
         const bool have = blk == 0 || blk1 >= 0;
-        const uint32_t sel_a = (t & 1) ? 0x1504u : 0x5140u, sel_b = (t & 1) ? 0x3726u : 0x7362u;
-        const uint32_t sel_lo = (t & 2) ? 0x1054u : 0x5410u, sel_hi = (t & 2) ? 0x3276u : 0x7632u;
+        const uint32_t codes = hi ? 0xC0C03030u : 0x0C0C0303u;
         int woff[4];                                           // word offsets of the four loads inside a 16-column-pair set
 #pragma unroll
         for (int u = 0; u < 4; ++u) woff[u] = (4 * t + (u ^ t)) * 8 + g;
@@ -389,20 +394,13 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
                     for (int u = 0; u < 4; ++u) W[4 * n + u] = (have && sp_ok) ? sP[n * 128 + woff[u]] : 0u;
                 uint32_t lo[16], up[16];                       // registers of the two stores: lanes 0-15 (jj = 0, 1) and 16-31 (jj = 2, 3)
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
-                    // 4x4 byte transpose: T[jj] = byte jj of the words of column pairs 16n + 4t + 0..3
-                    const uint32_t p0 = prmt(W[4 * n], W[4 * n + 1], sel_a), p1 = prmt(W[4 * n + 2], W[4 * n + 3], sel_a);
-                    const uint32_t p2 = prmt(W[4 * n], W[4 * n + 1], sel_b), p3 = prmt(W[4 * n + 2], W[4 * n + 3], sel_b);
-                    const uint32_t T[4] = {prmt(p0, p1, sel_lo), prmt(p0, p1, sel_hi), prmt(p2, p3, sel_lo), prmt(p2, p3, sel_hi)};
+                for (int n = 0; n < 4; ++n)
 #pragma unroll
-                    for (int jj = 0; jj < 4; ++jj) {
-                        const uint32_t nb = T[jj] >> (4 * hi);
-                        const uint32_t e = nb & 0x03030303u, o = (nb >> 2) & 0x03030303u;    // codes of the even / odd columns
+                    for (int jj = 0; jj < 4; ++jj) {           // byte jj of two words, twice, and its codes left where they are
                         uint32_t* dst = (jj < 2 ? lo : up) + 4 * n + 2 * (jj & 1);
-                        dst[0] = prmt(e, o, 0x5140u);
-                        dst[1] = prmt(e, o, 0x7362u);
+                        dst[0] = prmt(W[4 * n], W[4 * n + 1], 0x4040u + 0x1111u * jj) & codes;
+                        dst[1] = prmt(W[4 * n + 2], W[4 * n + 3], 0x4040u + 0x1111u * jj) & codes;
                     }
-                }
                 const uint32_t ta = tmem_base + tmem_a0 + (uint32_t)(32 * s) + ((uint32_t)(32 * q) << 16);
                 if (UCHK(tmem_a0 + 32 * s + 32 <= (uint32_t)kTmemCols && (tmem_base & 0xffffu) == 0u, 4, tmem_a0 + 32 * s, tmem_base)) {
                     tmem_st_16x256b_x4(ta, lo);
@@ -455,6 +453,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         const int m = 32 * q + lane;                         // TMEM lane
         const int rblk = q >> 1, rr = 32 * (q & 1) + 4 * (lane & 7) + (lane >> 3), row = 64 * rblk + rr;
         const int block = rblk ? blk1 : blk0;
+        const int shift = q & 1 ? 6 : 2;                     // the sums are 4 and 64 times the products (exactly)
         const float wscale = block >= 0 ? umma_seg_scale(a, block) : 0.0f;
         // Output columns [sequences][128 rows] (GLU: [..][64]) are assembled in shared memory the pipeline no longer
         // needs - the rings, which are contiguous; with a cluster behind the partial tile the peers are reading - and
@@ -498,9 +497,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             }
             float* unit_out = s_out + (size_t)16 * ob0 * row_floats;
             float* unit_glu = s_glu + (size_t)16 * ob0 * 64;
-            umma_epilogue_block<EPI>(a, r0, s_inv, s_sum, wscale, c0, seq0, block, rr, row, rblk == 1, unit_out, unit_glu, ok);
+            umma_epilogue_block<EPI>(a, r0, s_inv, s_sum, wscale, shift, c0, seq0, block, rr, row, rblk == 1, unit_out, unit_glu, ok);
             if (two)
-                umma_epilogue_block<EPI>(a, r1, s_inv, s_sum, wscale, c0 + 16, seq0, block, rr, row, rblk == 1, unit_out + 16 * row_floats,
+                umma_epilogue_block<EPI>(a, r1, s_inv, s_sum, wscale, shift, c0 + 16, seq0, block, rr, row, rblk == 1, unit_out + 16 * row_floats,
                                          unit_glu + 16 * 64, ok);
             if (glu) {
                 // gate and up halves of the unit are both in shared memory: out = ReLU(gate)^2 * up, four floats at a time
@@ -570,7 +569,7 @@ static int pick_umma_ksplit(int ctas, int n_chunks) {
     return k;
 }
 
-// a8 [batch][K] int8 (16-byte aligned), inv [batch], sum_a [batch] already produced on `st`.
+// a8 [batch][K] int8 in the order of act_quant_kernel's a_mma (16-byte aligned), inv [batch], sum_a [batch] already produced on `st`.
 int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float* inv, const int* sum_a, cudaStream_t st) {
     UmmaLaunch L;
     L.a = a;

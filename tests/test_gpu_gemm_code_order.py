@@ -1,0 +1,41 @@
+"""Tensor-core TL1 product: the order of K in which codes and activations meet (codes left in place, even activations times
+four, sums shifted back). Accumulators, plain activations and outputs bit for bit against the CPU, with the quantiser's
+register path and its element-by-element path (rows above 14336, rows not on a 16-byte boundary), the smallest K, all four K
+splits and weights and activations at their extremes, where the scaled sums are largest."""
+import numpy as np
+import pytest
+import torch
+from gpu_helpers import cpu_bitlinear, dev, host
+from helpers import ora, synth
+
+pytestmark = pytest.mark.gpu
+P = ora.ptr
+
+
+@pytest.mark.parametrize("N,K,batch,aligned,extreme", [
+    (128, 128, 9, True, False), (64, 256, 16, False, False), (192, 640, 17, True, True), (128, 2560, 70, True, False),
+    (128, 6912, 9, False, True), (2560, 1024, 33, True, False), (128, 14464, 12, True, True)])
+def test_order_of_codes_and_activations(cuda_lib, N, K, batch, aligned, extreme):
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([91, N, K, batch])
+    w = synth.random_tl1_packed(rng, N, K)
+    x = rng.standard_normal((batch, K)).astype(np.float32)
+    if extreme:                                              # every code 2, every activation +31: the largest sum there is
+        w = np.full_like(w, 0xAA)
+        x[:] = 1.0
+        x[1::2] = -1.0
+        x[2, ::3] = 0.5
+    flat = torch.zeros(batch * K + 1, device="cuda")
+    dx = flat[:-1] if aligned else flat[1:]                  # one float off a 16-byte boundary
+    dx = dx.view(batch, K)
+    dx.copy_(dev(x))
+    r = kernels.tl1_gemv(dx, dev(w), N // 64, K, [0.016], want_acc=True, want_act=True)
+    torch.cuda.synchronize()
+    acc, act, out = host(r["acc"]), host(r["a"]), host(r["out"])
+    for b in range(batch):
+        want_out, want_acc, inv = cpu_bitlinear(x[b], w, N, K, 0.016)
+        a = np.zeros(K, np.int8)
+        ora.load_oracle().ora_act_quant31(P(x[b], ora.c_f32p), K, P(a, ora.c_i8p))
+        assert np.array_equal(act[b], a)
+        assert np.array_equal(acc[b], want_acc), f"sequence {b}"
+        assert np.array_equal(out[b], want_out), f"sequence {b}"
