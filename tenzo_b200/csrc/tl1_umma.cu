@@ -10,8 +10,8 @@
 //   quantiser)
 //
 // One CTA per 128-row tile (two 64-row TL1 blocks; for the GLU epilogue the gate block and its up block, so the
-// activation is applied inside the CTA). K is walked in 128-byte chunks through a ring of 4, 8 or 12 slots (a multiple of
-// four: see UmmaSmem::slots_for); 21 warps per CTA:
+// activation is applied inside the CTA). K is walked in 128-byte chunks through two rings, 8 or 12 slots of codes in tensor
+// memory and 4, 8 or 12 activation tiles in shared memory (multiples of four: see UmmaSmem::a_slots_for); 21 warps per CTA:
 //   warp 0 (lane 0)     bulk-copies the packed 2-bit weights eight chunks at a time (2 x 16 KB) into a ring of two or
 //                       three groups; the first groups are requested by one lane each first thing in the kernel
 //                       (weights depend on no earlier kernel); lanes 1-31 fetch the per-sequence scale and sum for
@@ -22,16 +22,19 @@
 //                       proxy fence). Lane quarter q of a group takes one nibble half of one row block; a thread's
 //                       four TMEM lanes are the four rows of ONE packed word, so a thread loads sixteen words per
 //                       chunk and every byte of them is used. The row order inside a quarter is therefore permuted
-//                       (TMEM lane l holds row 4*(l&7) + (l>>3)); the epilogue undoes it. The warps of a group
-//                       take turns TMA-loading the chunk's activation tile [N][128 B] (128-byte swizzle) into the
-//                       slot right after they have seen it free: a dedicated thread doing a poll, an expect_tx and
-//                       a TMA issue per chunk was the slowest role of the pipeline (about 800 cycles per chunk);
+//                       (TMEM lane l holds row 4*(l&7) + (l>>3)); the epilogue undoes it. Up to 144 sequences there are as
+//                       many activation slots as code slots, and the warps of a group take turns TMA-loading the chunk's
+//                       activation tile [N][128 B] (128-byte swizzle) right after they have seen the slot free;
 //   warps 1, 18-20      (lane 0 each) take every fourth chunk: one poll of the slot's barrier (expand arrivals + the
 //                       TMA's bytes), four tcgen05.mma (K = 32 each, A from tensor memory), one commit that frees the
 //                       slot. A poll costs the issuing thread about 180 cycles, a commit about 80 and the loop
 //                       another 270 (measured), more than the MMAs of a chunk take below 256 sequences, so one
 //                       issuing thread bounds the loop; four hide it. Integer accumulation is order-free, so the only
-//                       ordering needed between them is that chunk 0 (which overwrites) completes first.
+//                       ordering needed between them is that chunk 0 (which overwrites) completes first. From 145
+//                       sequences on only four activation tiles fit. With one ring for both, codes and MMAs then took
+//                       turns (900 cycles a chunk for 516 of math); now the codes run eight chunks ahead, and each issuing
+//                       thread requests the next tile of its own slot as soon as its MMAs have completed (one thread that
+//                       requested all of them was the slowest role, 970 cycles a chunk): 640 cycles a chunk.
 // After the last chunk every issuing thread commits to one barrier, which starts the epilogue on all sixteen expand
 // warps (the groups on alternate 32-sequence column units; TMEM lane = weight row, tcgen05.ld 16 sequences at a
 // time, scale / residual / ReLU^2*GLU, the unit assembled in shared memory and sent off by its own TMA store while
@@ -77,7 +80,8 @@ struct UmmaLaunch {
     const int* sum_a;        // [batch] sum_k a_k
     int units;               // tiles along the rows
     int n_box;               // sequences per CTA, padded to a multiple of 16 (<= 256)
-    int n_slots;             // ring slots (A in tensor memory, activation tile in shared memory)
+    int n_slots;             // ring slots (A in tensor memory)
+    int b_slots;             // activation tiles in shared memory: as many, or four (then the issuing threads request them)
     int n_pgroups;           // groups of kPGroup chunks in the packed-weight ring
     int ksplit;              // CTAs of a cluster that share one tile's K range (1 = no cluster)
     int store_cols;          // sequences per TMA store of the epilogue (32; 16 with a cluster or up to 64 sequences)
@@ -118,21 +122,34 @@ __device__ __forceinline__ float umma_seg_scale(const tenzo_tl1_gemv_args& a, in
 }
 
 struct UmmaSmem {
-    // [1024-aligned] ring n_slots x { B n_box*128 } | packed ring n_pgroups x 2 blocks x 16 KB | barriers | tmem slot | inv[256] | sum_a[256]
+    // [1024-aligned] ring b_slots x { B n_box*128 } | packed ring n_pgroups x 2 blocks x 16 KB | barriers | tmem slot | inv[256] | sum_a[256]
     static __host__ __device__ int pgroups_for(int n_box) { return n_box <= 64 ? kMaxPGroups : 2; }
     static __host__ __device__ int tmem_a(int n_box) { return (n_box + 31) & ~31; }          // first column of the A slots
-    static __host__ __device__ int slots_for(int n_box) {
-        const int by_tmem = (kTmemCols - tmem_a(n_box)) / 32, by_smem = (kSmemBudget - pgroups_for(n_box) * kPGroup * kPBytes) / (n_box * kKc);
-        const int r = by_tmem < by_smem ? by_tmem : by_smem;
-        // A multiple of four (the expand groups and the issuing threads): slot s then always belongs to group s % 4 and
-        // thread s % 4, so every phase of a slot's barriers is seen, in order, by the same waiter. (A parity wait
-        // cannot tell phase k from phase k - 2: with five slots a thread that ran ahead of its neighbour took a slot's
-        // previous phase for the one it waited for and multiplied a tile that had not arrived.)
+    // Both numbers are multiples of four (the expand groups and the issuing threads): slot s then always belongs to group s % 4 and
+    // thread s % 4, so every phase of a slot's barriers is seen, in order, by the same waiter. (A parity wait
+    // cannot tell phase k from phase k - 2: with five slots a thread that ran ahead of its neighbour took a slot's
+    // previous phase for the one it waited for and multiplied a tile that had not arrived.)
+    static __host__ __device__ int a_slots_for(int n_box) {                                  // by tensor memory: 12 up to 128 sequences, 8 at 256
+        const int r = (kTmemCols - tmem_a(n_box)) / 32;
         return (r < kMaxSlots ? r : kMaxSlots) & ~3;
+    }
+    static __host__ __device__ int b_slots_for(int n_box) {                                  // by shared memory: 12 up to 96 sequences, 4 from 145 on
+        const int r = (kSmemBudget - pgroups_for(n_box) * kPGroup * kPBytes) / (n_box * kKc), a = a_slots_for(n_box);
+        return (r < a ? r : a) & ~3;
     }
     static constexpr int n_bars = 2 * kMaxSlots + 2 * kMaxPGroups + 3;
     static __host__ __device__ size_t bytes(int n_box) {
-        return 1024 + (size_t)slots_for(n_box) * n_box * kKc + (size_t)pgroups_for(n_box) * kPGroup * kPBytes + ((8 * n_bars + 15) & ~15) + 16 + 2 * kMaxN * 4;
+        return 1024 + (size_t)b_slots_for(n_box) * n_box * kKc + (size_t)pgroups_for(n_box) * kPGroup * kPBytes + ((8 * n_bars + 15) & ~15) + 16 + 2 * kMaxN * 4;
+    }
+};
+
+// Slot and round of a chunk in a ring of n slots, stepped without a division (by at most n): n is a run-time number, and the
+// divisions were on the way of every hand-over (13824 x 2560 with GLU at 12 sequences 13.9 -> 12.7 us, 28672 x 4096 29.2 -> 25.7).
+struct RingPos {
+    int slot, round;
+    __device__ __forceinline__ void step(int by, int n) {
+        slot += by;
+        if (slot >= n) { slot -= n; ++round; }
     }
 };
 
@@ -192,9 +209,10 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base_off = ((smem_addr(smem_raw) + 1023u) & ~1023u) - smem_addr(smem_raw);
     unsigned char* ring = smem_raw + base_off;
-    const int N = L.n_box, R = L.n_slots, slot_bytes = N * kKc;
+    const int N = L.n_box, R = L.n_slots, RB = L.b_slots, slot_bytes = N * kKc;
+    const bool b_ahead = RB < R;                       // the codes run further ahead than the activation tiles do
     const int PG = L.n_pgroups;
-    unsigned char* pring = ring + (size_t)R * slot_bytes;                       // [PG][2 row blocks][kPGroup chunks][64][32] packed weights
+    unsigned char* pring = ring + (size_t)RB * slot_bytes;                       // [PG][2 row blocks][kPGroup chunks][64][32] packed weights
     uint64_t* bars = reinterpret_cast<uint64_t*>(pring + (size_t)PG * kPGroup * kPBytes);
     const uint32_t tmem_a0 = (uint32_t)UmmaSmem::tmem_a(N);
     uint64_t* bar_full = bars;                         // [R] A expanded (one arrival per expanding warp) and the activation tile landed
@@ -252,7 +270,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             mbar_init(&bar_full[lane], 5);             // four expanding warps + the expect_tx of the warp that requests the activation tile
             mbar_init(&bar_empty[lane], 1);
         } else if (lane >= 16 && lane < 16 + kMaxPGroups) {
-            mbar_init(&bar_pfree[lane - 16], 4 * kExpandGroups * (R >= 8 ? 1 : 2));   // one arrival per expanding warp per iteration
+            mbar_init(&bar_pfree[lane - 16], 4 * kExpandGroups * (b_ahead ? 2 : 1));   // one arrival per expanding warp per iteration
         } else if (lane == 24) {
             mbar_init(bar_accum, kMmaThreads);
         } else if (lane == 25) {
@@ -301,22 +319,41 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         if (lane == 0) {
             // c = s32, a = u8, b = s8, both K-major, N at bit 17 (>>3), M at bit 24 (>>4)
             const uint32_t idesc = (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(kTileRows >> 4) << 24);
+            // With fewer activation slots than code slots (four) a thread also requests its chunks' tiles: the slot is its own,
+            // and the tile after next is due when the MMAs it has just issued have completed.
+            auto request_tile = [&](int j, int s) {
+                if (UCHK(ring + (size_t)(mma_t + 1) * slot_bytes <= pring, 2, mma_t, j)) {
+                    mbar_expect_tx(&bar_full[s], (unsigned)slot_bytes);
+                    tma_load_2d(ring + (size_t)mma_t * slot_bytes, &amap, (c_begin + j) * kKc, seq0, &bar_full[s]);
+                }
+            };
+            RingPos at = {mma_t, 0};
+            if (b_ahead && mma_t < n_chunks) {
+                if (a.use_pdl) pdl_wait();
+                request_tile(mma_t, mma_t);
+            }
             if (mma_t > 0 && mma_t < n_chunks && !mbar_spin_bounded(bar_first, 0u)) timed_out = true;
             for (int j = mma_t; j < n_chunks && !timed_out; j += kMmaThreads) {
-                const int s = j % R, use = j / R;
+                const int s = at.slot, sb = b_ahead ? mma_t : s;
+                const unsigned parity = (unsigned)at.round & 1u;
+                at.step(kMmaThreads, R);
                 UC(j, 4);
-                if (!mbar_spin_bounded(&bar_full[s], (unsigned)use & 1u)) { timed_out = true; break; }
+                if (!mbar_spin_bounded(&bar_full[s], parity)) { timed_out = true; break; }
                 tc_fence_after();
                 UC(j, 5);
                 const uint32_t ta = tmem_base + tmem_a0 + (uint32_t)(32 * s);
-                const uint64_t db = umma_desc_sw128(smem_addr(ring + (size_t)s * slot_bytes));
-                if (UCHK(tmem_a0 + 32 * s + 32 <= (uint32_t)kTmemCols && s < R && ring + (size_t)(s + 1) * slot_bytes <= pring, 5, s, j))
+                const uint64_t db = umma_desc_sw128(smem_addr(ring + (size_t)sb * slot_bytes));
+                if (UCHK(tmem_a0 + 32 * s + 32 <= (uint32_t)kTmemCols && s < R && ring + (size_t)(sb + 1) * slot_bytes <= pring, 5, s, j))
 #pragma unroll
                 for (int k4 = 0; k4 < kKc / 32; ++k4)
                     umma_i8_ta(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, (j > 0 || k4 > 0) ? 1u : 0u);
                 umma_commit(&bar_empty[s]);
                 UC(j, 6);
                 if (j == 0) umma_commit(bar_first);
+                if (b_ahead && j + kMmaThreads < n_chunks) {
+                    if (!mbar_spin_bounded(&bar_empty[s], parity)) { timed_out = true; break; }
+                    request_tile(j + kMmaThreads, at.slot);
+                }
             }
             umma_commit(bar_accum);
         }
@@ -340,23 +377,28 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
 #pragma unroll
         for (int u = 0; u < 4; ++u) woff[u] = (4 * t + (u ^ t)) * 8 + g;
         // An iteration costs a warp about two thousand cycles whatever it expands (a poll of a barrier that has long
-        // completed is 300 cycles, a tensor-memory store 500 until it has landed), so with eight or more slots it takes
-        // two chunks, j and j + 4: one poll for both slots (the same thread issues both chunks' MMAs in order, so the
+        // completed is 300 cycles, a tensor-memory store 500 until it has landed), so where the activation tiles have as many
+        // slots it takes two chunks, j and j + 4: one poll for both slots (the same thread issues both chunks' MMAs in order, so the
         // later one's completion implies the earlier one's), one for the weights (both lie in the same group of eight),
         // the two polls on different lanes, one wait for the four stores.
-        const int cpi = R >= 8 ? 2 : 1;
+        const int cpi = b_ahead ? 1 : 2;
         int seen_group = -1;
+        RingPos next = {grp, 0}, weights = {0, 0};           // of the iteration's first chunk and of its group of packed weights
         for (int it = 0, j0 = grp; j0 < n_chunks; ++it, j0 += kExpandGroups * cpi) {
             const int n_here = (cpi == 2 && j0 + kExpandGroups < n_chunks) ? 2 : 1;
-            const int j_last = j0 + kExpandGroups * (n_here - 1);
-            const int pg = j0 / kPGroup, ps = pg % PG, puse = pg / PG;
+            const int pg = j0 / kPGroup;
+            if (pg != seen_group && pg > 0) weights.step(1, PG);
+            const int ps = weights.slot;
+            RingPos at[2] = {next, next};
+            at[1].step(kExpandGroups, R);
+            next.step(kExpandGroups * cpi, R);
             bool ok = true;
             if (lane == 0 && q == 0) { UC(j0, 0); if (n_here == 2) UC(j0 + kExpandGroups, 0); }
             if (lane == 0) {
-                const int s = j_last % R, use = j_last / R;
-                ok = use == 0 || mbar_spin_bounded(&bar_empty[s], (unsigned)(use - 1) & 1u);
+                const RingPos last = n_here == 2 ? at[1] : at[0];
+                ok = last.round == 0 || mbar_spin_bounded(&bar_empty[last.slot], (unsigned)(last.round - 1) & 1u);
             } else if (lane == 1 && pg != seen_group) {
-                ok = mbar_spin_bounded(&bar_p[ps], (unsigned)puse & 1u);
+                ok = mbar_spin_bounded(&bar_p[ps], (unsigned)weights.round & 1u);
             }
             seen_group = pg;
             ok = __all_sync(0xffffffffu, ok);
@@ -370,8 +412,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             // the weights depend on nothing, and the previous kernel runs about as long as the first round of expansion.
             auto request_tiles = [&]() {
                 for (int c = 0; c < n_here; ++c) {
-                    const int j = j0 + kExpandGroups * c, s = j % R;
-                    if (lane == 0 && ((it * cpi + c) & 3) == q) {
+                    const int j = j0 + kExpandGroups * c, s = c ? at[1].slot : at[0].slot;
+                    if (!b_ahead && lane == 0 && ((it * cpi + c) & 3) == q) {
                         if (UCHK(s < R && ring + (size_t)(s + 1) * slot_bytes <= pring, 2, s, j)) {
                             mbar_expect_tx(&bar_full[s], (unsigned)slot_bytes);
                             tma_load_2d(ring + (size_t)s * slot_bytes, &amap, (c_begin + j) * kKc, seq0, &bar_full[s]);
@@ -382,7 +424,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             const bool request_last = it == 0 && a.use_pdl;
             if (!request_last) request_tiles();
             for (int c = 0; c < n_here; ++c) {
-                const int j = j0 + kExpandGroups * c, s = j % R;
+                const int j = j0 + kExpandGroups * c, s = c ? at[1].slot : at[0].slot;
                 const uint32_t* sP = reinterpret_cast<const uint32_t*>(pring + (size_t)ps * kPGroup * kPBytes + (size_t)blk * kPGroup * (kPBytes / 2) +
                                                                        (size_t)(j % kPGroup) * (kPBytes / 2));
                 uint32_t W[16];
@@ -410,14 +452,14 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             if (lane == 0 && q == 0) { UC(j0, 2); if (n_here == 2) UC(j0 + kExpandGroups, 2); }
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_pfree[ps]);       // every lane's packed words have been loaded and used
-            if (request_last) {
+            if (request_last && !b_ahead) {
                 if (lane == 0) pdl_wait();
                 request_tiles();
             }
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane < n_here) mbar_arrive(&bar_full[(j0 + kExpandGroups * lane) % R]);
+            if (lane < n_here) mbar_arrive(&bar_full[lane ? at[1].slot : at[0].slot]);
             if (lane == 0 && q == 0) { UC(j0, 3); if (n_here == 2) UC(j0 + kExpandGroups, 3); }
         }
         // ---- all of this CTA's MMAs have completed; in a cluster it parks its partial tile [N][128 TMEM lanes] int32
@@ -579,7 +621,9 @@ int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float*
     L.units = glu ? a.n_blocks / 2 : (a.n_blocks + 1) / 2;
     const int per_cta = a.batch < kMaxN ? a.batch : kMaxN;
     L.n_box = (per_cta + 15) & ~15;
-    L.n_slots = UmmaSmem::slots_for(L.n_box);
+    L.n_slots = UmmaSmem::a_slots_for(L.n_box);
+    L.b_slots = UmmaSmem::b_slots_for(L.n_box);
+    if (L.b_slots >= 8) L.n_slots = L.b_slots;                     // (enough of them: requested by the warps that expand the codes, two chunks at a time)
     L.n_pgroups = UmmaSmem::pgroups_for(L.n_box);
     const int seq_tiles = (a.batch + kMaxN - 1) / kMaxN;
     L.ksplit = pick_umma_ksplit(L.units * seq_tiles, a.K / kKc);
@@ -653,7 +697,7 @@ extern "C" __attribute__((visibility("default"))) int tenzo_trace_umma_chunks(lo
 extern "C" int tenzo_cuda_tl1_gemm_layout(int batch, int* slots, int* weight_groups, size_t* smem_bytes, size_t* epilogue_bytes) {
     if (batch < tz::kUmmaMinBatch) return -1;                    // the tensor-core path does not apply
     const int per_cta = batch < tz::kMaxN ? batch : tz::kMaxN, n_box = (per_cta + 15) & ~15;
-    if (slots) *slots = tz::UmmaSmem::slots_for(n_box);
+    if (slots) *slots = tz::UmmaSmem::b_slots_for(n_box);
     if (weight_groups) *weight_groups = tz::UmmaSmem::pgroups_for(n_box);
     if (smem_bytes) *smem_bytes = tz::UmmaSmem::bytes(n_box);
     // without a cluster: the output columns [n_box][128] fp32 (GLU: [n_box][64] twice); with one: behind the partial tile
