@@ -29,8 +29,9 @@
 //                       TMA's bytes), four tcgen05.mma (K = 32 each, A from tensor memory), one commit that frees the
 //                       slot. A poll costs the issuing thread about 180 cycles, a commit about 80 and the loop
 //                       another 270 (measured), more than the MMAs of a chunk take below 256 sequences, so one
-//                       issuing thread bounds the loop; four hide it. Integer accumulation is order-free, so the only
-//                       ordering needed between them is that chunk 0 (which overwrites) completes first. From 145
+//                       issuing thread bounds the loop; four hide it. Integer accumulation is order-free, and the
+//                       expanding warps zero the accumulators while they wait for weights, so the threads need no
+//                       order among them (when chunk 0 had to overwrite them first, the others lost 850 cycles). From 145
 //                       sequences on only four activation tiles fit. With one ring for both, codes and MMAs then took
 //                       turns (900 cycles a chunk for 516 of math); now the codes run eight chunks ahead, and each issuing
 //                       thread requests the next tile of its own slot as soon as its MMAs have completed (one thread that
@@ -220,8 +221,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
     uint64_t* bar_p = bars + 2 * kMaxSlots;            // [PG] packed weights have landed
     uint64_t* bar_pfree = bar_p + kMaxPGroups;         // [PG] packed weights consumed (one arrival per expanding warp per chunk)
     uint64_t* bar_accum = bar_pfree + kMaxPGroups;        // every issuing thread's MMAs have completed
-    uint64_t* bar_first = bar_accum + 1;               // chunk 0 (the one that overwrites the accumulators) has completed
-    uint64_t* bar_meta = bar_first + 1;                // per-sequence scale and sum are in shared memory
+    uint64_t* bar_zero = bar_accum + 1;                // the accumulators are zero (one arrival per expanding warp)
+    uint64_t* bar_meta = bar_zero + 1;                 // per-sequence scale and sum are in shared memory
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(bars) + ((8 * UmmaSmem::n_bars + 15) & ~15));   // 16-byte aligned
     float* s_inv = reinterpret_cast<float*>(tmem_slot + 4);   // [kMaxN] m/31 of this CTA's sequences
     int* s_sum = reinterpret_cast<int*>(s_inv + kMaxN);       // [kMaxN] sum_k a_k
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         } else if (lane == 24) {
             mbar_init(bar_accum, kMmaThreads);
         } else if (lane == 25) {
-            mbar_init(bar_first, 1);
+            mbar_init(bar_zero, 4 * kExpandGroups);
         } else if (lane == 26) {
             mbar_init(bar_meta, 1);
         }
@@ -332,7 +333,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
                 if (a.use_pdl) pdl_wait();
                 request_tile(mma_t, mma_t);
             }
-            if (mma_t > 0 && mma_t < n_chunks && !mbar_spin_bounded(bar_first, 0u)) timed_out = true;
+            if (mma_t < n_chunks && !mbar_spin_bounded(bar_zero, 0u)) timed_out = true;
             for (int j = mma_t; j < n_chunks && !timed_out; j += kMmaThreads) {
                 const int s = at.slot, sb = b_ahead ? mma_t : s;
                 const unsigned parity = (unsigned)at.round & 1u;
@@ -346,10 +347,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
                 if (UCHK(tmem_a0 + 32 * s + 32 <= (uint32_t)kTmemCols && s < R && ring + (size_t)(sb + 1) * slot_bytes <= pring, 5, s, j))
 #pragma unroll
                 for (int k4 = 0; k4 < kKc / 32; ++k4)
-                    umma_i8_ta(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, (j > 0 || k4 > 0) ? 1u : 0u);
+                    umma_i8_ta(tmem_base, ta + (uint32_t)(8 * k4), db + (uint64_t)(2 * k4), idesc, 1u);
                 umma_commit(&bar_empty[s]);
                 UC(j, 6);
-                if (j == 0) umma_commit(bar_first);
                 if (b_ahead && j + kMmaThreads < n_chunks) {
                     if (!mbar_spin_bounded(&bar_empty[s], parity)) { timed_out = true; break; }
                     request_tile(j + kMmaThreads, at.slot);
@@ -382,6 +382,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         // later one's completion implies the earlier one's), one for the weights (both lie in the same group of eight),
         // the two polls on different lanes, one wait for the four stores.
         const int cpi = b_ahead ? 1 : 2;
+        // While the first weights are on their way: zero the accumulators (the groups alternate 16-column blocks).
+        for (int c0 = 16 * grp; c0 < N; c0 += 16 * kExpandGroups) tmem_zero16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)c0);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_zero);
         int seen_group = -1;
         RingPos next = {grp, 0}, weights = {0, 0};           // of the iteration's first chunk and of its group of packed weights
         for (int it = 0, j0 = grp; j0 < n_chunks; ++it, j0 += kExpandGroups * cpi) {
@@ -394,11 +400,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             next.step(kExpandGroups * cpi, R);
             bool ok = true;
             if (lane == 0 && q == 0) { UC(j0, 0); if (n_here == 2) UC(j0 + kExpandGroups, 0); }
-            if (lane == 0) {
+            {   // lane 0 waits for the slot, lane 1 for the weights: the same code for both, or one would wait after the other
                 const RingPos last = n_here == 2 ? at[1] : at[0];
-                ok = last.round == 0 || mbar_spin_bounded(&bar_empty[last.slot], (unsigned)(last.round - 1) & 1u);
-            } else if (lane == 1 && pg != seen_group) {
-                ok = mbar_spin_bounded(&bar_p[ps], (unsigned)weights.round & 1u);
+                uint64_t* bar = lane == 0 ? &bar_empty[last.slot] : &bar_p[ps];
+                const int round = lane == 0 ? last.round - 1 : weights.round;
+                if (lane == 0 ? round >= 0 : lane == 1 && pg != seen_group) ok = mbar_spin_bounded(bar, (unsigned)round & 1u);
             }
             seen_group = pg;
             ok = __all_sync(0xffffffffu, ok);
