@@ -85,8 +85,10 @@ __device__ __forceinline__ int mma_place(int i) { return i ^ ((i >> 2) & 1); }
 
 // A thread holds kAqVec 16-byte pieces of the row in registers (launch_act_quant picks threads and pieces by K; longer rows
 // go through shared memory).
-template <int kAqThreads, int kAqVec>
-__global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
+// kAqResident: CTAs an SM must hold. With one the norm's weights are loaded ahead of the wait for the previous
+// kernel and held in registers as well, for the latency of few rows; with more they are loaded when they are used.
+template <int kAqThreads, int kAqVec, int kAqResident>
+__global__ void __launch_bounds__(kAqThreads, kAqResident) act_quant_kernel(
     const float* x, const float* __restrict__ norm_w, int do_norm, float eps, int K, int x_stride,
     uint32_t* words, float* inv, int8_t* a_out, int8_t* a_mma, int* sum_out, int use_pdl) {
     extern __shared__ __align__(16) float s_y[];   // K floats (or eight padded rows of K/8 squares) + 32 scratch
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
         const int k4 = K >> 2;
         float4 w4[kAqVec], v[kAqVec];
         const bool has_w = do_norm && norm_w;
-        if (has_w) {                                    // model constants: no need to wait for the previous kernel
+        if (kAqResident == 1 && has_w) {                // model constants: no need to wait for the previous kernel
 #pragma unroll
             for (int r = 0; r < kAqVec; ++r) {
                 const int i = tid + r * kAqThreads;
@@ -167,6 +169,10 @@ __global__ void __launch_bounds__(kAqThreads) act_quant_kernel(
 #pragma unroll
             for (int r = 0; r < kAqVec; ++r) {          // y = (x * inv_rms) * w, left to right (rms_apply)
                 v[r].x *= inv_rms; v[r].y *= inv_rms; v[r].z *= inv_rms; v[r].w *= inv_rms;
+                if (kAqResident > 1 && has_w) {
+                    const int i = tid + r * kAqThreads;
+                    w4[r] = i < k4 ? __ldg(reinterpret_cast<const float4*>(norm_w) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
                 if (has_w) { v[r].x *= w4[r].x; v[r].y *= w4[r].y; v[r].z *= w4[r].z; v[r].w *= w4[r].w; }
             }
         }
@@ -287,7 +293,14 @@ cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, f
     const size_t smem = (size_t)((rows > K ? rows : K) + 32) * sizeof(float);
     // 16-byte pieces a thread: as few as the row needs (registers: 1536 rows of 2560 in 21 us with seven, 13 with three), 512
     // threads for rows above 7168 (14336 went through shared memory element by element: 17 us, now 10)
-    auto kernel = K <= 3072 ? act_quant_kernel<256, 3> : K <= 4096 ? act_quant_kernel<256, 4> : K <= 7168 ? act_quant_kernel<256, 7> : act_quant_kernel<512, 7>;
+    // From 4097 elements on the registers with the weights leave room for two CTAs an SM (one of 512 threads), and more rows than that
+    // would come in rounds of a chain of additions each: then twice as many without them (1536 rows: 6912 elements 31.0 -> 22.0 us, 14336 92.7 -> 62.5;
+    // 512 rows 11.3 -> 9.4 and 32.3 -> 21.2; at 256 rows of 6912 no difference; shorter rows gain nothing: 512 of 2560 4.8 -> 5.6).
+    const bool many = batch > 148 * (K <= 7168 ? 2 : 1);
+    auto kernel = K <= 3072   ? act_quant_kernel<256, 3, 1>
+                  : K <= 4096 ? act_quant_kernel<256, 4, 1>
+                  : K <= 7168 ? (many ? act_quant_kernel<256, 7, 4> : act_quant_kernel<256, 7, 1>)
+                              : (many ? act_quant_kernel<512, 7, 2> : act_quant_kernel<512, 7, 1>);
     const int threads = K <= 7168 ? 256 : 512;
     if (smem > 48 * 1024) {
         cudaError_t ea = allow_smem(kernel, 96 * 1024);

@@ -5,7 +5,7 @@ splits and weights and activations at their extremes, where the scaled sums are 
 import numpy as np
 import pytest
 import torch
-from gpu_helpers import cpu_bitlinear, dev, host
+from gpu_helpers import cpu_bitlinear, cpu_rms_norm, dev, host
 from helpers import ora, synth
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +39,20 @@ def test_order_of_codes_and_activations(cuda_lib, N, K, batch, aligned, extreme)
         assert np.array_equal(act[b], a)
         assert np.array_equal(acc[b], want_acc), f"sequence {b}"
         assert np.array_equal(out[b], want_out), f"sequence {b}"
+
+
+@pytest.mark.parametrize("K,batch", [(6912, 297), (4224, 300), (14336, 149)])
+def test_many_rows_quantiser(cuda_lib, K, batch):
+    """More rows than the quantiser that holds the norm's weights has places for: the one that loads them late, same bits."""
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([92, K, batch])
+    N = 64
+    w, nw = synth.random_tl1_packed(rng, N, K), (1.0 + 0.1 * rng.standard_normal(K)).astype(np.float32)
+    x = rng.standard_normal((batch, K)).astype(np.float32)
+    r = kernels.tl1_gemv(dev(x), dev(w), N // 64, K, [0.016], norm_w=dev(nw), do_norm=True, want_acc=True, want_act=True)
+    few = kernels.tl1_gemv(dev(x[:12]), dev(w), N // 64, K, [0.016], norm_w=dev(nw), do_norm=True, want_acc=True, want_act=True)
+    torch.cuda.synchronize()
+    assert all(np.array_equal(host(r[k])[:12], host(few[k])) for k in ("a", "inv", "acc", "out"))
+    for b in (0, 1, batch // 2, batch - 1):
+        want_out, want_acc, _ = cpu_bitlinear(cpu_rms_norm(x[b], nw), w, N, K, 0.016)
+        assert np.array_equal(host(r["acc"])[b], want_acc) and np.array_equal(host(r["out"])[b], want_out), f"sequence {b}"
