@@ -259,10 +259,9 @@ __device__ __forceinline__ float expf_reference_bits_lanes(float x, uint32_t tab
     const unsigned long long ki = (unsigned long long)__double_as_longlong(kd);
     kd = __dadd_rn(kd, -shift);
     const double r = __fma_rn(inv_ln2_n, xd, -kd);
-    const int sel = (int)(ki & 31);
+    const int sel = (int)ki;                                   // a shuffle takes the lane modulo 32
     const uint32_t lo = __shfl_sync(0xffffffffu, tab_lo, sel), hi = __shfl_sync(0xffffffffu, tab_hi, sel);
-    const unsigned long long t = (((unsigned long long)hi << 32) | lo) + (ki << 47);
-    const double s = __longlong_as_double((long long)t);
+    const double s = __hiloint2double((int)(hi + ((uint32_t)ki << 15)), (int)lo);      // table entry + (ki << 47): no carry from below
     const double zz = __fma_rn(c0, r, c1);
     const double r2 = __dmul_rn(r, r);
     double y = __fma_rn(c2, r, 1.0);

@@ -14,42 +14,47 @@ namespace tz {
 // inside a binade by more than that is certain to stay in it. The few others (the sum can double only so often) are added
 // element by element, and so are the first 64, where it doubles all the time.
 //
-// Cycles for n values, this against the plain loop with its loads: 2048: 6 800 and 10 800; 864: 5 000 and 4 700 (about 300 a
-// segment that is added one by one, 315 a group of eight that is not).
+// HEAD = false: for a sum that goes on, where the first elements are like all others.
 //
-// `e` is in shared memory, 16-byte aligned, and readable up to ordered_sum_padded(n) floats, zeros beyond n. All 32 lanes
+// `e` is in shared memory, 16-byte aligned, and readable up to ordered_sum_padded(n, HEAD) floats, zeros beyond n. All 32 lanes
 // call it with the same arguments and get the same result.
 constexpr int kOrderedHead = 64;
-__host__ __device__ constexpr int ordered_sum_segment(int n) {          // elements a lane takes behind the head: whole 16-byte pieces, an odd number of them (no bank conflicts)
-    const int pieces = n > kOrderedHead ? (n - kOrderedHead + 127) >> 7 : 1;
-    return 4 * (pieces | 1);
+__host__ __device__ constexpr int ordered_sum_segment(int n) {          // elements a lane takes of n: whole 16-byte pieces, an odd number of them (no bank conflicts)
+    return 4 * ((n > 0 ? (n + 127) >> 7 : 1) | 1);
 }
-__host__ __device__ constexpr int ordered_sum_padded(int n) { return kOrderedHead + 32 * ordered_sum_segment(n); }
+__host__ __device__ constexpr int ordered_sum_padded(int n, bool head = true) {
+    return head ? kOrderedHead + 32 * ordered_sum_segment(n - kOrderedHead) : 32 * ordered_sum_segment(n);
+}
+// Two amounts in a row, each from an even and from an odd mantissa: again such a pair.
+__device__ __forceinline__ void join_steps(int& even, int& odd, int next_even, int next_odd) {
+    even += even & 1 ? next_odd : next_even;
+    odd += odd & 1 ? next_even : next_odd;
+}
 
-// The plain loop over n values (n a multiple of 4): eight 16-byte loads, then their 32 additions. Loading the next batch during
-// the additions is slower: a wait for one batch then also waits for the loads of the next.
+// The plain loop over n values (n a multiple of 4): eight 16-byte loads, then their 32 additions (of zeros behind the last value, which
+// change nothing). Loading the next batch during the additions is slower: a wait for one batch then also waits for the loads of
+// the next.
 __device__ __forceinline__ float chain_sum(const float* e, int n, float s) {
     const float4* p = reinterpret_cast<const float4*>(e);
-    int j = 0;
 #pragma unroll 1
-    for (; j + 8 <= n >> 2; j += 8) {
+    for (int j = 0; j < n >> 2; j += 8) {
         float4 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = p[j + u];
+        for (int u = 0; u < 8; ++u) v[u] = j + u < n >> 2 ? p[j + u] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int u = 0; u < 8; ++u) { s += v[u].x; s += v[u].y; s += v[u].z; s += v[u].w; }
     }
-#pragma unroll 1
-    for (; j < n >> 2; ++j) { const float4 v = p[j]; s += v.x; s += v.y; s += v.z; s += v.w; }
     return s;
 }
 
+template <bool HEAD>
 __device__ __forceinline__ float ordered_sum_warp(const float* e, int n, float s) {
     constexpr uint32_t kExp = 0x7f800000u;
+    constexpr int head = HEAD ? kOrderedHead : 0;
     const int lane = threadIdx.x & 31;
     if (n <= kOrderedHead) return chain_sum(e, (n + 3) & ~3, s);
-    const int L4 = ordered_sum_segment(n) >> 2;
-    const float4* segs = reinterpret_cast<const float4*>(e + kOrderedHead);
+    const int L4 = ordered_sum_segment(n - head) >> 2;
+    const float4* segs = reinterpret_cast<const float4*>(e + head);
     const float4* mine = segs + lane * L4;
     float p0 = 0.0f, p1 = 0.0f;
 #pragma unroll 4
@@ -65,7 +70,7 @@ __device__ __forceinline__ float ordered_sum_warp(const float* e, int n, float s
         const float up = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += up;
     }
-    s = chain_sum(e, kOrderedHead, s);
+    if (HEAD) s = chain_sum(e, kOrderedHead, s);
     const float margin = (float)n * 0x1p-23f;            // twice the bound
     const float from = s + (incl - part), to = s + incl;
     const uint32_t B = __float_as_uint(from) & kExp;
@@ -82,34 +87,45 @@ __device__ __forceinline__ float ordered_sum_warp(const float* e, int n, float s
     }
     // starting at B, not at s, the loop may leave the binade where the sum does not: then the segment is not used either
     const uint32_t use = __ballot_sync(0xffffffffu, inside && (__float_as_uint(c0) & kExp) == B && (__float_as_uint(c1) & kExp) == B);
-    // Inside a binade the sum's bits count units of u, so the amounts are integers: i0 from an even mantissa and, the two runs
-    // keeping a distance of 0, 1 or 2 units, i0 + (-1, 0 or 1) from an odd one. Nine cycles a segment: S + i0 + (S & 1) di.
-    const int i0 = (int)(__float_as_uint(c0) - B), di = (int)(__float_as_uint(c1) - (B | 1u)) - i0;
-    const int word = (i0 << 2) | (di + 1);
-    const int n_seg = (n - kOrderedHead + 4 * L4 - 1) / (4 * L4);
-    int S = __float_as_int(s);
-#pragma unroll 1
-    for (int i = 0; i < n_seg; i += 8) {
-        int w[8];
+    // Inside a binade the sum's bits count units of u, so the amounts are integers, and two segments in a row are one: five rounds of
+    // shuffles leave in the last lane of every run of sure lanes what the run comes to. (Walked one by one, the 32 segments took
+    // more instructions than their additions.) Segments behind the last are empty, their amounts zero.
+    int even = (int)(__float_as_uint(c0) - B), odd = (int)(__float_as_uint(c1) - (B | 1u));
+    if (use == 0xffffffffu) {                                // (most of a long sum's chunks)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] = __shfl_sync(0xffffffffu, word, i + k);
-        const uint32_t sure = use >> i & 0xffu;
-        if (sure == 0xffu) {                             // (segments behind the last are empty: i0 = 0)
+        for (int o = 1; o < 32; o <<= 1) {
+            const int ne = __shfl_down_sync(0xffffffffu, even, o), no = __shfl_down_sync(0xffffffffu, odd, o);
+            join_steps(even, odd, ne, no);
+        }
+        const int S = __float_as_int(s);
+        return __int_as_float(S + __shfl_sync(0xffffffffu, S & 1 ? odd : even, 0));
+    }
+    const uint32_t first = ~use | (~use << 1) | 1u;          // lanes that no sure lane's amounts are added to from below
+    int f = (int)(first >> lane & 1u);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) S += (w[k] >> 2) + (S & 1) * ((w[k] & 3) - 1);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (sure >> k & 1u) {
-                    S += (w[k] >> 2) + (S & 1) * ((w[k] & 3) - 1);
-                } else if (i + k < n_seg) {
-                    S = __float_as_int(chain_sum(reinterpret_cast<const float*>(segs + (i + k) * L4), 4 * L4, __int_as_float(S)));
-                }
-            }
+    for (int o = 1; o < 32; o <<= 1) {
+        int pe = __shfl_up_sync(0xffffffffu, even, o), po = __shfl_up_sync(0xffffffffu, odd, o);
+        const int pf = __shfl_up_sync(0xffffffffu, f, o);
+        if (!f && lane >= o) {
+            join_steps(pe, po, even, odd);
+            even = pe;
+            odd = po;
+            f = pf;
         }
     }
-    s = __int_as_float(S);
-    return s;
+    int S = __float_as_int(s);
+#pragma unroll 1
+    for (int k = 0; k < 32;) {
+        const uint32_t unsure = ~use & (0xffffffffu << k);
+        const int end = unsure ? __ffs(unsure) - 1 : 32;     // the first lane from k on that is not sure
+        if (end > k) {
+            const int je = __shfl_sync(0xffffffffu, even, end - 1), jo = __shfl_sync(0xffffffffu, odd, end - 1);
+            S += S & 1 ? jo : je;
+        }
+        if (end < 32) S = __float_as_int(chain_sum(reinterpret_cast<const float*>(segs + end * L4), 4 * L4, __int_as_float(S)));
+        k = end + 1;
+    }
+    return __int_as_float(S);
 }
 
 }  // namespace tz
