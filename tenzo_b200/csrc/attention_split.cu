@@ -389,9 +389,9 @@ __global__ void __launch_bounds__(SoftShape<HS, MANY>::threads, SoftShape<HS, MA
 // order (:842-851). Producer warps keep a three-stage ring of key chunks filled and form the weights p_t * s_v[t]
 // (:830, :844), so that the consumers only load, convert and multiply-add. Hand-over by named barriers (a poll of an
 // mbarrier costs its warp more than a chunk's barrier does). Two shapes (pick_values):
-//   heavy  two dims a lane and all heads: the fewest instructions and shared-memory cycles an item. Two items a CTA, two
-//          consumer warps each; V bytes by bulk copy, converted by the consumers (the sign-extending byte load and a
-//          32-bit conversion a dim);
+//   heavy  two neighbouring dims a lane and all heads: the fewest instructions and shared-memory cycles an item. Two items a CTA,
+//          two consumer warps each; V bytes by bulk copy, two to a load and converted by the consumers (one load a dim: 131 us
+//          against 126 at 64 x 8192 keys, 222 and 212 for 1536 prompt rows; what the kernel waits for most is shared memory);
 //   light  32 dims a CTA, one consumer warp of one or all heads: for when there are fewer items than schedulers. Four producer
 //          warps convert V to floats, which leaves the consumer a load, the weights and one FMA a chain and key. One
 //          consumer a CTA because the floats pass the shared-memory pipe twice: four of them, at 13 cycles a key, waited for it.
@@ -412,12 +412,11 @@ struct LightRing {
     static constexpr int bytes = kValueStages * 4 * (v_floats + w_floats);
 };
 
-// A sign-extended byte, converted as a 32-bit integer: that conversion issues like an FMA (one cycle), the one from a byte
-// goes through the special-function pipe (eight), which is what the compiler takes when it knows the range.
-__device__ __forceinline__ int byte_at(const int8_t* p) {
-    int x = *p;
-    asm("" : "+r"(x));
-    return x;
+// The two signed bytes of a sign-extended 16-bit load, one converted by the special-function pipe (from 8 bits) and one like an
+// FMA (from 32): both from 32 bits, with a permute for the lower byte, is slower (128 us against 126).
+__device__ __forceinline__ void bytes_of(int pair, int& lo, int& hi) {
+    lo = (int)(int8_t)pair;
+    hi = (int)(int8_t)(pair >> 8);
 }
 
 // What an item's value sums read.
@@ -537,13 +536,14 @@ __device__ __forceinline__ void split_values_heavy(const SplitLaunch& L, unsigne
     for (int c = 0; c < n_chunks; ++c) {
         const int st = c % kValueStages;
         named_barrier_sync(bar_full + st, kCount);
-        const int8_t* vp = reinterpret_cast<const int8_t*>(s_v + st * Ring::v_bytes) + 64 * part + lane;
+        const int8_t* vp = reinterpret_cast<const int8_t*>(s_v + st * Ring::v_bytes) + 64 * part + 2 * lane;
         const float* wp = s_w + st * Ring::w_floats;
         const int n = min(kValueKeys, it.T - c * kValueKeys);
+        auto load_v = [&](int k) { return (int)*reinterpret_cast<const int16_t*>(vp + k * kHd); };
         if (n == kValueKeys) {
             // three batches of eight keys under way, interleaved key by key: raw bytes on their way from shared memory,
             // bytes being converted, and values being summed
-            int raw[U][2];
+            int raw[U];
             float f[2][U][2], w[2][U][GH];
             auto load_w = [&](int k, int b, int i) {           // the i-th 16 bytes of eight keys' weights
                 const float4 q = reinterpret_cast<const float4*>(wp + k * GH)[i];
@@ -552,31 +552,32 @@ __device__ __forceinline__ void split_values_heavy(const SplitLaunch& L, unsigne
                 w[b][(4 * i + 2) / GH][(4 * i + 2) % GH] = q.z;
                 w[b][(4 * i + 3) / GH][(4 * i + 3) % GH] = q.w;
             };
+            auto convert = [&](int b, int u) {
+                int lo, hi;
+                bytes_of(raw[u], lo, hi);
+                f[b][u][0] = (float)lo;
+                f[b][u][1] = (float)hi;
+            };
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int d = 0; d < 2; ++d) raw[u][d] = byte_at(vp + u * kHd + 32 * d);
+            for (int u = 0; u < U; ++u) raw[u] = load_v(u);
 #pragma unroll
             for (int i = 0; i < U * GH / 4; ++i) load_w(0, 0, i);
 #pragma unroll
-            for (int u = 0; u < U; ++u)
-#pragma unroll
-                for (int d = 0; d < 2; ++d) {
-                    f[0][u][d] = (float)raw[u][d];
-                    raw[u][d] = byte_at(vp + (U + u) * kHd + 32 * d);
-                }
+            for (int u = 0; u < U; ++u) {
+                convert(0, u);
+                raw[u] = load_v(U + u);
+            }
 #pragma unroll
             for (int k = 0; k < kValueKeys; k += U) {
                 const int b = (k / U) & 1;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
 #pragma unroll
-                    for (int d = 0; d < 2; ++d) {
+                    for (int d = 0; d < 2; ++d)
 #pragma unroll
                         for (int g = 0; g < GH; ++g) acc[g][d] = __fmaf_rn(f[b][u][d], w[b][u][g], acc[g][d]);
-                        if (k + U < kValueKeys) f[b ^ 1][u][d] = (float)raw[u][d];
-                        if (k + 2 * U < kValueKeys) raw[u][d] = byte_at(vp + (k + 2 * U + u) * kHd + 32 * d);
-                    }
+                    if (k + U < kValueKeys) convert(b ^ 1, u);
+                    if (k + 2 * U < kValueKeys) raw[u] = load_v(k + 2 * U + u);
                     if (k + U < kValueKeys)
 #pragma unroll
                         for (int i = u * GH / 4; i < (u + 1) * GH / 4; ++i) load_w(k + U, b ^ 1, i);
@@ -584,21 +585,23 @@ __device__ __forceinline__ void split_values_heavy(const SplitLaunch& L, unsigne
             }
         } else {                                       // the last chunk
 #pragma unroll 4
-            for (int k = 0; k < n; ++k)
+            for (int k = 0; k < n; ++k) {
+                int lo, hi;
+                bytes_of(load_v(k), lo, hi);
 #pragma unroll
-                for (int d = 0; d < 2; ++d) {
-                    const float f = (float)byte_at(vp + k * kHd + 32 * d);
-#pragma unroll
-                    for (int g = 0; g < GH; ++g) acc[g][d] = __fmaf_rn(f, wp[k * GH + g], acc[g][d]);
+                for (int g = 0; g < GH; ++g) {
+                    acc[g][0] = __fmaf_rn((float)lo, wp[k * GH + g], acc[g][0]);
+                    acc[g][1] = __fmaf_rn((float)hi, wp[k * GH + g], acc[g][1]);
                 }
+            }
         }
         if (c + kValueStages < n_chunks) named_barrier_arrive(bar_free + st, kCount);
     }
-    float* out = L.a.out + ((size_t)it.seq * L.a.n_q + it.head0) * kHd + 64 * part + lane;
+    float* out = L.a.out + ((size_t)it.seq * L.a.n_q + it.head0) * kHd + 64 * part + 2 * lane;
 #pragma unroll
     for (int g = 0; g < GH; ++g)
 #pragma unroll
-        for (int d = 0; d < 2; ++d) out[g * kHd + 32 * d] = acc[g][d];
+        for (int d = 0; d < 2; ++d) out[g * kHd + d] = acc[g][d];
 }
 
 // GV heads and 32 dims of an item a CTA. Producer warp p converts keys 16 p .. 16 p + 15 of a chunk (in block pools: one block),
