@@ -43,7 +43,7 @@
 // Few row tiles (the out, down and q|k|v projections have 20 to 30) would leave most SMs idle, so K is then split
 // across the 2, 4 or 8 CTAs of a thread-block cluster: each accumulates its share of the chunks in its own tensor
 // memory and parks its int32 partial tile in shared memory; after a hardware cluster barrier every CTA takes the
-// 16-sequence column blocks b = rank, rank + ksplit, ..., adds its peers' partials for them through distributed
+// units of four sequences u = rank, rank + ksplit, ..., adds its peers' partials for them through distributed
 // shared memory (integer sums: order-free, exact), runs the epilogue on them and stores them (a reduce-scatter:
 // the epilogue work is spread over the cluster instead of queueing on one leader).
 // Every mbarrier wait is bounded; a wait that gives up sets g_umma_timeouts, the roles fall through
@@ -85,7 +85,7 @@ struct UmmaLaunch {
     int b_slots;             // activation tiles in shared memory: as many, or four (then the issuing threads request them)
     int n_pgroups;           // groups of kPGroup chunks in the packed-weight ring
     int ksplit;              // CTAs of a cluster that share one tile's K range (1 = no cluster)
-    int store_cols;          // sequences per TMA store of the epilogue (32; 16 with a cluster or up to 64 sequences)
+    int store_cols;          // sequences per TMA store of the epilogue (32; 16 up to 64 sequences, 4 with a cluster or up to 32)
 };
 
 __device__ int g_umma_timeouts = 0;
@@ -154,13 +154,13 @@ struct RingPos {
     }
 };
 
-// One 16-sequence block of the epilogue: r = accumulators of TMEM lane m (weight row `row`, `rr` inside its block).
-template <int EPI>
-__device__ __forceinline__ void umma_epilogue_block(const tenzo_tl1_gemv_args& a, uint32_t (&r)[16], const float* s_inv, const int* s_sum, float wscale,
+// NC sequences of the epilogue: r = accumulators of TMEM lane m (weight row `row`, `rr` inside its block).
+template <int EPI, int NC>
+__device__ __forceinline__ void umma_epilogue_block(const tenzo_tl1_gemv_args& a, uint32_t (&r)[NC], const float* s_inv, const int* s_sum, float wscale,
                                                     int shift, int c0, int seq0, int block, int rr, int row, bool up_half, float* s_out_cols, float* s_glu_cols, bool ok) {
-    float v[16];
+    float v[NC];
 #pragma unroll
-    for (int i = 0; i < 16; i += 4) {
+    for (int i = 0; i < NC; i += 4) {
         const int4 sv = *reinterpret_cast<const int4*>(s_sum + c0 + i);
         const float4 iv = *reinterpret_cast<const float4*>(s_inv + c0 + i);
         const int s4[4] = {sv.x, sv.y, sv.z, sv.w};
@@ -174,32 +174,32 @@ __device__ __forceinline__ void umma_epilogue_block(const tenzo_tl1_gemv_args& a
     }
     if (a.acc_out && ok && block >= 0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
+        for (int i = 0; i < NC; ++i)
             if (seq0 + c0 + i < a.batch) a.acc_out[(size_t)(seq0 + c0 + i) * a.n_blocks * 64 + block * 64 + rr] = (int)r[i];
     }
     if (EPI == TENZO_EPI_RELU2_GLU) {
         if (up_half) {                                   // the up value, and ReLU(gate)^2: multiplied once both are in place
 #pragma unroll
-            for (int i = 0; i < 16; ++i) s_glu_cols[i * 64 + rr] = v[i];
+            for (int i = 0; i < NC; ++i) s_glu_cols[i * 64 + rr] = v[i];
         } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            for (int i = 0; i < NC; ++i) {
                 const float rl = fmaxf(0.0f, v[i]);
                 s_out_cols[i * 64 + rr] = rl * rl;                               // :1618
             }
         }
     } else if (EPI == TENZO_EPI_RESIDUAL) {
-        float res[16];
+        float res[NC];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < NC; ++i) {
             const int seq = seq0 + c0 + i;
             res[i] = (seq < a.batch && block >= 0) ? __ldcg(a.resid + (size_t)seq * a.out_stride + block * 64 + rr) : 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) s_out_cols[i * 128 + row] = res[i] + v[i];                          // :1590
+        for (int i = 0; i < NC; ++i) s_out_cols[i * 128 + row] = res[i] + v[i];                          // :1590
     } else {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) s_out_cols[i * 128 + row] = v[i];
+        for (int i = 0; i < NC; ++i) s_out_cols[i * 128 + row] = v[i];
     }
 }
 
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             if (lane == 0 && q == 0) { UC(j0, 3); if (n_here == 2) UC(j0 + kExpandGroups, 3); }
         }
         // ---- all of this CTA's MMAs have completed; in a cluster it parks its partial tile [N][128 TMEM lanes] int32
-        //      (the column blocks its peers will reduce) in the ring memory the pipeline no longer needs -----------------
+        //      (the columns its peers will reduce) in the ring memory the pipeline no longer needs -----------------
         if (a.use_pdl) pdl_wait();                           // the residual rows come from an earlier kernel (long done by now)
         bool ok = true;
         if (lane == 0) ok = !timed_out && mbar_spin_bounded(bar_meta, 0u) && mbar_spin_bounded(bar_accum, 0u);
@@ -483,13 +483,13 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             const int m = 32 * q + lane;
             int* s_part = reinterpret_cast<int*>(ring);
             for (int c0 = 16 * grp; c0 < N; c0 += 16 * kExpandGroups) {
-                if ((c0 >> 4) % ksplit == split) continue;       // this CTA's own column blocks stay in tensor memory
                 uint32_t r[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) r[i] = 0u;
                 if (ok) tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, r);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) s_part[(c0 + i) * 128 + m] = (int)r[i];
+                for (int i = 0; i < 16; ++i)
+                    if ((((c0 + i) >> 2) & (ksplit - 1)) != split) s_part[(c0 + i) * 128 + m] = (int)r[i];      // (this CTA's own units stay in tensor memory)
             }
         }
     }
@@ -508,54 +508,22 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         // leave unit by unit through TMA stores: rows of 512 (256) contiguous bytes per sequence, clipped at the
         // matrix edge by the tensor map. GLU: the up half parks its values and the gate half its ReLU^2 side by side, then
         // the group multiplies them in place. Space: N*512 bytes without a cluster (at least four slots), N*512 plus 512 per
-        // own column with one (a rank owns at most every other block), which the two rings hold for every N.
+        // own column with one (a rank owns at most every other unit), which the two rings hold for every N.
+        // A unit is 32 sequences, 16 up to 64 and four with a cluster or up to 32, so that all groups of all ranks have some: with units
+        // of sixteen, 64 sequences on four ranks were one group's work in each, twelve one group's of one rank (quantiser and product,
+        // 2560 x 6912: 64 sequences 17.2 -> 15.2 us, 12 sequences 16.1 -> 14.1, 256 25.7 -> 22.9).
         constexpr int row_floats = glu ? 64 : 128;
-        const int SB = L.store_cols >> 4;                    // 16-sequence blocks per store unit: 2, or 1 (a cluster; few sequences)
         float* s_out = reinterpret_cast<float*>(ring + (CLUSTER ? (size_t)N * 512 : 0));            // behind the partial tile [N][128] int32
-        float* s_glu = s_out + (size_t)(CLUSTER ? 16 * ((N / 16 + 1) / 2) : N) * 64;                 // behind the GLU output columns (a rank owns at most every other block)
-        const int n_blocks16 = N / 16;
-        const int own_blocks = CLUSTER ? (n_blocks16 - split + ksplit - 1) / ksplit : n_blocks16;
-        const int n_units = (own_blocks + SB - 1) / SB;
+        float* s_glu = s_out + (size_t)(CLUSTER ? 4 * ((N / 4 + 1) / 2) : N) * 64;                   // behind the GLU output columns (a rank owns at most every other unit)
         const bool leader = lane == 0 && q == 0;
         const uint32_t t_lane = tmem_base + ((uint32_t)(32 * q) << 16);
-#pragma unroll 1
-        for (int un = grp; un < n_units; un += kExpandGroups) {
-            const int ob0 = un * SB;
-            const bool two = SB == 2 && ob0 + 1 < own_blocks;
-            const int c0 = 16 * (CLUSTER ? split + ksplit * ob0 : ob0);
-            uint32_t r0[16], r1[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) r0[i] = r1[i] = 0u;
-            if (ok) {
-                tmem_ld16_nowait(t_lane + (uint32_t)c0, r0);
-                if (two) tmem_ld16_nowait(t_lane + (uint32_t)(c0 + 16), r1);
-                tmem_wait_ld();
-            }
-            if (CLUSTER) {
-                // the peers' partials over distributed shared memory: every load issued before the first is
-                // used (ranks beyond the cluster and this CTA's own read its own tile and are masked out)
-#pragma unroll
-                for (int p = 0; p < 8; ++p) {
-                    const bool use_p = p < ksplit && p != split;
-                    const int* peer = cg::this_cluster().map_shared_rank(reinterpret_cast<int*>(ring), use_p ? p : split);
-                    const uint32_t mask = use_p ? 0xffffffffu : 0u;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) r0[i] += mask & (uint32_t)peer[(c0 + i) * 128 + m];
-                }
-            }
-            float* unit_out = s_out + (size_t)16 * ob0 * row_floats;
-            float* unit_glu = s_glu + (size_t)16 * ob0 * 64;
-            umma_epilogue_block<EPI>(a, r0, s_inv, s_sum, wscale, shift, c0, seq0, block, rr, row, rblk == 1, unit_out, unit_glu, ok);
-            if (two)
-                umma_epilogue_block<EPI>(a, r1, s_inv, s_sum, wscale, shift, c0 + 16, seq0, block, rr, row, rblk == 1, unit_out + 16 * row_floats,
-                                         unit_glu + 16 * 64, ok);
+        auto send = [&](float* unit_out, float* unit_glu, int cols, int c0) {      // a unit assembled by the group's four warps
             if (glu) {
                 // gate and up halves of the unit are both in shared memory: out = ReLU(gate)^2 * up, four floats at a time
                 named_barrier_sync(1 + grp, 128);
-                const int n4 = (two ? 32 : 16) * 64 / 4;
                 float4* o4 = reinterpret_cast<float4*>(unit_out);
                 const float4* g4 = reinterpret_cast<const float4*>(unit_glu);
-                for (int i = 32 * q + lane; i < n4; i += 128) {
+                for (int i = 32 * q + lane; i < cols * 16; i += 128) {
                     float4 o = o4[i];
                     const float4 u = g4[i];
                     o.x *= u.x; o.y *= u.y; o.z *= u.z; o.w *= u.w;             // :1619
@@ -566,11 +534,62 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
             fence_proxy_async_smem();
             named_barrier_sync(1 + grp, 128);
             if (leader && ok && seq0 + c0 < a.batch &&
-                UCHK(reinterpret_cast<unsigned char*>(unit_out) + 16 * SB * row_floats * 4 <= reinterpret_cast<unsigned char*>(bars), 6,
-                     reinterpret_cast<unsigned char*>(unit_out) - smem_raw, un)) {             // else nothing but padding
+                UCHK(reinterpret_cast<unsigned char*>(unit_out) + L.store_cols * row_floats * 4 <= reinterpret_cast<unsigned char*>(bars), 6,
+                     reinterpret_cast<unsigned char*>(unit_out) - smem_raw, c0)) {             // else nothing but padding
                 asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
                              ::"l"(&omap), "r"((glu ? tile : blk0) * 64), "r"(seq0 + c0), "r"(smem_addr(unit_out)) : "memory");
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            }
+        };
+        if (CLUSTER || L.store_cols == 4) {
+#pragma unroll 1
+            for (int k = grp;; k += kExpandGroups) {
+                const int c0 = 4 * (CLUSTER ? split + ksplit * k : k);
+                if (c0 >= N || seq0 + c0 >= a.batch) break;
+                uint32_t r[4] = {0u, 0u, 0u, 0u};
+                if (ok) {
+                    tmem_ld4_nowait(t_lane + (uint32_t)c0, r);
+                    tmem_wait_ld();
+                }
+                if (CLUSTER) {
+                    // the peers' partials over distributed shared memory, every load issued before the first is used
+                    uint32_t part[8][4];
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        const bool use_p = p < ksplit && p != split;
+                        const int* peer = cg::this_cluster().map_shared_rank(reinterpret_cast<int*>(ring), use_p ? p : split);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) part[p][i] = use_p ? (uint32_t)peer[(c0 + i) * 128 + m] : 0u;
+                    }
+#pragma unroll
+                    for (int p = 0; p < 8; ++p)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) r[i] += part[p][i];
+                }
+                float* unit_out = s_out + (size_t)4 * k * row_floats;
+                float* unit_glu = s_glu + (size_t)4 * k * 64;
+                umma_epilogue_block<EPI, 4>(a, r, s_inv, s_sum, wscale, shift, c0, seq0, block, rr, row, rblk == 1, unit_out, unit_glu, ok);
+                send(unit_out, unit_glu, 4, c0);
+            }
+        } else {
+#pragma unroll 1
+            for (int c0 = L.store_cols * grp; c0 < N; c0 += L.store_cols * kExpandGroups) {
+                const bool two = L.store_cols == 32 && c0 + 16 < N;
+                uint32_t r0[16], r1[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) r0[i] = r1[i] = 0u;
+                if (ok) {
+                    tmem_ld16_nowait(t_lane + (uint32_t)c0, r0);
+                    if (two) tmem_ld16_nowait(t_lane + (uint32_t)(c0 + 16), r1);
+                    tmem_wait_ld();
+                }
+                float* unit_out = s_out + (size_t)c0 * row_floats;
+                float* unit_glu = s_glu + (size_t)c0 * 64;
+                umma_epilogue_block<EPI, 16>(a, r0, s_inv, s_sum, wscale, shift, c0, seq0, block, rr, row, rblk == 1, unit_out, unit_glu, ok);
+                if (two)
+                    umma_epilogue_block<EPI, 16>(a, r1, s_inv, s_sum, wscale, shift, c0 + 16, seq0, block, rr, row, rblk == 1, unit_out + 16 * row_floats,
+                                                 unit_glu + 16 * 64, ok);
+                send(unit_out, unit_glu, two ? 32 : 16, c0);
             }
         }
         if (tid == 64) UT(8);
@@ -633,13 +652,12 @@ int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float*
     L.n_pgroups = UmmaSmem::pgroups_for(L.n_box);
     const int seq_tiles = (a.batch + kMaxN - 1) / kMaxN;
     L.ksplit = pick_umma_ksplit(L.units * seq_tiles, a.K / kKc);
-    L.store_cols = (L.ksplit > 1 || L.n_box <= 64) ? 16 : 32;      // few sequences: 16 per unit, so that every group gets one
+    L.store_cols = L.ksplit > 1 || L.n_box <= 32 ? 4 : L.n_box <= 64 ? 16 : 32;
     CUtensorMap amap, omap;
     // activations [batch][K] int8: B-operand tiles {128 bytes of K, n_box sequences}, 128-byte swizzle
     if (int rc = encode_2d(&amap, CU_TENSOR_MAP_DATA_TYPE_UINT8, a8, (uint64_t)a.K, (uint64_t)a.batch, (uint64_t)a.K, kKc, (uint32_t)L.n_box,
                            CU_TENSOR_MAP_SWIZZLE_128B)) return rc;
-    // output [batch][n_out] fp32: store units {128 (GLU: 64) rows of the weight matrix, 32 sequences (16: the column
-    // blocks a cluster's CTAs store separately)}
+    // output [batch][n_out] fp32: store units {128 (GLU: 64) rows of the weight matrix, 32, 16 or 4 sequences}
     const uint64_t n_out = (uint64_t)(glu ? a.n_blocks / 2 : a.n_blocks) * 64;
     if (int rc = encode_2d(&omap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.out, n_out, (uint64_t)a.batch, (uint64_t)a.out_stride * 4, glu ? 64u : 128u,
                            (uint32_t)L.store_cols, CU_TENSOR_MAP_SWIZZLE_NONE)) return rc;
@@ -707,8 +725,8 @@ extern "C" int tenzo_cuda_tl1_gemm_layout(int batch, int* slots, int* weight_gro
     if (weight_groups) *weight_groups = tz::UmmaSmem::pgroups_for(n_box);
     if (smem_bytes) *smem_bytes = tz::UmmaSmem::bytes(n_box);
     // without a cluster: the output columns [n_box][128] fp32 (GLU: [n_box][64] twice); with one: behind the partial tile
-    // [n_box][128] int32, the columns of the blocks a rank owns (at most every other 16-sequence block)
-    if (epilogue_bytes) *epilogue_bytes = (size_t)n_box * 512 + (size_t)16 * ((n_box / 16 + 1) / 2) * 512;
+    // [n_box][128] int32, the columns of the units a rank owns (at most every other four sequences)
+    if (epilogue_bytes) *epilogue_bytes = (size_t)n_box * 512 + (size_t)4 * ((n_box / 4 + 1) / 2) * 512;
     return 0;
 }
 
