@@ -661,11 +661,15 @@ bool attn_split_preferred(const tenzo_attention_args& a);
 int attn_split_kernels(const tenzo_attention_args& a);
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st);
 int attn_split_take_timeouts();
+// exact order, up to 256 keys (attention_short.cu)
+bool attn_short_chosen(const tenzo_attention_args& a);
+int attn_short_run(const tenzo_attention_args& a, cudaStream_t st);
+int attn_short_take_errors();
 
 static bool attn_split_chosen(const tenzo_attention_args& a) {
     return a.tiles == 3 || (a.tiles == 0 && a.heads_per_cta == 0 && attn_split_possible(a) && attn_split_preferred(a));
 }
-int attn_kernels(const tenzo_attention_args& a) { return a.mode == 1 ? 3 : attn_split_chosen(a) ? attn_split_kernels(a) : 1; }
+int attn_kernels(const tenzo_attention_args& a) { return a.mode == 1 ? 3 : !attn_short_chosen(a) && attn_split_chosen(a) ? attn_split_kernels(a) : 1; }
 }
 
 extern "C" int tenzo_cuda_attention_take_timeouts(void) {
@@ -674,7 +678,9 @@ extern "C" int tenzo_cuda_attention_take_timeouts(void) {
     if (v) cudaMemcpyToSymbol(tz::g_attn_timeouts, &zero, sizeof zero);
     const int f = tz::attn_fast_take_timeouts();
     const int p = tz::attn_split_take_timeouts();
-    if (f < 0 || p < 0) return -1;
+    const int s = tz::attn_short_take_errors();
+    if (f < 0 || p < 0 || s < 0) return -1;
+    if (s > v) v = s;
     return v > f ? (v > p ? v : p) : (f > p ? f : p);
 }
 
@@ -699,6 +705,7 @@ extern "C" int tenzo_cuda_attention_int8(const tenzo_attention_args* args, void*
     if (a.mode != 0) return -1;
     if ((size_t)a.max_len * sizeof(float) > (size_t)kScoreSmemBytes) return -5;   // one head's scores must fit on chip
     if (a.tiles == 3 && !attn_split_possible(a)) return -5;
+    if (attn_short_chosen(a)) return attn_short_run(a, static_cast<cudaStream_t>(stream));
     if (attn_split_chosen(a)) return attn_split_run(a, static_cast<cudaStream_t>(stream));
     AttnLaunch L;
     L.a = a;

@@ -858,11 +858,10 @@ int attn_split_kernels(const tenzo_attention_args& a) {
     return 3 * ((a.batch + per_pass - 1) / per_pass);
 }
 
-// With heads for nearly two CTAs an SM the three kernels win at any length (20/5 heads, 16 x 16 keys: 10.5 us against 13.2 in
-// one kernel, 64 x 64: 18.5 and 25.8, 256 x 256: 60 and 111; 32/8 heads alike), with heads for every SM from about 256 keys on
-// (8 x 128: 12.1 and 10.5; 12 x 1500: 34 and 50), with fewer from about 1000 (one sequence of 1024 keys: 17.5 us against 19,
-// of 512: 15 against 10, of 6003: 48 against 98). max_len is an upper bound that callers round up, so these lines lie one
-// step further.
+// Against the one kernel of attention.cu, above the 256 keys that attention_short.cu takes: with heads for every SM the three kernels win
+// (12 x 1500: 34 and 50 us; 8 x 128 keys 12.1 and 10.5, not reached), with fewer from about 1000 keys on (one sequence of 1024 keys:
+// 17.5 us against 19, of 512: 15 against 10, of 6003: 47 against 98). max_len is an upper bound that callers round up, so the line lies
+// one step further.
 bool attn_split_preferred(const tenzo_attention_args& a) {
     const long long heads = (long long)a.batch * a.n_q;
     return heads >= 256 || a.max_len > (heads >= 148 ? 256 : 1024);
