@@ -388,16 +388,14 @@ __global__ void __launch_bounds__(SoftShape<HS, MANY>::threads, SoftShape<HS, MA
 // Value sums: a consumer lane owns one or two output dims of GV heads, one chain per head and dim, and walks the keys in
 // order (:842-851). Producer warps keep a three-stage ring of key chunks filled and form the weights p_t * s_v[t]
 // (:830, :844), so that the consumers only load, convert and multiply-add. Hand-over by named barriers (a poll of an
-// mbarrier costs its warp more than a chunk's barrier does). Two shapes (pick_values):
+// mbarrier costs its warp more than a chunk's barrier does). Two shapes (heavy_items), and a third for a few heads in all:
 //   heavy  two neighbouring dims a lane and all heads: the fewest instructions and shared-memory cycles an item. Two items a CTA,
 //          two consumer warps each; V bytes by bulk copy, two to a load and converted by the consumers (one load a dim: 131 us
 //          against 126 at 64 x 8192 keys, 222 and 212 for 1536 prompt rows; what the kernel waits for most is shared memory);
-//   light  32 dims a CTA, one consumer warp of one or all heads: for when there are fewer items than schedulers. Four producer
-//          warps convert V to floats, which leaves the consumer a load, the weights and one FMA a chain and key. One
-//          consumer a CTA because the floats pass the shared-memory pipe twice: four of them, at 13 cycles a key, waited for it.
-//          One sequence: 8.8 cycles a key with one head (6003 to 12000 keys), twice the FMA's latency; neither side waits for the
-//          other (some 30 of 630 cycles a chunk), so the loop of the chain and the producers' conversion would both have to shorten.
-//          Attention of one sequence of 6003 keys 47 us, with the heavy shape 66.
+//   light  32 dims and all heads a CTA, one consumer warp: for when there are fewer items than schedulers. Four producer
+//          warps convert V to floats, which leaves the consumer a load, the weights and the FMAs. One
+//          consumer a CTA because the floats pass the shared-memory pipe twice: four of them, at 13 cycles a key, waited for it;
+//   few    one head and 64 dims a CTA, a dim a lane (split_values_few_kernel).
 constexpr int kValueThreads = 192;                    // heavy: four consumer warps, one a scheduler, and two producers; light: 1 + 4
 constexpr int kValueKeys = 64, kValueStages = 3;
 template <int GV>
@@ -463,6 +461,69 @@ __device__ __forceinline__ void load_vec(const float* p, float (&v)[GV]) {
     }
 }
 
+// The producer warp of a group of consumers: V rows as they come, weights of GV heads, a ring of kValueStages chunks of KEYS keys.
+template <int GH, int GV, int KEYS, bool PAGED>
+__device__ __forceinline__ void produce_values(const ValueItem<GH, PAGED>& it, int n_chunks, unsigned char* s_v, float* s_e, float* s_w, float* s_s,
+                                               uint64_t* s_bar, int bar_full, int bar_free, int count) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        for (int i = 0; i < kValueStages; ++i) mbar_init(&s_bar[i], 1);
+        mbar_init_fence();
+    }
+    __syncwarp();
+    float inv[GV];
+    load_vec<GV>(it.inv, inv);
+    // Block pools: lane l holds block l of the next chunk, fetched a chunk ahead (an address that waits for the table puts its round
+    // trip on every chunk).
+    auto block_of = [&](int c) { return PAGED && lane < KEYS / 16 && c * KEYS + 16 * lane < it.T ? __ldg(it.rows.table + c * (KEYS / 16) + lane) : 0; };
+    auto row_of = [&](int block) { return (((size_t)block * it.rows.n_layers + it.rows.layer) * it.rows.n_kv + it.rows.kvh) * 16; };
+    int next_block = block_of(0);
+    auto request = [&](int c) {
+        if (c < n_chunks) {
+            const int block = next_block;
+            next_block = block_of(c + 1);
+            const int st = c % kValueStages, t0 = c * KEYS, n = min(KEYS, it.T - t0);
+            if (lane == 0) mbar_expect_tx(&s_bar[st], (unsigned)n * kHd);
+            __syncwarp();
+            unsigned char* dst = s_v + st * (KEYS * kHd);
+            if constexpr (PAGED) {
+                if (16 * lane < n) bulk_g2s(dst + lane * 16 * kHd, it.cv + row_of(block) * kHd, (unsigned)min(16, n - 16 * lane) * kHd, &s_bar[st]);
+            } else {
+                if (lane == 0) bulk_g2s(dst, it.cv + it.rows.row(t0) * kHd, (unsigned)n * kHd, &s_bar[st]);
+            }
+#pragma unroll
+            for (int i = 0; i < KEYS / 32; ++i) {
+                const int k = 32 * i + lane;
+                const size_t r = PAGED ? row_of(__shfl_sync(0xffffffffu, block, k >> 4)) + (k & 15) : it.rows.row(t0 + k);
+                if (k < n) {
+                    cp_async<4 * GV>(s_e + st * (KEYS * GV) + k * GV, it.e + (size_t)(t0 + k) * GH);
+                    cp_async<4>(s_s + st * KEYS + k, it.sv + r);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");       // one group a chunk, empty behind the last
+    };
+    bool timed_out = false;
+    for (int c = 0; c < kValueStages - 1; ++c) request(c);
+    for (int c = 0; c < n_chunks; ++c) {
+        const int st = c % kValueStages;
+        asm volatile("cp.async.wait_group %0;" ::"n"(kValueStages - 2) : "memory");
+#pragma unroll
+        for (int i = 0; i < KEYS / 32; ++i) {                              // a lane's own copies
+            const int k = 32 * i + lane;
+            float ev[GV];
+#pragma unroll
+            for (int g = 0; g < GV; ++g) ev[g] = s_e[st * (KEYS * GV) + k * GV + g];
+            store_weights<GV, PAGED>(s_w + st * (KEYS * GV) + k * GV, ev, inv, s_s[st * KEYS + k]);
+        }
+        if (!mbar_wait_bounded(&s_bar[st], (unsigned)(c / kValueStages) & 1u)) timed_out = true;
+        named_barrier_arrive(bar_full + st, count);
+        if (c > 0 && c + kValueStages - 1 < n_chunks) named_barrier_sync(bar_free + (c - 1) % kValueStages, count);   // chunk c - 1 has been read
+        request(c + kValueStages - 1);
+    }
+    if (timed_out) atomicExch(&g_split_timeouts, 1);
+}
+
 template <int GH, bool PAGED>
 __device__ __forceinline__ void split_values_heavy(const SplitLaunch& L, unsigned char* smem, uint64_t (*s_bars)[kValueStages], int block, int n_items) {
     using Ring = HeavyRing<GH>;
@@ -478,55 +539,7 @@ __device__ __forceinline__ void split_values_heavy(const SplitLaunch& L, unsigne
     const int bar_full = 1 + grp * 2 * kValueStages, bar_free = bar_full + kValueStages;
     const int n_chunks = (it.T + kValueKeys - 1) / kValueKeys;
     if (warp >= 4) {
-        uint64_t* s_bar = s_bars[grp];
-        if (lane == 0) {
-            for (int i = 0; i < kValueStages; ++i) mbar_init(&s_bar[i], 1);
-            mbar_init_fence();
-        }
-        __syncwarp();
-        float inv[GH];
-        load_vec<GH>(it.inv, inv);
-        auto request = [&](int c) {
-            if (c < n_chunks) {
-                const int st = c % kValueStages, t0 = c * kValueKeys, n = min(kValueKeys, it.T - t0);
-                if (lane == 0) mbar_expect_tx(&s_bar[st], (unsigned)n * kHd);
-                __syncwarp();
-                unsigned char* dst = s_v + st * Ring::v_bytes;
-                if constexpr (PAGED) {
-                    if (16 * lane < n) bulk_g2s(dst + lane * 16 * kHd, it.cv + it.rows.row(t0 + 16 * lane) * kHd, (unsigned)min(16, n - 16 * lane) * kHd, &s_bar[st]);
-                } else {
-                    if (lane == 0) bulk_g2s(dst, it.cv + it.rows.row(t0) * kHd, (unsigned)n * kHd, &s_bar[st]);
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int k = 32 * i + lane;
-                    if (k < n) {
-                        cp_async<4 * GH>(s_e + st * Ring::w_floats + k * GH, it.e + (size_t)(t0 + k) * GH);
-                        cp_async<4>(s_s + st * kValueKeys + k, it.sv + it.rows.row(t0 + k));
-                    }
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");       // one group a chunk, empty behind the last
-        };
-        bool timed_out = false;
-        for (int c = 0; c < kValueStages - 1; ++c) request(c);
-        for (int c = 0; c < n_chunks; ++c) {
-            const int st = c % kValueStages;
-            asm volatile("cp.async.wait_group %0;" ::"n"(kValueStages - 2) : "memory");
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {                              // a lane's own copies
-                const int k = 32 * i + lane;
-                float ev[GH];
-#pragma unroll
-                for (int g = 0; g < GH; ++g) ev[g] = s_e[st * Ring::w_floats + k * GH + g];
-                store_weights<GH, PAGED>(s_w + st * Ring::w_floats + k * GH, ev, inv, s_s[st * kValueKeys + k]);
-            }
-            if (!mbar_wait_bounded(&s_bar[st], (unsigned)(c / kValueStages) & 1u)) timed_out = true;
-            named_barrier_arrive(bar_full + st, kCount);
-            if (c > 0 && c + kValueStages - 1 < n_chunks) named_barrier_sync(bar_free + (c - 1) % kValueStages, kCount);   // chunk c - 1 has been read
-            request(c + kValueStages - 1);
-        }
-        if (timed_out) atomicExch(&g_split_timeouts, 1);
+        produce_values<GH, GH, kValueKeys, PAGED>(it, n_chunks, s_v, s_e, s_w, s_s, s_bars[grp], bar_full, bar_free, kCount);
         return;
     }
     const int part = warp & 1;
@@ -604,18 +617,18 @@ __device__ __forceinline__ void split_values_heavy(const SplitLaunch& L, unsigne
         for (int d = 0; d < 2; ++d) out[g * kHd + d] = acc[g][d];
 }
 
-// GV heads and 32 dims of an item a CTA. Producer warp p converts keys 16 p .. 16 p + 15 of a chunk (in block pools: one block),
+// All heads and 32 dims of an item a CTA. Producer warp p converts keys 16 p .. 16 p + 15 of a chunk (in block pools: one block),
 // one 16-byte piece a lane, fetched four chunks ahead. Word j of piece q of key r goes to the 16 bytes (2 j + q) ^ 2 (r & 3)
 // of the key's row, which keeps the stores of a warp free of bank conflicts; consumer lane l reads the floats of dim
 // 16 ((l >> 2) & 1) + 4 (l >> 3) + (l & 3).
-template <int GH, int GV, bool PAGED>
+template <int GH, bool PAGED>
 __device__ __forceinline__ void split_values_light(const SplitLaunch& L, unsigned char* smem, int block, int item0) {
-    using Ring = LightRing<GV>;
-    constexpr int kSubs = GH / GV, kCount = 160, kAhead = 4;
+    using Ring = LightRing<GH>;
+    constexpr int GV = GH, kCount = 160, kAhead = 4;
     const int lane = threadIdx.x & 31, warp = ((threadIdx.x >> 5) + block) % 6;      // consumers of successive CTAs on different schedulers
     const int part = block & 3, group = block >> 2;
     if (warp == 5) return;
-    const ValueItem<GH, PAGED> it(L, item0 + group / kSubs, group % kSubs * GV);
+    const ValueItem<GH, PAGED> it(L, item0 + group, 0);
     if (it.T <= 0) return;
     float* s_v = reinterpret_cast<float*>(smem);                                                 // [stages][keys][32]
     float* s_w = s_v + kValueStages * Ring::v_floats;                                            // [stages][keys][GV]
@@ -737,15 +750,96 @@ __device__ __forceinline__ void split_values_light(const SplitLaunch& L, unsigne
     for (int g = 0; g < GV; ++g) out[g * kHd] = acc[g];
 }
 
-// The first `heavy` items in the heavy shape, the rest in the light one with GV heads a CTA.
-template <int GH, int GV, bool PAGED>
+// Few heads (one or two sequences): a CTA has one head and 64 dims, a dim a lane and a consumer warp a scheduler, so that a chain runs at
+// the multiply-add's latency: a byte load, a conversion and a quarter of a weight load fit beside it. A batch of eight keys is
+// summed while the next is converted and the one after that is on its way from shared memory, over the chunks' ends too.
+// Chunks of 256 keys: a chunk costs the producer warp some 700 cycles whatever it holds. One sequence of 6003 keys: 30.4 us with V
+// converted to floats by four producer warps (8.8 cycles a key, as long as the producers took), here 33.2 with chunks of 64 keys,
+// 25.7 of 128 and 24.0 of 256; two sequences up to 5000 32.0 -> 20.7.
+constexpr int kFewThreads = 96, kFewKeys = 256;
+constexpr int kFewBytes = kValueStages * (kFewKeys * kHd + 12 * kFewKeys);
+template <int GH, bool PAGED>
+__global__ void __launch_bounds__(kFewThreads) split_values_few_kernel(const SplitLaunch L) {
+    extern __shared__ __align__(128) unsigned char s_v[];                                        // [stages][keys][128]
+    __shared__ uint64_t s_bar[kValueStages];
+    float* s_e = reinterpret_cast<float*>(s_v + kValueStages * kFewKeys * kHd);                // [stages][keys]
+    float* s_w = s_e + kValueStages * kFewKeys;
+    float* s_s = s_w + kValueStages * kFewKeys;
+    constexpr int U = 8, kBatches = kFewKeys / U, bar_full = 1, bar_free = 1 + kValueStages;
+    if (L.a.use_pdl) pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = blockIdx.x & 1, unit = blockIdx.x >> 1;
+    const ValueItem<GH, PAGED> it(L, unit / GH, unit % GH);
+    if (it.T <= 0) return;
+    const int n_chunks = (it.T + kFewKeys - 1) / kFewKeys, full = it.T / kFewKeys;
+    if (warp == 2) {
+        produce_values<GH, 1, kFewKeys, PAGED>(it, n_chunks, s_v, s_e, s_w, s_s, s_bar, bar_full, bar_free, kFewThreads);
+        return;
+    }
+    const int dim = 64 * half + 32 * warp + lane;
+    float acc = 0.0f, f[2][U], w[2][U];
+    int raw[U];
+    auto load_v = [&](int st, int k) {                 // (a load that extends the sign, converted from 32 bits: that conversion issues like an FMA)
+        int x = reinterpret_cast<const int8_t*>(s_v)[(st * kFewKeys + k) * kHd + dim];
+        asm("" : "+r"(x));
+        return x;
+    };
+    auto load_w = [&](int st, int k, int b, int i) {   // the i-th four of eight weights
+        const float4 q = *reinterpret_cast<const float4*>(s_w + st * kFewKeys + k + 4 * i);
+        w[b][4 * i] = q.x; w[b][4 * i + 1] = q.y; w[b][4 * i + 2] = q.z; w[b][4 * i + 3] = q.w;
+    };
+    if (full > 0) {
+        named_barrier_sync(bar_full, kFewThreads);
+#pragma unroll
+        for (int u = 0; u < U; ++u) raw[u] = load_v(0, u);
+        load_w(0, 0, 0, 0);
+        load_w(0, 0, 0, 1);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f[0][u] = (float)raw[u];
+            raw[u] = load_v(0, U + u);
+        }
+    }
+    int st = 0;
+    for (int c = 0; c < full; ++c) {
+        const int next = st + 1 == kValueStages ? 0 : st + 1;
+        const bool more = c + 1 < full;
+#pragma unroll
+        for (int j = 0; j < kBatches; ++j) {           // batch j is summed, j + 1 converted, j + 2 loaded
+            const int b = j & 1;
+            if (j == kBatches - 2 && more) named_barrier_sync(bar_full + next, kFewThreads);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                acc = __fmaf_rn(f[b][u], w[b][u], acc);
+                if (j < kBatches - 1 || more) f[b ^ 1][u] = (float)raw[u];
+                if (j < kBatches - 2) raw[u] = load_v(st, (j + 2) * U + u);
+                else if (more) raw[u] = load_v(next, (j + 2 - kBatches) * U + u);
+                if ((u & 3) == 3) {
+                    if (j < kBatches - 1) load_w(st, (j + 1) * U, b ^ 1, u >> 2);
+                    else if (more) load_w(next, 0, b ^ 1, u >> 2);
+                }
+            }
+            if (j == kBatches - 2 && c + kValueStages < n_chunks) named_barrier_arrive(bar_free + st, kFewThreads);      // the chunk is in registers
+        }
+        st = next;
+    }
+    if (full < n_chunks) {                             // the keys behind the last whole chunk
+        const int n = it.T - full * kFewKeys;
+        named_barrier_sync(bar_full + st, kFewThreads);
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) acc = __fmaf_rn((float)load_v(st, k), s_w[st * kFewKeys + k], acc);
+    }
+    L.a.out[((size_t)it.seq * L.a.n_q + it.head0) * kHd + dim] = acc;
+}
+
+// The first `heavy` items in the heavy shape, the rest in the light one.
+template <int GH, bool PAGED>
 __global__ void __launch_bounds__(kValueThreads, 3) split_values_kernel(const SplitLaunch L, int heavy) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ uint64_t s_bars[2][kValueStages];
     if (L.a.use_pdl) pdl_wait();
     const int heavy_blocks = (heavy + 1) / 2;
     if ((int)blockIdx.x < heavy_blocks) split_values_heavy<GH, PAGED>(L, smem_raw, s_bars, blockIdx.x, heavy);
-    else split_values_light<GH, GV, PAGED>(L, smem_raw, blockIdx.x - heavy_blocks, heavy);
+    else split_values_light<GH, PAGED>(L, smem_raw, blockIdx.x - heavy_blocks, heavy);
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------
@@ -801,23 +895,27 @@ static cudaError_t split_launch(void (*kernel)(KArgs...), dim3 grid, int threads
 // How the value sums of `items` items are cut. Heavy items run best when each of the 592 schedulers (148 SMs) has the same
 // number of their warps, so whole rounds of 296 items are heavy; a rest that would leave most SMs idle for a round, and a
 // batch as small as that, is light (64 x 8192 keys, 20/5 heads: 276 us all heavy, 253 with 24 of the 320 items light; 60 items of
-// 1500 36.8 all heavy and 35.7 all light, 70 items 37.5 and 36.3, 80 items 42.1 and 48.1; 100 items of 2048 54.8 and 62.3). One
-// head a CTA only where even then few SMs have one. The cut goes by the number of items, whatever their lengths.
-struct ValueSplit { int heavy, gv; };
-static ValueSplit pick_values(long long items, int gh) {
+// 1500 36.8 all heavy and 35.7 all light, 70 items 37.5 and 36.3, 80 items 42.1 and 48.1; 100 items of 2048 54.8 and 62.3). The
+// cut goes by the number of items, whatever their lengths. Up to kFewHeads heads take the form of one head a CTA.
+constexpr int kFewHeads = 40;
+static int heavy_items(long long items) {
     const long long rest = items % 296;
-    const bool light = rest <= (items < 296 ? 70 : 100);
-    return {(int)(light ? items - rest : items), items * gh <= 40 ? 1 : gh};
+    return (int)(rest <= (items < 296 ? 70 : 100) ? items - rest : items);
 }
 
-template <int GH, int GV, bool PAGED>
-static cudaError_t launch_values(const SplitLaunch& L, int heavy, int items, cudaStream_t st) {
-    const int smem = heavy ? HeavyRing<GH>::bytes : LightRing<GV>::bytes;
-    static_assert(HeavyRing<GH>::bytes >= LightRing<GV>::bytes, "");
-    cudaError_t e = allow_smem(split_values_kernel<GH, GV, PAGED>, HeavyRing<GH>::bytes);
+template <int GH, bool PAGED>
+static cudaError_t launch_values(const SplitLaunch& L, int items, cudaStream_t st) {
+    if (items * GH <= kFewHeads) {
+        cudaError_t e = allow_smem(split_values_few_kernel<GH, PAGED>, kFewBytes);
+        if (e != cudaSuccess) return e;
+        return split_launch(split_values_few_kernel<GH, PAGED>, dim3((unsigned)(items * GH * 2)), kFewThreads, kFewBytes, st, L.a.use_pdl != 0, L);
+    }
+    const int heavy = heavy_items(items), smem = heavy ? HeavyRing<GH>::bytes : LightRing<GH>::bytes;
+    static_assert(HeavyRing<GH>::bytes >= LightRing<GH>::bytes, "");
+    cudaError_t e = allow_smem(split_values_kernel<GH, PAGED>, HeavyRing<GH>::bytes);
     if (e != cudaSuccess) return e;
-    const int blocks = (heavy + 1) / 2 + (items - heavy) * (GH / GV) * 4;
-    return split_launch(split_values_kernel<GH, GV, PAGED>, dim3((unsigned)blocks), kValueThreads, smem, st, L.a.use_pdl != 0, L, heavy);
+    const int blocks = (heavy + 1) / 2 + (items - heavy) * 4;
+    return split_launch(split_values_kernel<GH, PAGED>, dim3((unsigned)blocks), kValueThreads, smem, st, L.a.use_pdl != 0, L, heavy);
 }
 
 template <int GH, int HS, bool PAGED, bool MANY = false>
@@ -842,8 +940,7 @@ static cudaError_t split_pass(const SplitLaunch& L, int n_seq, cudaStream_t st) 
     if (GH > 1 && items > 3 * 148) e = launch_softmax<GH, GH, PAGED, GH != 1>(L, items, st);
     else e = GH == 1 || items >= 148 ? launch_softmax<GH, GH, PAGED>(L, items, st) : launch_softmax<GH, 1, PAGED>(L, items, st);
     if (e != cudaSuccess) return e;
-    const ValueSplit v = pick_values(items, GH);
-    return v.gv == GH ? launch_values<GH, GH, PAGED>(L, v.heavy, (int)items, st) : launch_values<GH, 1, PAGED>(L, v.heavy, (int)items, st);
+    return launch_values<GH, PAGED>(L, (int)items, st);
 }
 
 static int split_rows_per_pass(const tenzo_attention_args& a) {
