@@ -640,10 +640,11 @@ static size_t fa_smem_bytes(int stages) {
 // keys of streaming (32 x 4160: 93 us with 384 keys per CTA, 73 us with 1024), and a split costs the merge about 16. Up to
 // three rounds count whole, more of them less sharply. At least 256 keys, a multiple of the 128 the four warps take per round.
 // (64 x 8192 keys, 320 items: three splits, as by the rule of about three waves, are 2.2 rounds, four are 2.9.)
+// (2 x 1000 keys, 10 items: four splits of 256, the last one short, 5.7 us; three of 384 6.8.)
 static void fa_pick_split(int batch, int n_kv, int group, int max_len, int* n_splits, int* split_keys) {
     const long long items = (long long)batch * n_kv, places = 148 * (group <= 4 ? kFbResident : 2);
     double best = 0.0;
-    for (int want = 1; want <= 64 && (want == 1 || (max_len + want - 1) / want >= 256); ++want) {
+    for (int want = 1; want <= 64 && (want == 1 || (max_len + want - 1) / want > 128); ++want) {       // 129 and more round up to 256
         const int keys = ((max_len + want - 1) / want + 127) / 128 * 128, splits = (max_len + keys - 1) / keys;
         const long long ctas = items * splits;
         const double rounds = ctas <= 3 * places ? (double)((ctas + places - 1) / places) : (double)ctas / places + 0.5;
