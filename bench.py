@@ -319,7 +319,7 @@ def attention_roofline(B, ctx, steps, peak, mode=0):
     gbs = bytes_per / (ms * 1e-3) / 1e9
     del ck, cv, sk, sv
     torch.cuda.empty_cache()
-    return {"bound": "hbm", "kernel": "attn_fast_kernel (+ append, merge)" if mode == 1 else "split_scores, split_softmax and split_values kernels", "achieved": gbs, "peak": peak[0],
+    return {"bound": "hbm", "kernel": "attn_fast_t_kernel (+ append, merge)" if mode == 1 else "split_scores, split_softmax and split_values kernels", "achieved": gbs, "peak": peak[0],
             "peak_source": peak[1], "unit": "GB/s", "frac": gbs / peak[0],
             "traffic": bytes_per * (297.5 / 259.5) if mode == 0 else bytes_per * (265.6 / 259.5),
             "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.6 MB read + 5.9 MB written for 259.5 MB algorithmic, scaled by the keys read" if mode == 0 else

@@ -166,8 +166,8 @@ typedef struct {
     void* workspace;        /* 16-byte aligned, contents need not be kept. Mode 1: tenzo_cuda_attention_workspace_bytes(...)
                                bytes for the partial results of the splits. Mode 0: optional,
                                tenzo_cuda_attention_exact_workspace_bytes(...) bytes for the score vectors (room for one
-                               sequence at least); NULL keeps them in shared memory, which is slower for all but short
-                               contexts of few sequences. Same results either way */
+                               sequence at least); not used up to max_len 256. NULL keeps them in shared memory, which
+                               is slower for all but few sequences of some hundred keys. Same results either way */
     size_t workspace_bytes;
 } tenzo_attention_args;
 

@@ -332,7 +332,7 @@ def run_attn(args):
                      "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.6 MB read + 5.9 MB written for 259.5 MB algorithmic, scaled by the keys read",
                      "bytes_per_launch": bytes_per, "us_per_launch": ms * 1e3},
         "tolerance_mode": {"ms_per_step": ms_fast, "achieved": bytes_per / (ms_fast * 1e-3) / 1e9, "unit": "GB/s",
-                           "frac": bytes_per / (ms_fast * 1e-3) / 1e9 / peak[0], "kernel": "fa_append_kernel + attn_fast_kernel + attn_fast_merge_kernel",
+                           "frac": bytes_per / (ms_fast * 1e-3) / 1e9 / peak[0], "kernel": "fa_append_kernel + attn_fast_t_kernel + attn_fast_merge_kernel",
                            "max_rel_err_vs_exact": fast_err, "tolerance": 1e-3},
         "cpu_baseline": cpu,
     }), flush=True)

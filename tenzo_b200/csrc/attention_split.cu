@@ -11,16 +11,16 @@
 //            key row and 64 broadcast LDS.128 of the query per key pair;
 //   softmax  one CTA per item or head; the ordered sum of the exponentials in parallel segments (ordered_sum.cuh);
 //   values   consumer warps that own the chains of an (item, dims, heads) unit, fed by producer warps.
-// What bounds it. A (key, item) takes 74 warp instructions (35.6 in the scores, 9.2 in the softmax, 29.2 in the value sums; 16 + 16
-// of them are the multiply-adds whose order is fixed), so 592 schedulers need 64 us a million. 64 x 8192 keys, 20/5 heads:
-// 672 us in one kernel, here 277, 106 us a million; 1536 prompt rows 100; lengths spread over a factor of two 115 (256
-// sequences up to 4096) to 156 (32 up to 2048, 32/8 heads), equal ones of the same maximum 104 and 130. The distance to 64: the
-// three kernels follow one another without overlap (113, 48 and 134 us at 64 x 8192, each alone and cold), the softmax lasts as
-// long as its summing warps' chains (38 % of the issue slots), scores and value sums use 62 to 67 % of theirs, and the
-// last round of the value sums is as long as its longest item (they are dealt out by index). Packed f32x2 FMAs hold the
-// FMA pipe for two cycles but one issue slot: 16 of them and 16 byte permutes take 46 cycles of a scheduler, 32 plain FMAs and the
-// permutes 65, so the scores and conversions would gain by them; they are not written that way yet.
-// One sequence of 6003 keys: 98 us in one kernel, here 47 (8.6, 15.6 and 34.5 us, each alone and cold).
+// What bounds it. A (key, item) takes some 70 warp instructions (35.6 in the scores, 6.3 in the softmax, 28 in the value sums; 16 +
+// 16 of them are the multiply-adds whose order is fixed), so 592 schedulers need 60 us a million. 64 x 8192 keys, 20/5 heads:
+// 672 us in one kernel, here 272, 104 us a million (277 before the sums of the softmax were joined and the value sums took two dims
+// a load). The distance to 60: the three kernels follow one another without overlap (111, 35 and 126 us at 64 x 8192), the
+// softmax lasts as long as its summing warps' chains, and the last round of the value sums is as long as its longest item (they
+// are dealt out by index). The scores' loop cannot go below 30 cycles of a scheduler a (key, item): a byte permute or a logical
+// operation holds its pipe for two cycles and adds to the multiply-adds instead of hiding under them, and a packed f32x2 multiply-add holds its
+// pipe for as long as two plain ones. Four keys a lane, packed multiply-adds, conversion by an integer MMA and persistent CTAs
+// were all written and took 108 to 167 us against 111 here.
+// One sequence of 6003 keys: 98 us in one kernel, here 41 (6, 10.5 and 24 us).
 // Launched back to back with programmatic serialisation but without an early trigger: kernels that let their dependents in
 // before their own wait pile up on the SMs, and a small grid is then placed on the few that have room (one sequence of
 // 6003 keys took 211 us that way).
@@ -957,7 +957,7 @@ int attn_split_kernels(const tenzo_attention_args& a) {
 
 // Against the one kernel of attention.cu, above the 256 keys that attention_short.cu takes: with heads for every SM the three kernels win
 // (12 x 1500: 34 and 50 us; 8 x 128 keys 12.1 and 10.5, not reached), with fewer from about 1000 keys on (one sequence of 1024 keys:
-// 17.5 us against 19, of 512: 15 against 10, of 6003: 47 against 98). max_len is an upper bound that callers round up, so the line lies
+// 17.5 us against 19, of 512: 15 against 10, of 6003: 41 against 98). max_len is an upper bound that callers round up, so the line lies
 // one step further.
 bool attn_split_preferred(const tenzo_attention_args& a) {
     const long long heads = (long long)a.batch * a.n_q;
