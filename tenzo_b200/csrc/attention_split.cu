@@ -955,13 +955,18 @@ int attn_split_kernels(const tenzo_attention_args& a) {
     return 3 * ((a.batch + per_pass - 1) / per_pass);
 }
 
-// Against the one kernel of attention.cu, above the 256 keys that attention_short.cu takes: with heads for every SM the three kernels win
-// (12 x 1500: 34 and 50 us; 8 x 128 keys 12.1 and 10.5, not reached), with fewer from about 1000 keys on (one sequence of 1024 keys:
-// 17.5 us against 19, of 512: 15 against 10, of 6003: 41 against 98). max_len is an upper bound that callers round up, so the line lies
-// one step further.
+// Against the one kernel of attention.cu, above the 256 keys that attention_short.cu takes (us in a graph, one kernel and three). With heads
+// for every SM the three win (12 x 1500: 50 and 34). With fewer the one kernel is a chain as long as the context, the three have
+// their fixed cost: one sequence of 512 keys 10.1 and 11.9, of 640 13.0 and 12.8, of 768 15.1 and 12.6, of 1024 19.2 and 15.3; from block
+// pools, where the one kernel reads through the table key by key, 400 13.4 and 14.5, 512 15.4 and 14.3, 1024 26.0 and 17.0. Above kFewHeads heads the
+// value sums are those for many: 80 heads 1024 keys 20.0 and 20.8, pools 512 15.4 and 15.5, 640 18.6 and 17.5. max_len is an upper bound that
+// callers round up, so each line lies a step further.
 bool attn_split_preferred(const tenzo_attention_args& a) {
     const long long heads = (long long)a.batch * a.n_q;
-    return heads >= 256 || a.max_len > (heads >= 148 ? 256 : 1024);
+    if (heads >= 256) return true;
+    if (heads >= 148) return a.max_len > 256;
+    if (a.block_table) return a.max_len > (heads <= kFewHeads ? 512 : 640);
+    return a.max_len > (heads <= kFewHeads ? 768 : 1024);
 }
 
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st) {

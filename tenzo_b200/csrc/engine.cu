@@ -642,6 +642,7 @@ void Engine::prefill_chunk(const int* tokens, int M) {
 static int bucket_for(int len, int max_seq) {
     int b = 256;
     while (b < len) b <<= 1;
+    if (b == 1024 && len <= 768) b = 768;         // a few sequences change kernels here (attn_split_preferred)
     return b < max_seq ? b : max_seq;
 }
 

@@ -43,3 +43,27 @@ def test_few_heads(cuda_lib, nq, nkv, lens):
         assert np.array_equal(host(out)[b], o), f"sequence {b} (length {lens[b]})"
         o = oracle_paged(O, 0, int(pos[b]), nq, nkv, 1, q[b], k[b], v[b], opk, opv, osk, osv, table[b])
         assert np.array_equal(host(paged)[b], o), f"block pools, sequence {b} (length {lens[b]})"
+
+
+@pytest.mark.parametrize("paged,B,nq,last", [(False, 1, 20, 768), (False, 2, 20, 768), (False, 4, 20, 1024), (True, 1, 20, 512), (True, 4, 20, 640)])
+@pytest.mark.parametrize("over", [0, 1])
+def test_line_between_the_forms(cuda_lib, paged, B, nq, last, over):
+    """Either side of the line between one kernel and three: the bits of the other form."""
+    from tenzo_b200 import kernels
+    nkv, T = 5, last + over
+    ms = (T + 15) // 16 * 16
+    g = torch.Generator(device="cuda").manual_seed(T)
+    shape = (B * ms // 16, 1, nkv, 16, 128) if paged else (B, 1, nkv, ms, 128)
+    ck, cv = (torch.randint(-127, 128, shape, generator=g, device="cuda", dtype=torch.int8) for _ in range(2))
+    sk, sv = (0.01 + 0.02 * torch.rand(shape[:-1], generator=g, device="cuda") for _ in range(2))
+    q = torch.randn(B, nq * 128, generator=g, device="cuda")
+    pos = torch.full((B,), T - 1, dtype=torch.int32, device="cuda")
+    ws = torch.empty(cuda_lib.tenzo_cuda_attention_exact_workspace_bytes(B, nq, nkv, T), dtype=torch.uint8, device="cuda")
+    args = dict(layer=0, n_q=nq, n_kv=nkv, max_seq=ms, max_len=T, append=False)
+    if paged:
+        args.update(block_table=torch.randperm(B * ms // 16, generator=g, device="cuda").int().view(B, -1), n_layers=1)
+    got = kernels.attention_int8(q, None, None, ck, cv, sk, sv, pos, workspace=ws, **args)
+    other = kernels.attention_int8(q, None, None, ck, cv, sk, sv, pos, **(dict(args) if over else dict(args, tiles=3, workspace=ws)))
+    torch.cuda.synchronize()
+    assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
+    assert torch.equal(got, other)
