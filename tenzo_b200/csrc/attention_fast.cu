@@ -171,9 +171,11 @@ __global__ void __launch_bounds__(kFaThreads, 2) attn_fast_kernel(const FaLaunch
     const size_t item = ((size_t)seq * a.n_kv + kvh) * L.n_splits + split;
     float* po = L.part_o + item * G * kHd;
     float* pml = L.part_ml + item * G * 2;
-    if (pos < 0 || pos >= a.max_len || c_begin >= c_end) {                   // nothing here: a neutral partial
-        if (tid < G) { pml[tid * 2] = -INFINITY; pml[tid * 2 + 1] = 0.0f; }
-        for (int i = tid; i < G * kHd; i += kFaThreads) po[i] = 0.0f;
+    if (pos < 0 || pos >= a.max_len || c_begin >= c_end) {                   // nothing here: a neutral partial (one split has none, nor room for it)
+        if (L.n_splits > 1) {
+            if (tid < G) { pml[tid * 2] = -INFINITY; pml[tid * 2 + 1] = 0.0f; }
+            for (int i = tid; i < G * kHd; i += kFaThreads) po[i] = 0.0f;
+        }
         if (pos < 0 || pos >= a.max_len) atomicExch(&g_fa_timeouts, 2);
         return;
     }
@@ -386,9 +388,11 @@ __global__ void __launch_bounds__(kFaThreads, kFbResident) attn_fast_t_kernel(co
     const size_t item = ((size_t)seq * a.n_kv + kvh) * L.n_splits + split;
     float* po = L.part_o + item * G * kHd;
     float* pml = L.part_ml + item * G * 2;
-    if (pos < 0 || pos >= a.max_len || c_begin >= c_end) {                   // nothing here: a neutral partial
-        if (tid < G) { pml[tid * 2] = -INFINITY; pml[tid * 2 + 1] = 0.0f; }
-        for (int i = tid; i < G * kHd; i += kFaThreads) po[i] = 0.0f;
+    if (pos < 0 || pos >= a.max_len || c_begin >= c_end) {                   // nothing here: a neutral partial (one split has none, nor room for it)
+        if (L.n_splits > 1) {
+            if (tid < G) { pml[tid * 2] = -INFINITY; pml[tid * 2 + 1] = 0.0f; }
+            for (int i = tid; i < G * kHd; i += kFaThreads) po[i] = 0.0f;
+        }
         if (pos < 0 || pos >= a.max_len) atomicExch(&g_fa_timeouts, 2);
         return;
     }
