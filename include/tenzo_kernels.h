@@ -164,7 +164,9 @@ typedef struct {
     int mode;
     int split_keys;         /* mode 1: keys per CTA (rounded up to 128); 0 = choose automatically */
     void* workspace;        /* 16-byte aligned, contents need not be kept. Mode 1: tenzo_cuda_attention_workspace_bytes(...)
-                               bytes for the partial results of the splits. Mode 0: optional,
+                               bytes for the partial results of the splits; with less, or NULL, fewer splits are chosen,
+                               down to one that needs none (slower for few sequences of many keys), and split_keys that
+                               need more are refused (-1). Mode 0: optional,
                                tenzo_cuda_attention_exact_workspace_bytes(...) bytes for the score vectors (room for one
                                sequence at least); not used up to max_len 256. NULL keeps them in shared memory, which
                                is slower for all but few sequences of some hundred keys. Same results either way */

@@ -645,11 +645,13 @@ static size_t fa_smem_bytes(int stages) {
 // three rounds count whole, more of them less sharply. At least 256 keys, a multiple of the 128 the four warps take per round.
 // (64 x 8192 keys, 320 items: three splits, as by the rule of about three waves, are 2.2 rounds, four are 2.9.)
 // (2 x 1000 keys, 10 items: four splits of 256, the last one short, 5.7 us; three of 384 6.8.)
-static void fa_pick_split(int batch, int n_kv, int group, int max_len, int* n_splits, int* split_keys) {
+// `most`: as many splits as the caller's workspace holds partial results of, at least the one that needs none.
+static void fa_pick_split(int batch, int n_kv, int group, int max_len, int most, int* n_splits, int* split_keys) {
     const long long items = (long long)batch * n_kv, places = 148 * (group <= 4 ? kFbResident : 2);
     double best = 0.0;
     for (int want = 1; want <= 64 && (want == 1 || (max_len + want - 1) / want > 128); ++want) {       // 129 and more round up to 256
         const int keys = ((max_len + want - 1) / want + 127) / 128 * 128, splits = (max_len + keys - 1) / keys;
+        if (splits > most) continue;
         const long long ctas = items * splits;
         const double rounds = ctas <= 3 * places ? (double)((ctas + places - 1) / places) : (double)ctas / places + 0.5;
         const double cost = rounds * (keys + 500) + 16.0 * (splits - 1);
@@ -704,14 +706,17 @@ int attn_fast_run(const tenzo_attention_args& a, cudaStream_t st) {
     if (L.a.q_stride <= 0) L.a.q_stride = a.n_q * kHd;
     if (L.a.kv_stride <= 0) L.a.kv_stride = a.n_kv * kHd;
     L.group = a.n_q / a.n_kv;
-    fa_pick_split(a.batch, a.n_kv, L.group, a.max_len, &L.n_splits, &L.split_keys);
+    // Splits that the workspace has room for. A choice of the library's own keeps to it; a forced one is refused without.
+    const size_t per_split = (size_t)a.batch * a.n_q * (kHd + 2) * sizeof(float);
+    const size_t room = a.workspace && !(reinterpret_cast<uintptr_t>(a.workspace) & 15) ? a.workspace_bytes / per_split : 0;
     if (a.split_keys > 0) {
         L.split_keys = (a.split_keys + 127) / 128 * 128;
         L.n_splits = (a.max_len + L.split_keys - 1) / L.split_keys;
+        if (L.n_splits > 1 && room < (size_t)L.n_splits) return -1;
+    } else {
+        fa_pick_split(a.batch, a.n_kv, L.group, a.max_len, room > 1 ? (int)(room < 64 ? room : 64) : 1, &L.n_splits, &L.split_keys);
     }
     const size_t items = (size_t)a.batch * a.n_kv * L.n_splits;
-    const size_t need = items * L.group * (kHd + 2) * sizeof(float);
-    if (L.n_splits > 1 && (!a.workspace || a.workspace_bytes < need || (reinterpret_cast<uintptr_t>(a.workspace) & 15))) return -1;
     L.part_o = static_cast<float*>(a.workspace);
     L.part_ml = L.part_o + items * L.group * kHd;
     if (a.append) {

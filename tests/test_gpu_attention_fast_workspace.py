@@ -32,3 +32,25 @@ def test_position_outside_with_one_split(cuda_lib, nq, nkv, room):
         assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 2 and cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
         assert torch.equal(out[0], good[0]) and torch.equal(out[2], good[2]) and bool((out[1] == 7.0).all())
         assert bool((buf == 0x5a).all())
+
+
+@pytest.mark.parametrize("B,nq,nkv,T", [(2, 8, 2, 1000), (3, 16, 2, 2100), (56, 16, 16, 1500)])
+def test_fewer_splits_where_the_workspace_is_short(cuda_lib, B, nq, nkv, T):
+    """Every workspace gives a result, also one just short of another split; splits asked for by the caller still need their room."""
+    from tenzo_b200 import kernels
+    args, kw = setup(B, nq, nkv, T)
+    want = kernels.attention_int8(*args, **kw)
+    split = B * nq * 130 * 4                                # partial results of one split
+    buf = torch.empty(kernels.attention_workspace_bytes(B, nq, nkv, T) + 16, dtype=torch.uint8, device="cuda")
+    for room in (0, 64, split, 2 * split - 1, 2 * split, 3 * split, 4 * split - 4, 8 * split):
+        n = min(room, buf.numel() - 16)
+        buf.fill_(0x5a)
+        got = kernels.attention_int8(*args, **kw, mode=1, workspace=buf[:n])
+        torch.cuda.synchronize()
+        assert bool((buf[n:] == 0x5a).all())
+        assert max(rel_err(host(got[b]), host(want[b])) for b in range(B)) < TOL, f"room {room}"
+    kernels.attention_int8(*args, **kw, mode=1, workspace=buf[8:])                                   # off its alignment: not used
+    with pytest.raises(RuntimeError, match="rc=-1"):
+        kernels.attention_int8(*args, **kw, mode=1, workspace=buf[:split], split_keys=(T + 1) // 2)
+    torch.cuda.synchronize()
+    assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
