@@ -48,7 +48,7 @@ def test_few_heads(cuda_lib, nq, nkv, lens):
 @pytest.mark.parametrize("paged,B,nq,last", [(False, 1, 20, 768), (False, 2, 20, 768), (False, 4, 20, 1024), (True, 1, 20, 512), (True, 4, 20, 640)])
 @pytest.mark.parametrize("over", [0, 1])
 def test_line_between_the_forms(cuda_lib, paged, B, nq, last, over):
-    """Either side of the line between one kernel and three: the bits of the other form."""
+    """Either side of the line between one kernel and three: the three use the workspace, and the bits are the other form's."""
     from tenzo_b200 import kernels
     nkv, T = 5, last + over
     ms = (T + 15) // 16 * 16
@@ -58,12 +58,13 @@ def test_line_between_the_forms(cuda_lib, paged, B, nq, last, over):
     sk, sv = (0.01 + 0.02 * torch.rand(shape[:-1], generator=g, device="cuda") for _ in range(2))
     q = torch.randn(B, nq * 128, generator=g, device="cuda")
     pos = torch.full((B,), T - 1, dtype=torch.int32, device="cuda")
-    ws = torch.empty(cuda_lib.tenzo_cuda_attention_exact_workspace_bytes(B, nq, nkv, T), dtype=torch.uint8, device="cuda")
-    args = dict(layer=0, n_q=nq, n_kv=nkv, max_seq=ms, max_len=T, append=False)
+    ws = torch.full((cuda_lib.tenzo_cuda_attention_exact_workspace_bytes(B, nq, nkv, T),), 0x5a, dtype=torch.uint8, device="cuda")
+    args = dict(layer=0, n_q=nq, n_kv=nkv, max_seq=ms, max_len=T, append=False, workspace=ws)
     if paged:
         args.update(block_table=torch.randperm(B * ms // 16, generator=g, device="cuda").int().view(B, -1), n_layers=1)
-    got = kernels.attention_int8(q, None, None, ck, cv, sk, sv, pos, workspace=ws, **args)
-    other = kernels.attention_int8(q, None, None, ck, cv, sk, sv, pos, **(dict(args) if over else dict(args, tiles=3, workspace=ws)))
+    got = kernels.attention_int8(q, None, None, ck, cv, sk, sv, pos, **args)
+    assert bool((ws != 0x5a).any()) == bool(over)
+    other = kernels.attention_int8(q, None, None, ck, cv, sk, sv, pos, tiles=2 if over else 3, **args)
     torch.cuda.synchronize()
     assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
     assert torch.equal(got, other)
