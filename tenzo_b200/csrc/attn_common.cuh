@@ -122,7 +122,8 @@ __device__ __forceinline__ float sequential_sum(const float* e, int T) {
 }
 
 // e[g][t] = expf(e[g][t] - max[g]) for t < T, by all `n_threads` threads of the CTA (whole warps: the table
-// lookup is a shuffle, so every lane makes every call).
+// lookup is a shuffle, so every lane makes every call). The wide form of the exponential: one sequence of 512 keys 11.70 us
+// with it and 11.76 without, of 768 16.44 and 16.53; block pools of 400 keys 12.52 and 12.51.
 template <int GH>
 __device__ __forceinline__ void exp_in_place(float* e, int T, int tp, const float* mx, int tid, int n_threads) {
     const int lane = tid & 31;
@@ -141,7 +142,7 @@ __device__ __forceinline__ void exp_in_place(float* e, int T, int tp, const floa
                 x[u] = t < T ? row[t] - m : 0.0f;
             }
 #pragma unroll
-            for (int u = 0; u < U; ++u) x[u] = expf_reference_bits_lanes(x[u], tab_lo, tab_hi);
+            for (int u = 0; u < U; ++u) x[u] = expf_reference_bits_lanes<true>(x[u], tab_lo, tab_hi);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int t = base + u * n_threads + tid;
