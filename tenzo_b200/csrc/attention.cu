@@ -650,6 +650,8 @@ extern "C" __attribute__((visibility("default"))) int tenzo_cuda_attention_trace
 }
 #endif
 
+#include "attention_short.cuh"       // exact order, up to 256 keys; sets g_attn_timeouts
+
 namespace tz {
 // tolerance mode (attention_fast.cu)
 bool attn_fast_applicable(const tenzo_attention_args& a);
@@ -661,10 +663,6 @@ bool attn_split_preferred(const tenzo_attention_args& a);
 int attn_split_kernels(const tenzo_attention_args& a);
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st);
 int attn_split_take_timeouts();
-// exact order, up to 256 keys (attention_short.cu)
-bool attn_short_chosen(const tenzo_attention_args& a);
-int attn_short_run(const tenzo_attention_args& a, cudaStream_t st);
-int attn_short_take_errors();
 
 static bool attn_split_chosen(const tenzo_attention_args& a) {
     return a.tiles == 3 || (a.tiles == 0 && a.heads_per_cta == 0 && attn_split_possible(a) && attn_split_preferred(a));
@@ -678,9 +676,7 @@ extern "C" int tenzo_cuda_attention_take_timeouts(void) {
     if (v) cudaMemcpyToSymbol(tz::g_attn_timeouts, &zero, sizeof zero);
     const int f = tz::attn_fast_take_timeouts();
     const int p = tz::attn_split_take_timeouts();
-    const int s = tz::attn_short_take_errors();
-    if (f < 0 || p < 0 || s < 0) return -1;
-    if (s > v) v = s;
+    if (f < 0 || p < 0) return -1;
     return v > f ? (v > p ? v : p) : (f > p ? f : p);
 }
 

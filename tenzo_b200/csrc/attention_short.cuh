@@ -11,6 +11,9 @@
 // for many): one sequence of 64 keys 4.8 -> 3.6, of 211 6.7 -> 5.6; 63 prompt rows 16.6 -> 7.2, 255 44.6 -> 39.1; 12 sequences up to 200 keys
 // 12.6 -> 6.8, 64 up to 256 23.5 -> 19.2, 256 up to 256 54.5 -> 52.5; block pools, 64 up to 200 25.9 -> 18.3. At 256 keys and many items it is
 // bound by its instructions as the three kernels are, and the line lies there.
+// Part of attention.cu, whose error flag it sets: a flag of its own would be one more synchronising copy, 13 us, wherever the flags are
+// read (each greedy call, each step of several sequences).
+#pragma once
 #include <cuda.h>
 
 #include "attn_common.cuh"
@@ -25,8 +28,6 @@ struct ShortLaunch {
     tenzo_attention_args a;
     bool early;                      // position, cache rows and scales are read before the wait for the previous kernel
 };
-
-__device__ int g_short_errors = 0;   // 2: a position outside [0, max_len) was refused
 
 // [K rows][V rows] | exponentials [GH][stride] | weights [keys][GH] | queries [GH][128] | new rows [2][128]
 struct ShortSmem {
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(kShortThreads) attn_short_kernel(const ShortLa
     if (a.use_pdl && !L.early) pdl_wait();
     const int pos = __ldcg(a.pos + seq), T = pos + 1;
     if (pos < 0 || pos >= a.max_len) {
-        if (tid == 0) atomicExch(&g_short_errors, 2);
+        if (tid == 0) atomicExch(&g_attn_timeouts, 2);
         return;
     }
     const size_t base = ((size_t)a.layer * a.n_kv + kvh) * a.max_seq;
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(kShortThreads) attn_short_kernel(const ShortLa
 }
 
 // Up to 256 keys. `tiles` and `heads_per_cta` ask for one of the other forms; the rows go to shared memory in 16-byte pieces.
-bool attn_short_chosen(const tenzo_attention_args& a) {
+static bool attn_short_chosen(const tenzo_attention_args& a) {
     if (a.mode != 0 || a.tiles != 0 || a.heads_per_cta != 0 || a.max_len > kShortKeys) return false;
     if ((reinterpret_cast<uintptr_t>(a.cache_k) & 15) || (reinterpret_cast<uintptr_t>(a.cache_v) & 15)) return false;
     return a.block_table || a.seq_stride_kv % 16 == 0;
@@ -303,7 +304,7 @@ static int short_launch(const ShortLaunch& L, cudaStream_t st) {
     return (int)cudaLaunchKernelEx(&cfg, attn_short_kernel<GH, PAGED>, L);
 }
 
-int attn_short_run(const tenzo_attention_args& a, cudaStream_t st) {
+static int attn_short_run(const tenzo_attention_args& a, cudaStream_t st) {
     ShortLaunch L;
     L.a = a;
     if (L.a.q_stride <= 0) L.a.q_stride = a.n_q * kHd;
@@ -315,13 +316,6 @@ int attn_short_run(const tenzo_attention_args& a, cudaStream_t st) {
     while (gh > 1 && (long long)a.batch * (a.n_q / gh) < 148) gh >>= 1;
     if (a.block_table) return gh == 4 ? short_launch<4, true>(L, st) : gh == 2 ? short_launch<2, true>(L, st) : short_launch<1, true>(L, st);
     return gh == 4 ? short_launch<4, false>(L, st) : gh == 2 ? short_launch<2, false>(L, st) : short_launch<1, false>(L, st);
-}
-
-int attn_short_take_errors() {
-    int v = 0, zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_short_errors, sizeof v) != cudaSuccess) return -1;
-    if (v) cudaMemcpyToSymbol(g_short_errors, &zero, sizeof zero);
-    return v;
 }
 
 }  // namespace tz

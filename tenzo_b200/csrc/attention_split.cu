@@ -955,7 +955,7 @@ int attn_split_kernels(const tenzo_attention_args& a) {
     return 3 * ((a.batch + per_pass - 1) / per_pass);
 }
 
-// Against the one kernel of attention.cu, above the 256 keys that attention_short.cu takes (us in a graph, one kernel and three). With heads
+// Against the one kernel of attention.cu, above the 256 keys that attention_short.cuh takes (us in a graph, one kernel and three). With heads
 // for every SM the three win (12 x 1500: 50 and 34). With fewer the one kernel is a chain as long as the context, the three have
 // their fixed cost: one sequence of 512 keys 10.1 and 11.9, of 640 13.0 and 12.8, of 768 15.1 and 12.6, of 1024 19.2 and 15.3; from block
 // pools, where the one kernel reads through the table key by key, 400 13.4 and 14.5, 512 15.4 and 14.3, 1024 26.0 and 17.0. Above kFewHeads heads the
