@@ -655,6 +655,7 @@ extern "C" __attribute__((visibility("default"))) int tenzo_cuda_attention_trace
 namespace tz {
 // tolerance mode (attention_fast.cu)
 bool attn_fast_applicable(const tenzo_attention_args& a);
+int attn_fast_kernels(const tenzo_attention_args& a);
 int attn_fast_run(const tenzo_attention_args& a, cudaStream_t st);
 int attn_fast_take_timeouts();
 // exact order over the whole machine, with scratch (attention_split.cu)
@@ -667,7 +668,7 @@ int attn_split_take_timeouts();
 static bool attn_split_chosen(const tenzo_attention_args& a) {
     return a.tiles == 3 || (a.tiles == 0 && a.heads_per_cta == 0 && attn_split_possible(a) && attn_split_preferred(a));
 }
-int attn_kernels(const tenzo_attention_args& a) { return a.mode == 1 ? 3 : !attn_short_chosen(a) && attn_split_chosen(a) ? attn_split_kernels(a) : 1; }
+int attn_kernels(const tenzo_attention_args& a) { return a.mode == 1 ? attn_fast_kernels(a) : !attn_short_chosen(a) && attn_split_chosen(a) ? attn_split_kernels(a) : 1; }
 }
 
 extern "C" int tenzo_cuda_attention_take_timeouts(void) {

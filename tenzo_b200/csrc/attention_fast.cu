@@ -700,22 +700,31 @@ bool attn_fast_applicable(const tenzo_attention_args& a) {
     return true;
 }
 
+// The launch's splits, chosen or asked for; false: the workspace has no room for those asked for.
+static bool fa_plan(const tenzo_attention_args& a, int* n_splits, int* split_keys) {
+    const size_t per_split = (size_t)a.batch * a.n_q * (kHd + 2) * sizeof(float);
+    const size_t room = a.workspace && !(reinterpret_cast<uintptr_t>(a.workspace) & 15) ? a.workspace_bytes / per_split : 0;
+    if (a.split_keys > 0) {
+        *split_keys = (a.split_keys + 127) / 128 * 128;
+        *n_splits = (a.max_len + *split_keys - 1) / *split_keys;
+        return *n_splits == 1 || room >= (size_t)*n_splits;
+    }
+    fa_pick_split(a.batch, a.n_kv, a.n_q / a.n_kv, a.max_len, room > 1 ? (int)(room < 64 ? room : 64) : 1, n_splits, split_keys);
+    return true;
+}
+
+int attn_fast_kernels(const tenzo_attention_args& a) {
+    int n_splits, split_keys;
+    return fa_plan(a, &n_splits, &split_keys) ? (a.append ? 1 : 0) + (n_splits > 1 ? 2 : 1) : 0;
+}
+
 int attn_fast_run(const tenzo_attention_args& a, cudaStream_t st) {
     FaLaunch L;
     L.a = a;
     if (L.a.q_stride <= 0) L.a.q_stride = a.n_q * kHd;
     if (L.a.kv_stride <= 0) L.a.kv_stride = a.n_kv * kHd;
     L.group = a.n_q / a.n_kv;
-    // Splits that the workspace has room for. A choice of the library's own keeps to it; a forced one is refused without.
-    const size_t per_split = (size_t)a.batch * a.n_q * (kHd + 2) * sizeof(float);
-    const size_t room = a.workspace && !(reinterpret_cast<uintptr_t>(a.workspace) & 15) ? a.workspace_bytes / per_split : 0;
-    if (a.split_keys > 0) {
-        L.split_keys = (a.split_keys + 127) / 128 * 128;
-        L.n_splits = (a.max_len + L.split_keys - 1) / L.split_keys;
-        if (L.n_splits > 1 && room < (size_t)L.n_splits) return -1;
-    } else {
-        fa_pick_split(a.batch, a.n_kv, L.group, a.max_len, room > 1 ? (int)(room < 64 ? room : 64) : 1, &L.n_splits, &L.split_keys);
-    }
+    if (!fa_plan(a, &L.n_splits, &L.split_keys)) return -1;
     const size_t items = (size_t)a.batch * a.n_kv * L.n_splits;
     L.part_o = static_cast<float*>(a.workspace);
     L.part_ml = L.part_o + items * L.group * kHd;

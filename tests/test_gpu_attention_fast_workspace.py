@@ -54,3 +54,21 @@ def test_fewer_splits_where_the_workspace_is_short(cuda_lib, B, nq, nkv, T):
         kernels.attention_int8(*args, **kw, mode=1, workspace=buf[:split], split_keys=(T + 1) // 2)
     torch.cuda.synchronize()
     assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
+
+
+def test_launches_are_counted(cuda_lib):
+    """A step whose attention is one split launches no merge: a kernel fewer a layer than one with several."""
+    from helpers import synth
+    from tenzo_b200.engine import Engine
+    cfg = dict(hidden_size=512, num_q_heads=4, num_kv_heads=2, head_dim=128, num_layers=3, ffn_dim=1536, vocab_size=4096, max_seq_len=512)
+    m = synth.SyntheticModel(cfg, seed=5)
+    with Engine(m.config_struct(), batch=2, attention_mode=1).load_synthetic(m) as e:
+        e.kv_fill_random(400, seed=1)
+        n = []
+        for length in (100, 400, 100, 400):
+            for s in range(2):
+                e.set_seq_len(s, length)
+            before = e.kernel_launches()
+            e.decode_greedy([1, 2], 1)
+            n.append(e.kernel_launches() - before)
+    assert n[:2] == n[2:] and n[1] - n[0] == cfg["num_layers"]
