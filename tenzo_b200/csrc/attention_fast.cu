@@ -641,20 +641,26 @@ static size_t fa_smem_bytes(int stages) {
 
 // Keys per CTA: the number of splits whose rounds of CTAs (444 places for the kernel with three an SM, 296 for the one with two)
 // take least, at the longest length: a CTA's fixed cost - barriers, query rotation, the first tiles' latency - is worth some 500
-// keys of streaming (32 x 4160: 93 us with 384 keys per CTA, 73 us with 1024), and a split costs the merge about 16. Up to
-// three rounds count whole, more of them less sharply. At least 256 keys, a multiple of the 128 the four warps take per round.
-// (64 x 8192 keys, 320 items: three splits, as by the rule of about three waves, are 2.2 rounds, four are 2.9.)
-// (2 x 1000 keys, 10 items: four splits of 256, the last one short, 5.7 us; three of 384 6.8.)
+// keys of streaming, 600 with eight heads a kv head, and a split costs the merge about 16. Up to three rounds count whole, more
+// of them less sharply. At least 256 keys, a multiple of the 128 the four warps take per round.
+// In a graph, us by the former rule (three waves, 1024 keys at least) and by this one, and of the best split of any number:
+//   20/5 heads   1 x 1000 7.6, 7.6, 7.1   1 x 16384 20.5, 17.1, 16.8   1 x 36864 38.5, 23.6, 22.7   8 x 16384 46.9, 38.0, 38.0
+//                24 x 8192 61.3, 50.6, 50.6   64 x 8192 132.5, 118.7, 118.7
+//   16/8, 16/16  4 x 16000 38.4, 30.0, 30.0   64 x 16384 366, 337, 328   1 x 36864 43.3, 34.5, 34.4   56 x 8192 338, 309, 288
+//   40/5, 8 heads a kv head  1 x 16384 30.4, 22.2, 21.3   1 x 36864 58.1, 31.0, 30.4   12 x 1500 19.2, 16.1, 16.1
+//                24 x 8192 84.4, 67.7, 67.7   64 x 8192 169, 169, 166 (500 for these as well: four splits, 173)
+//   64/8, 32/4   4 x 16000 48.0, 39.5, 39.5   64 x 4096 141, 125, 125   100 x 2500 81.5, 77.9, 77.9   256 x 4096 244, 244, 242
 // `most`: as many splits as the caller's workspace holds partial results of, at least the one that needs none.
 static void fa_pick_split(int batch, int n_kv, int group, int max_len, int most, int* n_splits, int* split_keys) {
     const long long items = (long long)batch * n_kv, places = 148 * (group <= 4 ? kFbResident : 2);
+    const double fixed = group <= 4 ? 500.0 : 600.0;
     double best = 0.0;
     for (int want = 1; want <= 64 && (want == 1 || (max_len + want - 1) / want > 128); ++want) {       // 129 and more round up to 256
         const int keys = ((max_len + want - 1) / want + 127) / 128 * 128, splits = (max_len + keys - 1) / keys;
         if (splits > most) continue;
         const long long ctas = items * splits;
         const double rounds = ctas <= 3 * places ? (double)((ctas + places - 1) / places) : (double)ctas / places + 0.5;
-        const double cost = rounds * (keys + 500) + 16.0 * (splits - 1);
+        const double cost = rounds * (keys + fixed) + 16.0 * (splits - 1);
         if (want == 1 || cost < best) {
             best = cost;
             *split_keys = keys;
