@@ -321,9 +321,9 @@ def attention_roofline(B, ctx, steps, peak, mode=0):
     torch.cuda.empty_cache()
     return {"bound": "hbm", "kernel": "attn_fast_t_kernel (+ append, merge)" if mode == 1 else "split_scores, split_softmax and split_values kernels", "achieved": gbs, "peak": peak[0],
             "peak_source": peak[1], "unit": "GB/s", "frac": gbs / peak[0],
-            "traffic": bytes_per * (297.5 / 259.5) if mode == 0 else bytes_per * (265.6 / 259.5),
-            "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.6 MB read + 5.9 MB written for 259.5 MB algorithmic, scaled by the keys read" if mode == 0 else
-                              "ncu at 24 sequences x 8192 keys: 259.8 MB read + 5.8 MB of partial outputs written for 259.5 MB algorithmic, scaled by the keys read",
+            "traffic": bytes_per * (303.7 / 259.5) if mode == 0 else bytes_per * (346.3 / 343.0),
+            "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.5 MB read + 12.2 MB written for 259.5 MB algorithmic, scaled by the keys read" if mode == 0 else
+                              "ncu of attn_fast_t_kernel at 250 sequences x 1024 keys, one split: 340.5 MB read + 4.9 to 6.7 MB written for 343.0 MB algorithmic, scaled by the keys read",
             "bytes_per_launch": bytes_per, "us_per_launch": ms * 1e3, "launches_timed": steps,
             "l2": f"{bytes_per / 1e6:.0f} MB of KV per launch, larger than L2" if bytes_per > 130e6 else "smaller than L2: an upper bound"}
 

@@ -328,8 +328,8 @@ def run_attn(args):
                    "l2": f"KV {bytes_per / 1e6:.0f} MB per step, larger than L2"},
         "gpu_launches": args.steps,
         "roofline": {"bound": "hbm", "kernel": "split_scores, split_softmax and split_values kernels", "achieved": gbs, "peak": peak[0], "peak_source": peak[1], "unit": "GB/s",
-                     "frac": gbs / peak[0], "traffic": bytes_per * (297.5 / 259.5),
-                     "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.6 MB read + 5.9 MB written for 259.5 MB algorithmic, scaled by the keys read",
+                     "frac": gbs / peak[0], "traffic": bytes_per * (303.7 / 259.5),
+                     "traffic_source": "ncu at 24 sequences x 8192 keys, each kernel cold: 291.5 MB read + 12.2 MB written for 259.5 MB algorithmic, scaled by the keys read",
                      "bytes_per_launch": bytes_per, "us_per_launch": ms * 1e3},
         "tolerance_mode": {"ms_per_step": ms_fast, "achieved": bytes_per / (ms_fast * 1e-3) / 1e9, "unit": "GB/s",
                            "frac": bytes_per / (ms_fast * 1e-3) / 1e9 / peak[0], "kernel": "fa_append_kernel + attn_fast_t_kernel + attn_fast_merge_kernel",
