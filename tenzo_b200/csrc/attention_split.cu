@@ -750,9 +750,11 @@ __device__ __forceinline__ void split_values_light(const SplitLaunch& L, unsigne
     for (int g = 0; g < GV; ++g) out[g * kHd] = acc[g];
 }
 
-// Few heads (one or two sequences): a CTA has one head and 64 dims, a dim a lane and a consumer warp a scheduler, so that a chain runs at
-// the multiply-add's latency: a byte load, a conversion and a quarter of a weight load fit beside it. A batch of eight keys is
+// Few heads (one or two sequences): a CTA has one head and 64 dims, a dim a lane and a consumer warp a scheduler, and beside a chain's
+// multiply-add there is only a byte load, a conversion and a quarter of a weight load a key. A batch of eight keys is
 // summed while the next is converted and the one after that is on its way from shared memory, over the chunks' ends too.
+// 24.2 us for one sequence of 6003 keys and 44.9 for 12000 are 3.5 us and 6.8 cycles a key, where the chain alone would take the
+// multiply-add's 4.6: 3.9 warp instructions a key (producers included), 37 % of the issue slots used, stalls mostly fixed latencies.
 // Chunks of 256 keys: a chunk costs the producer warp some 700 cycles whatever it holds. One sequence of 6003 keys: 30.4 us with V
 // converted to floats by four producer warps (8.8 cycles a key, as long as the producers took), here 33.2 with chunks of 64 keys,
 // 25.7 of 128 and 24.0 of 256; two sequences up to 5000 32.0 -> 20.7.

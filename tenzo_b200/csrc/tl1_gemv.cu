@@ -937,7 +937,7 @@ extern "C" int tenzo_cuda_tl1_gemv_take_repeats(void) {
 extern "C" size_t tenzo_cuda_tl1_gemv_workspace_bytes(int batch, int K) {
     if (batch <= 1 || K <= 0) return 0;
     const size_t nsets = ((size_t)(K >> 1) + 15) / 16;
-    // packed activations (words path) or the plain int8 matrix (tensor-core path), then inv[batch], then sum_a[batch]
+    // packed activations (words path) or the int8 matrix in act_quant_kernel's a_mma order (tensor-core path), then inv[batch], then sum_a[batch]
     const size_t act = (size_t)batch * nsets * 32 > (size_t)batch * K ? (size_t)batch * nsets * 32 : (size_t)batch * K;
     return ((act + 15) & ~(size_t)15) + 2 * (size_t)batch * sizeof(float) + 64;
 }
