@@ -84,7 +84,7 @@ EXT_SYMBOLS = [
 ]
 KERNEL_SYMBOLS = [
     "tenzo_cuda_tl1_gemv", "tenzo_cuda_tl1_gemv_ksplit", "tenzo_cuda_tl1_gemm_ksplit", "tenzo_cuda_tl1_gemm_layout", "tenzo_cuda_tl1_gemv_workspace_bytes", "tenzo_cuda_tl1_gemv_take_timeouts", "tenzo_cuda_tl1_gemv_take_repeats", "tenzo_cuda_selftest_wait_expiry", "tenzo_cuda_rmsnorm_quant", "tenzo_cuda_attention_int8",
-    "tenzo_cuda_attention_heads_per_cta", "tenzo_cuda_attention_take_timeouts", "tenzo_cuda_attention_workspace_bytes", "tenzo_cuda_attention_exact_workspace_bytes", "tenzo_cuda_lm_head_i8", "tenzo_cuda_lm_head_scratch_bytes",
+    "tenzo_cuda_attention_heads_per_cta", "tenzo_cuda_attention_take_timeouts", "tenzo_cuda_attention_workspace_bytes", "tenzo_cuda_attention_exact_workspace_bytes", "tenzo_cuda_attention_rows_workspace_bytes", "tenzo_cuda_lm_head_i8", "tenzo_cuda_lm_head_scratch_bytes",
     "tenzo_cuda_embedding_i8", "tenzo_cuda_tl1_pack_rows2bit", "tenzo_cuda_lm_head_i8_static",
     "tenzo_cuda_lm_head_static_max_batch", "tenzo_cuda_lm_head_take_timeouts", "tenzo_cuda_repetition_penalty",
     "tenzo_cuda_topk_candidates", "tenzo_cuda_topk_max_candidates",
@@ -164,6 +164,7 @@ def declare_kernel_abi(L):
     L.tenzo_cuda_attention_take_timeouts.restype, L.tenzo_cuda_attention_take_timeouts.argtypes = i32, []
     L.tenzo_cuda_attention_heads_per_cta.restype, L.tenzo_cuda_attention_heads_per_cta.argtypes = i32, [i32, i32, i32, i32]
     L.tenzo_cuda_attention_exact_workspace_bytes.restype = L.tenzo_cuda_attention_workspace_bytes.restype = sz
+    L.tenzo_cuda_attention_rows_workspace_bytes.restype, L.tenzo_cuda_attention_rows_workspace_bytes.argtypes = sz, [i32, i32, i32, i32]
     L.tenzo_cuda_attention_exact_workspace_bytes.argtypes = L.tenzo_cuda_attention_workspace_bytes.argtypes = [i32, i32, i32, i32]
     L.tenzo_cuda_lm_head_i8.restype = i32
     L.tenzo_cuda_lm_head_i8.argtypes = [vp, vp, i32, f32, vp, vp, i32, i32, i32, i32, vp, vp, vp, vp, i32, vp]

@@ -905,6 +905,10 @@ static int heavy_items(long long items) {
     return (int)(rest <= (items < 296 ? 70 : 100) ? items - rest : items);
 }
 
+}  // namespace tz
+#include "attention_rows.cuh"        // many query rows over one cache
+namespace tz {
+
 template <int GH, bool PAGED>
 static cudaError_t launch_values(const SplitLaunch& L, int items, cudaStream_t st) {
     if (items * GH <= kFewHeads) {
@@ -953,6 +957,7 @@ static int split_rows_per_pass(const tenzo_attention_args& a) {
 }
 
 int attn_split_kernels(const tenzo_attention_args& a) {
+    if (const int rows = attn_rows_per_pass(a)) return 4 * ((a.batch + rows - 1) / rows);
     const int per_pass = split_rows_per_pass(a);
     return 3 * ((a.batch + per_pass - 1) / per_pass);
 }
@@ -972,6 +977,7 @@ bool attn_split_preferred(const tenzo_attention_args& a) {
 }
 
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st) {
+    if (const int rows = attn_rows_per_pass(a)) return attn_rows_run(a, rows, st);
     SplitLaunch L;
     L.a = a;
     if (L.a.q_stride <= 0) L.a.q_stride = a.n_q * kHd;
@@ -1012,6 +1018,12 @@ int attn_split_take_timeouts() {
 }
 
 }  // namespace tz
+
+extern "C" size_t tenzo_cuda_attention_rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
+    if (batch <= 0 || n_q <= 0 || n_kv <= 0 || n_q % n_kv || n_q / n_kv > 8 || max_len <= 0) return 0;
+    const size_t split = tz::attn_split_workspace_bytes(batch, n_q, max_len), rows = tz::rows_workspace_bytes(batch, n_q, n_kv, max_len);
+    return split > rows ? split : rows;
+}
 
 extern "C" size_t tenzo_cuda_attention_exact_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
     if (batch <= 0 || n_q <= 0 || n_kv <= 0 || n_q % n_kv || max_len <= 0) return 0;

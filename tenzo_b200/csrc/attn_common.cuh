@@ -15,6 +15,39 @@ __device__ __forceinline__ float s8_to_f(uint32_t word_xor80, int byte) {
     return __uint_as_float(prmt(word_xor80, 0x4B000000u, sel)) - 8388736.0f;
 }
 
+// Two floats side by side and their packed operations, each half rounded as the plain operation rounds it. A packed multiply-add
+// holds its pipe for 2.3 cycles, two plain ones for 3.1 (loops of independent accumulators, four warps a scheduler).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
+// The four signed bytes of a word as floats: byte b of the lower half is masked, its sign bit turned over and a float's exponent put
+// around it, one logical operation, so that the float reads 2^23 + 128 + b (bits 0-7) or 2^15 + 128 + b (bits 8-15); the upper
+// half by way of a shift. (A byte permute takes the pipe of logical operations twice as long.) The exponents are kept where
+// the compiler does not see them as constants: with two constants it makes two operations of one.
+struct ByteFloats {
+    uint32_t m0, m1;
+    f32x2 off;
+    __device__ __forceinline__ ByteFloats() {
+        asm volatile("mov.u32 %0, 0x4B000080;" : "=r"(m0));
+        asm volatile("mov.u32 %0, 0x47008000;" : "=r"(m1));
+        off = pack2(-8388736.0f, -32896.0f);
+    }
+    template <uint32_t MASK>
+    static __device__ __forceinline__ float masked(uint32_t v, uint32_t m) {
+        uint32_t r;
+        asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(r) : "r"(v), "n"(MASK), "r"(m));       // (v & MASK) ^ m
+        return __uint_as_float(r);
+    }
+    __device__ __forceinline__ void pairs(uint32_t v, f32x2& lo, f32x2& hi) const {
+        const uint32_t u = v >> 16;
+        lo = add2(pack2(masked<0xffu>(v, m0), masked<0xff00u>(v, m1)), off);
+        hi = add2(pack2(masked<0xffu>(u, m0), masked<0xff00u>(u, m1)), off);
+    }
+};
+
 __device__ __forceinline__ void rope_pair(float x0, float x1, const float* cs, const float* sn, int i, float& r0, float& r1) {
     r0 = x0;
     r1 = x1;
