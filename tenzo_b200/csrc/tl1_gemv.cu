@@ -409,7 +409,11 @@ __global__ void __launch_bounds__((FUSED ? kFusedWarps : kBatchedWarps) * 32, FU
 // The chain warp is warp 0: the scheduler prefers it.
 // What bounds it: latency. Of the 2.9 us of a K = 2560 product 0.5 us are the load of x, 0.2 the maximum, 0.6 the quantiser, 0.7
 // the product, 0.8 the rest of the chain and the check. In a decode step (launches overlapped) 3840 x 2560 4.8 -> 4.3 us,
-// 2560 x 2560 4.9 -> 3.9, gate|up 13824 x 2560 6.1 -> 5.2, 2560 x 6912 8.8 -> 7.2, against the kernel above.
+// 2560 x 2560 4.9 -> 3.9, gate|up 13824 x 2560 6.1 -> 5.2, 2560 x 6912 8.8 -> 7.2, against the kernel above. Then three
+// waits less, 24.51 -> 24.02 ms for 32 tokens of a 2B-shaped model: the presumed maximum's element is handed over in shared memory (it
+// was read again from L2, and 300 to 1000 cycles of every product waited for that: 24.31), the chain's loads run a batch ahead of its
+// additions (24.10), and one block's MMAs go to two sums in turn. In cycles after the wait, 2560 x 2560: 960 for x and its squares, 700
+// quantiser, 240 barrier and weights, 1600 product, 700 check, 600 scale and store.
 constexpr int kOneWorkers = kFusedWarps * 32, kOneThreads = kOneWorkers + 32;
 constexpr int kOneMaxK = 8192;
 
@@ -437,7 +441,7 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
     int* s_d = reinterpret_cast<int*>(smem);                         // [nb_cta][kRows] accumulators: low-nibble rows x4, high-nibble rows x64
     float* s_f = reinterpret_cast<float*>(smem + 128);               // [0,16) maxima, 32: 1/rms
     int* s_sa = reinterpret_cast<int*>(s_f + 36);                    // sum of the activations
-    int* s_top = s_sa + 1;                                           // element of the presumed maximum
+    unsigned long long* s_top = reinterpret_cast<unsigned long long*>(s_f + 38);   // x and its weight where x * w is largest (one 64-bit word: stores of equal ones do not mix)
     uint32_t* s_b = smem + OneSmem::head_words;                      // [sets][8]: word c of set b holds activations 32 b + c + 8 j as bytes j, even c times 4
     float* s_sq = reinterpret_cast<float*>(s_b + (a.K >> 2));        // [8][stride]
     const int stride = OneSmem::stride(a.K), n_pieces = a.K >> 2, kh = a.K >> 1, n_sets = a.K >> 5;
@@ -452,28 +456,9 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
         if (a.use_pdl) pdl_wait();
         if (!a.do_norm) return;
         named_barrier_sync(3, kOneThreads);                          // the squares are in place
-        float sum = 0.0f;
-        if (lane < 8) {
-            const float4* p = reinterpret_cast<const float4*>(s_sq + lane * stride);
-            const int n4 = a.K >> 5;
-            auto add4 = [&](const float4& v) {
-                sum = __fadd_rn(sum, v.x);
-                sum = __fadd_rn(sum, v.y);
-                sum = __fadd_rn(sum, v.z);
-                sum = __fadd_rn(sum, v.w);
-            };
-            int j = 0;
-#pragma unroll 1
-            for (; j + 8 <= n4; j += 8) {                            // eight loads, then their 32 additions
-                float4 v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = p[j + u];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) add4(v[u]);
-            }
-#pragma unroll 1
-            for (; j < n4; ++j) add4(p[j]);
-        }
+        // The fixed cost of every faster form is more than it saves here: 320 additions are 1666 cycles (864: 3900); sixteen segments of
+        // the chains by eight warps, walked from presumed sums and joined, 2270 (2840), five parts by three warps 1930 (3250).
+        const float sum = lane < 8 ? sequential_sum(s_sq + lane * stride, a.K >> 3) : 0.0f;
         float ss = __shfl_sync(0xffffffffu, sum, 0);
 #pragma unroll
         for (int j = 1; j < 8; ++j) ss = __fadd_rn(ss, __shfl_sync(0xffffffffu, sum, j));      // the eight lanes left to right (common.cuh)
@@ -494,7 +479,10 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
     asm volatile("cp.async.commit_group;" ::: "memory");
     l2_prefetch_workers(a.prefetch, a.prefetch_bytes, tid, kOneWorkers);
     if (tid < 128) s_d[tid] = 0;
-    if (tid == 0) *s_sa = *s_top = 0;
+    if (tid == 0) {
+        *s_sa = 0;
+        *s_top = 0x7fffffffull;                                      // no number, if no element is one
+    }
     const bool has_w = a.do_norm && a.norm_w;
     constexpr bool kKeep = P <= 2;                                   // w and the result stay in registers for the check, else they are read again
     // Pieces beyond the vector read its first one: a load under a condition would be waited for before the next.
@@ -618,7 +606,7 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
                 if (tid + j * kOneWorkers < n_pieces)
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        if (fabsf(z(j, k)) == m) *s_top = 4 * (tid + j * kOneWorkers) + k;
+                        if (fabsf(z(j, k)) == m) *s_top = (unsigned long long)__float_as_uint(wr[j][k]) << 32 | __float_as_uint(xr[j][k]);
         }
         forget();
         const float to_q = __fdividef(31.0f, fmaxf(m, 1e-30f));
@@ -655,11 +643,6 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
 #pragma unroll 1
     for (;;) {
         named_barrier_sync(1, kOneWorkers);                          // packed words and weights are in place
-        float top_x = 0.0f, top_w = 1.0f;
-        if (!checked) {
-            top_x = __ldcg(a.x + *s_top);
-            if (has_w) top_w = __ldg(a.norm_w + *s_top);
-        }
         int acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
         auto product = [&](auto blocks) {
             constexpr int NB = decltype(blocks)::value;
@@ -684,13 +667,16 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
 #pragma unroll
                     for (int bk = 0; bk < NB; ++bk) {
                         const uint32_t w = W[bk][i];
-                        mma_u8s8(acc[bk], w & 0x03030303u, w & 0x30303030u, w & 0x0C0C0C0Cu, w & 0xC0C0C0C0u, be, bo);
+                        mma_u8s8(acc[NB == 1 ? i & 1 : bk], w & 0x03030303u, w & 0x30303030u, w & 0x0C0C0C0Cu, w & 0xC0C0C0C0u, be, bo);
                     }
                 }
             }
         };
         if (glu) product(std::integral_constant<int, 2>{});
         else product(std::integral_constant<int, 1>{});
+        if (!glu)                                                    // (of one block: two sums, for MMAs that do not wait for the one before)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[0][e] += acc[1][e];
         // D: rows g (low nibbles) and g + 8 (high ones), columns 2 t4, 2 t4 + 1: byte rows 4 g + column; of halves, columns 4-7
         // belong to the words of lanes g >= 4 and the other columns to those below. The warps meet.
         if (HB == 2 ? t4 < 2 : (t4 >> 1) == (g >> 2)) {
@@ -714,7 +700,8 @@ __global__ void __launch_bounds__(kOneThreads, 2) tl1_one_kernel(const GemvLaunc
             for (int j = 0; j < P; ++j) load_w(j, wr[j]);
         named_barrier_sync(4, kOneThreads);
         float inv_rms = s_f[32];
-        const float m_top = fabsf(normed(top_x, inv_rms, top_w)), to_q = 31.0f / fmaxf(m_top, 1e-6f);
+        const unsigned long long top = *s_top;
+        const float m_top = fabsf(normed(__uint_as_float((uint32_t)top), inv_rms, __uint_as_float((uint32_t)(top >> 32)))), to_q = 31.0f / fmaxf(m_top, 1e-6f);
         bool good = true;
 #pragma unroll
         for (int j = 0; j < P; ++j)
