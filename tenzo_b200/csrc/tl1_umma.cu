@@ -11,18 +11,18 @@
 //
 // One CTA per 128-row tile (two 64-row TL1 blocks; for the GLU epilogue the gate block and its up block, so the
 // activation is applied inside the CTA). K is walked in 128-byte chunks through two rings, 8 or 12 slots of codes in tensor
-// memory and 4, 8 or 12 activation tiles in shared memory (multiples of four: see UmmaSmem::a_slots_for); 21 warps per CTA:
+// memory and 4 or 12 activation tiles in shared memory (multiples of four: see UmmaSmem::a_slots_for); 21 warps per CTA:
 //   warp 0 (lane 0)     bulk-copies the packed 2-bit weights eight chunks at a time (2 x 16 KB) into a ring of two or
 //                       three groups; the first groups are requested by one lane each first thing in the kernel
 //                       (weights depend on no earlier kernel); lanes 1-31 fetch the per-sequence scale and sum for
 //                       the epilogue;
 //   warps 2-17          (four groups of four; group g takes chunks g, g + 4, ..., two per iteration when there are
-//                       eight or more slots) expand the 2-bit codes to bytes in registers and write them straight into
+//                       twelve activation tiles) expand the 2-bit codes to bytes in registers and write them straight into
 //                       the slot's 32 columns of tensor memory (tcgen05.st 16x256b: no shared-memory A tile, no
 //                       proxy fence). Lane quarter q of a group takes one nibble half of one row block; a thread's
 //                       four TMEM lanes are the four rows of ONE packed word, so a thread loads sixteen words per
 //                       chunk and every byte of them is used. The row order inside a quarter is therefore permuted
-//                       (TMEM lane l holds row 4*(l&7) + (l>>3)); the epilogue undoes it. Up to 144 sequences there are as
+//                       (TMEM lane l holds row 4*(l&7) + (l>>3)); the epilogue undoes it. Up to 96 sequences there are as
 //                       many activation slots as code slots, and the warps of a group take turns TMA-loading the chunk's
 //                       activation tile [N][128 B] (128-byte swizzle) right after they have seen the slot free;
 //   warps 1, 18-20      (lane 0 each) take every fourth chunk: one poll of the slot's barrier (expand arrivals + the
@@ -31,8 +31,8 @@
 //                       another 270 (measured), more than the MMAs of a chunk take below 256 sequences, so one
 //                       issuing thread bounds the loop; four hide it. Integer accumulation is order-free, and the
 //                       expanding warps zero the accumulators while they wait for weights, so the threads need no
-//                       order among them (when chunk 0 had to overwrite them first, the others lost 850 cycles). From 145
-//                       sequences on only four activation tiles fit. With one ring for both, codes and MMAs then took
+//                       order among them (when chunk 0 had to overwrite them first, the others lost 850 cycles). From 97
+//                       sequences on there are four activation tiles only. With one ring for both, codes and MMAs then took
 //                       turns (900 cycles a chunk for 516 of math); now the codes run eight chunks ahead, and each issuing
 //                       thread requests the next tile of its own slot as soon as its MMAs have completed (one thread that
 //                       requested all of them was the slowest role, 970 cycles a chunk): 640 cycles a chunk.
@@ -40,7 +40,8 @@
 // warps (the groups on alternate 32-sequence column units; TMEM lane = weight row, tcgen05.ld 16 sequences at a
 // time, scale / residual / ReLU^2*GLU, the unit assembled in shared memory and sent off by its own TMA store while
 // the next one is computed).
-// Few row tiles (the out, down and q|k|v projections have 20 to 30) would leave most SMs idle, so K is then split
+// Few row tiles (the out, down and q|k|v projections have 20 to 30) would leave most SMs idle, so many sequences are then spread over
+// several CTAs a row tile, or K is split (pick_umma_shape)
 // across the 2, 4 or 8 CTAs of a thread-block cluster: each accumulates its share of the chunks in its own tensor
 // memory and parks its int32 partial tile in shared memory; after a hardware cluster barrier every CTA takes the
 // units of four sequences u = rank, rank + ksplit, ..., adds its peers' partials for them through distributed
@@ -65,7 +66,7 @@ constexpr int kUmmaThreads = 32 * (2 + 4 * kExpandGroups + 3);   // warp 0 produ
 // 11.9 for 2560 x 6912; here 8.9 and 13.2), with more it takes four (21 and 25 us; here 9.0 and 13.5).
 constexpr int kUmmaMinBatch = 9;
 constexpr int kMmaThreads = 4;
-constexpr int kMaxSlots = 16;                  // ring of chunk slots: as many as tensor memory and shared memory allow (4 at 256 sequences, 12 at 64)
+constexpr int kMaxSlots = 16;                  // ring of chunk slots: as many as tensor memory and shared memory allow
 constexpr int kPGroup = 8;                     // chunks of packed weights per bulk copy (16 KB per row block)
 constexpr int kMaxPGroups = 3;                 // such groups in the ring (3 up to 64 sequences, else 2): 64 KB of packed weights in flight behind the group in use
 constexpr int kKc = 128;                       // bytes of K per chunk (one swizzle atom row)
@@ -80,7 +81,7 @@ struct UmmaLaunch {
     const float* inv;        // [batch] m/31
     const int* sum_a;        // [batch] sum_k a_k
     int units;               // tiles along the rows
-    int n_box;               // sequences per CTA, padded to a multiple of 16 (<= 256)
+    int n_box;               // sequences per CTA, a multiple of 16 (<= 256)
     int n_slots;             // ring slots (A in tensor memory)
     int b_slots;             // activation tiles in shared memory: as many, or four (then the issuing threads request them)
     int n_pgroups;           // groups of kPGroup chunks in the packed-weight ring
@@ -134,9 +135,12 @@ struct UmmaSmem {
         const int r = (kTmemCols - tmem_a(n_box)) / 32;
         return (r < kMaxSlots ? r : kMaxSlots) & ~3;
     }
-    static __host__ __device__ int b_slots_for(int n_box) {                                  // by shared memory: 12 up to 96 sequences, 4 from 145 on
-        const int r = (kSmemBudget - pgroups_for(n_box) * kPGroup * kPBytes) / (n_box * kKc), a = a_slots_for(n_box);
-        return (r < a ? r : a) & ~3;
+    // By shared memory: 12 or more up to 96 sequences, else 4. Eight, which would fit up to 144, are one iteration of all expanding warps: with four
+    // the codes run ahead of the tiles instead (28672 x 4096 with GLU at 128 sequences 30.7 -> 28.4 us, 2560 x 6912 24.0 -> 22.4; at 96, from twelve
+    // to four, 25.6 -> 26.8).
+    static __host__ __device__ int b_slots_for(int n_box) {
+        const int r = (kSmemBudget - pgroups_for(n_box) * kPGroup * kPBytes) / (n_box * kKc), a = a_slots_for(n_box), b = (r < a ? r : a) & ~3;
+        return b < 12 ? 4 : b;
     }
     static constexpr int n_bars = 2 * kMaxSlots + 2 * kMaxPGroups + 3;
     static __host__ __device__ size_t bytes(int n_box) {
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
     UCHK(reinterpret_cast<const unsigned char*>(s_sum + kMaxN) <= smem_end, 7, reinterpret_cast<const unsigned char*>(s_sum + kMaxN) - smem_raw, dyn_bytes);
 #endif
     constexpr bool glu = EPI == TENZO_EPI_RELU2_GLU;
-    const int tile = blockIdx.x, seq0 = blockIdx.y * kMaxN;
+    const int tile = blockIdx.x, seq0 = blockIdx.y * L.n_box;
     const int blk0 = glu ? tile : 2 * tile;
     const int blk1 = glu ? tile + L.units : (2 * tile + 1 < a.n_blocks ? 2 * tile + 1 : -1);
     const int ksplit = CLUSTER ? L.ksplit : 1;
@@ -488,8 +492,9 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
                 for (int i = 0; i < 16; ++i) r[i] = 0u;
                 if (ok) tmem_ld16(tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)c0, r);
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if ((((c0 + i) >> 2) & (ksplit - 1)) != split) s_part[(c0 + i) * 128 + m] = (int)r[i];      // (this CTA's own units stay in tensor memory)
+                for (int i = 0; i < 16; i += 4)
+                    if ((((c0 + i) >> 2) & (ksplit - 1)) != split)                                              // (this CTA's own units stay in tensor memory)
+                        *reinterpret_cast<uint4*>(s_part + (c0 + i) * 128 + 4 * m) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
             }
         }
     }
@@ -553,18 +558,15 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
                 }
                 if (CLUSTER) {
                     // the peers' partials over distributed shared memory, every load issued before the first is used
-                    uint32_t part[8][4];
+                    uint4 part[8];
 #pragma unroll
                     for (int p = 0; p < 8; ++p) {
                         const bool use_p = p < ksplit && p != split;
                         const int* peer = cg::this_cluster().map_shared_rank(reinterpret_cast<int*>(ring), use_p ? p : split);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) part[p][i] = use_p ? (uint32_t)peer[(c0 + i) * 128 + m] : 0u;
+                        part[p] = use_p ? *reinterpret_cast<const uint4*>(peer + c0 * 128 + 4 * m) : make_uint4(0u, 0u, 0u, 0u);
                     }
 #pragma unroll
-                    for (int p = 0; p < 8; ++p)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) r[i] += part[p][i];
+                    for (int p = 0; p < 8; ++p) { r[0] += part[p].x; r[1] += part[p].y; r[2] += part[p].z; r[3] += part[p].w; }
                 }
                 float* unit_out = s_out + (size_t)4 * k * row_floats;
                 float* unit_glu = s_glu + (size_t)4 * k * 64;
@@ -618,9 +620,19 @@ bool tl1_umma_applicable(const tenzo_tl1_gemv_args& a) {
     return a.batch >= kUmmaMinBatch && a.K % kKc == 0 && a.K >= kKc && a.out_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
-// CTAs of a cluster that split one tile's K range: doubled while the grid still fits the SMs (one CTA per SM) and
-// every CTA keeps at least four 128-byte chunks. TENZO_UMMA_KSPLIT = 1, 2, 4 or 8 overrides the choice (measurement aid).
-static int pick_umma_ksplit(int ctas, int n_chunks) {
+// Sequences a CTA holds (a multiple of 16) and CTAs of a cluster that split one tile's K range. Fewer sequences a CTA use SMs that
+// few row tiles leave idle as a split of K does, for the expansion of the weights once more a tile of sequences but without an exchange: a
+// cluster's partial tiles move at some 14 bytes a cycle and SM (2560 x 2560 at 256 sequences over clusters of four: 98 KB into each
+// CTA, 6900 cycles of 21000). The candidates' costs are compared in units of 10 ns: a CTA's start, its chunks, its
+// sequences' epilogue, the exchange; rounds of CTAs, which overlap in part; and launching them. Clusters that do not fit the
+// SMs at once (GPCs hold whole ones only) are a round more. The constants were fitted to 1049 timed pairs of quantiser and product, 16 to 1536
+// sequences, 12 matrices: the choice is 0.6 % from the best of a size on average, and on none slower than what was taken before (up to
+// 256 sequences a CTA and as large a cluster as the SMs hold). In us, before and now: 3840 x 2560 at 96 sequences 10.8 and 9.1, 256 14.8 and
+// 11.8, 384 17.2 and 12.6; 2560 x 2560 at 256 15.2 and 12.2, 512 21.0 and 15.8; 2560 x 6912 at 256 20.5 and 18.5; 13824 x 2560 GLU at 384
+// 29.7 and 26.1; 4096 x 14336 at 320 46.6 and 41.4. Up to 64 sequences a CTA holds them all and the cluster is as large as the SMs allow,
+// the best within 3 % but for 3840 x 2560 at 64 (9.1; 8.6 in two tiles of sequences). TENZO_UMMA_KSPLIT = 1, 2, 4 or 8 overrides the cluster's size (measurement aid).
+struct UmmaShape { int n_box, ksplit; };
+static UmmaShape pick_umma_shape(int units, int n_chunks, int batch, int epilogue) {
     static const int forced = [] {
         const char* e = std::getenv("TENZO_UMMA_KSPLIT");
         const int v = e ? std::atoi(e) : 0;
@@ -630,10 +642,34 @@ static int pick_umma_ksplit(int ctas, int n_chunks) {
         int dev = 0, n = 0;
         return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && n > 0 ? n : 148;
     }();
-    if (forced) return forced <= n_chunks ? forced : 1;
-    int k = 1;
-    while (k < 8 && ctas * k * 2 <= n_sm && n_chunks / (k * 2) >= 4) k *= 2;
-    return k;
+    if (batch <= 64) {                                       // one CTA, or the largest cluster that fits
+        UmmaShape one = {(batch + 15) & ~15, 1};
+        if (forced) one.ksplit = forced <= n_chunks ? forced : 1;
+        else while (one.ksplit < 8 && units * one.ksplit * 2 <= n_sm && n_chunks / (one.ksplit * 2) >= 4) one.ksplit *= 2;
+        return one;
+    }
+    UmmaShape best = {0, 1};
+    float best_cost = 0.0f;
+    for (int tiles = (batch + kMaxN - 1) / kMaxN, last = 0;; ++tiles) {
+        int n = ((batch + tiles - 1) / tiles + 15) & ~15;
+        // (tiles of 240 are stored in units of 16 sequences; 14208 x 5760 with a residual at 466 sequences 65.5 us, in tiles of 256 62.8, plain ones 46.2 and 48.1)
+        if (n == 240 && tiles > 1 && epilogue != TENZO_EPI_STORE) n = kMaxN;
+        if (n < 32) break;
+        if (n == last) continue;
+        last = n;
+        const long long ctas = (long long)units * ((batch + n - 1) / n);
+        for (int k = 1; k <= 8; k *= 2) {
+            if (forced ? k != (forced <= n_chunks ? forced : 1) : k > 1 && (n_chunks / k < 4 || ctas * k > n_sm)) continue;
+            const int fit = k == 8 ? n_sm - n_sm * 3 / 16 : k == 4 ? n_sm - n_sm / 9 : n_sm;
+            const float rounds = (float)((ctas * k + fit - 1) / fit);
+            const float one = 88.0f + 26.0f * (float)((n_chunks + k - 1) / k) + 3.62f * (float)n +
+                              (k > 1 ? 156.0f + 0.55f * (float)(n * (k - 1)) / (float)k : 0.0f) + (k == 8 ? 38.0f : 0.0f);
+            const float cost = (0.41f + 0.59f * rounds) * one + 1.61f * (float)(ctas * k);
+            if (!best.n_box || cost < best_cost) { best = {n, k}; best_cost = cost; }
+        }
+        if (n <= 32) break;
+    }
+    return best;
 }
 
 // a8 [batch][K] int8 in the order of act_quant_kernel's a_mma (16-byte aligned), inv [batch], sum_a [batch] already produced on `st`.
@@ -644,15 +680,16 @@ int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float*
     L.sum_a = sum_a;
     const bool glu = a.epilogue == TENZO_EPI_RELU2_GLU;
     L.units = glu ? a.n_blocks / 2 : (a.n_blocks + 1) / 2;
-    const int per_cta = a.batch < kMaxN ? a.batch : kMaxN;
-    L.n_box = (per_cta + 15) & ~15;
+    const UmmaShape shape = pick_umma_shape(L.units, a.K / kKc, a.batch, a.epilogue);
+    L.n_box = shape.n_box;
+    L.ksplit = shape.ksplit;
     L.n_slots = UmmaSmem::a_slots_for(L.n_box);
     L.b_slots = UmmaSmem::b_slots_for(L.n_box);
-    if (L.b_slots >= 8) L.n_slots = L.b_slots;                     // (enough of them: requested by the warps that expand the codes, two chunks at a time)
+    if (L.b_slots > 4) L.n_slots = L.b_slots;                      // (enough of them: requested by the warps that expand the codes, two chunks at a time)
     L.n_pgroups = UmmaSmem::pgroups_for(L.n_box);
-    const int seq_tiles = (a.batch + kMaxN - 1) / kMaxN;
-    L.ksplit = pick_umma_ksplit(L.units * seq_tiles, a.K / kKc);
-    L.store_cols = L.ksplit > 1 || L.n_box <= 32 ? 4 : L.n_box <= 64 ? 16 : 32;
+    const int seq_tiles = (a.batch + L.n_box - 1) / L.n_box;
+    // (A store is not to reach into the next tile's sequences.)
+    L.store_cols = L.ksplit > 1 || L.n_box <= 32 ? 4 : L.n_box <= 64 || (seq_tiles > 1 && (L.n_box & 31)) ? 16 : 32;
     CUtensorMap amap, omap;
     // activations [batch][K] int8: B-operand tiles {128 bytes of K, n_box sequences}, 128-byte swizzle
     if (int rc = encode_2d(&amap, CU_TENSOR_MAP_DATA_TYPE_UINT8, a8, (uint64_t)a.K, (uint64_t)a.batch, (uint64_t)a.K, kKc, (uint32_t)L.n_box,
@@ -733,5 +770,5 @@ extern "C" int tenzo_cuda_tl1_gemm_layout(int batch, int* slots, int* weight_gro
 extern "C" int tenzo_cuda_tl1_gemm_ksplit(int n_blocks, int K, int batch, int epilogue) {
     if (n_blocks <= 0 || K < tz::kKc || K % tz::kKc || batch < tz::kUmmaMinBatch) return 0;       // the tensor-core path does not apply
     const int units = epilogue == TENZO_EPI_RELU2_GLU ? n_blocks / 2 : (n_blocks + 1) / 2;
-    return tz::pick_umma_ksplit(units * ((batch + tz::kMaxN - 1) / tz::kMaxN), K / tz::kKc);
+    return tz::pick_umma_shape(units, K / tz::kKc, batch, epilogue).ksplit;
 }

@@ -56,3 +56,24 @@ def test_many_rows_quantiser(cuda_lib, K, batch):
     for b in (0, 1, batch // 2, batch - 1):
         want_out, want_acc, _ = cpu_bitlinear(cpu_rms_norm(x[b], nw), w, N, K, 0.016)
         assert np.array_equal(host(r["acc"])[b], want_acc) and np.array_equal(host(r["out"])[b], want_out), f"sequence {b}"
+
+
+@pytest.mark.parametrize("N,K,B", [(2560, 2560, 65), (2560, 2560, 97), (3840, 2560, 129), (3840, 2560, 257), (640, 5120, 161), (2560, 1280, 337),
+                                   (640, 2560, 513), (13824, 384, 385), (1344, 2560, 305), (3840, 1280, 1537)])
+def test_tiles_of_sequences_match_one_tile(cuda_lib, N, K, B):
+    """Sequences over several CTAs a row tile, the last tile of them ragged: every epilogue gives what a call for up to 64 of the sequences does."""
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([97, N, K, B])
+    w, x = dev(synth.random_tl1_packed(rng, N, K)), dev(rng.standard_normal((B, K)).astype(np.float32))
+    res, nw = dev(rng.standard_normal((B, N)).astype(np.float32)), dev((1 + 0.1 * rng.standard_normal(K)).astype(np.float32))
+    for epi in (kernels.EPI_STORE, kernels.EPI_RESIDUAL) + ((kernels.EPI_RELU2_GLU,) if N // 64 % 2 == 0 else ()):
+        glu = epi == kernels.EPI_RELU2_GLU
+
+        def run(a, r):
+            return kernels.tl1_gemv(a, w, N // 64, K, [0.02, 0.03] if glu else [0.02], [N // 128, N // 64] if glu else None, epilogue=epi,
+                                    resid=r if epi == kernels.EPI_RESIDUAL else None, norm_w=nw, do_norm=True)["out"]
+
+        many = run(x, res)
+        few = torch.cat([run(x[i:i + 64].contiguous(), res[i:i + 64].contiguous()) for i in range(0, B, 64)])
+        assert torch.equal(many, few), f"epilogue {epi}: {int((many != few).any(1).sum())} sequences differ"
+    assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
