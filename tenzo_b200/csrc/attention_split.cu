@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(SoftShape<HS, MANY>::threads, SoftShape<HS, MA
 // Value sums: a consumer lane owns one or two output dims of GV heads, one chain per head and dim, and walks the keys in
 // order (:842-851). Producer warps keep a three-stage ring of key chunks filled and form the weights p_t * s_v[t]
 // (:830, :844), so that the consumers only load, convert and multiply-add. Hand-over by named barriers (a poll of an
-// mbarrier costs its warp more than a chunk's barrier does). Two shapes (heavy_items), and a third for a few heads in all:
+// mbarrier costs its warp more than a chunk's barrier does). Two shapes (heavy_items), and a third for up to 160 heads in all:
 //   heavy  two neighbouring dims a lane and all heads: the fewest instructions and shared-memory cycles an item. Two items a CTA,
 //          two consumer warps each; V bytes by bulk copy, two to a load and converted by the consumers (one load a dim: 131 us
 //          against 126 at 64 x 8192 keys, 222 and 212 for 1536 prompt rows; what the kernel waits for most is shared memory);
@@ -750,7 +750,7 @@ __device__ __forceinline__ void split_values_light(const SplitLaunch& L, unsigne
     for (int g = 0; g < GV; ++g) out[g * kHd] = acc[g];
 }
 
-// Few heads (one or two sequences): a CTA has one head and 64 dims, a dim a lane and a consumer warp a scheduler, and beside a chain's
+// Few heads (up to eight sequences of 20): a CTA has one head and 64 dims, a dim a lane and a consumer warp a scheduler, and beside a chain's
 // multiply-add there is only a byte load, a conversion and a quarter of a weight load a key. A batch of eight keys is
 // summed while the next is converted and the one after that is on its way from shared memory, over the chunks' ends too.
 // 24.2 us for one sequence of 6003 keys and 44.9 for 12000 are 3.5 us and 6.8 cycles a key, where the chain alone would take the
@@ -898,8 +898,10 @@ static cudaError_t split_launch(void (*kernel)(KArgs...), dim3 grid, int threads
 // number of their warps, so whole rounds of 296 items are heavy; a rest that would leave most SMs idle for a round, and a
 // batch as small as that, is light (64 x 8192 keys, 20/5 heads: 276 us all heavy, 253 with 24 of the 320 items light; 60 items of
 // 1500 36.8 all heavy and 35.7 all light, 70 items 37.5 and 36.3, 80 items 42.1 and 48.1; 100 items of 2048 54.8 and 62.3). The
-// cut goes by the number of items, whatever their lengths. Up to kFewHeads heads take the form of one head a CTA.
-constexpr int kFewHeads = 40;
+// cut goes by the number of items, whatever their lengths. Up to kFewHeads heads, a consumer warp a scheduler, take the form of one head a CTA
+// (light and this form, value sums in us: 60 heads up to 3000 keys 20.1 and 14.4, 80 heads of 6000 44.2 and 35.0, 120 heads up to 1500 13.8 and 11.2, 128
+// of 16/16 up to 2000 18.1 and 14.0, 160 up to 1500 15.8 and 12.7 and of 6000 66.1 and 66.4; 240 heads up to 1500 16.9 and 17.9).
+constexpr int kFewHeads = 160;
 static int heavy_items(long long items) {
     const long long rest = items % 296;
     return (int)(rest <= (items < 296 ? 70 : 100) ? items - rest : items);
@@ -965,15 +967,16 @@ int attn_split_kernels(const tenzo_attention_args& a) {
 // Against the one kernel of attention.cu, above the 256 keys that attention_short.cuh takes (us in a graph, one kernel and three). With heads
 // for every SM the three win (12 x 1500: 50 and 34). With fewer the one kernel is a chain as long as the context, the three have
 // their fixed cost: one sequence of 512 keys 10.1 and 11.9, of 640 13.0 and 12.8, of 768 15.1 and 12.6, of 1024 19.2 and 15.3; from block
-// pools, where the one kernel reads through the table key by key, 400 13.4 and 14.5, 512 15.4 and 14.3, 1024 26.0 and 17.0. Above kFewHeads heads the
-// value sums are those for many: 80 heads 1024 keys 20.0 and 20.8, pools 512 15.4 and 15.5, 640 18.6 and 17.5. max_len is an upper bound that
+// pools, where the one kernel reads through the table key by key, 400 13.4 and 14.5, 512 15.4 and 14.3, 1024 26.0 and 17.0. Above two sequences'
+// heads it is less: 80 heads 768 keys 15.3 and 15.5, 900 18.3 and 17.6, pools 512 15.3 and 15.0, 640 18.5 and 17.5. max_len is an upper bound that
 // callers round up, so each line lies a step further.
+constexpr int kLineHeads = 40;
 bool attn_split_preferred(const tenzo_attention_args& a) {
     const long long heads = (long long)a.batch * a.n_q;
     if (heads >= 256) return true;
     if (heads >= 148) return a.max_len > 256;
-    if (a.block_table) return a.max_len > (heads <= kFewHeads ? 512 : 640);
-    return a.max_len > (heads <= kFewHeads ? 768 : 1024);
+    if (a.block_table) return a.max_len > (heads <= kLineHeads ? 512 : 640);
+    return a.max_len > (heads <= kLineHeads ? 768 : 1024);
 }
 
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st) {

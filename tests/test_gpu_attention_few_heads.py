@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 P = ora.ptr
 
 
-@pytest.mark.parametrize("nq,nkv", [(8, 2), (4, 4)])
+@pytest.mark.parametrize("nq,nkv", [(8, 2), (4, 4), (40, 10)])
 @pytest.mark.parametrize("lens", [[1, 255, 256, 257], [263, 264, 511, 512], [513, 767, 769, 1030], [1281, 1536, 1537, 40]])
 def test_few_heads(cuda_lib, nq, nkv, lens):
     from tenzo_b200 import kernels
