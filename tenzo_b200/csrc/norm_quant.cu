@@ -178,6 +178,8 @@ __global__ void __launch_bounds__(kAqThreads, kAqResident) act_quant_kernel(
         }
 #pragma unroll
         for (int r = 0; r < kAqVec; ++r) m = fmaxf(fmaxf(m, fmaxf(fabsf(v[r].x), fabsf(v[r].y))), fmaxf(fabsf(v[r].z), fabsf(v[r].w)));
+        int* s_i = reinterpret_cast<int*>(s_f + 31);
+        if (tid == 0) *s_i = 0;                          // (the maximum's barriers come before the sum)
         m = fmaxf(block_max_nonneg(m, s_f), 1e-6f);      // TenzoEngine.cpp:28-32
         AQT(4);
         const float to_q = 31.0f / m;             // :34
@@ -218,14 +220,10 @@ __global__ void __launch_bounds__(kAqThreads, kAqResident) act_quant_kernel(
                 }
             }
             if (sum_out) {                        // sum_k a_k, for kernels that multiply by the unsigned codes w+1
-                int* s_i = reinterpret_cast<int*>(s_f);
-                __syncthreads();
-                if (tid == 0) s_i[0] = 0;
-                __syncthreads();
                 part = __reduce_add_sync(0xffffffffu, part);
-                if ((tid & 31) == 0) atomicAdd(&s_i[0], part);
+                if ((tid & 31) == 0) atomicAdd(s_i, part);
                 __syncthreads();
-                if (tid == 0) sum_out[seq] = s_i[0];
+                if (tid == 0) sum_out[seq] = *s_i;
             }
         }
         AQT(5);

@@ -246,13 +246,13 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
     const int ksplit = CLUSTER ? L.ksplit : 1;
     const int split = CLUSTER ? (int)cg::this_cluster().block_rank() : 0;         // cluster = the CTAs with this tile's blockIdx.z = 0..ksplit-1
     const int all_chunks = a.K / kKc;
-    const int c_begin = split * all_chunks / ksplit;                                // this CTA's chunks of K: never empty (all_chunks >= ksplit)
-    const int n_chunks = (split + 1) * all_chunks / ksplit - c_begin;
+    const int ks_shift = 31 - __clz(ksplit);                                        // (a power of two; a division would be on the way of the first copies)
+    const int c_begin = split * all_chunks >> ks_shift;                             // this CTA's chunks of K: never empty (all_chunks >= ksplit)
+    const int n_chunks = ((split + 1) * all_chunks >> ks_shift) - c_begin;
 
     const size_t blk_bytes = (size_t)(a.K / 2) * 32;
     const int n_groups = (n_chunks + kPGroup - 1) / kPGroup;
-    auto request_group = [&](int g) {                      // packed weights of chunks kPGroup*g .. kPGroup*g + kPGroup-1, both row blocks
-        const int slot = g % PG;
+    auto request_group = [&](int g, int slot) {            // packed weights of chunks kPGroup*g .. kPGroup*g + kPGroup-1, both row blocks
         const int chunks = min(kPGroup, n_chunks - g * kPGroup);
         const unsigned bytes = (unsigned)chunks * (kPBytes / 2);
         unsigned char* sP = pring + (size_t)slot * kPGroup * kPBytes;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
         // over a hundred cycles; the other barriers are initialised by another warp meanwhile).
         mbar_init(&bar_p[lane], 1);
         mbar_init_fence();
-        if (lane < n_groups) request_group(lane);
+        if (lane < n_groups) request_group(lane, lane);
         if (lane == 0) UT(2);
     } else if (warp == 2) {
         if (lane < R) {
@@ -300,10 +300,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) tl1_umma_kernel(const UmmaLau
     if (warp == 0) {
         if (lane == 0) {
             // ---- producer: the remaining groups of packed weights, each as soon as its ring half is free -------
+            RingPos at = {0, 1};
             for (int gp = PG; gp < n_groups; ++gp) {
-                const int slot = gp % PG, guse = gp / PG;
-                if (!mbar_spin_bounded(&bar_pfree[slot], (unsigned)(guse - 1) & 1u)) { timed_out = true; break; }
-                request_group(gp);
+                if (!mbar_spin_bounded(&bar_pfree[at.slot], (unsigned)(at.round - 1) & 1u)) { timed_out = true; break; }
+                request_group(gp, at.slot);
+                at.step(1, PG);
             }
         } else {
             // ---- per-sequence epilogue operands (quantiser outputs) ---------------------------------------
