@@ -899,14 +899,15 @@ static cudaError_t split_launch(void (*kernel)(KArgs...), dim3 grid, int threads
 // batch as small as that, is light (64 x 8192 keys, 20/5 heads: 276 us all heavy, 253 with 24 of the 320 items light; 60 items of
 // 1500 36.8 all heavy and 35.7 all light, 70 items 37.5 and 36.3, 80 items 42.1 and 48.1; 100 items of 2048 54.8 and 62.3). Behind a whole round
 // an SM takes one light CTA, 37 items in all; two of them are slower than another heavy one (value sums of 3000 keys a sequence in us, the rest
-// light and all heavy: 320 items 49.2 and 58.9, 335 75.6 and 59.0, 370 75.4 and 59.4; of 1800 keys 640 items 57.9 and 55.2, 690 65.5 and 55.5; of 1000 keys 900
-// items 38.7 and 41.6, 950 44.2 and 42.3). The cut goes by the number of items, whatever their lengths. Up to kFewHeads heads, a consumer warp a scheduler, take the form of one head a CTA
+// light and all heavy: 320 items 49.2 and 58.9, 335 75.6 and 59.0, 370 75.4 and 59.4). Behind
+// two rounds and more it matters less (1800 keys: 640 items 57.9 and 55.2, lengths spread over a factor of two 48.4 and 49.9; 690 65.5 and 55.5, spread
+// 51.7 and 51.4). The cut goes by the number of items, whatever their lengths. Up to kFewHeads heads, a consumer warp a scheduler, take the form of one head a CTA
 // (light and this form, value sums in us: 60 heads up to 3000 keys 20.1 and 14.4, 80 heads of 6000 44.2 and 35.0, 120 heads up to 1500 13.8 and 11.2, 128
 // of 16/16 up to 2000 18.1 and 14.0, 160 up to 1500 15.8 and 12.7 and of 6000 66.1 and 66.4; 240 heads up to 1500 16.9 and 17.9).
 constexpr int kFewHeads = 160;
 static int heavy_items(long long items) {
     const long long rest = items % 296;
-    return (int)(rest <= (items < 296 ? 70 : 37) ? items - rest : items);
+    return (int)(rest <= (items < 296 ? 70 : items < 592 ? 37 : 60) ? items - rest : items);
 }
 
 }  // namespace tz

@@ -651,6 +651,7 @@ static UmmaShape pick_umma_shape(int units, int n_chunks, int batch, int epilogu
     }
     UmmaShape best = {0, 1};
     float best_cost = 0.0f;
+    const float per_sm = 1.0f / (float)n_sm;
     for (int tiles = (batch + kMaxN - 1) / kMaxN, last = 0;; ++tiles) {
         int n = ((batch + tiles - 1) / tiles + 15) & ~15;
         // (tiles of 240 are stored in units of 16 sequences; 14208 x 5760 with a residual at 466 sequences 65.5 us, in tiles of 256 62.8, plain ones 46.2 and 48.1)
@@ -658,17 +659,19 @@ static UmmaShape pick_umma_shape(int units, int n_chunks, int batch, int epilogu
         if (n < 32) break;
         if (n == last) continue;
         last = n;
-        const long long ctas = (long long)units * ((batch + n - 1) / n);
-        for (int k = 1; k <= 8; k *= 2) {
-            if (forced ? k != (forced <= n_chunks ? forced : 1) : k > 1 && (n_chunks / k < 4 || ctas * k > n_sm)) continue;
+        const int ctas = units * ((batch + n - 1) / n);
+        for (int k = forced ? (forced <= n_chunks ? forced : 1) : 1;; k *= 2) {
+            if (!forced && k > 1 && (k > 8 || n_chunks < 4 * k || ctas * k > n_sm)) break;
             const int fit = k == 8 ? n_sm - n_sm * 3 / 16 : k == 4 ? n_sm - n_sm / 9 : n_sm;
-            const float rounds = (float)((ctas * k + fit - 1) / fit);
+            const float rounds = ctas * k <= fit ? 1.0f : k > 1 ? 2.0f : (float)(int)((float)(ctas + n_sm - 1) * per_sm);
             const float one = 88.0f + 26.0f * (float)((n_chunks + k - 1) / k) + 3.62f * (float)n +
                               (k > 1 ? 156.0f + 0.55f * (float)(n * (k - 1)) / (float)k : 0.0f) + (k == 8 ? 38.0f : 0.0f);
             const float cost = (0.41f + 0.59f * rounds) * one + 1.61f * (float)(ctas * k);
             if (!best.n_box || cost < best_cost) { best = {n, k}; best_cost = cost; }
+            if (forced) break;
         }
-        if (n <= 32) break;
+        // (more CTAs than SMs already, and each tile more is a round more: a call outside a graph waits for this)
+        if (n <= 32 || (best.n_box && ctas > 16 * n_sm)) break;
     }
     return best;
 }
