@@ -664,6 +664,11 @@ bool attn_split_preferred(const tenzo_attention_args& a);
 int attn_split_kernels(const tenzo_attention_args& a);
 int attn_split_run(const tenzo_attention_args& a, cudaStream_t st);
 int attn_split_take_timeouts();
+// (where a kernel sets its flag on the current device; null if the query failed)
+const int* attn_timeouts_flag() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_attn_timeouts) == cudaSuccess ? static_cast<const int*>(p) : nullptr;
+}
 
 static bool attn_split_chosen(const tenzo_attention_args& a) {
     return a.tiles == 3 || (a.tiles == 0 && a.heads_per_cta == 0 && attn_split_possible(a) && attn_split_preferred(a));

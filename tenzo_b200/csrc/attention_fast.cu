@@ -756,6 +756,10 @@ int attn_fast_run(const tenzo_attention_args& a, cudaStream_t st) {
     return 0;
 }
 
+const int* attn_fast_timeouts_flag() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_fa_timeouts) == cudaSuccess ? static_cast<const int*>(p) : nullptr;
+}
 int attn_fast_take_timeouts() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_fa_timeouts, sizeof v) != cudaSuccess) return -1;

@@ -1016,6 +1016,10 @@ int attn_split_run(const tenzo_attention_args& a, cudaStream_t st) {
     return 0;
 }
 
+const int* attn_split_timeouts_flag() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_split_timeouts) == cudaSuccess ? static_cast<const int*>(p) : nullptr;
+}
 int attn_split_take_timeouts() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_split_timeouts, sizeof v) != cudaSuccess) return -1;

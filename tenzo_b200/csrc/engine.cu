@@ -36,6 +36,13 @@
 
 namespace tz {
 
+// the kernels' error flags on the current device
+const int* attn_timeouts_flag();
+const int* attn_fast_timeouts_flag();
+const int* attn_split_timeouts_flag();
+const int* lm_head_umma_timeouts_flag();
+const int* tl1_timeouts_flag();
+const int* tl1_umma_timeouts_flag();
 int attn_kernels(const tenzo_attention_args& a);         // how many kernels one attention call launches (attention.cu)
 
 // cos/sin [max_seq][head_dim/2] with the reference's float expressions (TenzoEngine.cpp:466-469).
@@ -74,9 +81,16 @@ __global__ void advance_kernel(int* pos, int* tokens, const int* next, int batch
     }
 }
 
-__global__ void record_tokens_kernel(const int* next, int* history, int step, int batch) {
+// `any`, behind the last step: whether a kernel has set its error flag by now.
+__global__ void record_tokens_kernel(const int* next, int* history, int step, int batch, const StatusFlags flags, int* any) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < batch) history[(size_t)step * batch + i] = next[i];
+    if (any && i == 0) {
+        int v = 0;
+#pragma unroll
+        for (int f = 0; f < StatusFlags::n; ++f) v |= __ldcg(flags.at[f]);
+        *any = v;
+    }
 }
 
 // Chunked prefill: rotate and quantise the K rows, quantise the V rows of M consecutive tokens of one sequence and
@@ -267,7 +281,15 @@ void Engine::init(const tenzo_config_t& c, const tenzo_ext_options_t& o) {
     }
     attn_ws = dalloc(attn_ws_bytes);
 
+    const int* flags[StatusFlags::n] = {tz::attn_timeouts_flag(), tz::attn_fast_timeouts_flag(), tz::attn_split_timeouts_flag(),
+                                        tz::lm_head_umma_timeouts_flag(), tz::tl1_timeouts_flag(), tz::tl1_umma_timeouts_flag()};
+    status_flags.known = true;
+    for (int i = 0; i < StatusFlags::n; ++i) {
+        status_flags.at[i] = flags[i];
+        if (!flags[i]) status_flags.known = false;
+    }
     TZ_CUDA(cudaMallocHost(&h_pin, (3 * B + 16) * sizeof(int)));
+    h_status = h_pin + 3 * B;
     h_tokens = h_pin;
     h_pos = h_pin + B;
     h_next = h_pin + 2 * B;
@@ -773,14 +795,15 @@ void Engine::decode_greedy(const int* first, int n_steps, int* out) {
     TZ_CUDA(cudaEventRecord(ev0, stream));
     for (int i = 0; i < n_steps; ++i) {
         run_step(true, true);
-        record_tokens_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(d_next, d_history, i, batch);
+        record_tokens_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(d_next, d_history, i, batch, status_flags, status_flags.known && i + 1 == n_steps ? h_status : nullptr);
         launches += 1;
     }
     TZ_CUDA(cudaEventRecord(ev1, stream));
     TZ_CUDA(cudaMemcpyAsync(out, d_history, (size_t)n_steps * batch * 4, cudaMemcpyDeviceToHost, stream));
     TZ_CUDA(cudaStreamSynchronize(stream));
     pc_check();
-    check_device_status(true);
+    // (Six synchronising copies of 13 us each only where there is something to report.)
+    if (!status_flags.known || *h_status) check_device_status(true);
 }
 
 void Engine::kv_fill(int len, unsigned long long seed) {

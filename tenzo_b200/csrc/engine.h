@@ -40,6 +40,13 @@ struct LayerDev {
     bool has_mlp = false, set = false;
 };
 
+// Where the kernels of the library set their error flags on the engine's device.
+struct StatusFlags {
+    static constexpr int n = 6;
+    const int* at[n] = {};
+    bool known = false;
+};
+
 class Engine {
 public:
     Engine(const tenzo_config_t& cfg, const tenzo_ext_options_t& opt);
@@ -119,7 +126,8 @@ public:
     int* h_sample_past = nullptr;                        // pinned: distinct past tokens, then their counts
     std::vector<int> past_count;                         // [V], zero between calls
     size_t sample_past_cap = 0;
-    int *h_pin = nullptr, *h_tokens = nullptr, *h_pos = nullptr, *h_next = nullptr;
+    int *h_pin = nullptr, *h_tokens = nullptr, *h_pos = nullptr, *h_next = nullptr, *h_status = nullptr;
+    StatusFlags status_flags;
     std::vector<int> seq_len;
     std::vector<void*> owned;
     std::map<int, cudaGraphExec_t> graphs;

@@ -226,6 +226,10 @@ int launch_lm_head_umma(const int8_t* q8, const float* sx, const int8_t* w, cons
     return e == cudaSuccess ? 0 : (int)e;
 }
 
+const int* lm_head_umma_timeouts_flag() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_lmu_timeouts) == cudaSuccess ? static_cast<const int*>(p) : nullptr;
+}
 int lm_head_umma_take_timeouts() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_lmu_timeouts, sizeof v) != cudaSuccess) return -1;

@@ -794,6 +794,10 @@ cudaError_t launch_act_quant(const float* x, const float* norm_w, int do_norm, f
 bool tl1_umma_applicable(const tenzo_tl1_gemv_args& a);
 int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float* inv, const int* sum_a, cudaStream_t st);
 int tl1_umma_take_timeouts();
+const int* tl1_timeouts_flag() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_tl1_timeouts) == cudaSuccess ? static_cast<const int*>(p) : nullptr;
+}
 
 template <int NT, bool FUSED>
 static cudaError_t launch_gemv(const GemvLaunch& L, cudaStream_t st) {

@@ -736,6 +736,10 @@ int launch_tl1_umma(const tenzo_tl1_gemv_args& a, const int8_t* a8, const float*
 }
 
 
+const int* tl1_umma_timeouts_flag() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_umma_timeouts) == cudaSuccess ? static_cast<const int*>(p) : nullptr;
+}
 int tl1_umma_take_timeouts() {
     int v = 0, zero = 0;
     if (cudaMemcpyFromSymbol(&v, g_umma_timeouts, sizeof v) != cudaSuccess) return -1;
