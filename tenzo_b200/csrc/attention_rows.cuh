@@ -180,8 +180,12 @@ __global__ void __launch_bounds__(kRowThreads, 2) rows_scores_kernel(const RowsL
         request(0);
         request(1);
     }
-    // warps 2 x 4 over (32 vectors, 32 keys); lanes 4 x 8: vectors 4 vg .. and 16 + 4 vg .., keys 4 kg ..
-    const int kg = lane & 7, vq = 8 * (warp >> 2) + (lane >> 3), k0 = 32 * (warp & 3) + 4 * kg;
+    // warps 2 x 4 over (32 vectors, 32 keys); lanes 4 x 8: vectors 4 vg .. and 16 + 4 vg .., keys 4 kg .. The second four go through the keys'
+    // quarters the other way round, so that the warps whose quarter of the last key tile is behind every row's last key, and which leave it out,
+    // are of different schedulers (300 rows 49.8 -> 47.7 us in all, 600 rows 94.9 -> 91.8, 1000 of 32/8 heads 261.8 -> 259.0, 1537 355.2 -> 352.2; a branch
+    // around the products instead of a shorter loop: 1537 rows 357.3).
+    const int kg = lane & 7, vq = 8 * (warp >> 2) + (lane >> 3), kw = 32 * (warp < 4 ? warp : 7 - warp), k0 = kw + 4 * kg;
+    const int n_mine = (first + (n_halves >> 1) - 1) * kRowKeys + kw < T ? n_halves : n_halves - 2;
     const float* sk = a.scale_k + ((size_t)a.layer * a.n_kv + kvh) * a.max_seq;
     const float sm_scale = 1.0f / sqrtf((float)kHd);             // :660
     f32x2 sum[4][4];
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rows_scores_kernel(const RowsL
     __syncthreads();
     if (lane == 0 && !mbar_wait_bounded(&s_bar[2], 0u)) timed_out = true;
 #pragma unroll 1
-    for (int h = 0; h < n_halves; ++h) {
+    for (int h = 0; h < n_mine; ++h) {
         if (lane == 0 && !mbar_wait_bounded(&s_bar[h & 1], (unsigned)(h >> 1) & 1u)) timed_out = true;
         __syncwarp();
         const float* sh = s_k + (h & 1) * kRowHalf + k0;
@@ -245,8 +249,9 @@ __global__ void __launch_bounds__(kRowThreads, 2) rows_scores_kernel(const RowsL
                 m[i] = fmaxf(mine, other);
             }
         const int vec = 4 * (kg < 4 ? vq : vq + 4) + (kg & 3), r = vec / L.G;
-        if (s_keys[r] > t0 + 32 * (warp & 3)) atomicMax(L.max + (size_t)(tile * L.rows + r) * a.n_q + kvh * L.G + vec % L.G, ordered_bits(m[0]));
+        if (s_keys[r] > t0 + kw) atomicMax(L.max + (size_t)(tile * L.rows + r) * a.n_q + kvh * L.G + vec % L.G, ordered_bits(m[0]));
     }
+    for (int h = n_mine; h < n_halves; ++h) __syncthreads();     // (thread 0 never comes here: its quarter is the first)
     if (timed_out) atomicExch(&g_split_timeouts, 1);
 }
 
