@@ -15,9 +15,9 @@
 // copy. (Converted by every CTA on its way into shared memory, 1536 rows took 383 us, with 37 % of the value sums' time in it.)
 //
 // What bounds it: the pipe of the multiply-adds. A key of a kv head's four vectors is 8 packed multiply-adds of 2.3 cycles a warp in either
-// product, 92 us each for 1536 rows (20/5 heads); the loops in place take 156 and 126 (pipe 66 % busy; a loop of this shape alone takes 105: what
-// it copies into register pairs and loads shares the issue slots). 1536 rows 564 -> 341 us against attention_split.cu (scores 273 -> 156, softmax
-// 99 -> 54, values 210 -> 126, preparation 15), 600 rows 124 -> 89, 300 rows 51 -> 45, 256 rows at 3000 keys 340 -> 289, 600 rows of 16/16 heads 288 -> 81.
+// product, 92 us each for 1536 rows (20/5 heads); the loops in place take 153 and 126 (pipe 66 % busy; a loop of this shape alone takes 105: what
+// it copies into register pairs and loads shares the issue slots). 1536 rows 564 -> 338 us against attention_split.cu (scores 273 -> 153, softmax
+// 99 -> 54, values 210 -> 126, preparation 15), 600 rows 124 -> 86, 300 rows 51 -> 43, 256 rows at 3000 keys 340 -> 289, 600 rows of 16/16 heads 288 -> 81.
 #pragma once
 #include "attn_common.cuh"
 #include "../../include/tenzo_kernels.h"
@@ -182,7 +182,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) rows_scores_kernel(const RowsL
     }
     // warps 2 x 4 over (32 vectors, 32 keys); lanes 4 x 8: vectors 4 vg .. and 16 + 4 vg .., keys 4 kg .. The second four go through the keys'
     // quarters the other way round, so that the warps whose quarter of the last key tile is behind every row's last key, and which leave it out,
-    // are of different schedulers (300 rows 49.8 -> 47.7 us in all, 600 rows 94.9 -> 91.8, 1000 of 32/8 heads 261.8 -> 259.0, 1537 355.2 -> 352.2; a branch
+    // are of different schedulers (300 rows 49.8 -> 47.7 us in all, 600 rows 94.9 -> 91.8, 1000 of 32/8 heads 261.8 -> 259.0, 1537 355.2 -> 352.2, 256 behind 2744 keys 297.4
+    // and 298.3; a branch
     // around the products instead of a shorter loop: 1537 rows 357.3).
     const int kg = lane & 7, vq = 8 * (warp >> 2) + (lane >> 3), kw = 32 * (warp < 4 ? warp : 7 - warp), k0 = kw + 4 * kg;
     const int n_mine = (first + (n_halves >> 1) - 1) * kRowKeys + kw < T ? n_halves : n_halves - 2;
