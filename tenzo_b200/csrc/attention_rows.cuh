@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(32 * (kRowSoftWarps + 1), 2) rows_softmax_kern
 #pragma unroll
         for (int h = 0; h < kOwn; ++h)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) x[h][u] = t + 32 * u + lane < T[h] ? __ldcg(row[h] + t + 32 * u) : -1e30f;
+            for (int u = 0; u < 4; ++u) x[h][u] = t + 32 * u + lane < T[h] ? __ldcg(row[h] + t + 32 * u) : -INFINITY;
     };
     load(0);
     for (int c = 0; c < n_chunks; ++c) {
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(32 * (kRowSoftWarps + 1), 2) rows_softmax_kern
 #pragma unroll
         for (int h = 0; h < kOwn; ++h)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) e[h][u] = x[h][u] - mx[h];               // (behind the last key: underflows to zero)
+            for (int u = 0; u < 4; ++u) e[h][u] = x[h][u] - mx[h];               // (behind the last key -inf for every maximum, which is -1e30 at least: zero)
         if (c + 1 < n_chunks) load(t + kRowSoftChunk);
 #pragma unroll
         for (int h = 0; h < kOwn; ++h)

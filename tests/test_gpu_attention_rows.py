@@ -87,3 +87,32 @@ def test_rows_equal_three_kernels(cuda_lib, n, max_len, nq, nkv, passes):
     a, b = call(0), call(3)
     assert torch.isnan(b).any() and torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(), b.nan_to_num())
     cuda_lib.tenzo_cuda_attention_take_timeouts()
+
+
+@pytest.mark.parametrize("blown,nq,nkv", [(1, 20, 5), (37, 16, 16)])
+def test_rows_whose_scores_all_lie_below_the_maximums_start(cuda_lib, blown, nq, nkv):
+    """The first keys of kv head 0 score -1e34 with their own queries, those of kv head 1 -inf: the reference's maximum stays at its start, -1e30, every
+    exponential is 0, and the row is 0 / 0. Slots behind such a row's last key are no keys, whatever rows lie beside it."""
+    O = ora.load_oracle()
+    n, ms = 300, 303
+    rng = np.random.default_rng([132, blown, nq])
+    ck, cv = (np.zeros((2, nkv, ms, 128), np.int8) for _ in range(2))
+    sk, sv = (np.ones((2, nkv, ms), np.float32) for _ in range(2))
+    q, k, v = (rng.standard_normal((n, h * 128)).astype(np.float32) for h in (nq, nkv, nkv))
+    k[:blown, :128], k[:blown, 128:256] = 1e30, 3e38
+    q[:blown, :2 * (nq // nkv) * 128] = -1000.0
+    want = np.zeros((n, nq * 128), np.float32)
+    for t in range(n):
+        O.ora_attention_int8(1, t, nq, nkv, 128, ms, 10000.0, P(q[t].copy(), ora.c_f32p), P(k[t].copy(), ora.c_f32p), P(v[t].copy(), ora.c_f32p), P(want[t], ora.c_f32p),
+                             P(ck, ora.c_i8p), P(cv, ora.c_i8p), P(sk, ora.c_f32p), P(sv, ora.c_f32p))
+    assert np.isnan(want[0, :2 * (nq // nkv) * 128]).all() and np.isfinite(want[0, 2 * (nq // nkv) * 128:]).all()
+    order = rng.permutation(n)
+    cs, sn = (dev(t) for t in rope_tables(ms, 10000.0))
+    ws = torch.full((cuda_lib.tenzo_cuda_attention_rows_workspace_bytes(n, nq, nkv, n),), 0x5a, dtype=torch.uint8, device="cuda")
+    args = [dev(a) for a in (q[order], ck, cv, sk, sv, order.astype(np.int32))]
+    call = lambda tiles: host(attend(cuda_lib, *args, nq, nkv, ms, n, cs, sn, ws, tiles))
+    got = call(0)
+    assert took_rows(ws, args[1], nkv, n)
+    assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
+    assert np.array_equal(got, want[order], equal_nan=True)
+    assert np.array_equal(call(3), want[order], equal_nan=True)
