@@ -441,8 +441,8 @@ static size_t rows_tile_bytes(int n_q, int n_kv, int max_len) {                 
     const size_t tp = ((size_t)max_len + 3) & ~(size_t)3;
     return ((size_t)kRowVecs / (n_q / n_kv) * n_q * (tp + 2) + (size_t)n_kv * kRowQFloats) * sizeof(float);
 }
-// Scratch of one pass at most, beside the keys'. It is as large as a prompt of 1600 rows needs whole, of which about half is touched: 1536 rows
-// take 344 us in one pass, 451 in three (whose last tiles leave SMs idle three times), 587 in six; the three kernels 564.
+// Scratch of one pass at most, beside the keys'. It is as large as a prompt of 1700 rows needs whole (20/5 heads), of which about half is touched: 1536 rows
+// take 338 us in one pass, 384 in two, 444 in three (whose last tiles leave SMs idle three times), 575 in six; the three kernels 565.
 constexpr size_t kRowsPassBytes = (size_t)256 << 20;
 
 static size_t rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
@@ -453,8 +453,11 @@ static size_t rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
 }
 
 // Rows of a pass in the caller's scratch; 0: another form. A CTA of the value sums has the whole chains of 32 vectors, so there has to be one for
-// every SM, or a few SMs take as long for the last key (64 rows at 3000 keys, 40 CTAs: 107 us as items, 190 here; 257 rows, 165 CTAs: 44 and 42), and
-// three in each of several passes (512 rows a pass: 451 us of 564 as items).
+// every SM in a pass, or a few SMs take as long for the last key (64 rows at 3000 keys, 40 CTAs: 107 us as items, 190 here). In us here and as items, 20/5
+// heads, one pass: 225 rows 31 and 36, 240 behind 3000 keys 302 and 320; several, by the CTAs of each: 512 rows behind 6000 keys 160 CTAs 1178 and 1517,
+// 1024 behind 8000 220 CTAs 2645 and 3939, behind 3000 320 CTAs 1131 and 1544, 8000 from the start 250 CTAs 9304 and 14444, 4500 410 CTAs 3029 and 4791.
+// A whole prompt's few last tiles at each pass' end cost most where the scratch holds little of it: 1536 rows in 160 CTAs a pass 575 and 565, in 240 448;
+// 32/8 heads, 1000 rows, 176 CTAs 409 and 418.
 constexpr int kRowsValueCtas = 148;
 static int attn_rows_per_pass(const tenzo_attention_args& a) {
     if (a.tiles != 0 || a.batch < 2 || a.block_table || a.seq_stride_kv != 0 || a.append || a.heads_per_cta != 0) return 0;
@@ -464,9 +467,7 @@ static int attn_rows_per_pass(const tenzo_attention_args& a) {
     size_t fit = (a.workspace_bytes - 64 - keys) / tile;
     if (fit > kRowsPassBytes / tile) fit = kRowsPassBytes > tile ? kRowsPassBytes / tile : 1;
     const int passes = fit < (size_t)tiles ? (int)((tiles + fit - 1) / fit) : 1, tiles_pass = (tiles + passes - 1) / passes;
-    const int ctas = tiles_pass * (kRowVecs / kRowValueVecs) * a.n_kv;
-    if (ctas < (passes > 1 ? 3 : 1) * kRowsValueCtas) return 0;
-    return tiles_pass * per_tile;
+    return tiles_pass * (kRowVecs / kRowValueVecs) * a.n_kv < kRowsValueCtas ? 0 : tiles_pass * per_tile;
 }
 
 static int attn_rows_run(const tenzo_attention_args& a, int rows_per_pass, cudaStream_t st) {

@@ -116,3 +116,20 @@ def test_rows_whose_scores_all_lie_below_the_maximums_start(cuda_lib, blown, nq,
     assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
     assert np.array_equal(got, want[order], equal_nan=True)
     assert np.array_equal(call(3), want[order], equal_nan=True)
+
+
+@pytest.mark.parametrize("n,max_len,nq,nkv,scratch_rows", [(700, 640, 20, 5, 352), (1000, 300, 32, 8, 176), (520, 517, 16, 16, 320)])
+def test_rows_in_several_passes_of_one_value_cta_an_sm(cuda_lib, n, max_len, nq, nkv, scratch_rows):
+    """Scratch for 160 to 220 CTAs of the value sums: two passes and more, the last one smaller, give what the three kernels do."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ck, cv = (torch.randint(-128, 128, (2, nkv, max_len, 128), generator=g, device="cuda", dtype=torch.int8) for _ in range(2))
+    sk, sv = (0.001 + 0.02 * torch.rand(2, nkv, max_len, generator=g, device="cuda") for _ in range(2))
+    q = torch.randn(n, nq * 128, generator=g, device="cuda")
+    pos = torch.randint(0, max_len, (n,), generator=g, device="cuda", dtype=torch.int32)
+    cs, sn = (torch.from_numpy(t).cuda() for t in rope_tables(max_len, 10000.0))
+    ws = torch.full((cuda_lib.tenzo_cuda_attention_rows_workspace_bytes(scratch_rows, nq, nkv, max_len),), 0x5a, dtype=torch.uint8, device="cuda")
+    call = lambda tiles: attend(cuda_lib, q, ck, cv, sk, sv, pos, nq, nkv, max_len, max_len, cs, sn, ws, tiles)
+    got = call(0)
+    assert took_rows(ws, ck, nkv, max_len)
+    assert torch.equal(got, call(3))
+    assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
