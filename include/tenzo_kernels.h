@@ -182,8 +182,9 @@ TENZO_API size_t tenzo_cuda_attention_workspace_bytes(int batch, int n_q, int n_
 /* Scratch bytes with which mode 0 takes whole batches at its best; bounded (about 64 MB, or one sequence's scores). */
 TENZO_API size_t tenzo_cuda_attention_exact_workspace_bytes(int batch, int n_q, int n_kv, int max_len);
 /* The same for mode 0 with many query rows over one contiguous cache (seq_stride_kv 0, append 0: a prompt's rows), whose scores
- * are worked out tile by tile; never less than the above. Bounded as well (about 256 MB and 1 KB a key and kv head, or one tile's
- * scores). With less scratch such calls take smaller passes, or the form that other batches take: same results. */
+ * are worked out tile by tile; for calls of `batch` rows and of up to max_len keys. Never less than the above, and no more where no such call
+ * has rows enough for the form. Bounded as well (about 256 MB and 1 KB a key and kv head). With less scratch such calls take smaller passes,
+ * or the form that other batches take: same results. */
 TENZO_API size_t tenzo_cuda_attention_rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len);
 /* Query heads one CTA will process for this shape (1..n_q/n_kv); informational. */
 TENZO_API int tenzo_cuda_attention_heads_per_cta(int batch, int n_q, int n_kv, int max_len);

@@ -434,7 +434,6 @@ __global__ void __launch_bounds__(kRowValueThreads, 4) rows_values_kernel(const 
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------------
-static int rows_per_tile(const tenzo_attention_args& a) { return kRowVecs / (a.n_q / a.n_kv); }
 static int rows_key_tiles(int max_len) { return (max_len + kRowKeys - 1) / kRowKeys; }
 static size_t rows_key_bytes(int n_kv, int max_len) { return (size_t)2 * rows_key_tiles(max_len) * n_kv * kHd * kRowKeys * sizeof(float); }
 static size_t rows_tile_bytes(int n_q, int n_kv, int max_len) {                    // of one tile's queries, scores, maxima and sums
@@ -445,13 +444,6 @@ static size_t rows_tile_bytes(int n_q, int n_kv, int max_len) {                 
 // take 338 us in one pass, 384 in two, 444 in three (whose last tiles leave SMs idle three times), 575 in six; the three kernels 565.
 constexpr size_t kRowsPassBytes = (size_t)256 << 20;
 
-static size_t rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
-    const int per_tile = kRowVecs / (n_q / n_kv);
-    const size_t tile = rows_tile_bytes(n_q, n_kv, max_len), all = tile * (size_t)((batch + per_tile - 1) / per_tile);
-    const size_t cap = kRowsPassBytes > tile ? kRowsPassBytes : tile;
-    return rows_key_bytes(n_kv, max_len) + (all < cap ? all : cap) + 64;
-}
-
 // Rows of a pass in the caller's scratch; 0: another form. A CTA of the value sums has the whole chains of 32 vectors, so there has to be one for
 // every SM in a pass, or a few SMs take as long for the last key (64 rows at 3000 keys, 40 CTAs: 107 us as items, 190 here). In us here and as items, 20/5
 // heads, one pass: 225 rows 31 and 36, 240 behind 3000 keys 302 and 320; several, by the CTAs of each: 512 rows behind 6000 keys 160 CTAs 1178 and 1517,
@@ -459,15 +451,31 @@ static size_t rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
 // A whole prompt's few last tiles at each pass' end cost most where the scratch holds little of it: 1536 rows in 160 CTAs a pass 575 and 565, in 240 448;
 // 32/8 heads, 1000 rows, 176 CTAs 409 and 418.
 constexpr int kRowsValueCtas = 148;
-static int attn_rows_per_pass(const tenzo_attention_args& a) {
-    if (a.tiles != 0 || a.batch < 2 || a.block_table || a.seq_stride_kv != 0 || a.append || a.heads_per_cta != 0) return 0;
-    const int per_tile = rows_per_tile(a), tiles = (a.batch + per_tile - 1) / per_tile;
-    const size_t keys = rows_key_bytes(a.n_kv, a.max_len), tile = rows_tile_bytes(a.n_q, a.n_kv, a.max_len);
-    if (a.workspace_bytes < keys + tile + 64) return 0;
-    size_t fit = (a.workspace_bytes - 64 - keys) / tile;
+static int rows_in_pass(int batch, int n_q, int n_kv, int max_len, size_t scratch) {
+    const int per_tile = kRowVecs / (n_q / n_kv), tiles = (batch + per_tile - 1) / per_tile;
+    const size_t keys = rows_key_bytes(n_kv, max_len), tile = rows_tile_bytes(n_q, n_kv, max_len);
+    if (scratch < keys + tile + 64) return 0;
+    size_t fit = (scratch - 64 - keys) / tile;
     if (fit > kRowsPassBytes / tile) fit = kRowsPassBytes > tile ? kRowsPassBytes / tile : 1;
     const int passes = fit < (size_t)tiles ? (int)((tiles + fit - 1) / fit) : 1, tiles_pass = (tiles + passes - 1) / passes;
-    return tiles_pass * (kRowVecs / kRowValueVecs) * a.n_kv < kRowsValueCtas ? 0 : tiles_pass * per_tile;
+    return tiles_pass * (kRowVecs / kRowValueVecs) * n_kv < kRowsValueCtas ? 0 : tiles_pass * per_tile;
+}
+static int attn_rows_per_pass(const tenzo_attention_args& a) {
+    if (a.tiles != 0 || a.batch < 2 || a.block_table || a.seq_stride_kv != 0 || a.append || a.heads_per_cta != 0) return 0;
+    return rows_in_pass(a.batch, a.n_q, a.n_kv, a.max_len, a.workspace_bytes);
+}
+
+// Scratch for `batch` rows and up to max_len keys: what the longest cache wants that this form takes with it; 0 if it takes none (fewer
+// rows than it has CTAs for).
+static size_t rows_workspace_bytes(int batch, int n_q, int n_kv, int max_len) {
+    const int per_tile = kRowVecs / (n_q / n_kv), tiles = (batch + per_tile - 1) / per_tile;
+    if ((long long)tiles * (kRowVecs / kRowValueVecs) * n_kv < kRowsValueCtas) return 0;
+    for (int len = max_len; len > 0; len = (len - 1) / kRowKeys * kRowKeys) {
+        const size_t tile = rows_tile_bytes(n_q, n_kv, len), all = tile * (size_t)tiles, cap = kRowsPassBytes > tile ? kRowsPassBytes : tile;
+        const size_t bytes = rows_key_bytes(n_kv, len) + (all < cap ? all : cap) + 64;
+        if (rows_in_pass(batch, n_q, n_kv, len, bytes)) return bytes;
+    }
+    return 0;
 }
 
 static int attn_rows_run(const tenzo_attention_args& a, int rows_per_pass, cudaStream_t st) {

@@ -572,8 +572,14 @@ void Engine::prefill_chunk(const int* tokens, int M) {
             TZ_CUDA(cudaMalloc((void**)&pf_tokens, m * 4));
             TZ_CUDA(cudaMalloc((void**)&pf_pos, m * 4));
             TZ_CUDA(cudaMalloc(&pf_ws, tenzo_cuda_tl1_gemv_workspace_bytes(M > 1 ? M : 2, h > ffn ? h : ffn)));
-            pf_attn_ws_bytes = (paged ? tenzo_cuda_attention_exact_workspace_bytes : tenzo_cuda_attention_rows_workspace_bytes)(M, cfg.num_q_heads, cfg.num_kv_heads, cfg.max_seq_len);
-            TZ_CUDA(cudaMalloc(&pf_attn_ws, pf_attn_ws_bytes));
+            const size_t least = tenzo_cuda_attention_exact_workspace_bytes(M, cfg.num_q_heads, cfg.num_kv_heads, cfg.max_seq_len);
+            pf_attn_ws_bytes = paged ? least : tenzo_cuda_attention_rows_workspace_bytes(M, cfg.num_q_heads, cfg.num_kv_heads, cfg.max_seq_len);
+            if (pf_attn_ws_bytes > least && cudaMalloc(&pf_attn_ws, pf_attn_ws_bytes) != cudaSuccess) {      // the rows' form is the faster one, not the only one
+                cudaGetLastError();
+                pf_attn_ws = nullptr;
+                pf_attn_ws_bytes = least;
+            }
+            if (!pf_attn_ws) TZ_CUDA(cudaMalloc(&pf_attn_ws, pf_attn_ws_bytes));
         } catch (...) {
             free_prefill_rows();
             throw;

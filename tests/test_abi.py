@@ -164,3 +164,17 @@ def test_engine_creation_fails_loudly_without_a_gpu(lib):
         pytest.skip("a GPU is present")
     assert not lib.tenzo_create_engine(None)
     assert b"no CPU path" in lib.tenzo_ext_last_error() or b"CUDA" in lib.tenzo_ext_last_error()
+
+
+def test_scratch_of_a_prompts_rows(lib):
+    """No more than any batch's where the rows have no form of their own (here one CTA an SM: 224 rows of 20/5 heads), whatever the cache; else enough for
+    every shorter cache too."""
+    rows, exact = lib.tenzo_cuda_attention_rows_workspace_bytes, lib.tenzo_cuda_attention_exact_workspace_bytes
+    for batch, n_q, n_kv in ((1, 20, 5), (16, 20, 5), (64, 20, 5), (224, 20, 5), (64, 32, 8), (144, 32, 8), (64, 16, 16), (256, 16, 16)):
+        for max_len in (1, 300, 4096, 32768, 131072):
+            assert rows(batch, n_q, n_kv, max_len) == exact(batch, n_q, n_kv, max_len), (batch, n_q, n_kv, max_len)
+    for batch, n_q, n_kv in ((225, 20, 5), (600, 20, 5), (4000, 20, 5), (160, 32, 8), (1000, 32, 4), (300, 16, 16)):
+        lens = (1, 127, 128, 129, 600, 1500, 4096, 10000, 32768, 131072)
+        got = [rows(batch, n_q, n_kv, n) for n in lens]
+        assert got == sorted(got) and all(g >= exact(batch, n_q, n_kv, n) for g, n in zip(got, lens)), (batch, n_q, n_kv, got)
+        assert got[4] > exact(batch, n_q, n_kv, 600) and got[-1] < (512 << 20)

@@ -133,3 +133,34 @@ def test_rows_in_several_passes_of_one_value_cta_an_sm(cuda_lib, n, max_len, nq,
     assert took_rows(ws, ck, nkv, max_len)
     assert torch.equal(got, call(3))
     assert cuda_lib.tenzo_cuda_attention_take_timeouts() == 0
+
+
+def rows_engine(max_seq):
+    from tenzo_b200 import synth
+    from tenzo_b200.engine import Engine
+    m = synth.SyntheticModel(dict(synth.TINY, hidden_size=2560, num_q_heads=20, num_kv_heads=5, ffn_dim=768, num_layers=2, vocab_size=2048, max_seq_len=max_seq), seed=43)
+    return lambda: Engine(m.config_struct(max_seq_len=max_seq)).load_synthetic(m)
+
+
+def test_engine_without_memory_for_the_rows_scratch_takes_the_smaller_one(cuda_lib):
+    """A prompt whose rows' scratch (243 MB here) does not fit on the device any more runs in the scratch of any batch (64 MB): same cache, same tokens."""
+    from tenzo_b200 import synth
+    new, prompt, left = rows_engine(8192), synth.prompt_tokens(13, 301, 2048), 160 << 20
+    assert cuda_lib.tenzo_cuda_attention_rows_workspace_bytes(300, 20, 5, 8192) > left + (64 << 20)
+
+    def run(e):
+        e.prefill_chunk(prompt[:-1])
+        return [e.kv_export(0, l, 300) for l in range(2)], e.decode_greedy([int(prompt[-1])], 8)
+
+    with new() as e:
+        kv, tokens = run(e)
+    with new() as e:
+        hog = []
+        try:
+            while (free := torch.cuda.mem_get_info()[0]) > left + (8 << 20):
+                hog.append(torch.empty(min(free - left, 8 << 30), dtype=torch.uint8, device="cuda"))
+            kv_few, tokens_few = run(e)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+    assert np.array_equal(tokens, tokens_few) and all(np.array_equal(a, b) for x, y in zip(kv, kv_few) for a, b in zip(x, y))
