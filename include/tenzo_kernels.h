@@ -77,7 +77,10 @@ TENZO_API int tenzo_cuda_tl1_gemv_ksplit(int n_blocks, int K, int epilogue);
  * (1, 2, 4 or 8; more than 1 when the row tiles alone would leave most SMs idle); 0 if that path does not take the
  * shape. Informational. */
 TENZO_API int tenzo_cuda_tl1_gemm_ksplit(int n_blocks, int K, int batch, int epilogue);
-/* The tensor-core path's per-CTA layout for `batch` sequences (of a CTA that holds min(batch, 256) padded to 16, the most of any):
+/* Sequences a CTA of the tensor-core path holds for this shape (a multiple of 16, at most 256; several CTAs share the batch where it is fewer
+ * than `batch`); 0 if that path does not take the shape. Informational; no counterpart in the reference. */
+TENZO_API int tenzo_cuda_tl1_gemm_sequences(int n_blocks, int K, int batch, int epilogue);
+/* The tensor-core path's layout of a CTA that holds min(batch, 256) sequences padded to 16 (tenzo_cuda_tl1_gemm_sequences says how many a shape's CTA holds):
  * ring slots (a multiple of four), groups of eight weight chunks in flight, dynamic shared memory in bytes, and the
  * bytes the epilogue may need in the two rings. Host arithmetic only (no device call); returns 0, or -1 for
  * fewer than nine sequences. Informational; no counterpart in the reference. */

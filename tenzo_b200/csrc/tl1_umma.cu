@@ -775,8 +775,10 @@ extern "C" int tenzo_cuda_tl1_gemm_layout(int batch, int* slots, int* weight_gro
     return 0;
 }
 
-extern "C" int tenzo_cuda_tl1_gemm_ksplit(int n_blocks, int K, int batch, int epilogue) {
-    if (n_blocks <= 0 || K < tz::kKc || K % tz::kKc || batch < tz::kUmmaMinBatch) return 0;       // the tensor-core path does not apply
+static tz::UmmaShape gemm_shape(int n_blocks, int K, int batch, int epilogue) {
+    if (n_blocks <= 0 || K < tz::kKc || K % tz::kKc || batch < tz::kUmmaMinBatch) return {0, 0};       // the tensor-core path does not apply
     const int units = epilogue == TENZO_EPI_RELU2_GLU ? n_blocks / 2 : (n_blocks + 1) / 2;
-    return tz::pick_umma_shape(units, K / tz::kKc, batch, epilogue).ksplit;
+    return tz::pick_umma_shape(units, K / tz::kKc, batch, epilogue);
 }
+extern "C" int tenzo_cuda_tl1_gemm_ksplit(int n_blocks, int K, int batch, int epilogue) { return gemm_shape(n_blocks, K, batch, epilogue).ksplit; }
+extern "C" int tenzo_cuda_tl1_gemm_sequences(int n_blocks, int K, int batch, int epilogue) { return gemm_shape(n_blocks, K, batch, epilogue).n_box; }

@@ -77,3 +77,30 @@ def test_tiles_of_sequences_match_one_tile(cuda_lib, N, K, B):
         few = torch.cat([run(x[i:i + 64].contiguous(), res[i:i + 64].contiguous()) for i in range(0, B, 64)])
         assert torch.equal(many, few), f"epilogue {epi}: {int((many != few).any(1).sum())} sequences differ"
     assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
+
+
+@pytest.mark.parametrize("N,K,B,sequences,ksplit", [(4096, 14336, 128, 128, 4), (4096, 14336, 144, 144, 4), (4096, 14336, 240, 240, 4), (4096, 14336, 256, 256, 4),
+                                                    (4096, 14336, 320, 160, 2), (4096, 14336, 497, 256, 2), (768, 16384, 206, 112, 8), (768, 16384, 320, 160, 8),
+                                                    (512, 14336, 390, 144, 8)])
+def test_clusters_with_four_activation_tiles(cuda_lib, N, K, B, sequences, ksplit):
+    """K split over a cluster whose CTAs hold more than 96 sequences each (four activation tiles, the partial tiles in the rings): every epilogue gives
+    what calls for up to 64 of the sequences do, and those of eight on the other path. The shapes are the chosen ones, for 148 SMs."""
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([98, N, K, B])
+    w, x = dev(synth.random_tl1_packed(rng, N, K)), dev(rng.standard_normal((B, K)).astype(np.float32))
+    res, nw = dev(rng.standard_normal((B, N)).astype(np.float32)), dev((1 + 0.1 * rng.standard_normal(K)).astype(np.float32))
+    for epi in (kernels.EPI_STORE, kernels.EPI_RESIDUAL, kernels.EPI_RELU2_GLU):
+        glu = epi == kernels.EPI_RELU2_GLU
+        assert cuda_lib.tenzo_cuda_tl1_gemm_sequences(N // 64, K, B, epi) == sequences > 96
+        assert cuda_lib.tenzo_cuda_tl1_gemm_ksplit(N // 64, K, B, epi) == ksplit > 1
+
+        def run(i, n):
+            return kernels.tl1_gemv(x[i:i + n].contiguous(), w, N // 64, K, [0.02, 0.03] if glu else [0.02], [N // 128, N // 64] if glu else None, epilogue=epi,
+                                    resid=res[i:i + n].contiguous() if epi == kernels.EPI_RESIDUAL else None, norm_w=nw, do_norm=True)["out"]
+
+        many = run(0, B)
+        few = torch.cat([run(i, 64) for i in range(0, B, 64)])
+        assert torch.equal(many, few), f"epilogue {epi}: {int((many != few).any(1).sum())} sequences differ"
+        for i in (0, sequences - 8, B - 8):
+            assert torch.equal(many[i:i + 8], run(i, 8)), f"epilogue {epi}, sequences from {i}"
+    assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
