@@ -653,14 +653,21 @@ static UmmaShape pick_umma_shape(int units, int n_chunks, int batch, int epilogu
     float best_cost = 0.0f;
     const float per_sm = 1.0f / (float)n_sm;
     for (int tiles = (batch + kMaxN - 1) / kMaxN, last = 0;; ++tiles) {
-        int n = ((batch + tiles - 1) / tiles + 15) & ~15;
-        // (tiles of 240 are stored in units of 16 sequences; 14208 x 5760 with a residual at 466 sequences 65.5 us, in tiles of 256 62.8, plain ones 46.2 and 48.1)
-        if (n == 240 && tiles > 1 && epilogue != TENZO_EPI_STORE) n = kMaxN;
-        if (n < 32) break;
-        if (n == last) continue;
-        last = n;
-        const int ctas = units * ((batch + n - 1) / n);
+        const int even = ((batch + tiles - 1) / tiles + 15) & ~15;
+        if (even < 32) break;
+        if (even == last) continue;
+        last = even;
+        // An odd multiple of 16 among several tiles is stored in units of 16 sequences, others in units of 32 (store_cols), by four groups of warps in
+        // turn: 208 and 240 take four rounds where 224 and 256 take two, and where a unit also loads residuals or joins gate and up, a round costs more than 16
+        // sequences do (us, residual and GLU, 208 and 224: 13824 x 2560 GLU at 385 sequences 28.0 and 27.5, 14208 x 5760 at 416 53.2 and 51.9, 2560 x 6912 at 1345
+        // 47.5 and 46.9; 240 and 256: 14208 x 5760 at 480 61.9 and 59.5, 13824 x 2560 GLU at 1200 61.6 and 61.1, 4096 x 4096 at 960 31.7 and 32.0;
+        // plain stores 14208 x 5760 at 480 46.0 and 47.9). One round more, 80 to 176, does not (176 and 192: 13824 x 2560 GLU at 673 sequences 39.5 and 39.4, 2560 x
+        // 2560 at 1200 22.0 and 22.7).
+        const int padded = tiles > 1 && epilogue != TENZO_EPI_STORE && (even & 31) && (even + 63) / 64 > (even + 127) / 128 + 1 ? even + 16 : even;
+        const int ctas_even = units * ((batch + even - 1) / even);
         for (int k = forced ? (forced <= n_chunks ? forced : 1) : 1;; k *= 2) {
+            const int n = k == 1 ? padded : even;                // (clusters store in units of four)
+            const int ctas = n == even ? ctas_even : units * ((batch + n - 1) / n);
             if (!forced && k > 1 && (k > 8 || n_chunks < 4 * k || ctas * k > n_sm)) break;
             const int fit = k == 8 ? n_sm - n_sm * 3 / 16 : k == 4 ? n_sm - n_sm / 9 : n_sm;
             const float rounds = ctas * k <= fit ? 1.0f : k > 1 ? 2.0f : (float)(int)((float)(ctas + n_sm - 1) * per_sm);
@@ -671,7 +678,7 @@ static UmmaShape pick_umma_shape(int units, int n_chunks, int batch, int epilogu
             if (forced) break;
         }
         // (more CTAs than SMs already, and each tile more is a round more: a call outside a graph waits for this)
-        if (n <= 32 || (best.n_box && ctas > 16 * n_sm)) break;
+        if (even <= 32 || (best.n_box && ctas_even > 16 * n_sm)) break;
     }
     return best;
 }

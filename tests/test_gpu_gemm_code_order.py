@@ -104,3 +104,23 @@ def test_clusters_with_four_activation_tiles(cuda_lib, N, K, B, sequences, kspli
         for i in (0, sequences - 8, B - 8):
             assert torch.equal(many[i:i + 8], run(i, 8)), f"epilogue {epi}, sequences from {i}"
     assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
+
+
+@pytest.mark.parametrize("N,K,B,plain", [(13824, 2560, 385, 208), (13824, 384, 416, 208), (4096, 4096, 897, 240), (2560, 2560, 1345, 208)])
+def test_tiles_of_sequences_by_the_rounds_of_their_stores(cuda_lib, N, K, B, plain):
+    """Tiles whose stores would take two rounds more than those of 16 sequences more give way to them where a unit does more than store; all give what a
+    call for up to 64 of the sequences does."""
+    from tenzo_b200 import kernels
+    rng = np.random.default_rng([99, N, K, B])
+    w, x = dev(synth.random_tl1_packed(rng, N, K)), dev(rng.standard_normal((B, K)).astype(np.float32))
+    res = dev(rng.standard_normal((B, N)).astype(np.float32))
+    for epi in (kernels.EPI_STORE, kernels.EPI_RESIDUAL, kernels.EPI_RELU2_GLU):
+        glu = epi == kernels.EPI_RELU2_GLU
+        assert cuda_lib.tenzo_cuda_tl1_gemm_sequences(N // 64, K, B, epi) == (plain if epi == kernels.EPI_STORE else plain + 16)
+
+        def run(i, n):
+            return kernels.tl1_gemv(x[i:i + n].contiguous(), w, N // 64, K, [0.02, 0.03] if glu else [0.02], [N // 128, N // 64] if glu else None, epilogue=epi,
+                                    resid=res[i:i + n].contiguous() if epi == kernels.EPI_RESIDUAL else None)["out"]
+
+        assert torch.equal(run(0, B), torch.cat([run(i, 64) for i in range(0, B, 64)])), f"epilogue {epi}"
+    assert cuda_lib.tenzo_cuda_tl1_gemv_take_timeouts() == 0
