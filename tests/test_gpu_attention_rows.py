@@ -164,3 +164,27 @@ def test_engine_without_memory_for_the_rows_scratch_takes_the_smaller_one(cuda_l
             del hog
             torch.cuda.empty_cache()
     assert np.array_equal(tokens, tokens_few) and all(np.array_equal(a, b) for x, y in zip(kv, kv_few) for a, b in zip(x, y))
+
+
+@pytest.mark.parametrize("chunks", [[700], [300, 400], [20, 680]])
+def test_engine_chunks_take_the_rows_form(cuda_lib, chunks):
+    """A prompt through the engine as it runs by default (overlapped launches, every layer on one scratch, a cache longer than the prompt, 20/5 heads):
+    the cache and the tokens that follow are those of the prompt fed token by token."""
+    from tenzo_b200 import synth
+    new, prompt = rows_engine(1100), synth.prompt_tokens(14, 701, 2048)
+    with new() as e:
+        for t in prompt[:-1]:
+            e.prefill_token(int(t))
+        kv = [e.kv_export(0, l, 700) for l in range(2)]
+        tokens = e.decode_greedy([int(prompt[-1])], 8)
+    with new() as e:
+        done = 0
+        for c in chunks:
+            before = e.kernel_launches()
+            e.prefill_chunk(prompt[done:done + c])
+            done += c
+            if c >= 300:
+                assert e.kernel_launches() - before == 1 + 2 * (1 + 4 * 2 + 4)          # the embedding; a layer's append, products and four attention kernels
+        for l in range(2):
+            assert all(np.array_equal(got, want) for got, want in zip(e.kv_export(0, l, 700), kv[l])), f"layer {l}"
+        assert np.array_equal(e.decode_greedy([int(prompt[-1])], 8), tokens)
