@@ -329,11 +329,12 @@ __global__ void __launch_bounds__(32 * (kRowSoftWarps + 1), 2) rows_softmax_kern
 }
 
 // Value sums of 32 vectors x 128 dims: chunks of 32 keys; V's floats by bulk copies into three buffers, the weights [32 keys][vectors] (quads of
-// vectors exchanged by the key's quad) through registers into two.
+// vectors exchanged by the key's quad) through registers into two. Three CTAs an SM: the buffers are 56 KB, and a fourth lacks 512 bytes for its barriers.
+// With two buffers there are four, and they wait more for their copies: 1024 rows 171 -> 180 us in all, 4000 2289 -> 2335, 1536 336 -> 338.
 constexpr int kRowValueVecs = 32, kRowValueThreads = 4 * kRowValueVecs, kRowValueStages = 3;
 constexpr int kRowVFloats = kRowChunk * kHd, kRowWFloats = kRowChunk * kRowValueVecs;
 constexpr int kRowValueBytes = (kRowValueStages * kRowVFloats + 2 * kRowWFloats) * 4;
-__global__ void __launch_bounds__(kRowValueThreads, 4) rows_values_kernel(const RowsLaunch L) {
+__global__ void __launch_bounds__(kRowValueThreads, 3) rows_values_kernel(const RowsLaunch L) {
     const tenzo_attention_args& a = L.a;
     extern __shared__ __align__(128) float smem[];
     __shared__ uint64_t s_bar[kRowValueStages];
