@@ -8,16 +8,17 @@
 // whose order of summation is the reference's:
 //   scores   chain j of eight (elements j, j + 8, ...) is a product over 16 elements; a lane holds 8 vectors x 8 keys of one
 //            chain, runs its 16 multiply-adds, adds it to the sum of the chains before, and goes on with the next chain;
-//   softmax  a warp a (row, head): maximum, exponentials, their sum in order (ordered_sum.cuh), and the weights e / sum * scale_v;
-//   values   a lane holds 8 vectors x 8 dims, one chain each, and walks the keys; weights are zero behind a row's last key, which
-//            changes no sum.
+//   softmax  sixteen warps evaluate the exponentials of 32 (row, head) pairs, a lane of another adds up a pair's in order;
+//   values   a lane holds 8 vectors x 8 dims, one chain each, and walks the keys; the weights e / sum * scale_v are zero behind a row's
+//            last key, which changes no sum.
 // The cache's bytes become floats once a call (rows_prepare_kernel), in the order in which a tile holds them, so that a tile's half is one bulk
 // copy. (Converted by every CTA on its way into shared memory, 1536 rows took 383 us, with 37 % of the value sums' time in it.)
 //
 // What bounds it: the pipe of the multiply-adds. A key of a kv head's four vectors is 8 packed multiply-adds of 2.3 cycles a warp in either
-// product, 92 us each for 1536 rows (20/5 heads); the loops in place take 153 and 126 (pipe 66 % busy; a loop of this shape alone takes 105: what
-// it copies into register pairs and loads shares the issue slots). 1536 rows 564 -> 338 us against attention_split.cu (scores 273 -> 153, softmax
-// 99 -> 54, values 210 -> 126, preparation 15), 600 rows 124 -> 86, 300 rows 51 -> 43, 256 rows at 3000 keys 340 -> 289, 600 rows of 16/16 heads 288 -> 81.
+// product, 92 us each for 1536 rows (20/5 heads); the loops in place take 158 and 133 (the kernels by themselves under a profiler; pipe 66 and 73 % busy; a loop of
+// this shape alone takes 105: what it copies into register pairs and loads shares the issue slots), the softmax 55, the preparation 15. A whole call, back to back in
+// a graph, in us, as items (attention_split.cu) and here: 1536 rows 565 and 336, 600 rows 123 and 82, 300 rows 50 and 40, 256 rows behind 2744 keys 323 and 288, 4000 rows
+// 3751 and 2289; 16/16 heads, 300 rows 119 and 39, 1500 rows 1122 and 279; 32/8, 1000 rows 418 and 251.
 #pragma once
 #include "attn_common.cuh"
 #include "../../include/tenzo_kernels.h"
@@ -182,9 +183,8 @@ __global__ void __launch_bounds__(kRowThreads, 2) rows_scores_kernel(const RowsL
     }
     // warps 2 x 4 over (32 vectors, 32 keys); lanes 4 x 8: vectors 4 vg .. and 16 + 4 vg .., keys 4 kg .. The second four go through the keys'
     // quarters the other way round, so that the warps whose quarter of the last key tile is behind every row's last key, and which leave it out,
-    // are of different schedulers (300 rows 49.8 -> 47.7 us in all, 600 rows 94.9 -> 91.8, 1000 of 32/8 heads 261.8 -> 259.0, 1537 355.2 -> 352.2, 256 behind 2744 keys 297.4
-    // and 298.3; a branch
-    // around the products instead of a shorter loop: 1537 rows 357.3).
+    // are of different schedulers (calls apart, each waited for: 300 rows 49.8 -> 47.7 us, 600 rows 94.9 -> 91.8, 1000 of 32/8 heads 261.8 -> 259.0, 1537 355.2 -> 352.2, 256 behind 2744 keys 297.4
+    // and 298.3; a branch around the products instead of a shorter loop: 1537 rows 357.3).
     const int kg = lane & 7, vq = 8 * (warp >> 2) + (lane >> 3), kw = 32 * (warp < 4 ? warp : 7 - warp), k0 = kw + 4 * kg;
     const int n_mine = (first + (n_halves >> 1) - 1) * kRowKeys + kw < T ? n_halves : n_halves - 2;
     const float* sk = a.scale_k + ((size_t)a.layer * a.n_kv + kvh) * a.max_seq;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kRowThreads, 2) rows_scores_kernel(const RowsL
 // Scores -> exponentials (in place) and 1 / sum. There are more (row, head) pairs than the machine has lanes for, so a lane of the summing warp
 // adds up a pair's exponentials one after another as the reference does, while the other warps evaluate the next chunk: 32 pairs a
 // CTA, chunks of 128 keys through two buffers. (A warp a pair with ordered_sum.cuh's segments: 139 us for 1536 rows, some thousand
-// instructions a pair beside the exponentials; here 54.) Bound by the instructions of the exponential.
+// instructions a pair beside the exponentials; here 55.) Bound by the instructions of the exponential.
 constexpr int kRowSoftWarps = 16, kRowSoftChunk = 128, kRowSoftStride = kRowSoftChunk + 4;
 __global__ void __launch_bounds__(32 * (kRowSoftWarps + 1), 2) rows_softmax_kernel(const RowsLaunch L) {
     const tenzo_attention_args& a = L.a;

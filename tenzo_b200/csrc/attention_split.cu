@@ -900,8 +900,11 @@ static cudaError_t split_launch(void (*kernel)(KArgs...), dim3 grid, int threads
 // 1500 36.8 all heavy and 35.7 all light, 70 items 37.5 and 36.3, 80 items 42.1 and 48.1; 100 items of 2048 54.8 and 62.3). Behind a whole round
 // an SM takes one light CTA, 37 items in all; two of them are slower than another heavy one (value sums of 3000 keys a sequence in us, the rest
 // light and all heavy: 320 items 49.2 and 58.9, 335 75.6 and 59.0, 370 75.4 and 59.4). Behind
-// two rounds and more it matters less (1800 keys: 640 items 57.9 and 55.2, lengths spread over a factor of two 48.4 and 49.9; 690 65.5 and 55.5, spread
-// 51.7 and 51.4). The cut goes by the number of items, whatever their lengths. Up to kFewHeads heads, a consumer warp a scheduler, take the form of one head a CTA
+// two rounds and more it is a few per cent either way, and which depends on the lengths, which the host does not know: two light CTAs an SM cost equal lengths
+// what a heavy round saves, and ragged ones end sooner with them. The line is a compromise between those (whole calls in us, the rest light and all heavy; equal 1800 keys,
+// spread over a factor of two, spread from 100 to 3000 keys: 630 items 127.4 and 127.7, 112.0 and 108.0, 144.2 and 156.0; 640 130.8 and 128.0, 108.1 and 109.5,
+// 132.8 and 130.2; 650 133.6 and 128.5, 113.8 and 114.7, 149.0 and 156.4; 675 140.3 and 131.7, 114.7 and 113.2, 150.4 and 160.3; 690 141.8 and 133.2, 119.5 and 115.7, 139.3 and
+// 148.2; 945 175.7 and 174.1, 149.1 and 148.2, 178.6 and 186.6; 1240 214.9 and 213.5, 178.7 and 177.7, 226.0 and 224.6). Up to kFewHeads heads, a consumer warp a scheduler, take the form of one head a CTA
 // (light and this form, value sums in us: 60 heads up to 3000 keys 20.1 and 14.4, 80 heads of 6000 44.2 and 35.0, 120 heads up to 1500 13.8 and 11.2, 128
 // of 16/16 up to 2000 18.1 and 14.0, 160 up to 1500 15.8 and 12.7 and of 6000 66.1 and 66.4; 240 heads up to 1500 16.9 and 17.9).
 constexpr int kFewHeads = 160;
